@@ -247,13 +247,12 @@ class _Plan:
     """A grouped plan that is destroyed with the state that holds it."""
 
     def __init__(self, arr):
-        self.handle = C.c_void_p()
+        self.handle, self.destroy = C.c_void_p(), _lib.lib().b2_grouped_plan_destroy
         _lib.check(_lib.lib().b2_grouped_plan_create(len(arr), arr, C.byref(self.handle)),
                    "b2_grouped_plan_create")
 
     def __del__(self):
-        torch.cuda.synchronize()
-        _lib.lib().b2_grouped_plan_destroy(self.handle)
+        self.destroy(self.handle)
 
 
 # --------------------------------------------------------------- one pass --
