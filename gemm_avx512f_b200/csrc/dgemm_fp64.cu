@@ -208,34 +208,73 @@ __global__ void __launch_bounds__(WM *WN * 32, 1)
         }
     return;
   }
+  // C is read before any of it is written, 16 rows of the warp tile at a
+  // time: interleaved with the stores, each load would wait for the one before
+  // it (the compiler keeps their order), 32 round trips to memory in a row --
+  // 8 us of the 11 us of a 64x64x64 product on B200.
   const bool beta_one = (beta == 1.0);
 #pragma unroll
-  for (int i = 0; i < MT; ++i)
+  for (int i = 0; i < MT; ++i) {
+    double c_old[NTL][4];
 #pragma unroll
     for (int j = 0; j < NTL; ++j)
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         const int m = m0 + wm0 + i * 16 + g + 8 * (v >> 1);
         const int n = n0 + wn0 + j * 8 + 2 * t + (v & 1);
-        if (m < M && n < N) {
-          double *p = C + (size_t)n * ldc + m;
-          const double c_old = *p;
-          *p = beta_one ? fma(alpha, acc[i][j][v], c_old) : fma(alpha, acc[i][j][v], beta * c_old);
-        }
+        c_old[j][v] = (m < M && n < N) ? C[(size_t)n * ldc + m] : 0.0;
       }
+#pragma unroll
+    for (int j = 0; j < NTL; ++j)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const int m = m0 + wm0 + i * 16 + g + 8 * (v >> 1);
+        const int n = n0 + wn0 + j * 8 + 2 * t + (v & 1);
+        if (m < M && n < N)
+          C[(size_t)n * ldc + m] = beta_one ? fma(alpha, acc[i][j][v], c_old[j][v])
+                                            : fma(alpha, acc[i][j][v], beta * c_old[j][v]);
+      }
+  }
 }
 
-__global__ void splitk_reduce_kernel(int M, int N, int splits, const double *__restrict__ P,
-                                     int ldp, double alpha, double beta, double *__restrict__ C,
-                                     int ldc) {
-  const size_t total = (size_t)M * N;
-  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (size_t)gridDim.x * blockDim.x) {
-    const int m = (int)(idx % M), n = (int)(idx / M);
-    double s = 0.0;
-    for (int z = 0; z < splits; ++z) s += P[(size_t)z * ldp * N + (size_t)n * ldp + m];
-    double *p = C + (size_t)n * ldc + m;
-    *p = (beta == 1.0) ? fma(alpha, s, *p) : fma(alpha, s, beta * *p);
+// C = alpha * (sum of the slices' partials, in slice order) + beta * C: one row
+// pair per thread along x, columns along y.  Launched as a programmatic
+// dependent of the GEMM: its blocks start while the GEMM's last ones finish and
+// wait here for its writes.
+__global__ void __launch_bounds__(256)
+    splitk_reduce_kernel(int M, int N, int splits, const double *__restrict__ P, int ldp,
+                         double alpha, double beta, double *__restrict__ C, int ldc) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int pairs = (M + 1) / 2;
+  const long long total = (long long)pairs * N;
+  const size_t plane = (size_t)ldp * N;
+  const bool cvec = (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldc & 1) == 0;
+  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
+       idx += (long long)gridDim.x * blockDim.x) {
+    const int n = (int)(idx / pairs), m = (int)(idx - (long long)n * pairs) * 2;
+    const double *p = P + (size_t)n * ldp + m;  // ldp is even: 16-byte aligned
+    double *q = C + (size_t)n * ldc + m;
+    const bool two = m + 1 < M;
+    double2 c;
+    if (two && cvec) c = *reinterpret_cast<const double2 *>(q);
+    else c = make_double2(q[0], two ? q[1] : 0.0);
+    double s0 = 0.0, s1 = 0.0;
+    for (int z = 0; z < splits; z += 4) {
+      double2 x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (z + u < splits) x[u] = *reinterpret_cast<const double2 *>(p + (size_t)(z + u) * plane);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (z + u < splits) s0 += x[u].x, s1 += x[u].y;
+    }
+    c.x = (beta == 1.0) ? fma(alpha, s0, c.x) : fma(alpha, s0, beta * c.x);
+    c.y = (beta == 1.0) ? fma(alpha, s1, c.y) : fma(alpha, s1, beta * c.y);
+    if (two && cvec) *reinterpret_cast<double2 *>(q) = c;
+    else {
+      q[0] = c.x;
+      if (two) q[1] = c.y;
+    }
   }
 }
 
@@ -303,24 +342,34 @@ inline bool is_notrans(char c) { return c == 'N' || c == 'n'; }
 }  // namespace
 
 Fp64Cfg fp64_default_cfg(int m, int n, int k, int sm_count) {
-  // Measured on B200: the 64x64 tile with two CTAs per SM is best from 1024^3
-  // to 8192^3 (31.5 TF at 4096^3); in the exhaustive sweep over 22000 shapes
-  // with M, N, K in [16, 1024] split-K 8 on that tile was the best single
-  // choice, so grids below ~1024 tiles split K up to 8 ways as long as every
-  // slice keeps >= 8 of K (2.6 % mean regret against the per-shape best of
-  // all 36 FP64 configurations; 32 % when slices had to keep >= 32: small-K
-  // products are latency-bound and gain from any split).  The split also
-  // stops at 1024 work units (tiles x slices): 1024^3 runs in 83 us with 4
-  // slices (25.9 TFLOPS) against 87 us unsplit and 90 us with 8; the
-  // partials' extra reduction traffic outweighs the finer wave fit.
-  (void)sm_count;
+  // The 64x64 tile (three CTAs per SM) is the best of the three tiles from
+  // 1024^3 to 8192^3 and in the exhaustive sweep over M, N, K in [16, 1024].
+  // The K split is the one of 1, 2, 4, 8 with the smallest modelled time:
+  // q = work units (tiles x slices) per SM, each of `kit` K blocks of 16 that
+  // take the FP64 pipe 0.53 us; a lone CTA per SM reaches 74 % of that rate,
+  // two 91 %; 3 us to fill and drain, 1 us per further wave of three; a split
+  // adds a second launch and 64 KB of partials per unit, written and read at
+  // about 8 TB/s (they stay in L2).  Measured (B200, us, graph replays):
+  //   128x4096x128   S=1 9.7  2 11.7  4 12.7  8 15.4     512^3  28.3 17.6 15.5 17.5
+  //   512x1024x512   28.4 26.1 27.6 27.4     256^3  15.7 10.5 7.4 6.2
+  // (one fixed rule, 8 slices up to 1024 units, took the last column of the
+  // first three).
   Fp64Cfg c;
   c.tile = 2;
   c.mmak = 8;
-  const long t64 = (long)((m + 63) / 64) * ((n + 63) / 64);
+  const long long t64 = (long long)((m + 63) / 64) * ((n + 63) / 64);
+  const int sms = sm_count > 0 ? sm_count : 148;
   int sk = 1;
-  if (t64 < 1024)
-    while (sk < 8 && k / (2 * sk) >= 8 && t64 * sk * 2 <= 1024) sk *= 2;
+  double best = 1e300;
+  for (int s = 1; s <= 8 && t64 < 8192; s *= 2) {
+    if (s > 1 && k < 8 * s) break;
+    const long long units = t64 * s, q = (units + sms - 1) / sms;
+    const int kit = ((k + s - 1) / s + 15) / 16;
+    const double rate = q == 1 ? 0.74 : q == 2 ? 0.91 : 0.98;
+    double us = (double)q * kit * 0.53 / rate + 3.0 + (double)((q + 2) / 3 - 1);
+    if (s > 1) us += 2.0 + units * 65536.0 / 8e6;
+    if (us < best) best = us, sk = s;
+  }
   c.split_k = sk;
   return c;
 }
@@ -373,11 +422,12 @@ int dgemm_fp64(char ta, char tb, int m, int n, int k, double alpha, const double
     a.kchunk = chunk;
     a.splits = splits;
     if (splits > 1) {
-      const size_t bytes = (size_t)splits * m * n * sizeof(double);
+      const int ldp = (m + 1) & ~1;  // even: 16-byte row pairs in the reduction
+      const size_t bytes = (size_t)splits * ldp * n * sizeof(double);
       double *P = (double *)workspace(cx, WS_MISC, bytes);
       if (!P) return B2_ERR_NOMEM;
       a.P = P;
-      a.ldp = m;
+      a.ldp = ldp;
     } else {
       a.kchunk = k;
     }
@@ -395,10 +445,20 @@ int dgemm_fp64(char ta, char tb, int m, int n, int k, double alpha, const double
   }
   if (e != cudaSuccess) return cuda_fail(e, "dgemm_dmma_kernel");
   if (a.P) {
-    const size_t total = (size_t)m * n;
-    const int blocks = (int)((total + 255) / 256 > 4096 ? 4096 : (total + 255) / 256);
+    const long long total = (long long)((m + 1) / 2) * n;
+    const long long want = (total + 255) / 256;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)(want > 8192 ? 8192 : want));
+    lc.blockDim = dim3(256);
+    lc.stream = s;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
     B2_PROF("dgemm_splitk_reduce", s);
-    splitk_reduce_kernel<<<blocks, 256, 0, s>>>(m, n, a.splits, a.P, a.ldp, alpha, beta, C, ldc);
+    B2_CUDA_TRY(cudaLaunchKernelEx(&lc, splitk_reduce_kernel, m, n, a.splits, (const double *)a.P,
+                                   a.ldp, alpha, beta, C, ldc));
     B2_CUDA_TRY(cudaGetLastError());
   }
   return B2_OK;
