@@ -1,0 +1,49 @@
+"""GPU tests of the FP64 split-K forms (csrc/dgemm_fp64.cu): up to 8 slices
+meet in one thread-block cluster, more write partials to workspace.
+
+Tile edges, slice counts that are not powers of two, a last slice shorter than
+the others, odd leading dimensions (8-byte copies, scalar C) and padding rows
+of C; each result against the double-double yardstick of numpy's extended
+precision, bar ||C - C_ref||_F <= 8 K u ||A||_F ||B||_F (the parity bar of the
+other GEMM tests)."""
+import numpy as np
+import pytest
+
+from gemm_avx512f_b200 import _lib, blas
+from tests._util import fmat, normalized
+
+pytestmark = pytest.mark.gpu
+U = 2.0 ** -53
+
+
+@pytest.mark.parametrize("splits", [2, 3, 4, 5, 6, 7, 8, 9])
+@pytest.mark.parametrize("tile", [0, 1, 2])
+def test_every_slice_count_of_every_tile(cuda, tile, splits):
+    import torch
+
+    L = _lib.lib()
+    rng = np.random.default_rng(100 * tile + splits)
+    # K: `splits` slices of 16 or 32, the last one short; M, N around the tile edges
+    for m, n, k, ta, tb, pad, beta in ((64, 64, 16 * splits, "N", "N", 0, 0.0),
+                                       (129, 63, 16 * splits - 7, "T", "N", 1, 1.0),
+                                       (1, 131, 32 * splits - 31, "N", "T", 3, -0.5),
+                                       (200, 66, 32 * splits, "T", "T", 2, 0.5)):
+        a = fmat(rng, *((m, k) if ta == "N" else (k, m)), pad=pad)
+        b = fmat(rng, *((k, n) if tb == "N" else (n, k)), pad=pad)
+        c = fmat(rng, m, n, pad=pad)
+        opa = a[:m] if ta == "N" else a[:k].T
+        opb = b[:k] if tb == "N" else b[:n].T
+        ref = (1.25 * (opa.astype(np.longdouble) @ opb.astype(np.longdouble))
+               + beta * c[:m].astype(np.longdouble)).astype(np.float64)
+        da, db, dc = (torch.from_numpy(x.T.copy()).to(cuda) for x in (a, b, c))
+        torch.cuda.synchronize()
+        assert L.b2_set_fp64_config(tile, 8, splits) == 0
+        try:
+            blas.dgemm_device(ta, tb, m, n, k, 1.25, da, a.shape[0], db, b.shape[0], beta, dc,
+                              m + pad)
+            torch.cuda.synchronize()
+        finally:
+            L.b2_set_fp64_config(-1, 0, 0)
+        got = dc.cpu().numpy().T
+        assert np.array_equal(got[m:], c[m:]), "padding rows of C were written"
+        assert normalized(got[:m], ref, k, opa, opb, U) <= 8, (m, n, k, ta, tb)
