@@ -7,7 +7,8 @@
 // mma.sync.aligned.m16n8k{4,8,16}.row.col.f64 with accumulators in registers.
 //
 // Design:
-//  * CTA tile BM x BN (128x128 / 128x64 / 64x64), warp tile 64x32 or 32x32.
+//  * CTA tile BM x BN (128x128 / 128x64 / 64x64), warp tile 64x32 or 32x32;
+//    fragments double-buffered in registers (DMMA K 4 and 8).
 //  * op(A)/op(B) tiles streamed global->shared with cp.async (16 B when the
 //    leading dimension and base allow it, else 8 B) through a STAGES-deep ring;
 //    the reference's packing (src/gemm_copy.c) disappears: the smem tile keeps
@@ -37,47 +38,74 @@ __device__ __forceinline__ void cp_async(uint32_t dst, const void *src, int src_
                  "r"(src_bytes));
   }
 }
+template <int BYTES>
+__device__ __forceinline__ void cp_async_full(uint32_t dst, const void *src) {
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-// Load an OUTER x BK operand tile.  Element (o, k) of the operand lives at
-// g[o*ld + k] when KCONT (k contiguous in memory) else g[k*ld + o].
-// Shared layout: KCONT -> [o][BK+4], else [k][OUTER+4].
+// Chunk i of an OUTER x BK operand tile (VEC consecutive elements per thread).
+// Element (o, k) of the operand lives at g[o*ld + k] when KCONT (k contiguous
+// in memory) else g[k*ld + o].  Shared layout: KCONT -> [o][BK+4], else
+// [k][OUTER+4].
+template <int OUTER, int BK, int VEC, int NT>
+__host__ __device__ constexpr int tile_chunks() {
+  static_assert(OUTER * BK / VEC % NT == 0, "tile/thread mismatch");
+  return OUTER * BK / VEC / NT;
+}
 template <int OUTER, int BK, bool KCONT, int VEC, int NT>
-__device__ __forceinline__ void load_tile(uint32_t sbase, const double *__restrict__ g, int ld,
-                                          int o0, int k0, int olim, int klim, int tid) {
+__device__ __forceinline__ void load_chunk(uint32_t sbase, const double *__restrict__ g, int ld,
+                                           int o0, int k0, int olim, int klim, int tid, int i) {
+  const int c = tid + i * NT;
   if constexpr (KCONT) {
     constexpr int CPR = BK / VEC;
-    constexpr int TOTAL = OUTER * CPR;
-    static_assert(TOTAL % NT == 0, "tile/thread mismatch");
-#pragma unroll
-    for (int i = 0; i < TOTAL / NT; ++i) {
-      const int c = tid + i * NT;
-      const int o = c / CPR, kc = (c % CPR) * VEC;
-      const int go = o0 + o, gk = k0 + kc;
-      int valid = (go < olim) ? min(VEC, klim - gk) : 0;
-      valid = valid < 0 ? 0 : valid;
-      const double *src = valid ? g + (size_t)go * ld + gk : g;
-      cp_async<VEC * 8>(sbase + (uint32_t)(o * (BK + 4) + kc) * 8u, src, valid * 8);
-    }
+    const int o = c / CPR, kc = (c % CPR) * VEC;
+    const int go = o0 + o, gk = k0 + kc;
+    int valid = (go < olim) ? min(VEC, klim - gk) : 0;
+    valid = valid < 0 ? 0 : valid;
+    const double *src = valid ? g + (size_t)go * ld + gk : g;
+    cp_async<VEC * 8>(sbase + (uint32_t)(o * (BK + 4) + kc) * 8u, src, valid * 8);
   } else {
     constexpr int CPR = OUTER / VEC;
-    constexpr int TOTAL = BK * CPR;
-    static_assert(TOTAL % NT == 0, "tile/thread mismatch");
-#pragma unroll
-    for (int i = 0; i < TOTAL / NT; ++i) {
-      const int c = tid + i * NT;
-      const int kr = c / CPR, oc = (c % CPR) * VEC;
-      const int go = o0 + oc, gk = k0 + kr;
-      int valid = (gk < klim) ? min(VEC, olim - go) : 0;
-      valid = valid < 0 ? 0 : valid;
-      const double *src = valid ? g + (size_t)gk * ld + go : g;
-      cp_async<VEC * 8>(sbase + (uint32_t)(kr * (OUTER + 4) + oc) * 8u, src, valid * 8);
-    }
+    const int kr = c / CPR, oc = (c % CPR) * VEC;
+    const int go = o0 + oc, gk = k0 + kr;
+    int valid = (gk < klim) ? min(VEC, olim - go) : 0;
+    valid = valid < 0 ? 0 : valid;
+    const double *src = valid ? g + (size_t)gk * ld + go : g;
+    cp_async<VEC * 8>(sbase + (uint32_t)(kr * (OUTER + 4) + oc) * 8u, src, valid * 8);
   }
+}
+
+// The same map for tiles without an edge: element offset of the thread's chunk
+// 0 in the operand, its shared-memory byte offset, and the distances from one
+// chunk to the next.
+template <int OUTER, int BK, bool KCONT, int VEC>
+__device__ __forceinline__ size_t run_offset(int o0, int k0, int ld, int tid) {
+  constexpr int CPR = (KCONT ? BK : OUTER) / VEC;
+  const int hi = tid / CPR, lo = (tid % CPR) * VEC;
+  return KCONT ? (size_t)(o0 + hi) * ld + (k0 + lo) : (size_t)(k0 + hi) * ld + (o0 + lo);
+}
+template <int OUTER, int BK, bool KCONT, int VEC>
+__device__ __forceinline__ uint32_t run_dst(int tid) {
+  constexpr int CPR = (KCONT ? BK : OUTER) / VEC;
+  return (uint32_t)((tid / CPR) * (KCONT ? BK + 4 : OUTER + 4) + (tid % CPR) * VEC) * 8u;
+}
+template <int OUTER, int BK, bool KCONT, int VEC, int NT>
+__device__ __forceinline__ size_t run_step(int ld) {
+  constexpr int CPR = (KCONT ? BK : OUTER) / VEC;
+  static_assert(NT % CPR == 0, "chunk rows must be whole");
+  return (size_t)(NT / CPR) * ld;
+}
+template <int OUTER, int BK, bool KCONT, int VEC, int NT>
+__host__ __device__ constexpr uint32_t run_dst_step() {
+  return (uint32_t)(NT / ((KCONT ? BK : OUTER) / VEC) * (KCONT ? BK + 4 : OUTER + 4)) * 8u;
 }
 
 template <int MMAK>
@@ -109,7 +137,7 @@ __device__ __forceinline__ void dmma(double (&c)[4], const double *a, const doub
 // P + z*ldp*N (split-K partial); otherwise C = alpha*acc + beta*C (beta==1: C += alpha*acc).
 template <int BM, int BN, int BK, int WM, int WN, int STAGES, int MMAK, bool A_KCONT,
           bool B_KCONT, int VEC>
-__global__ void __launch_bounds__(WM *WN * 32, 1)
+__global__ void __launch_bounds__(WM *WN * 32, BM * BN <= 64 * 64 && MMAK == 4 ? 3 : 1)
     dgemm_dmma_kernel(int M, int N, int K, int kchunk, double alpha,
                       const double *__restrict__ A, int lda, const double *__restrict__ B,
                       int ldb, double beta, double *__restrict__ C, int ldc,
@@ -143,10 +171,43 @@ __global__ void __launch_bounds__(WM *WN * 32, 1)
 #pragma unroll
       for (int v = 0; v < 4; ++v) acc[i][j][v] = 0.0;
 
+  constexpr int A_CH = tile_chunks<BM, BK, VEC, NT>(), B_CH = tile_chunks<BN, BK, VEC, NT>();
+  // Tiles that lie wholly inside the matrices copy from running pointers (a
+  // few instructions per copy); edge tiles and a last short K block take the
+  // bounds-checked form.
+  const bool inside = m0 + BM <= M && n0 + BN <= N;
+  const double *pa = A + run_offset<BM, BK, A_KCONT, VEC>(m0, kbeg, lda, tid);
+  const double *pb = B + run_offset<BN, BK, B_KCONT, VEC>(n0, kbeg, ldb, tid);
+  const uint32_t da = sA_u + run_dst<BM, BK, A_KCONT, VEC>(tid);
+  const uint32_t db = sB_u + run_dst<BN, BK, B_KCONT, VEC>(tid);
+  const size_t ia = run_step<BM, BK, A_KCONT, VEC, NT>(lda);  // chunk to chunk
+  const size_t ib = run_step<BN, BK, B_KCONT, VEC, NT>(ldb);
+  const size_t ka = A_KCONT ? (size_t)BK : (size_t)BK * lda;  // stage to stage
+  const size_t kb = B_KCONT ? (size_t)BK : (size_t)BK * ldb;
+  // Copies stage kt (called once per kt, in order) into ring slot st.
   auto load_stage = [&](int st, int kt) {
     const int k0 = kbeg + kt * BK;
-    load_tile<BM, BK, A_KCONT, VEC, NT>(sA_u + st * A_ST * 8, A, lda, m0, k0, M, kend, tid);
-    load_tile<BN, BK, B_KCONT, VEC, NT>(sB_u + st * B_ST * 8, B, ldb, n0, k0, N, kend, tid);
+    if (inside && k0 + BK <= kend) {
+#pragma unroll
+      for (int c = 0; c < A_CH; ++c)
+        cp_async_full<VEC * 8>(da + st * (A_ST * 8) + c * run_dst_step<BM, BK, A_KCONT, VEC, NT>(),
+                               pa + c * ia);
+#pragma unroll
+      for (int c = 0; c < B_CH; ++c)
+        cp_async_full<VEC * 8>(db + st * (B_ST * 8) + c * run_dst_step<BN, BK, B_KCONT, VEC, NT>(),
+                               pb + c * ib);
+    } else {
+#pragma unroll
+      for (int c = 0; c < A_CH; ++c)
+        load_chunk<BM, BK, A_KCONT, VEC, NT>(sA_u + st * A_ST * 8, A, lda, m0, k0, M, kend, tid,
+                                             c);
+#pragma unroll
+      for (int c = 0; c < B_CH; ++c)
+        load_chunk<BN, BK, B_KCONT, VEC, NT>(sB_u + st * B_ST * 8, B, ldb, n0, k0, N, kend, tid,
+                                             c);
+    }
+    pa += ka;
+    pb += kb;
   };
 
 #pragma unroll
@@ -155,41 +216,65 @@ __global__ void __launch_bounds__(WM *WN * 32, 1)
     cp_async_commit();
   }
 
-  for (int kt = 0; kt < KT; ++kt) {
-    cp_async_wait<STAGES - 2>();
-    __syncthreads();
-    {
-      const int kn = kt + STAGES - 1;
-      if (kn < KT) load_stage(kn % STAGES, kn);
-      cp_async_commit();
-    }
-    const double *As = sA + (kt % STAGES) * A_ST;
-    const double *Bs = sB + (kt % STAGES) * B_ST;
+  // Bound: the FP64 pipe (0.533 us per 64x64x16 block and SM at 1.92 GHz).
+  // Fragments are double-buffered in registers: the next K step's shared loads
+  // (across a stage's edge too, so the barrier sits before the last step's
+  // DMMAs) are in flight while the current step's DMMAs issue.  With the
+  // running copy pointers and DMMA K 4 (whose fragments leave three CTAs per
+  // SM) a block takes 0.553 us where it took 0.597 (K = 4096, 10 tiles per SM;
+  // 4096^3 4228 -> 3886 us); one CTA alone on an SM 0.72 instead of 1.0.
+  // Copies placed one by one between the DMMAs were slower (0.70).
+  constexpr int KS = BK / MMAK;
+  // (DMMA K 16 has one step per stage and twice the fragments: single-buffered.)
+  constexpr bool PIPE = KS % 2 == 0;
+  double af[PIPE ? 2 : 1][MT][MMAK / 2], bf[PIPE ? 2 : 1][NTL][MMAK / 4];
+  auto load_frags = [&](int buf, int st, int kk) {
+    const double *As = sA + st * A_ST;
+    const double *Bs = sB + st * B_ST;
 #pragma unroll
-    for (int kk = 0; kk < BK; kk += MMAK) {
-      double af[MT][MMAK / 2];
-      double bf[NTL][MMAK / 4];
+    for (int i = 0; i < MT; ++i)
 #pragma unroll
-      for (int i = 0; i < MT; ++i)
+      for (int v1 = 0; v1 < MMAK / 4; ++v1)
 #pragma unroll
-        for (int v1 = 0; v1 < MMAK / 4; ++v1)
-#pragma unroll
-          for (int v0 = 0; v0 < 2; ++v0) {
-            const int m = wm0 + i * 16 + g + 8 * v0, k = kk + t + 4 * v1;
-            af[i][v0 + 2 * v1] = A_KCONT ? As[m * (BK + 4) + k] : As[k * (BM + 4) + m];
-          }
-#pragma unroll
-      for (int j = 0; j < NTL; ++j)
-#pragma unroll
-        for (int v = 0; v < MMAK / 4; ++v) {
-          const int n = wn0 + j * 8 + g, k = kk + t + 4 * v;
-          bf[j][v] = B_KCONT ? Bs[n * (BK + 4) + k] : Bs[k * (BN + 4) + n];
+        for (int v0 = 0; v0 < 2; ++v0) {
+          const int m = wm0 + i * 16 + g + 8 * v0, k = kk + t + 4 * v1;
+          af[buf][i][v0 + 2 * v1] = A_KCONT ? As[m * (BK + 4) + k] : As[k * (BM + 4) + m];
         }
 #pragma unroll
+    for (int j = 0; j < NTL; ++j)
+#pragma unroll
+      for (int v = 0; v < MMAK / 4; ++v) {
+        const int n = wn0 + j * 8 + g, k = kk + t + 4 * v;
+        bf[buf][j][v] = B_KCONT ? Bs[n * (BK + 4) + k] : Bs[k * (BN + 4) + n];
+      }
+  };
+  cp_async_wait<STAGES - 2>();
+  __syncthreads();
+  if (PIPE) load_frags(0, 0, 0);
+  int st = 0, st_fill = STAGES - 1;  // stage being multiplied, stage refilled next
+  for (int kt = 0; kt < KT; ++kt) {
+    const int st_next = st + 1 == STAGES ? 0 : st + 1;
+    // every warp has issued its last reads of stage kt - 1, which is refilled here
+    const bool fill = kt + STAGES - 1 < KT;
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      const int cur = PIPE ? (ks & 1) : 0;
+      if (!PIPE) load_frags(0, st, ks * MMAK);
+      if (PIPE && ks + 1 < KS) load_frags(cur ^ 1, st, (ks + 1) * MMAK);
+      if (ks == 0 && fill) load_stage(st_fill, kt + STAGES - 1);
+      if (ks + 1 == KS) {
+        cp_async_commit();
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();
+        if (PIPE && kt + 1 < KT) load_frags(cur ^ 1, st_next, 0);
+      }
+#pragma unroll
       for (int i = 0; i < MT; ++i)
 #pragma unroll
-        for (int j = 0; j < NTL; ++j) dmma<MMAK>(acc[i][j], af[i], bf[j]);
+        for (int j = 0; j < NTL; ++j) dmma<MMAK>(acc[i][j], af[cur][i], bf[cur][j]);
     }
+    st = st_next;
+    st_fill = st_fill + 1 == STAGES ? 0 : st_fill + 1;
   }
   cp_async_wait<0>();
 
@@ -322,7 +407,10 @@ cudaError_t launch_one(const LaunchArgs &a, cudaStream_t s) {
 
 template <int BM, int BN, int WM, int WN, int STAGES, int MMAK, int VEC>
 cudaError_t launch_layout(bool ak, bool bk, const LaunchArgs &a, cudaStream_t s) {
-  if (ak && bk) return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, true, true, VEC>(a, s);
+  // 64x64, both operands K-contiguous: 80 KB in four stages would leave two
+  // CTAs per SM; three stages keep three
+  constexpr int ST_TN = BM * BN <= 64 * 64 ? 3 : STAGES;
+  if (ak && bk) return launch_one<BM, BN, 16, WM, WN, ST_TN, MMAK, true, true, VEC>(a, s);
   if (ak && !bk) return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, true, false, VEC>(a, s);
   if (!ak && bk) return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, false, true, VEC>(a, s);
   return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, false, false, VEC>(a, s);
@@ -356,7 +444,7 @@ Fp64Cfg fp64_default_cfg(int m, int n, int k, int sm_count) {
   // first three).
   Fp64Cfg c;
   c.tile = 2;
-  c.mmak = 8;
+  c.mmak = 4;
   const long long t64 = (long long)((m + 63) / 64) * ((n + 63) / 64);
   const int sms = sm_count > 0 ? sm_count : 148;
   int sk = 1;
