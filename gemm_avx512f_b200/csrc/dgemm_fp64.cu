@@ -9,8 +9,8 @@
 // Design:
 //  * CTA tile BM x BN (128x128 / 128x64 / 64x64), warp tile 64x32 or 32x32;
 //    fragments double-buffered in registers (DMMA K 4 and 8).
-//  * op(A)/op(B) tiles streamed global->shared with cp.async (16 B when the
-//    leading dimension and base allow it, else 8 B) through a STAGES-deep ring;
+//  * op(A)/op(B) tiles streamed global->shared with 16-byte cp.async (rows off
+//    a 16-byte boundary shifted by one element) through a STAGES-deep ring;
 //    the reference's packing (src/gemm_copy.c) disappears: the smem tile keeps
 //    the global orientation, padded so every DMMA fragment load is
 //    bank-conflict free for both orientations (+4 doubles per row).
@@ -51,61 +51,89 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-// Chunk i of an OUTER x BK operand tile (VEC consecutive elements per thread).
-// Element (o, k) of the operand lives at g[o*ld + k] when KCONT (k contiguous
-// in memory) else g[k*ld + o].  Shared layout: KCONT -> [o][BK+4], else
-// [k][OUTER+4].
-template <int OUTER, int BK, int VEC, int NT>
-__host__ __device__ constexpr int tile_chunks() {
-  static_assert(OUTER * BK / VEC % NT == 0, "tile/thread mismatch");
-  return OUTER * BK / VEC / NT;
+// Operand tiles are copied as 16-byte chunks (two elements) of the rows that are
+// contiguous in memory.  SH: the operand's base or leading dimension is odd, so
+// rows may start 8 bytes off a 16-byte boundary; such a row is copied from one
+// element earlier (one chunk more) and sits one element later in its shared
+// row, whose padding has room for both.  Tiles start at even elements, so a
+// row's shift is row_shift(p0, ld, row), and the row distances between one
+// thread's chunks, and between its fragment reads, are even: the shift is a
+// constant of the thread.  Odd leading dimensions took 8-byte copies before:
+// 2501x1777x1999 668 -> FILL us on B200.
+__device__ __forceinline__ int row_shift(const double *g, int ld, int row) {
+  return (int)(((reinterpret_cast<uintptr_t>(g) >> 3) + (unsigned)row * (unsigned)ld) & 1u);
 }
-template <int OUTER, int BK, bool KCONT, int VEC, int NT>
-__device__ __forceinline__ void load_chunk(uint32_t sbase, const double *__restrict__ g, int ld,
-                                           int o0, int k0, int olim, int klim, int tid, int i) {
-  const int c = tid + i * NT;
-  if constexpr (KCONT) {
-    constexpr int CPR = BK / VEC;
-    const int o = c / CPR, kc = (c % CPR) * VEC;
-    const int go = o0 + o, gk = k0 + kc;
-    int valid = (go < olim) ? min(VEC, klim - gk) : 0;
-    valid = valid < 0 ? 0 : valid;
-    const double *src = valid ? g + (size_t)go * ld + gk : g;
-    cp_async<VEC * 8>(sbase + (uint32_t)(o * (BK + 4) + kc) * 8u, src, valid * 8);
-  } else {
-    constexpr int CPR = OUTER / VEC;
-    const int kr = c / CPR, oc = (c % CPR) * VEC;
-    const int go = o0 + oc, gk = k0 + kr;
-    int valid = (gk < klim) ? min(VEC, olim - go) : 0;
-    valid = valid < 0 ? 0 : valid;
-    const double *src = valid ? g + (size_t)gk * ld + go : g;
-    cp_async<VEC * 8>(sbase + (uint32_t)(kr * (OUTER + 4) + oc) * 8u, src, valid * 8);
+
+// Chunk i of an OUTER x BK operand tile.  Element (o, k) of the operand lives
+// at g[o*ld + k] when KCONT (k contiguous in memory) else g[k*ld + o].  Shared
+// layout: KCONT -> [o][BK+4], else [k][OUTER+4].
+template <int OUTER, int BK, int NT>
+__host__ __device__ constexpr int tile_chunks() {
+  static_assert(OUTER * BK / 2 % NT == 0, "tile/thread mismatch");
+  return OUTER * BK / 2 / NT;
+}
+// One bounds-checked chunk: elements e0, e0 + 1 (e0 may be -1: not needed) of
+// row `row`, zero beyond the row's lim elements and for rows >= rows.
+template <bool SH>
+__device__ __forceinline__ void copy_pair(uint32_t dst, const double *__restrict__ g, int ld,
+                                          int row, int rows, int e0, int lim) {
+  int valid = row < rows ? min(2, lim - e0) : 0;
+  valid = valid < 0 ? 0 : valid;
+  if (SH && e0 < 0 && row == 0) {  // the element before the operand's first is not read
+    cp_async<8>(dst + 8, g, valid > 1 ? 8 : 0);
+    return;
   }
+  const double *none = reinterpret_cast<const double *>(reinterpret_cast<uintptr_t>(g) &
+                                                        ~(uintptr_t)15);
+  cp_async<16>(dst, valid ? g + (size_t)row * ld + e0 : none, valid * 8);
+}
+template <int OUTER, int BK, bool KCONT, bool SH, int NT>
+__device__ __forceinline__ void load_chunk(uint32_t sbase, const double *__restrict__ g, int ld,
+                                           int o0, int k0, int olim, int klim, int tid, int i,
+                                           int sh) {
+  const int c = tid + i * NT;
+  constexpr int CPR = (KCONT ? BK : OUTER) / 2;
+  const int hi = c / CPR, lo = (c % CPR) * 2;
+  const uint32_t dst = sbase + (uint32_t)(hi * (KCONT ? BK + 4 : OUTER + 4) + lo) * 8u;
+  if (KCONT) copy_pair<SH>(dst, g, ld, o0 + hi, olim, k0 + lo - sh, klim);
+  else copy_pair<SH>(dst, g, ld, k0 + hi, klim, o0 + lo - sh, olim);
+}
+// The chunk past the end of each shifted row (its first element is the row's last).
+template <int OUTER, int BK, bool KCONT, int NT>
+__device__ __forceinline__ void load_tails(uint32_t sbase, const double *__restrict__ g, int ld,
+                                           int o0, int k0, int olim, int klim, int tid) {
+  constexpr int ROWS = KCONT ? OUTER : BK, LEN = KCONT ? BK : OUTER;
+  static_assert(ROWS <= NT, "one tail per thread");
+  const int row = (KCONT ? o0 : k0) + tid;
+  if (tid >= ROWS || !row_shift(g, ld, row)) return;
+  const uint32_t dst = sbase + (uint32_t)(tid * (LEN + 4) + LEN) * 8u;
+  if (KCONT) copy_pair<true>(dst, g, ld, row, olim, k0 + LEN - 1, klim);
+  else copy_pair<true>(dst, g, ld, row, klim, o0 + LEN - 1, olim);
 }
 
 // The same map for tiles without an edge: element offset of the thread's chunk
 // 0 in the operand, its shared-memory byte offset, and the distances from one
 // chunk to the next.
-template <int OUTER, int BK, bool KCONT, int VEC>
+template <int OUTER, int BK, bool KCONT>
 __device__ __forceinline__ size_t run_offset(int o0, int k0, int ld, int tid) {
-  constexpr int CPR = (KCONT ? BK : OUTER) / VEC;
-  const int hi = tid / CPR, lo = (tid % CPR) * VEC;
+  constexpr int CPR = (KCONT ? BK : OUTER) / 2;
+  const int hi = tid / CPR, lo = (tid % CPR) * 2;
   return KCONT ? (size_t)(o0 + hi) * ld + (k0 + lo) : (size_t)(k0 + hi) * ld + (o0 + lo);
 }
-template <int OUTER, int BK, bool KCONT, int VEC>
+template <int OUTER, int BK, bool KCONT>
 __device__ __forceinline__ uint32_t run_dst(int tid) {
-  constexpr int CPR = (KCONT ? BK : OUTER) / VEC;
-  return (uint32_t)((tid / CPR) * (KCONT ? BK + 4 : OUTER + 4) + (tid % CPR) * VEC) * 8u;
+  constexpr int CPR = (KCONT ? BK : OUTER) / 2;
+  return (uint32_t)((tid / CPR) * (KCONT ? BK + 4 : OUTER + 4) + (tid % CPR) * 2) * 8u;
 }
-template <int OUTER, int BK, bool KCONT, int VEC, int NT>
+template <int OUTER, int BK, bool KCONT, int NT>
 __device__ __forceinline__ size_t run_step(int ld) {
-  constexpr int CPR = (KCONT ? BK : OUTER) / VEC;
-  static_assert(NT % CPR == 0, "chunk rows must be whole");
+  constexpr int CPR = (KCONT ? BK : OUTER) / 2;
+  static_assert(NT % CPR == 0 && (NT / CPR) % 2 == 0, "an even number of whole rows per step");
   return (size_t)(NT / CPR) * ld;
 }
-template <int OUTER, int BK, bool KCONT, int VEC, int NT>
+template <int OUTER, int BK, bool KCONT, int NT>
 __host__ __device__ constexpr uint32_t run_dst_step() {
-  return (uint32_t)(NT / ((KCONT ? BK : OUTER) / VEC) * (KCONT ? BK + 4 : OUTER + 4)) * 8u;
+  return (uint32_t)(NT / ((KCONT ? BK : OUTER) / 2) * (KCONT ? BK + 4 : OUTER + 4)) * 8u;
 }
 
 template <int MMAK>
@@ -136,7 +164,7 @@ __device__ __forceinline__ void dmma(double (&c)[4], const double *a, const doub
 // Output: when P != nullptr the raw product of this CTA's K range is written to
 // P + z*ldp*N (split-K partial); otherwise C = alpha*acc + beta*C (beta==1: C += alpha*acc).
 template <int BM, int BN, int BK, int WM, int WN, int STAGES, int MMAK, bool A_KCONT,
-          bool B_KCONT, int VEC>
+          bool B_KCONT, bool SH>
 __global__ void __launch_bounds__(WM *WN * 32, BM * BN <= 64 * 64 && MMAK == 4 ? 3 : 1)
     dgemm_dmma_kernel(int M, int N, int K, int kchunk, double alpha,
                       const double *__restrict__ A, int lda, const double *__restrict__ B,
@@ -171,40 +199,52 @@ __global__ void __launch_bounds__(WM *WN * 32, BM * BN <= 64 * 64 && MMAK == 4 ?
 #pragma unroll
       for (int v = 0; v < 4; ++v) acc[i][j][v] = 0.0;
 
-  constexpr int A_CH = tile_chunks<BM, BK, VEC, NT>(), B_CH = tile_chunks<BN, BK, VEC, NT>();
+  constexpr int A_CH = tile_chunks<BM, BK, NT>(), B_CH = tile_chunks<BN, BK, NT>();
+  // row shifts of this thread's chunks and of its fragment reads (A rows are k
+  // or m: the fragments' rows are t or g plus even numbers)
+  const int sha = SH ? row_shift(A, lda, (A_KCONT ? m0 : kbeg) + tid / ((A_KCONT ? BK : BM) / 2)) : 0;
+  const int shb = SH ? row_shift(B, ldb, (B_KCONT ? n0 : kbeg) + tid / ((B_KCONT ? BK : BN) / 2)) : 0;
+  const int fsa = SH ? row_shift(A, lda, A_KCONT ? g : t) : 0;
+  const int fsb = SH ? row_shift(B, ldb, B_KCONT ? g : t) : 0;
   // Tiles that lie wholly inside the matrices copy from running pointers (a
-  // few instructions per copy); edge tiles and a last short K block take the
+  // few instructions per copy); edge tiles, a last short K block and, when
+  // shifted, whatever touches the operand's first row's start take the
   // bounds-checked form.
   const bool inside = m0 + BM <= M && n0 + BN <= N;
-  const double *pa = A + run_offset<BM, BK, A_KCONT, VEC>(m0, kbeg, lda, tid);
-  const double *pb = B + run_offset<BN, BK, B_KCONT, VEC>(n0, kbeg, ldb, tid);
-  const uint32_t da = sA_u + run_dst<BM, BK, A_KCONT, VEC>(tid);
-  const uint32_t db = sB_u + run_dst<BN, BK, B_KCONT, VEC>(tid);
-  const size_t ia = run_step<BM, BK, A_KCONT, VEC, NT>(lda);  // chunk to chunk
-  const size_t ib = run_step<BN, BK, B_KCONT, VEC, NT>(ldb);
+  const bool a_first = SH && (A_KCONT ? m0 : kbeg) == 0, b_first = SH && (B_KCONT ? n0 : kbeg) == 0;
+  const double *pa = A + run_offset<BM, BK, A_KCONT>(m0, kbeg, lda, tid) - sha;
+  const double *pb = B + run_offset<BN, BK, B_KCONT>(n0, kbeg, ldb, tid) - shb;
+  const uint32_t da = sA_u + run_dst<BM, BK, A_KCONT>(tid);
+  const uint32_t db = sB_u + run_dst<BN, BK, B_KCONT>(tid);
+  const size_t ia = run_step<BM, BK, A_KCONT, NT>(lda);  // chunk to chunk
+  const size_t ib = run_step<BN, BK, B_KCONT, NT>(ldb);
   const size_t ka = A_KCONT ? (size_t)BK : (size_t)BK * lda;  // stage to stage
   const size_t kb = B_KCONT ? (size_t)BK : (size_t)BK * ldb;
   // Copies stage kt (called once per kt, in order) into ring slot st.
   auto load_stage = [&](int st, int kt) {
     const int k0 = kbeg + kt * BK;
-    if (inside && k0 + BK <= kend) {
+    if (inside && k0 + BK <= kend && !(kt == 0 && (a_first || b_first))) {
 #pragma unroll
       for (int c = 0; c < A_CH; ++c)
-        cp_async_full<VEC * 8>(da + st * (A_ST * 8) + c * run_dst_step<BM, BK, A_KCONT, VEC, NT>(),
-                               pa + c * ia);
+        cp_async_full<16>(da + st * (A_ST * 8) + c * run_dst_step<BM, BK, A_KCONT, NT>(),
+                          pa + c * ia);
 #pragma unroll
       for (int c = 0; c < B_CH; ++c)
-        cp_async_full<VEC * 8>(db + st * (B_ST * 8) + c * run_dst_step<BN, BK, B_KCONT, VEC, NT>(),
-                               pb + c * ib);
+        cp_async_full<16>(db + st * (B_ST * 8) + c * run_dst_step<BN, BK, B_KCONT, NT>(),
+                          pb + c * ib);
     } else {
 #pragma unroll
       for (int c = 0; c < A_CH; ++c)
-        load_chunk<BM, BK, A_KCONT, VEC, NT>(sA_u + st * A_ST * 8, A, lda, m0, k0, M, kend, tid,
-                                             c);
+        load_chunk<BM, BK, A_KCONT, SH, NT>(sA_u + st * A_ST * 8, A, lda, m0, k0, M, kend, tid, c,
+                                            sha);
 #pragma unroll
       for (int c = 0; c < B_CH; ++c)
-        load_chunk<BN, BK, B_KCONT, VEC, NT>(sB_u + st * B_ST * 8, B, ldb, n0, k0, N, kend, tid,
-                                             c);
+        load_chunk<BN, BK, B_KCONT, SH, NT>(sB_u + st * B_ST * 8, B, ldb, n0, k0, N, kend, tid, c,
+                                            shb);
+    }
+    if (SH) {
+      load_tails<BM, BK, A_KCONT, NT>(sA_u + st * A_ST * 8, A, lda, m0, k0, M, kend, tid);
+      load_tails<BN, BK, B_KCONT, NT>(sB_u + st * B_ST * 8, B, ldb, n0, k0, N, kend, tid);
     }
     pa += ka;
     pb += kb;
@@ -229,8 +269,8 @@ __global__ void __launch_bounds__(WM *WN * 32, BM * BN <= 64 * 64 && MMAK == 4 ?
   constexpr bool PIPE = KS % 2 == 0;
   double af[PIPE ? 2 : 1][MT][MMAK / 2], bf[PIPE ? 2 : 1][NTL][MMAK / 4];
   auto load_frags = [&](int buf, int st, int kk) {
-    const double *As = sA + st * A_ST;
-    const double *Bs = sB + st * B_ST;
+    const double *As = sA + st * A_ST + fsa;
+    const double *Bs = sB + st * B_ST + fsb;
 #pragma unroll
     for (int i = 0; i < MT; ++i)
 #pragma unroll
@@ -389,12 +429,12 @@ struct LaunchArgs {
 };
 
 template <int BM, int BN, int BK, int WM, int WN, int STAGES, int MMAK, bool AK, bool BKc,
-          int VEC>
+          bool SH>
 cudaError_t launch_one(const LaunchArgs &a, cudaStream_t s) {
   constexpr int A_ST = AK ? BM * (BK + 4) : BK * (BM + 4);
   constexpr int B_ST = BKc ? BN * (BK + 4) : BK * (BN + 4);
   constexpr size_t SMEM = (size_t)STAGES * (A_ST + B_ST) * sizeof(double);
-  auto kern = dgemm_dmma_kernel<BM, BN, BK, WM, WN, STAGES, MMAK, AK, BKc, VEC>;
+  auto kern = dgemm_dmma_kernel<BM, BN, BK, WM, WN, STAGES, MMAK, AK, BKc, SH>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)SMEM);
   if (e != cudaSuccess) return e;
@@ -405,23 +445,23 @@ cudaError_t launch_one(const LaunchArgs &a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-template <int BM, int BN, int WM, int WN, int STAGES, int MMAK, int VEC>
+template <int BM, int BN, int WM, int WN, int STAGES, int MMAK, bool SH>
 cudaError_t launch_layout(bool ak, bool bk, const LaunchArgs &a, cudaStream_t s) {
   // 64x64, both operands K-contiguous: 80 KB in four stages would leave two
   // CTAs per SM; three stages keep three
   constexpr int ST_TN = BM * BN <= 64 * 64 ? 3 : STAGES;
-  if (ak && bk) return launch_one<BM, BN, 16, WM, WN, ST_TN, MMAK, true, true, VEC>(a, s);
-  if (ak && !bk) return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, true, false, VEC>(a, s);
-  if (!ak && bk) return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, false, true, VEC>(a, s);
-  return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, false, false, VEC>(a, s);
+  if (ak && bk) return launch_one<BM, BN, 16, WM, WN, ST_TN, MMAK, true, true, SH>(a, s);
+  if (ak && !bk) return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, true, false, SH>(a, s);
+  if (!ak && bk) return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, false, true, SH>(a, s);
+  return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, false, false, SH>(a, s);
 }
 
-template <int MMAK, int VEC>
+template <int MMAK, bool SH>
 cudaError_t launch_tile(int tile, bool ak, bool bk, const LaunchArgs &a, cudaStream_t s) {
   switch (tile) {
-    case 0: return launch_layout<128, 128, 2, 4, 4, MMAK, VEC>(ak, bk, a, s);
-    case 1: return launch_layout<128, 64, 2, 2, 4, MMAK, VEC>(ak, bk, a, s);
-    default: return launch_layout<64, 64, 2, 2, 4, MMAK, VEC>(ak, bk, a, s);
+    case 0: return launch_layout<128, 128, 2, 4, 4, MMAK, SH>(ak, bk, a, s);
+    case 1: return launch_layout<128, 64, 2, 2, 4, MMAK, SH>(ak, bk, a, s);
+    default: return launch_layout<64, 64, 2, 2, 4, MMAK, SH>(ak, bk, a, s);
   }
 }
 
@@ -523,13 +563,13 @@ int dgemm_fp64(char ta, char tb, int m, int n, int k, double alpha, const double
   cudaError_t e;
   const int mk = cfg.mmak;
   if (vec2) {
-    e = mk == 16 ? launch_tile<16, 2>(cfg.tile, ak, bk, a, s)
-        : mk == 8 ? launch_tile<8, 2>(cfg.tile, ak, bk, a, s)
-                  : launch_tile<4, 2>(cfg.tile, ak, bk, a, s);
+    e = mk == 16 ? launch_tile<16, false>(cfg.tile, ak, bk, a, s)
+        : mk == 8 ? launch_tile<8, false>(cfg.tile, ak, bk, a, s)
+                  : launch_tile<4, false>(cfg.tile, ak, bk, a, s);
   } else {
-    e = mk == 16 ? launch_tile<16, 1>(cfg.tile, ak, bk, a, s)
-        : mk == 8 ? launch_tile<8, 1>(cfg.tile, ak, bk, a, s)
-                  : launch_tile<4, 1>(cfg.tile, ak, bk, a, s);
+    e = mk == 16 ? launch_tile<16, true>(cfg.tile, ak, bk, a, s)
+        : mk == 8 ? launch_tile<8, true>(cfg.tile, ak, bk, a, s)
+                  : launch_tile<4, true>(cfg.tile, ak, bk, a, s);
   }
   if (e != cudaSuccess) return cuda_fail(e, "dgemm_dmma_kernel");
   if (a.P) {

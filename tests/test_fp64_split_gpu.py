@@ -47,3 +47,42 @@ def test_every_slice_count_of_every_tile(cuda, tile, splits):
         got = dc.cpu().numpy().T
         assert np.array_equal(got[m:], c[m:]), "padding rows of C were written"
         assert normalized(got[:m], ref, k, opa, opb, U) <= 8, (m, n, k, ta, tb)
+
+
+@pytest.mark.parametrize("ta,tb", [("N", "N"), ("N", "T"), ("T", "N"), ("T", "T")])
+@pytest.mark.parametrize("offs", [(0, 0), (1, 0), (0, 1), (1, 1)])
+def test_operands_off_a_16_byte_boundary(cuda, ta, tb, offs):
+    """Bases 8 bytes off and odd / even leading dimensions in every pairing:
+    rows are then copied with a shift of one element."""
+    import torch
+
+    rng = np.random.default_rng(17)
+    for m, n, k, pa, pb in ((129, 130, 77, 0, 1), (64, 128, 64, 1, 1), (257, 65, 160, 2, 3),
+                            (63, 64, 5, 1, 0), (1, 2, 1, 0, 0)):
+        ar, ac = (m, k) if ta == "N" else (k, m)
+        br, bc = (k, n) if tb == "N" else (n, k)
+        a, b, c = fmat(rng, ar, ac, pad=pa), fmat(rng, br, bc, pad=pb), fmat(rng, m, n, pad=1)
+        opa = a[:ar] if ta == "N" else a[:ar].T
+        opb = b[:br] if tb == "N" else b[:br].T
+        ref = (opa.astype(np.longdouble) @ opb.astype(np.longdouble)
+               + 0.5 * c[:m].astype(np.longdouble)).astype(np.float64)
+
+        def up(x, off):
+            # NaN around the operand: a value read from outside would show
+            t = torch.full((x.size + 4,), float("nan"), dtype=torch.float64, device=cuda)
+            t[off:off + x.size] = torch.from_numpy(x.T.copy().reshape(-1)).to(cuda)
+            return t[off:]
+
+        for tile in (0, 1, 2):
+            da, db, dc = up(a, offs[0]), up(b, offs[1]), up(c, 1)
+            torch.cuda.synchronize()
+            assert _lib.lib().b2_set_fp64_config(tile, 4, 1) == 0
+            try:
+                blas.dgemm_device(ta, tb, m, n, k, 1.0, da, a.shape[0], db, b.shape[0], 0.5, dc,
+                                  m + 1)
+                torch.cuda.synchronize()
+            finally:
+                _lib.lib().b2_set_fp64_config(-1, 0, 0)
+            got = dc[:c.size].cpu().numpy().reshape(n, m + 1).T
+            assert np.array_equal(got[m:], c[m:])
+            assert normalized(got[:m], ref, k, opa, opb, U) <= 8, (m, n, k, tile)
