@@ -58,8 +58,9 @@ __device__ __forceinline__ void cp_async_wait() {
 // row, whose padding has room for both.  Tiles start at even elements, so a
 // row's shift is row_shift(p0, ld, row), and the row distances between one
 // thread's chunks, and between its fragment reads, are even: the shift is a
-// constant of the thread.  Odd leading dimensions took 8-byte copies before:
-// 2501x1777x1999 668 -> FILL us on B200.
+// constant of the thread.  Odd leading dimensions took twice the copies, of 8
+// bytes, before: 2501x1777x1999 671 -> 647 us on B200 (578 with even ones: the
+// shifted rows' shared reads meet 2-way bank conflicts).
 __device__ __forceinline__ int row_shift(const double *g, int ld, int row) {
   return (int)(((reinterpret_cast<uintptr_t>(g) >> 3) + (unsigned)row * (unsigned)ld) & 1u);
 }
@@ -136,6 +137,17 @@ __host__ __device__ constexpr uint32_t run_dst_step() {
   return (uint32_t)(NT / ((KCONT ? BK : OUTER) / 2) * (KCONT ? BK + 4 : OUTER + 4)) * 8u;
 }
 
+// Operand offset and shared byte offset of the chunk past the end of row tid.
+template <int OUTER, int BK, bool KCONT>
+__device__ __forceinline__ size_t run_tail(int o0, int k0, int ld, int tid) {
+  return KCONT ? (size_t)(o0 + tid) * ld + (k0 + BK - 1) : (size_t)(k0 + tid) * ld + (o0 + OUTER - 1);
+}
+template <int OUTER, int BK, bool KCONT>
+__device__ __forceinline__ uint32_t run_tail_dst(int tid) {
+  constexpr int LEN = KCONT ? BK : OUTER;
+  return (uint32_t)(tid * (LEN + 4) + LEN) * 8u;
+}
+
 template <int MMAK>
 __device__ __forceinline__ void dmma(double (&c)[4], const double *a, const double *b) {
   if constexpr (MMAK == 4) {
@@ -206,12 +218,14 @@ __global__ void __launch_bounds__(WM *WN * 32, BM * BN <= 64 * 64 && MMAK == 4 ?
   const int shb = SH ? row_shift(B, ldb, (B_KCONT ? n0 : kbeg) + tid / ((B_KCONT ? BK : BN) / 2)) : 0;
   const int fsa = SH ? row_shift(A, lda, A_KCONT ? g : t) : 0;
   const int fsb = SH ? row_shift(B, ldb, B_KCONT ? g : t) : 0;
-  // Tiles that lie wholly inside the matrices copy from running pointers (a
-  // few instructions per copy); edge tiles, a last short K block and, when
-  // shifted, whatever touches the operand's first row's start take the
-  // bounds-checked form.
-  const bool inside = m0 + BM <= M && n0 + BN <= N;
+  // An operand's tile that lies wholly inside it is copied from running
+  // pointers (a few instructions per copy); an edge tile, a last short K block
+  // and, when shifted, whatever touches the start of the operand's first row
+  // take the bounds-checked form.
+  const bool in_a = m0 + BM <= M, in_b = n0 + BN <= N;
   const bool a_first = SH && (A_KCONT ? m0 : kbeg) == 0, b_first = SH && (B_KCONT ? n0 : kbeg) == 0;
+  const bool tail_a = SH && tid < (A_KCONT ? BM : BK) && row_shift(A, lda, (A_KCONT ? m0 : kbeg) + tid);
+  const bool tail_b = SH && tid < (B_KCONT ? BN : BK) && row_shift(B, ldb, (B_KCONT ? n0 : kbeg) + tid);
   const double *pa = A + run_offset<BM, BK, A_KCONT>(m0, kbeg, lda, tid) - sha;
   const double *pb = B + run_offset<BN, BK, B_KCONT>(n0, kbeg, ldb, tid) - shb;
   const uint32_t da = sA_u + run_dst<BM, BK, A_KCONT>(tid);
@@ -223,28 +237,39 @@ __global__ void __launch_bounds__(WM *WN * 32, BM * BN <= 64 * 64 && MMAK == 4 ?
   // Copies stage kt (called once per kt, in order) into ring slot st.
   auto load_stage = [&](int st, int kt) {
     const int k0 = kbeg + kt * BK;
-    if (inside && k0 + BK <= kend && !(kt == 0 && (a_first || b_first))) {
+    const bool full = k0 + BK <= kend;
+    if (full && in_a && !(a_first && kt == 0)) {
 #pragma unroll
       for (int c = 0; c < A_CH; ++c)
         cp_async_full<16>(da + st * (A_ST * 8) + c * run_dst_step<BM, BK, A_KCONT, NT>(),
                           pa + c * ia);
-#pragma unroll
-      for (int c = 0; c < B_CH; ++c)
-        cp_async_full<16>(db + st * (B_ST * 8) + c * run_dst_step<BN, BK, B_KCONT, NT>(),
-                          pb + c * ib);
+      // (the element after the tile is in the row, or is not read)
+      if (SH && tail_a)
+        cp_async<16>(sA_u + st * (A_ST * 8) + run_tail_dst<BM, BK, A_KCONT>(tid),
+                     A + run_tail<BM, BK, A_KCONT>(m0, k0, lda, tid),
+                     (A_KCONT ? k0 + BK < kend : m0 + BM < M) ? 16 : 8);
     } else {
 #pragma unroll
       for (int c = 0; c < A_CH; ++c)
         load_chunk<BM, BK, A_KCONT, SH, NT>(sA_u + st * A_ST * 8, A, lda, m0, k0, M, kend, tid, c,
                                             sha);
+      if (SH) load_tails<BM, BK, A_KCONT, NT>(sA_u + st * A_ST * 8, A, lda, m0, k0, M, kend, tid);
+    }
+    if (full && in_b && !(b_first && kt == 0)) {
+#pragma unroll
+      for (int c = 0; c < B_CH; ++c)
+        cp_async_full<16>(db + st * (B_ST * 8) + c * run_dst_step<BN, BK, B_KCONT, NT>(),
+                          pb + c * ib);
+      if (SH && tail_b)
+        cp_async<16>(sB_u + st * (B_ST * 8) + run_tail_dst<BN, BK, B_KCONT>(tid),
+                     B + run_tail<BN, BK, B_KCONT>(n0, k0, ldb, tid),
+                     (B_KCONT ? k0 + BK < kend : n0 + BN < N) ? 16 : 8);
+    } else {
 #pragma unroll
       for (int c = 0; c < B_CH; ++c)
         load_chunk<BN, BK, B_KCONT, SH, NT>(sB_u + st * B_ST * 8, B, ldb, n0, k0, N, kend, tid, c,
                                             shb);
-    }
-    if (SH) {
-      load_tails<BM, BK, A_KCONT, NT>(sA_u + st * A_ST * 8, A, lda, m0, k0, M, kend, tid);
-      load_tails<BN, BK, B_KCONT, NT>(sB_u + st * B_ST * 8, B, ldb, n0, k0, N, kend, tid);
+      if (SH) load_tails<BN, BK, B_KCONT, NT>(sB_u + st * B_ST * 8, B, ldb, n0, k0, N, kend, tid);
     }
     pa += ka;
     pb += kb;
