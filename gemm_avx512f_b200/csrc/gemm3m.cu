@@ -18,7 +18,7 @@
 // tiles are de-interleaved into shared memory; the post-additions and the
 // complex alpha/beta happen in the epilogue.  beta follows the reference
 // drivers (C scaled whenever beta != 1, src/gemm_driver.c:131).
-//   zgemm3m: FP64 DMMA (mma.sync.m16n8k4.f64), 64x64 tile, 8 warps of 32x16.
+//   zgemm3m: FP64 DMMA (mma.sync.m16n8k4.f64), 64x32 tile, 8 warps of 16x16.
 //   cgemm3m: FP32 FFMA, 64x64 tile, 256 threads of 4x4 outputs.
 #include <stdlib.h>
 
@@ -246,12 +246,12 @@ __global__ void __launch_bounds__(256)
 
 // --------------------------------------- zgemm3m: one-launch FP64 DMMA --
 // The fused 3M product for complex128 at any size, on the FP64 tensor path
-// (mma.sync.m16n8k8.f64; tcgen05 has no f64 kind).  CTA tile 64 x 64 complex
-// outputs, 16 warps of 16 x 16, K in blocks of 16 complex elements streamed
-// global -> shared by cp.async (one 16-byte complex element per copy, zero
-// filled outside the matrix) through a 4-deep ring.  The smem tile keeps the
-// interleaved (re, im) pairs, so one 16-byte shared load gives a fragment
-// element's real and imaginary part; per K step every warp issues
+// (mma.sync.m16n8k4.f64; tcgen05 has no f64 kind).  CTA tile 64 x 32 complex
+// outputs, 8 warps of 16 x 16, two CTAs per SM; K in blocks of 16 complex
+// elements streamed global -> shared by cp.async (one 16-byte complex element
+// per copy, zero filled outside the matrix) through a 3-deep ring.  The smem
+// tile keeps the interleaved (re, im) pairs, so one 16-byte shared load gives a
+// fragment element's real and imaginary part; per K step every warp issues
 //     P1 += Ar Br,   P2 += Ai Bi,   P3 += (Ar + sa Ai)(Br + sb Bi)
 // with the pre-additions made on the fragments in registers (sa, sb = -1 for
 // conjugated operands), and the epilogue forms
@@ -260,42 +260,54 @@ __global__ void __launch_bounds__(256)
 // reference drivers do: src/gemm_driver.c:131).  Padding: +4 complex per row
 // when K is contiguous, +2 otherwise, so both orientations' 16-byte fragment
 // loads are conflict free.
-constexpr int Z_BM = 64, Z_BN = 64, Z_BK = 16, Z_WM = 4, Z_WN = 4, Z_STAGES = 4;
+// Bound: the FP64 pipe.  As in the real kernel (dgemm_fp64.cu) the next step's
+// fragments are loaded, across a stage's edge too, before the current step's
+// DMMAs issue, and tiles inside the matrices copy from running pointers.  The
+// earlier form (one 512-thread CTA of 64 x 64 per SM, fragments loaded at
+// their use) kept the pipe 75 % busy: 2048^3 1886 -> 1682 us on B200 (84 % busy).
+constexpr int Z_BM = 64, Z_BN = 32, Z_BK = 16, Z_WM = 4, Z_WN = 2, Z_STAGES = 3;
 constexpr int Z_NT = Z_WM * Z_WN * 32;
 
 template <bool KC>
+__host__ __device__ constexpr int z_pitch(int outer) {
+  return KC ? Z_BK + 4 : outer + 2;
+}
+template <bool KC>
 __host__ __device__ constexpr int z_stage_elems(int outer) {
-  return KC ? outer * (Z_BK + 4) : Z_BK * (outer + 2);
+  return (KC ? outer : Z_BK) * z_pitch<KC>(outer);
 }
 
-// One OUTER x BK complex tile; element (o, k) at g[o*ld + k] when KC (K
-// contiguous) else g[k*ld + o] (complex units).  Shared: KC -> [o][BK+4],
-// else [k][OUTER+2].
+// Chunk i (one complex element per thread) of an OUTER x BK tile; element
+// (o, k) at g[o*ld + k] when KC (K contiguous) else g[k*ld + o] (complex
+// units).  Shared: KC -> [o][BK+4], else [k][OUTER+2].
 template <int OUTER, bool KC>
-__device__ __forceinline__ void z_load_tile(uint32_t sbase, const double2 *__restrict__ g, int ld,
-                                            int o0, int k0, int olim, int klim, int tid) {
-  constexpr int TOTAL = OUTER * Z_BK;
-  static_assert(TOTAL % Z_NT == 0, "tile/thread mismatch");
-#pragma unroll
-  for (int i = 0; i < TOTAL / Z_NT; ++i) {
-    const int c = tid + i * Z_NT;
-    int o, k;
-    if (KC) { o = c / Z_BK; k = c % Z_BK; } else { k = c / OUTER; o = c % OUTER; }
-    const int go = o0 + o, gk = k0 + k;
-    const bool ok = go < olim && gk < klim;
-    const double2 *src = ok ? g + (KC ? (size_t)go * ld + gk : (size_t)gk * ld + go) : g;
-    const uint32_t dst = sbase + (uint32_t)(KC ? o * (Z_BK + 4) + k : k * (OUTER + 2) + o) * 16u;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src),
-                 "r"(ok ? 16 : 0));
-  }
+__device__ __forceinline__ void z_load_chunk(uint32_t sbase, const double2 *__restrict__ g, int ld,
+                                             int o0, int k0, int olim, int klim, int tid, int i) {
+  constexpr int CPR = KC ? Z_BK : OUTER;
+  const int c = tid + i * Z_NT, hi = c / CPR, lo = c % CPR;
+  const int go = o0 + (KC ? hi : lo), gk = k0 + (KC ? lo : hi);
+  const bool ok = go < olim && gk < klim;
+  const double2 *src = ok ? g + (KC ? (size_t)go * ld + gk : (size_t)gk * ld + go) : g;
+  const uint32_t dst = sbase + (uint32_t)(hi * z_pitch<KC>(OUTER) + lo) * 16u;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src),
+               "r"(ok ? 16 : 0));
+}
+
+__device__ __forceinline__ void z_mma(double (&c)[4], double a0, double a1, double b0) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+      "{%0,%1,%2,%3};\n"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a0), "d"(a1), "d"(b0));
 }
 
 template <bool A_KC, bool B_KC>
-__global__ void __launch_bounds__(Z_NT, 1)
+__global__ void __launch_bounds__(Z_NT, 2)
     zgemm3m_dmma_kernel(int M, int N, int K, const double2 *__restrict__ A, int lda,
                         const double2 *__restrict__ B, int ldb, double2 *__restrict__ C, int ldc,
                         double ar, double ai, double br, double bi, double sa, double sb) {
   constexpr int A_ST = z_stage_elems<A_KC>(Z_BM), B_ST = z_stage_elems<B_KC>(Z_BN);
+  constexpr int A_LD = z_pitch<A_KC>(Z_BM), B_LD = z_pitch<B_KC>(Z_BN);
   extern __shared__ __align__(16) double2 zsh[];
   double2 *sA = zsh;
   double2 *sB = zsh + Z_STAGES * A_ST;
@@ -315,80 +327,108 @@ __global__ void __launch_bounds__(Z_NT, 1)
 #pragma unroll
       for (int v = 0; v < 4; ++v) acc[p][j][v] = 0.0;
 
+  constexpr int A_CPR = A_KC ? Z_BK : Z_BM, B_CPR = B_KC ? Z_BK : Z_BN;
+  constexpr int A_CH = Z_BM * Z_BK / Z_NT, B_CH = Z_BN * Z_BK / Z_NT;
+  static_assert(Z_NT % A_CPR == 0 && Z_NT % B_CPR == 0, "whole rows per chunk");
+  const bool in_a = m0 + Z_BM <= M, in_b = n0 + Z_BN <= N;
+  const double2 *pa = A + (A_KC ? (size_t)(m0 + tid / A_CPR) * lda + tid % A_CPR
+                                : (size_t)(tid / A_CPR) * lda + m0 + tid % A_CPR);
+  const double2 *pb = B + (B_KC ? (size_t)(n0 + tid / B_CPR) * ldb + tid % B_CPR
+                                : (size_t)(tid / B_CPR) * ldb + n0 + tid % B_CPR);
+  const uint32_t da = sA_u + (uint32_t)((tid / A_CPR) * A_LD + tid % A_CPR) * 16u;
+  const uint32_t db = sB_u + (uint32_t)((tid / B_CPR) * B_LD + tid % B_CPR) * 16u;
+  const size_t ia = (size_t)(Z_NT / A_CPR) * lda, ib = (size_t)(Z_NT / B_CPR) * ldb;
+  const size_t ka = A_KC ? (size_t)Z_BK : (size_t)Z_BK * lda;
+  const size_t kb = B_KC ? (size_t)Z_BK : (size_t)Z_BK * ldb;
+  // Copies stage kt (called once per kt, in order) into ring slot st.
   auto load_stage = [&](int st, int kt) {
-    const int k0 = kt * Z_BK;
-    z_load_tile<Z_BM, A_KC>(sA_u + st * A_ST * 16, A, lda, m0, k0, M, K, tid);
-    z_load_tile<Z_BN, B_KC>(sB_u + st * B_ST * 16, B, ldb, n0, k0, N, K, tid);
+    const bool full = (kt + 1) * Z_BK <= K;
+#pragma unroll
+    for (int c = 0; c < A_CH; ++c) {
+      if (full && in_a)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                         da + (uint32_t)(st * A_ST + c * (Z_NT / A_CPR) * A_LD) * 16u),
+                     "l"(pa + c * ia));
+      else
+        z_load_chunk<Z_BM, A_KC>(sA_u + st * A_ST * 16, A, lda, m0, kt * Z_BK, M, K, tid, c);
+    }
+#pragma unroll
+    for (int c = 0; c < B_CH; ++c) {
+      if (full && in_b)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                         db + (uint32_t)(st * B_ST + c * (Z_NT / B_CPR) * B_LD) * 16u),
+                     "l"(pb + c * ib));
+      else
+        z_load_chunk<Z_BN, B_KC>(sB_u + st * B_ST * 16, B, ldb, n0, kt * Z_BK, N, K, tid, c);
+    }
+    pa += ka;
+    pb += kb;
   };
+  // Fragments of K step kk (4 complex k) of stage st: A rows g, g + 8, B
+  // columns g of the two 8-column blocks, k = kk + t.
+  double2 af[2][2], bf[2][2];
+  auto load_frags = [&](int buf, int st, int kk) {
+    const double2 *As = sA + st * A_ST, *Bs = sB + st * B_ST;
+    const int k = kk + t;
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      const int m = wm0 + g + 8 * v, n = wn0 + g + 8 * v;
+      af[buf][v] = A_KC ? As[m * A_LD + k] : As[k * A_LD + m];
+      bf[buf][v] = B_KC ? Bs[n * B_LD + k] : Bs[k * B_LD + n];
+    }
+  };
+
 #pragma unroll
   for (int st = 0; st < Z_STAGES - 1; ++st) {
     if (st < KT) load_stage(st, st);
     asm volatile("cp.async.commit_group;\n" ::);
   }
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(Z_STAGES - 2));
+  __syncthreads();
+  load_frags(0, 0, 0);
+  int st = 0, st_fill = Z_STAGES - 1;
   for (int kt = 0; kt < KT; ++kt) {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(Z_STAGES - 2));
-    __syncthreads();
-    {
-      const int kn = kt + Z_STAGES - 1;
-      if (kn < KT) load_stage(kn % Z_STAGES, kn);
-      asm volatile("cp.async.commit_group;\n" ::);
-    }
-    const double2 *As = sA + (kt % Z_STAGES) * A_ST;
-    const double2 *Bs = sB + (kt % Z_STAGES) * B_ST;
+    const int st_next = st + 1 == Z_STAGES ? 0 : st + 1;
 #pragma unroll
-    for (int kk = 0; kk < Z_BK; kk += 8) {
-      double are[4], aim[4], bre[2][2], bim[2][2];
-#pragma unroll
-      for (int v1 = 0; v1 < 2; ++v1)
-#pragma unroll
-        for (int v0 = 0; v0 < 2; ++v0) {
-          const int m = wm0 + g + 8 * v0, k = kk + t + 4 * v1;
-          const double2 x = A_KC ? As[m * (Z_BK + 4) + k] : As[k * (Z_BM + 2) + m];
-          are[v0 + 2 * v1] = x.x;
-          aim[v0 + 2 * v1] = x.y;
-        }
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int v = 0; v < 2; ++v) {
-          const int n = wn0 + j * 8 + g, k = kk + t + 4 * v;
-          const double2 x = B_KC ? Bs[n * (Z_BK + 4) + k] : Bs[k * (Z_BN + 2) + n];
-          bre[j][v] = x.x;
-          bim[j][v] = x.y;
-        }
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        asm volatile(
-            "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-            "{%8,%9}, {%0,%1,%2,%3};\n"
-            : "+d"(acc[0][j][0]), "+d"(acc[0][j][1]), "+d"(acc[0][j][2]), "+d"(acc[0][j][3])
-            : "d"(are[0]), "d"(are[1]), "d"(are[2]), "d"(are[3]), "d"(bre[j][0]), "d"(bre[j][1]));
-        asm volatile(
-            "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-            "{%8,%9}, {%0,%1,%2,%3};\n"
-            : "+d"(acc[1][j][0]), "+d"(acc[1][j][1]), "+d"(acc[1][j][2]), "+d"(acc[1][j][3])
-            : "d"(aim[0]), "d"(aim[1]), "d"(aim[2]), "d"(aim[3]), "d"(bim[j][0]), "d"(bim[j][1]));
+    for (int ks = 0; ks < Z_BK / 4; ++ks) {
+      const int cur = ks & 1;
+      if (ks + 1 < Z_BK / 4) load_frags(cur ^ 1, st, 4 * (ks + 1));
+      // every warp has issued its last reads of stage kt - 1, which is refilled here
+      if (ks == 0 && kt + Z_STAGES - 1 < KT) load_stage(st_fill, kt + Z_STAGES - 1);
+      if (ks + 1 == Z_BK / 4) {
+        asm volatile("cp.async.commit_group;\n" ::);
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(Z_STAGES - 2));
+        __syncthreads();
+        if (kt + 1 < KT) load_frags(cur ^ 1, st_next, 0);
       }
+      const double2 a0 = af[cur][0], a1 = af[cur][1];
 #pragma unroll
-      for (int v = 0; v < 4; ++v) are[v] = fma(sa, aim[v], are[v]);
+      for (int j = 0; j < 2; ++j) z_mma(acc[0][j], a0.x, a1.x, bf[cur][j].x);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) z_mma(acc[1][j], a0.y, a1.y, bf[cur][j].y);
+      const double s0 = fma(sa, a0.y, a0.x), s1 = fma(sa, a1.y, a1.x);
 #pragma unroll
       for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int v = 0; v < 2; ++v) bre[j][v] = fma(sb, bim[j][v], bre[j][v]);
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-        asm volatile(
-            "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-            "{%8,%9}, {%0,%1,%2,%3};\n"
-            : "+d"(acc[2][j][0]), "+d"(acc[2][j][1]), "+d"(acc[2][j][2]), "+d"(acc[2][j][3])
-            : "d"(are[0]), "d"(are[1]), "d"(are[2]), "d"(are[3]), "d"(bre[j][0]), "d"(bre[j][1]));
+        z_mma(acc[2][j], s0, s1, fma(sb, bf[cur][j].y, bf[cur][j].x));
     }
+    st = st_next;
+    st_fill = st_fill + 1 == Z_STAGES ? 0 : st_fill + 1;
   }
   asm volatile("cp.async.wait_group 0;\n" ::);
 
   // Fragment (j, v): row g + 8 (v >> 1), column 2t + (v & 1) of the warp tile.
+  // All of C is read before any of it is written (a load between two stores
+  // would wait for the one before it).
   const double s2 = sa * sb;
   const bool beta_one = br == 1.0 && bi == 0.0;
+  double2 cv[2][4];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const int m = m0 + wm0 + g + 8 * (v >> 1), n = n0 + wn0 + j * 8 + 2 * t + (v & 1);
+      cv[j][v] = (m < M && n < N) ? C[(size_t)n * ldc + m] : make_double2(0.0, 0.0);
+    }
 #pragma unroll
   for (int j = 0; j < 2; ++j)
 #pragma unroll
@@ -398,10 +438,10 @@ __global__ void __launch_bounds__(Z_NT, 1)
       if (m < M && n < N) {
         const double p1 = acc[0][j][v], p2 = s2 * acc[1][j][v], p3 = acc[2][j][v];
         const double re = p1 - p2, im = p3 - p1 - p2;
-        double2 *c = C + (size_t)n * ldc + m;
-        double2 cv = *c;
-        if (!beta_one) cv = make_double2(br * cv.x - bi * cv.y, br * cv.y + bi * cv.x);
-        *c = make_double2(cv.x + (ar * re - ai * im), cv.y + (ar * im + ai * re));
+        double2 c = cv[j][v];
+        if (!beta_one) c = make_double2(br * c.x - bi * c.y, br * c.y + bi * c.x);
+        C[(size_t)n * ldc + m] =
+            make_double2(c.x + (ar * re - ai * im), c.y + (ar * im + ai * re));
       }
     }
 }
@@ -616,11 +656,10 @@ int gemm3m_device(char ta, char tb, int m, int n, int k, const T *alpha, const T
     // multiply-adds, 2048^3 included: the pre-adds, the three products and
     // the combination never leave the SM, and no intermediate planes are
     // allocated (the three-GEMM form needs 3 (m k + k n + m n) doubles of
-    // workspace, 302 MB at 2048^3).  It runs 4 % below the three DMMA GEMMs
-    // there (36.4 against 38.0 TFLOPS effective; tensor pipe 75 % against 84 %
-    // active: the 512-thread fused CTA holds one CTA per SM).  The three
-    // GEMMs take over from 2^35: at 4096^3 they run at 41.8 TFLOPS effective
-    // against 36.9 for the one launch.  B2_Z3M_FUSED_MAX (multiply-adds)
+    // workspace, 302 MB at 2048^3).  It runs 2 % below the three DMMA GEMMs
+    // there (40.8 against 41.6 TFLOPS effective).  The three GEMMs take over
+    // from 2^35: at 4096^3 they run at 45.1 TFLOPS effective against 41.5 for
+    // the one launch.  B2_Z3M_FUSED_MAX (multiply-adds)
     // moves the limit.
     static const double fused_max = [] {
       const char *e = getenv("B2_Z3M_FUSED_MAX");
