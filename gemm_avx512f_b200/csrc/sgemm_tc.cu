@@ -17,6 +17,8 @@
 // is an L2 hit a few K' blocks later).
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "b2_methods.cuh"
 #include "b2_profile.cuh"
 #include "umma.cuh"
@@ -30,145 +32,151 @@ __device__ __forceinline__ float tf32_round(float x) {  // round to nearest, tie
   return __uint_as_float(r);
 }
 
-// Writes `terms` K-segments per row of the operand viewed as R x K (element
-// (r,k) at X[r*sr + k*sk]) into out[r][terms*kp] (elements of type T).
-// pattern: which split part each segment holds (0 = big/high, 1 = small/low).
-// vec (checked on the host: X 16-byte aligned and the strided dimension a
-// multiple of 4 elements, unit stride along the other): 16-byte loads of 4
-// consecutive rows (ROWCONT) or 4 consecutive k; otherwise scalar loads.
-template <typename T, bool ROWCONT>
+// One operand of a split pass: R rows of K elements, element (r, k) at
+// X[r + k*ld] (rowcont) or X[r*ld + k]; vec: 16-byte loads are legal (X 16-byte
+// aligned, ld a multiple of 4).
+struct SplitOp {
+  const float *X;
+  long long ld;
+  int R, rowcont, vec;
+  void *out;
+};
+
+// Writes every row of both operands as [big | small] (segs = 2) or [big]
+// segments of kp elements of type T, zero beyond K: out[r][segs*kp].  One
+// block turns 64 rows x 64 k around in shared memory; blocks that follow each
+// other read neighbouring memory.
+// Bound: HBM, 4 bytes read and segs*sizeof(T) written per element.  FILL
+template <typename T>
 __global__ void __launch_bounds__(256)
-    split_kernel(const float *__restrict__ X, long long sr, long long sk, int R, int K, int kp,
-                 int terms, unsigned pattern, T *__restrict__ out, int vec) {
-  __shared__ float tile[32][65];
-  const int k0 = blockIdx.x * 64, r0 = blockIdx.y * 32;
+    split_kernel(const SplitOp a, const SplitOp b, unsigned blocks_a, int K, int kp, int segs) {
+  __shared__ float tile[64][65];
+  const bool second = blockIdx.x >= blocks_a;
+  const float *X = second ? b.X : a.X;
+  const long long ld = second ? b.ld : a.ld;
+  const int R = second ? b.R : a.R;
+  const bool rowcont = second ? b.rowcont : a.rowcont, vec = second ? b.vec : a.vec;
+  T *out = (T *)(second ? b.out : a.out);
+  const unsigned id = second ? blockIdx.x - blocks_a : blockIdx.x;
+  const unsigned kt = (unsigned)(kp + 63) / 64, rt = (unsigned)(R + 63) / 64;
+  const int r0 = (int)(rowcont ? id % rt : id / kt) * 64;
+  const int k0 = (int)(rowcont ? id / rt : id % kt) * 64;
   const int tid = threadIdx.x;
   if (vec) {
+    float v[4][4];
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
+    for (int e = 0; e < 4; ++e) {
       const int idx = tid + 256 * e;
-      float v[4] = {0.f, 0.f, 0.f, 0.f};
-      if (ROWCONT) {  // 32 rows x 64 k: 8 float4 per k column
-        const int kk = idx >> 3, rr = (idx & 7) * 4;
-        const int r = r0 + rr, k = k0 + kk;
-        if (k < K) {
-          const float *src = X + r + (long long)k * sk;
-          if (r + 3 < R) {
-            const float4 q = __ldg(reinterpret_cast<const float4 *>(src));
-            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-          } else {
+      const int hi = idx >> 4, lo = (idx & 15) * 4;  // lo along the contiguous dimension
+      const int rr = rowcont ? lo : hi, kk = rowcont ? hi : lo;
+      const int r = r0 + rr, k = k0 + kk;
+      const int left = rowcont ? (k < K ? R - r : 0) : (r < R ? K - k : 0);
+      const float *src = X + (rowcont ? r + k * ld : r * ld + k);
+      if (left >= 4) {
+        const float4 q = __ldg(reinterpret_cast<const float4 *>(src));
+        v[e][0] = q.x, v[e][1] = q.y, v[e][2] = q.z, v[e][3] = q.w;
+      } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (r + j < R) v[j] = __ldg(src + j);
-          }
-        }
+        for (int j = 0; j < 4; ++j) v[e][j] = j < left ? __ldg(src + j) : 0.f;
+      }
+    }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) tile[rr + j][kk] = v[j];
-      } else {  // 32 rows x 64 k: 16 float4 per row
-        const int rr = idx >> 4, kk = (idx & 15) * 4;
-        const int r = r0 + rr, k = k0 + kk;
-        if (r < R) {
-          const float *src = X + (long long)r * sr + k;
-          if (k + 3 < K) {
-            const float4 q = __ldg(reinterpret_cast<const float4 *>(src));
-            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-          } else {
+    for (int e = 0; e < 4; ++e) {
+      const int idx = tid + 256 * e;
+      const int hi = idx >> 4, lo = (idx & 15) * 4;
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (k + j < K) v[j] = __ldg(src + j);
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) tile[rr][kk + j] = v[j];
+      for (int j = 0; j < 4; ++j) {
+        if (rowcont) tile[lo + j][hi] = v[e][j];
+        else tile[hi][lo + j] = v[e][j];
       }
     }
   } else {
+    float v[16];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int idx = tid + 256 * e;
-      int rr, kk;
-      if (ROWCONT) { rr = idx & 31; kk = idx >> 5; } else { kk = idx & 63; rr = idx >> 6; }
-      const int r = r0 + rr, k = k0 + kk;
-      float v = 0.f;
-      if (r < R && k < K) v = __ldg(X + (long long)r * sr + (long long)k * sk);
-      tile[rr][kk] = v;
+    for (int e = 0; e < 16; ++e) {
+      const int idx = tid + 256 * e, hi = idx >> 6, lo = idx & 63;
+      const int r = r0 + (rowcont ? lo : hi), k = k0 + (rowcont ? hi : lo);
+      v[e] = (r < R && k < K) ? __ldg(X + (rowcont ? r + k * ld : r * ld + k)) : 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      const int idx = tid + 256 * e, hi = idx >> 6, lo = idx & 63;
+      if (rowcont) tile[lo][hi] = v[e];
+      else tile[hi][lo] = v[e];
     }
   }
   __syncthreads();
-  const int rr = tid >> 3, q = tid & 7;
-  const int r = r0 + rr;
-  if (r >= R) return;
-  T *row = out + (long long)r * terms * kp;
-  // 16-byte stores of 16-byte groups of consecutive k: FP32 writes groups
-  // k0 + 4q and k0 + 32 + 4q (the second only where kp reaches it; kp is a
-  // multiple of 32), so each store instruction covers whole 128-byte lines
-  // of a row; BF16 writes one group of 8 at k0 + 8q (kp is a multiple of 64).
-  // Pad columns [K, kp) are written as zeros.
-  constexpr int GW = sizeof(T) == 4 ? 4 : 8;   // elements per 16-byte group
-  constexpr int NG = sizeof(T) == 4 ? 2 : 1;   // groups per thread
+  // 16-byte stores: 4 floats or 8 bfloat16 of one row; kp is a multiple of 32
+  // (float) or 64 (bfloat16) elements, and the tile is zero beyond K.
+  constexpr int GW = 16 / (int)sizeof(T), GPR = 64 / GW;
 #pragma unroll
-  for (int g = 0; g < NG; ++g) {
-    const int kl = (sizeof(T) == 4) ? g * 32 + 4 * q : 8 * q;  // offset within the 64-k tile
-    if (k0 + kl >= kp) break;
-    T big[GW], small[GW];
+  for (int e = 0; e < 64 * GPR / 256; ++e) {
+    const int idx = tid + 256 * e, rr = idx / GPR, kl = (idx % GPR) * GW;
+    const int r = r0 + rr;
+    if (r >= R || k0 + kl >= kp) continue;
+    T *dst = out + (long long)r * segs * kp + k0 + kl;
+    if constexpr (sizeof(T) == 4) {
+      float big[4], small[4];
 #pragma unroll
-    for (int j = 0; j < GW; ++j) {
-      const float v = (k0 + kl + j < K) ? tile[rr][kl + j] : 0.f;
-      if constexpr (sizeof(T) == 4) {
-        const float bv = tf32_round(v);
-        big[j] = bv;
-        small[j] = tf32_round(v - bv);
-      } else {
-        const __nv_bfloat16 h = __float2bfloat16_rn(v);
-        big[j] = h;
-        small[j] = __float2bfloat16_rn(v - __bfloat162float(h));
+      for (int j = 0; j < 4; ++j) {
+        const float x = tile[rr][kl + j];
+        big[j] = tf32_round(x);
+        small[j] = tf32_round(x - big[j]);
       }
-    }
-    for (int t = 0; t < terms; ++t) {
-      const T *src = ((pattern >> t) & 1u) ? small : big;
-      T *dst = row + (long long)t * kp + k0 + kl;
-      if constexpr (sizeof(T) == 4) {
-        *reinterpret_cast<float4 *>(dst) = make_float4(src[0], src[1], src[2], src[3]);
-      } else {
-        uint4 p;
-        p.x = (uint32_t)__bfloat16_as_ushort(src[0]) | ((uint32_t)__bfloat16_as_ushort(src[1]) << 16);
-        p.y = (uint32_t)__bfloat16_as_ushort(src[2]) | ((uint32_t)__bfloat16_as_ushort(src[3]) << 16);
-        p.z = (uint32_t)__bfloat16_as_ushort(src[4]) | ((uint32_t)__bfloat16_as_ushort(src[5]) << 16);
-        p.w = (uint32_t)__bfloat16_as_ushort(src[6]) | ((uint32_t)__bfloat16_as_ushort(src[7]) << 16);
-        *reinterpret_cast<uint4 *>(dst) = p;
+      *reinterpret_cast<float4 *>(dst) = make_float4(big[0], big[1], big[2], big[3]);
+      if (segs == 2)
+        *reinterpret_cast<float4 *>(dst + kp) = make_float4(small[0], small[1], small[2], small[3]);
+    } else {
+      uint32_t hw[4], lw[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint32_t h2 = 0, l2 = 0;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float x = tile[rr][kl + 2 * j + i];
+          const __nv_bfloat16 h = __float2bfloat16_rn(x);
+          const __nv_bfloat16 l = __float2bfloat16_rn(x - __bfloat162float(h));
+          h2 |= (uint32_t)__bfloat16_as_ushort(h) << (16 * i);
+          l2 |= (uint32_t)__bfloat16_as_ushort(l) << (16 * i);
+        }
+        hw[j] = h2;
+        lw[j] = l2;
       }
+      *reinterpret_cast<uint4 *>(dst) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+      if (segs == 2)
+        *reinterpret_cast<uint4 *>(dst + kp) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
     }
   }
 }
 
-// FP32 epilogue: lane p = column n of C, columns q = rows m (contiguous in C).
+// FP32 epilogue: lane p = row m of C, v[j] = column q0 + j: a warp reads and
+// writes 32 consecutive rows of a column, all of C's reads before its writes.
 struct F32Epi {
   float *C;
   int ldc;
   int M, N;
   float alpha, beta;
-  __device__ __forceinline__ void operator()(int, int p, int q0, const uint32_t (&v)[32]) const {
-    if (p >= N || q0 >= M) return;
-    float *col = C + (long long)p * ldc + q0;
-    const int nq = min(32, M - q0);
-    const bool one = (beta == 1.f);
-    if (nq == 32 && ((((uintptr_t)col) & 15) == 0)) {
+  __device__ __forceinline__ void operator()(int, int p, int q0, const float (&v)[16]) const {
+    if (p >= M || q0 >= N) return;
+    // (the volatile asms keep the compiler from holding the addresses of many
+    // columns at once beside the 128 sums, which spills)
+    long long ld = ldc;
+    asm volatile("" : "+l"(ld));
+    float *c = C + q0 * ld + p;
+    const int nq = min(16, N - q0);
+    float old[16];
 #pragma unroll
-      for (int g = 0; g < 8; ++g) {
-        float4 c = reinterpret_cast<float4 *>(col)[g];
-        const float a0 = __uint_as_float(v[4 * g]), a1 = __uint_as_float(v[4 * g + 1]);
-        const float a2 = __uint_as_float(v[4 * g + 2]), a3 = __uint_as_float(v[4 * g + 3]);
-        c.x = one ? fmaf(alpha, a0, c.x) : fmaf(alpha, a0, beta * c.x);
-        c.y = one ? fmaf(alpha, a1, c.y) : fmaf(alpha, a1, beta * c.y);
-        c.z = one ? fmaf(alpha, a2, c.z) : fmaf(alpha, a2, beta * c.z);
-        c.w = one ? fmaf(alpha, a3, c.w) : fmaf(alpha, a3, beta * c.w);
-        reinterpret_cast<float4 *>(col)[g] = c;
-      }
-    } else {
-      for (int j = 0; j < nq; ++j) {
-        const float a = __uint_as_float(v[j]);
-        col[j] = one ? fmaf(alpha, a, col[j]) : fmaf(alpha, a, beta * col[j]);
-      }
+    for (int j = 0; j < 16; ++j) {
+      old[j] = j < nq ? *c : 0.f;
+      c += ld;
+    }
+    asm volatile("" : "+l"(ld));
+    c -= 16 * ld;
+    const bool one = (beta == 1.f);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      if (j < nq) *c = one ? fmaf(alpha, v[j], old[j]) : fmaf(alpha, v[j], beta * old[j]);
+      c += ld;
     }
   }
 };
@@ -181,13 +189,13 @@ struct F32PartialEpi {
   long long plane;
   int ldw;
   int M, N;
-  __device__ __forceinline__ void operator()(int ks, int p, int q0, const uint32_t (&v)[32]) const {
-    if (p >= N || q0 >= M) return;
-    float4 *dst = reinterpret_cast<float4 *>(W + ks * plane + (long long)p * ldw + q0);
+  __device__ __forceinline__ void operator()(int ks, int p, int q0, const float (&v)[16]) const {
+    if (p >= M || q0 >= N) return;
+    float *w = W + ks * plane + (long long)q0 * ldw + p;
+    const int nq = min(16, N - q0);
 #pragma unroll
-    for (int g = 0; g < 8; ++g)
-      dst[g] = make_float4(__uint_as_float(v[4 * g]), __uint_as_float(v[4 * g + 1]),
-                           __uint_as_float(v[4 * g + 2]), __uint_as_float(v[4 * g + 3]));
+    for (int j = 0; j < 16; ++j)
+      if (j < nq) w[(long long)j * ldw] = v[j];
   }
 };
 
@@ -228,19 +236,47 @@ int choose_ksplit(long long tiles, int kblocks, int sms) {
 
 inline long long round_up(long long x, long long a) { return (x + a - 1) / a * a; }
 
-template <typename T>
-int run_split(const float *Xp, long long sr, long long sk, int R, int K, int kp, int terms,
-              unsigned pattern, T *out, cudaStream_t s) {
-  dim3 grid((kp + 63) / 64, (R + 31) / 32);
-  B2_PROF("sgemm_split", s);
-  const bool aligned = ((uintptr_t)Xp & 15) == 0;
-  if (sr == 1) {
-    const int vec = aligned && (sk % 4 == 0);
-    split_kernel<T, true><<<grid, 256, 0, s>>>(Xp, sr, sk, R, K, kp, terms, pattern, out, vec);
-  } else {
-    const int vec = aligned && sk == 1 && (sr % 4 == 0);
-    split_kernel<T, false><<<grid, 256, 0, s>>>(Xp, sr, sk, R, K, kp, terms, pattern, out, vec);
+// Work units of a product whose K is accumulated in S ranges of kbps blocks:
+// each unit takes `per` consecutive ranges of its tile (adding them in its
+// epilogue), so that ceil(S / per) partials per tile go through memory.
+// Modelled time (us): waves of units at t_kb per K block (measured MMA rate of
+// the engine) and 3 us of fill and epilogue, plus the partials written and read
+// at about 4 TB/s and a second launch.  2048^3 3xTF32 (64 pair tiles on 74
+// pairs, 8 ranges): one unit per tile instead of 8 partials of 16.8 MB.
+int ranges_per_unit(long long tiles, int S, int kbps, int kblocks, int slots, double t_kb, int m,
+                    int n) {
+  int best = S;
+  double best_us = 1e300;
+  for (int per = S; per >= 1; --per) {
+    const int E = (S + per - 1) / per;
+    if (per < S && (S + per) / (per + 1) == E) continue;  // same E with fewer ranges: no better
+    const long long waves = (tiles * E + slots - 1) / slots;
+    const int kb = per * kbps < kblocks ? per * kbps : kblocks;
+    double us = (double)waves * (kb * t_kb + 3.0);
+    if (E > 1) us += 3.0 + (double)E * m * n * 8.0 / 4e6;
+    if (us < best_us) best_us = us, best = per;
   }
+  return best;
+}
+
+SplitOp split_op(const float *X, long long sr, long long sk, int R, void *out) {
+  SplitOp o;
+  o.X = X;
+  o.rowcont = sr == 1;
+  o.ld = o.rowcont ? sk : sr;
+  o.R = R;
+  o.vec = ((uintptr_t)X & 15) == 0 && o.ld % 4 == 0;
+  o.out = out;
+  return o;
+}
+
+// Split pass over one or two operands (b.R = 0: one).
+template <typename T>
+int run_split(const SplitOp &a, const SplitOp &b, int K, int kp, int segs, cudaStream_t s) {
+  const unsigned kt = (unsigned)(kp + 63) / 64;
+  const unsigned ba = kt * ((unsigned)(a.R + 63) / 64), bb = kt * ((unsigned)(b.R + 63) / 64);
+  B2_PROF("sgemm_split", s);
+  split_kernel<T><<<ba + bb, 256, 0, s>>>(a, b, ba, K, kp, segs);
   B2_CUDA_TRY(cudaGetLastError());
   return B2_OK;
 }
@@ -249,7 +285,7 @@ int run_split(const float *Xp, long long sr, long long sk, int R, int K, int kp,
 
 int sgemm_split_tf32x3(const float *X, long long sr, long long sk, int R, int K, int kp,
                        float *out, cudaStream_t s) {
-  return run_split<float>(X, sr, sk, R, K, kp, 2, 0x2u, out, s);
+  return run_split<float>(split_op(X, sr, sk, R, out), SplitOp{}, K, kp, 2, s);
 }
 
 // Tensor-core engine of an SGEMM call: 0 = single CTA, 128 x 256 tile, 4
@@ -297,80 +333,72 @@ int sgemm_tensor_cfg(char ta, char tb, int m, int n, int k, float alpha, const f
   const long long kt = (long long)terms * kp;               // K' of the one GEMM
   const int segs = terms == 3 ? 2 : 1;                      // stored segments per row
   const long long ks_ = (long long)segs * kp;
-  void *Yp = workspace(cx, WS_SPLIT_Y, (size_t)m * ks_ * esz);
-  void *Xp = workspace(cx, WS_SPLIT_X, (size_t)n * ks_ * esz);
+  void *Xp = workspace(cx, WS_SPLIT_X, (size_t)m * ks_ * esz);
+  void *Yp = workspace(cx, WS_SPLIT_Y, (size_t)n * ks_ * esz);
   if (!Yp || !Xp) return B2_ERR_NOMEM;
-  // stored segments: [big] or [big, small]; terms read (Bb, Ab), (Bs, Ab), (Bb, As)
-  const unsigned pat = 0x2u;                      // segment 1 holds the small part
-  const unsigned segX = 0x2u, segY = 0x4u;        // term -> segment, B side / A side
-  int rc;
-  if (bf16) {
-    rc = run_split<__nv_bfloat16>(A, asr, ask, m, k, kp, segs, pat, (__nv_bfloat16 *)Yp, s);
-    if (rc == B2_OK)
-      rc = run_split<__nv_bfloat16>(B, bsr, bsk, n, k, kp, segs, pat, (__nv_bfloat16 *)Xp, s);
-  } else {
-    rc = run_split<float>(A, asr, ask, m, k, kp, segs, pat, (float *)Yp, s);
-    if (rc == B2_OK) rc = run_split<float>(B, bsr, bsk, n, k, kp, segs, pat, (float *)Xp, s);
-  }
+  // The engine's X (accumulator lanes) is op(A): a warp's 32 lanes are then 32
+  // consecutive rows of a column of C.  Stored segments: [big] or [big, small];
+  // terms read (Ab, Bb), (Ab, Bs), (As, Bb).
+  const unsigned segX = 0x4u, segY = 0x2u;        // term -> segment, A side / B side
+  const SplitOp oa = split_op(A, asr, ask, m, Xp), ob = split_op(B, bsr, bsk, n, Yp);
+  int rc = bf16 ? run_split<__nv_bfloat16>(oa, ob, k, kp, segs, s)
+                : run_split<float>(oa, ob, k, kp, segs, s);
   if (rc != B2_OK) return rc;
   const int kind = bf16 ? umma::KIND_BF16 : umma::KIND_TF32;
   const int eng = (cfg.engine >= 0 && cfg.engine <= 2) ? cfg.engine : 0;
-  // tile: X rows (n side) per tile x Y rows (m side) per tile; TMA boxes per CTA
+  // tile: X rows (m) x Y rows (n) per tile; TMA boxes per CTA
   const int tile_p = eng == 2 ? 256 : umma::BM, tile_q = eng == 1 ? 128 : 256;
   const int ybox = eng == 0 ? 256 : 128;
   CUtensorMap tmX, tmY;
-  rc = umma::make_kmajor_map(&tmX, kind, Xp, ks_, n, 1, ks_ * esz, (long long)n * ks_ * esz,
+  rc = umma::make_kmajor_map(&tmX, kind, Xp, ks_, m, 1, ks_ * esz, (long long)m * ks_ * esz,
                              umma::BM);
   if (rc == B2_OK)
-    rc = umma::make_kmajor_map(&tmY, kind, Yp, ks_, m, 1, ks_ * esz, (long long)m * ks_ * esz, ybox);
+    rc = umma::make_kmajor_map(&tmY, kind, Yp, ks_, n, 1, ks_ * esz, (long long)n * ks_ * esz, ybox);
   if (rc != B2_OK) return rc;
   const int seg_kb = terms == 3 ? (int)((long long)kp * esz / umma::KBLOCK_BYTES) : 0;
-  const long long tiles = ((n + tile_p - 1) / tile_p) * (long long)((m + tile_q - 1) / tile_q);
+  const long long tiles = ((n + tile_q - 1) / tile_q) * (long long)((m + tile_p - 1) / tile_p);
   const int kblocks = (int)((kt * esz + umma::KBLOCK_BYTES - 1) / umma::KBLOCK_BYTES);
   const int slots = eng == 2 ? cx->sm_count / 2 : cx->sm_count;
+  // K is accumulated in S ranges of kbps blocks; a unit adds `per` of them
   int S = cfg.split > 0 ? cfg.split : choose_ksplit(tiles, kblocks, slots);
   if (S > kblocks) S = kblocks > 0 ? kblocks : 1;
-  if (S > 1) {
-    // the engine may merge ranges; size W for S and pass the count it uses
-    const int kbps = (kblocks + S - 1) / S;
-    S = (kblocks + kbps - 1) / kbps;
-  }
-  auto run = [&](auto &&epi) -> int {
+  const int kbps = (kblocks + S - 1) / S;
+  S = (kblocks + kbps - 1) / kbps;
+  const int per = ranges_per_unit(tiles, S, kbps, kblocks, slots, eng == 1 ? 0.17 : 0.28, m, n);
+  const int E = (S + per - 1) / per;  // partials per tile
+  auto run = [&](auto epi) -> int {
+    using Epi = decltype(epi);
     const char *nm = bf16 ? "sgemm_umma_bf16" : "sgemm_umma_tf32";
-    if (eng == 2)
-      return bf16 ? umma::launch_pair<umma::KIND_BF16, 256, 6>(tmX, tmY, n, m, kt, 1, epi,
-                                                               cx->device, cx->derr, s, nm,
-                                                               nullptr, S, seg_kb, segX, segY)
-                  : umma::launch_pair<umma::KIND_TF32, 256, 6>(tmX, tmY, n, m, kt, 1, epi,
-                                                               cx->device, cx->derr, s, nm,
-                                                               nullptr, S, seg_kb, segX, segY);
-    if (eng == 1)
-      return bf16 ? umma::launch<umma::KIND_BF16, 128, 6>(tmX, tmY, n, m, kt, 1, epi,
-                                                          cx->sm_count, cx->derr, s, nm, 0,
-                                                          nullptr, S, seg_kb, segX, segY)
-                  : umma::launch<umma::KIND_TF32, 128, 6>(tmX, tmY, n, m, kt, 1, epi,
-                                                          cx->sm_count, cx->derr, s, nm, 0,
-                                                          nullptr, S, seg_kb, segX, segY);
-    return bf16 ? umma::launch<umma::KIND_BF16, 256, 4>(tmX, tmY, n, m, kt, 1, epi, cx->sm_count,
-                                                        cx->derr, s, nm, 0, nullptr, S, seg_kb,
-                                                        segX, segY)
-                : umma::launch<umma::KIND_TF32, 256, 4>(tmX, tmY, n, m, kt, 1, epi, cx->sm_count,
-                                                        cx->derr, s, nm, 0, nullptr, S, seg_kb,
-                                                        segX, segY);
+    const int kbr = per * kbps;
+    auto pair = [&](auto kd) {
+      return umma::launch_pair<decltype(kd)::value, 256, 6, Epi, true>(
+          tmX, tmY, m, n, kt, 1, epi, cx->device, cx->derr, s, nm, nullptr, E, seg_kb, segX, segY,
+          kbr, kbps);
+    };
+    auto single = [&](auto kd, auto bn, auto st) {
+      return umma::launch<decltype(kd)::value, decltype(bn)::value, decltype(st)::value, Epi, 1,
+                          true>(tmX, tmY, m, n, kt, 1, epi, cx->sm_count, cx->derr, s, nm, 0,
+                                nullptr, E, seg_kb, segX, segY, kbr, kbps);
+    };
+    using BF = std::integral_constant<int, umma::KIND_BF16>;
+    using TF = std::integral_constant<int, umma::KIND_TF32>;
+    using I4 = std::integral_constant<int, 4>;
+    using I6 = std::integral_constant<int, 6>;
+    using I128 = std::integral_constant<int, 128>;
+    using I256 = std::integral_constant<int, 256>;
+    if (eng == 2) return bf16 ? pair(BF{}) : pair(TF{});
+    if (eng == 1) return bf16 ? single(BF{}, I128{}, I6{}) : single(TF{}, I128{}, I6{});
+    return bf16 ? single(BF{}, I256{}, I4{}) : single(TF{}, I256{}, I4{});
   };
-  if (S == 1) {
-    F32Epi epi{C, ldc, m, n, alpha, beta};
-    return run(epi);
-  }
-  // Split-K: S partial products of K ranges, then one fixed-order reduction.
-  const int ldw = (int)round_up(m, 256);  // whole 256-column tiles stay in bounds
+  if (E == 1) return run(F32Epi{C, ldc, m, n, alpha, beta});
+  // E partial products of K ranges, then one fixed-order reduction.
+  const int ldw = (int)round_up(m, 32);
   const long long plane = (long long)n * ldw;
-  float *W = (float *)workspace(cx, WS_MISC, (size_t)plane * S * sizeof(float));
+  float *W = (float *)workspace(cx, WS_MISC, (size_t)plane * E * sizeof(float));
   if (!W) return B2_ERR_NOMEM;
-  F32PartialEpi pe{W, plane, ldw, m, n};
-  rc = run(pe);
+  rc = run(F32PartialEpi{W, plane, ldw, m, n});
   if (rc != B2_OK) return rc;
-  return sgemm_splitk_reduce(W, plane, ldw, S, m, n, alpha, beta, C, ldc, s);
+  return sgemm_splitk_reduce(W, plane, ldw, E, m, n, alpha, beta, C, ldc, s);
 }
 
 int sgemm_splitk_reduce(const float *W, long long plane, int ldw, int S, int m, int n,

@@ -10,13 +10,19 @@
 // memory, and the 24x8 FMA register tile of src/kernel/gemm_kernel.S becomes
 // 128 x BN x 32-byte tcgen05.mma instructions accumulating in TMEM.
 //
-// Roles (192 threads, one CTA per SM):
+// Roles (192 threads, 320 in SUM kernels with BN = 256; one CTA per SM):
 //   warp 0      TMA producer: fills a STAGES-deep ring of (X, Y) K-blocks.
 //   warp 1      TMEM owner + MMA issuer (one elected lane).
-//   warps 2..5  epilogue: tcgen05.ld of their 32-lane quarter of the
+//   warps 2..   epilogue: tcgen05.ld of their 32-lane quarter of the
 //               accumulator, then the functor.
 // TMEM holds two accumulators (2 x BN columns) so the epilogue of tile i
 // overlaps the MMAs of tile i+1.
+// SUM kernels cut a unit's K range into sub-ranges that go through the two
+// accumulators in turn; the epilogue adds each to FP32 sums in its registers
+// (128 columns a thread: 8 epilogue warps for BN = 256) while the next one is
+// multiplied.  The tensor core's accumulation error grows with the length of a
+// chain, so the split forms of SGEMM keep chains short; this keeps them short
+// without writing the partial products to memory.
 //
 // Every mbarrier wait is bounded (Problem::wait_ns of wall time from
 // %globaltimer, 2 s unless a test shortens it); on expiry the waiter stores
@@ -45,7 +51,6 @@ enum Kind { KIND_I8 = 0, KIND_BF16 = 1, KIND_TF32 = 2, KIND_U8 = 3 };
 
 constexpr int BM = 128;            // accumulator lanes (X rows) per tile
 constexpr int KBLOCK_BYTES = 128;  // one 128B swizzle atom along K per stage
-constexpr int THREADS = 192;
 constexpr uint64_t B2_WAIT_NS = 2000000000ull;  // 2 s per wait: far above any legal wait
 
 // Wait limit (ns) given to the next launches and the number of launches that
@@ -232,12 +237,32 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[32]) {
                : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld16_wait(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
+                 "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]),
+                 "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
+}
+
 // ---------------------------------------------------------------- kernel --
 struct Problem {
   int P, Q;        // rows of X and of Y (output tile space P x Q)
   int kblocks;     // K extent in 128-byte blocks
   int ksplit;      // K ranges per output tile (split-K; 1 = whole K in one accumulator)
   int kb_per_split;  // K blocks per range (every range is non-empty)
+  int sub_kb;        // K blocks accumulated at a time within a unit's range (kernels
+                     // with SUM add the sub-ranges in registers; else the whole range)
   int nbatch;      // independent products (3-D tensor maps, batch = outer coordinate)
   const int *nbatch_dev;  // if set: the batch count actually run (<= nbatch), read on the device
   int tiles_p, tiles_q;
@@ -285,13 +310,53 @@ __host__ __device__ constexpr int tmem_cols(int need) {
   return need <= 32 ? 32 : need <= 64 ? 64 : need <= 128 ? 128 : need <= 256 ? 256 : 512;
 }
 
+// Epilogue warps and threads: SUM kernels hold BN / (warps / 4) = 128 sums a thread.
+__host__ __device__ constexpr int epi_warps(int bn, bool sum) { return sum && bn > 128 ? 8 : 4; }
+__host__ __device__ constexpr int threads_for(int bn, bool sum) { return 64 + 32 * epi_warps(bn, sum); }
+
+// Epilogue of one work unit of a SUM kernel for one warp: `nsub` accumulators
+// in turn, their columns [c0, c0 + 128) of this lane quarter added up, then
+// handed to the functor 16 columns at a time.  wait(it) waits for accumulator
+// it & 1 (false: abandoned), done(it) frees it.
+template <class Wait, class Done, class Out>
+__device__ __forceinline__ bool sum_epilogue(uint32_t tmem_quarter, int bn, int c0, int nsub,
+                                             int &it, Wait wait, Done done, Out out) {
+  // 16 columns at a time: 128 sums and one load's registers fit the 168 a
+  // thread that 8 + 2 warps leave
+  float s[8][16];
+  for (int i = 0; i < nsub; ++i, ++it) {
+    if (!__all_sync(0xffffffffu, wait(it))) return false;
+    tc_fence_after();
+    const uint32_t taddr = tmem_quarter + (uint32_t)((it & 1) * bn + c0);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      uint32_t v[16];
+      tmem_ld16(taddr + (uint32_t)(c * 16), v);
+      tmem_ld16_wait(v);
+      if (i == 0) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) s[c][j] = __uint_as_float(v[j]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) s[c][j] += __uint_as_float(v[j]);
+      }
+    }
+    tc_fence_before();
+    __syncwarp();
+    done(it);
+  }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) out(c0 + 16 * c, s[c]);
+  return true;
+}
+
 // NACC = 1: every (batch, tile, K range) is its own work unit.  NACC > 1: a
 // work unit is a tile, and the unit multiplies batches 0 .. NACC-1 of the
 // operands into NACC accumulators that its epilogue receives together
 // (epi(p, q0, v0, v1, v2) for NACC = 3: the three real products of the 3M
 // method); no split-K.
-template <int KIND, int BN, int STAGES, class Epi, int NACC = 1>
-__global__ void __launch_bounds__(THREADS, 1)
+template <int KIND, int BN, int STAGES, class Epi, int NACC = 1, bool SUM = false>
+__global__ void __launch_bounds__(threads_for(BN, SUM), 1)
     umma_gemm_kernel(const __grid_constant__ CUtensorMap tmX,
                      const __grid_constant__ CUtensorMap tmY, const Problem pr, const Epi epi) {
   using L = SmemLayout<BN, STAGES>;
@@ -302,6 +367,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   static_assert(NACC == 1 || NACC == 3, "one accumulator, or three for the 3M products");
   static_assert(NACC == 3 || SETS == 2, "the single-accumulator engine double-buffers");
   constexpr int TCOLS = tmem_cols(SETS * NACC * BN);
+  static_assert(!SUM || (NACC == 1 && BN % 128 == 0), "summed epilogue: 128 columns a thread");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -328,7 +394,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);
-      mbar_init(tempty_bar(a), 4);  // one arrival per epilogue warp
+      mbar_init(tempty_bar(a), epi_warps(BN, SUM));  // one arrival per epilogue warp
     }
     mbar_init(drain_bar, 1);
     *abort_flag = 0;
@@ -397,37 +463,40 @@ __global__ void __launch_bounds__(THREADS, 1)
       uint32_t phase = 0;
       int it = 0;
       bool ok = true;
-      for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x, ++it) {
+      for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
         const int ks = u % pr.ksplit;
         const int kb0 = ks * pr.kb_per_split, kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
-        const int acc = it % SETS;
-        const uint32_t acc_phase = (uint32_t)((it / SETS) & 1);
-        if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, pr.derr, pr.wait_ns)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        for (int kbb = kb0; kbb < kb0 + NACC * (kb1 - kb0); ++kbb) {
-          const int bi = NACC > 1 ? (kbb - kb0) % NACC : 0;
-          const int kb = NACC > 1 ? kb0 + (kbb - kb0) / NACC : kbb;
-          const uint32_t d_tmem = tmem_base + (uint32_t)((acc * NACC + bi) * BN);
-          if (!mbar_wait(full_bar(stage), phase, abort_flag, pr.derr, pr.wait_ns)) {
+        for (int kr = kb0; kr < kb1 && ok; kr += pr.sub_kb, ++it) {
+          const int ke = min(kb1, kr + pr.sub_kb);
+          const int acc = it % SETS;
+          const uint32_t acc_phase = (uint32_t)((it / SETS) & 1);
+          if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, pr.derr, pr.wait_ns)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t sx = base + stage * L::STAGE_BYTES;
-          const uint32_t sy = sx + L::X_BYTES;
+          for (int kbb = kr; kbb < kr + NACC * (ke - kr); ++kbb) {
+            const int bi = NACC > 1 ? (kbb - kr) % NACC : 0;
+            const int kb = NACC > 1 ? kr + (kbb - kr) / NACC : kbb;
+            const uint32_t d_tmem = tmem_base + (uint32_t)((acc * NACC + bi) * BN);
+            if (!mbar_wait(full_bar(stage), phase, abort_flag, pr.derr, pr.wait_ns)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t sx = base + stage * L::STAGE_BYTES;
+            const uint32_t sy = sx + L::X_BYTES;
 #pragma unroll
-          for (int kk = 0; kk < KBLOCK_BYTES / 32; ++kk) {
-            tc_mma<KIND>(d_tmem, sw128_desc(sx + kk * 32), sw128_desc(sy + kk * 32), idesc,
-                         (kb != kb0 || kk) ? 1u : 0u);
+            for (int kk = 0; kk < KBLOCK_BYTES / 32; ++kk) {
+              tc_mma<KIND>(d_tmem, sw128_desc(sx + kk * 32), sw128_desc(sy + kk * 32), idesc,
+                           (kb != kr || kk) ? 1u : 0u);
+            }
+            tc_commit(empty_bar(stage));  // frees the stage once these MMAs have read it
+            if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           }
-          tc_commit(empty_bar(stage));  // frees the stage once these MMAs have read it
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          if (!ok) break;
+          tc_commit(tfull_bar(acc));
         }
-        if (!ok) break;
-        tc_commit(tfull_bar(acc));
       }
       // All MMAs issued so far complete before the drain barrier flips.
       tc_commit(drain_bar);
@@ -437,10 +506,27 @@ __global__ void __launch_bounds__(THREADS, 1)
     // ---------------------------------------------------------- epilogue
     const int quarter = warp & 3;  // TMEM lanes this warp may access
     int it = 0;
-    for (int u = blockIdx.x; u < total_units; u += gridDim.x, ++it) {
+    for (int u = blockIdx.x; u < total_units; u += gridDim.x) {
       const int t = u / pr.ksplit, ks = u - t * pr.ksplit;
       int b, tp, tq;
       tile_coords(pr, t, b, tp, tq);
+      if constexpr (SUM) {
+        const int kb0 = ks * pr.kb_per_split, kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
+        const int p = tp * BM + quarter * 32 + lane;
+        if (!sum_epilogue(
+                tmem_base + ((uint32_t)(quarter * 32) << 16), BN, (warp - 2) / 4 * 128,
+                (kb1 - kb0 + pr.sub_kb - 1) / pr.sub_kb, it,
+                [&](int i) {
+                  return mbar_wait(tfull_bar(i & 1), (uint32_t)((i >> 1) & 1), abort_flag, pr.derr,
+                                   pr.wait_ns);
+                },
+                [&](int i) {
+                  if (lane == 0) mbar_arrive(tempty_bar(i & 1));
+                },
+                [&](int c, const float(&v)[16]) { epi(b * pr.ksplit + ks, p, tq * BN + c, v); }))
+          break;
+        continue;
+      }
       const int acc = it % SETS;
       const bool ok =
           mbar_wait(tfull_bar(acc), (uint32_t)((it / SETS) & 1), abort_flag, pr.derr, pr.wait_ns);
@@ -455,7 +541,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           uint32_t v[32];
           tmem_ld32(taddr + (uint32_t)(c * 32), v);
           tmem_ld_wait(v);
-          epi(b * pr.ksplit + ks, p, tq * BN + c * 32, v);  // batch x K range
+          if constexpr (!SUM) epi(b * pr.ksplit + ks, p, tq * BN + c * 32, v);  // batch x K range
         } else {
           uint32_t v0[32], v1[32], v2[32];
           tmem_ld32(taddr + (uint32_t)(c * 32), v0);
@@ -464,12 +550,13 @@ __global__ void __launch_bounds__(THREADS, 1)
           tmem_ld_wait(v0);
           tmem_ld_wait(v1);
           tmem_ld_wait(v2);
-          epi(p, tq * BN + c * 32, v0, v1, v2);
+          if constexpr (NACC > 1) epi(p, tq * BN + c * 32, v0, v1, v2);
         }
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(tempty_bar(acc));
+      ++it;
     }
   }
 
@@ -604,14 +691,15 @@ __device__ __forceinline__ bool mbar_wait_pair(uint32_t bar, uint32_t parity,
 
 constexpr int PAIR_BM = 2 * BM;  // output rows per pair tile
 
-template <int KIND, int BN, int STAGES, class Epi>
-__global__ void __launch_bounds__(THREADS, 1)
+template <int KIND, int BN, int STAGES, class Epi, bool SUM = false>
+__global__ void __launch_bounds__(threads_for(BN, SUM), 1)
     umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX,
                           const __grid_constant__ CUtensorMap tmY, const Problem pr,
                           const Epi epi) {
   using L = SmemLayout<BN / 2, STAGES>;  // per CTA: 128 X rows + BN/2 Y rows per stage
   static_assert(BN % 32 == 0 && BN >= 64 && BN <= 256, "pair MMA N in [64, 256]");
   static_assert(2 * BN <= 512, "two accumulators must fit in TMEM");
+  static_assert(!SUM || BN % 128 == 0, "summed epilogue: 128 columns a thread");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -645,7 +733,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);
-      mbar_init(tempty_bar(a), 8);  // 4 epilogue warps in each CTA of the pair
+      mbar_init(tempty_bar(a), 2 * epi_warps(BN, SUM));  // the epilogue warps of both CTAs
     }
     mbar_init(drain_bar, 1);
     *abort_flag = 0;
@@ -718,37 +806,40 @@ __global__ void __launch_bounds__(THREADS, 1)
       uint32_t phase = 0;
       int it = 0;
       bool ok = true;
-      for (int u = pair; u < total_units && ok; u += npairs, ++it) {
+      for (int u = pair; u < total_units && ok; u += npairs) {
         const int ks = u % pr.ksplit;
         const int kb0 = ks * pr.kb_per_split, kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
-        const int acc = it & 1;
-        const uint32_t acc_phase = (uint32_t)((it >> 1) & 1);
-        if (!mbar_wait_pair(tempty_bar(acc), acc_phase ^ 1u, abort_flag, peer_abort, pr.derr,
-                            pr.wait_ns)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait_pair(full_bar(stage), phase, abort_flag, peer_abort, pr.derr,
+        for (int kr = kb0; kr < kb1 && ok; kr += pr.sub_kb, ++it) {
+          const int ke = min(kb1, kr + pr.sub_kb);
+          const int acc = it & 1;
+          const uint32_t acc_phase = (uint32_t)((it >> 1) & 1);
+          if (!mbar_wait_pair(tempty_bar(acc), acc_phase ^ 1u, abort_flag, peer_abort, pr.derr,
                               pr.wait_ns)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t sx = base + stage * L::STAGE_BYTES;
-          const uint32_t sy = sx + L::X_BYTES;
+          const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
+          for (int kb = kr; kb < ke; ++kb) {
+            if (!mbar_wait_pair(full_bar(stage), phase, abort_flag, peer_abort, pr.derr,
+                                pr.wait_ns)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t sx = base + stage * L::STAGE_BYTES;
+            const uint32_t sy = sx + L::X_BYTES;
 #pragma unroll
-          for (int kk = 0; kk < KBLOCK_BYTES / 32; ++kk) {
-            tc_mma_pair<KIND>(d_tmem, sw128_desc(sx + kk * 32), sw128_desc(sy + kk * 32), idesc,
-                              (kb != kb0 || kk) ? 1u : 0u);
+            for (int kk = 0; kk < KBLOCK_BYTES / 32; ++kk) {
+              tc_mma_pair<KIND>(d_tmem, sw128_desc(sx + kk * 32), sw128_desc(sy + kk * 32), idesc,
+                                (kb != kr || kk) ? 1u : 0u);
+            }
+            tc_commit_pair(empty_bar(stage), (uint16_t)3);  // frees the stage in both CTAs
+            if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           }
-          tc_commit_pair(empty_bar(stage), (uint16_t)3);  // frees the stage in both CTAs
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          if (!ok) break;
+          tc_commit_pair(tfull_bar(acc), (uint16_t)3);
         }
-        if (!ok) break;
-        tc_commit_pair(tfull_bar(acc), (uint16_t)3);
       }
       tc_commit_pair(drain_bar, (uint16_t)1);
       mbar_wait_drain(drain_bar, 0, pr.wait_ns);
@@ -757,10 +848,27 @@ __global__ void __launch_bounds__(THREADS, 1)
     // ---------------------------------------------------------- epilogue
     const int quarter = warp & 3;
     int it = 0;
-    for (int u = pair; u < total_units; u += npairs, ++it) {
+    for (int u = pair; u < total_units; u += npairs) {
       const int t = u / pr.ksplit, ks = u - t * pr.ksplit;
       int b, tp, tq;
       tile_coords(pr, t, b, tp, tq);
+      if constexpr (SUM) {
+        const int kb0 = ks * pr.kb_per_split, kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
+        const int p = tp * PAIR_BM + (int)rank * BM + quarter * 32 + lane;
+        if (!sum_epilogue(
+                tmem_base + ((uint32_t)(quarter * 32) << 16), BN, (warp - 2) / 4 * 128,
+                (kb1 - kb0 + pr.sub_kb - 1) / pr.sub_kb, it,
+                [&](int i) {
+                  return mbar_wait_pair(tfull_bar(i & 1), (uint32_t)((i >> 1) & 1), abort_flag,
+                                        peer_abort, pr.derr, pr.wait_ns);
+                },
+                [&](int i) {
+                  if (lane == 0) mbar_arrive_remote(map_rank(tempty_bar(i & 1), 0));
+                },
+                [&](int c, const float(&v)[16]) { epi(b * pr.ksplit + ks, p, tq * BN + c, v); }))
+          break;
+        continue;
+      }
       const int acc = it & 1;
       const bool ok = mbar_wait_pair(tfull_bar(acc), (uint32_t)((it >> 1) & 1), abort_flag,
                                      peer_abort, pr.derr, pr.wait_ns);
@@ -773,11 +881,12 @@ __global__ void __launch_bounds__(THREADS, 1)
         uint32_t v[32];
         tmem_ld32(taddr + (uint32_t)(c * 32), v);
         tmem_ld_wait(v);
-        epi(b * pr.ksplit + ks, p, tq * BN + c * 32, v);  // batch x K range
+        if constexpr (!SUM) epi(b * pr.ksplit + ks, p, tq * BN + c * 32, v);  // batch x K range
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(map_rank(tempty_bar(acc), 0));
+      ++it;
     }
   }
 
@@ -824,11 +933,25 @@ __global__ void __launch_bounds__(THREADS, 1)
 int make_kmajor_map(CUtensorMap *map, int kind, const void *base, long long kelems, long long rows,
                     long long nbatch, long long row_bytes, long long plane_bytes, int box_rows);
 
-template <int KIND, int BN, int STAGES, class Epi, int NACC = 1>
+// K ranges of a launch: `ksplit` of ceil(kblocks / ksplit) blocks, their count
+// recomputed so that none is empty (an empty range would leave its accumulator
+// unwritten); or, with kb_range, ranges of kb_range blocks.  sub_kb: the part
+// of a range accumulated at a time (0: all of it).
+inline void set_split(Problem &pr, int ksplit, int kb_range, int sub_kb) {
+  if (ksplit < 1) ksplit = 1;
+  if (ksplit > pr.kblocks) ksplit = pr.kblocks > 0 ? pr.kblocks : 1;
+  pr.kb_per_split = kb_range > 0 ? kb_range : (pr.kblocks + ksplit - 1) / ksplit;
+  pr.ksplit = pr.kb_per_split > 0 ? (pr.kblocks + pr.kb_per_split - 1) / pr.kb_per_split : 1;
+  if (pr.ksplit < 1) pr.ksplit = 1;
+  pr.sub_kb = sub_kb > 0 ? sub_kb : (pr.kb_per_split > 0 ? pr.kb_per_split : 1);
+}
+
+template <int KIND, int BN, int STAGES, class Epi, int NACC = 1, bool SUM = false>
 int launch(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, long long kelems,
            int nbatch, const Epi &epi, int sm_count, int *derr, cudaStream_t s,
            const char *prof_name, int max_ctas = 0, const int *nbatch_dev = nullptr,
-           int ksplit = 1, int seg_kb = 0, unsigned seg_x = 0, unsigned seg_y = 0) {
+           int ksplit = 1, int seg_kb = 0, unsigned seg_x = 0, unsigned seg_y = 0,
+           int kb_range = 0, int sub_kb = 0) {
   if (NACC > 1 && (ksplit > 1 || nbatch != NACC || nbatch_dev)) return B2_ERR_ARG;
   using L = SmemLayout<BN, STAGES>;
   Problem pr;
@@ -845,23 +968,17 @@ int launch(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, long lo
   pr.group = 8;
   pr.derr = derr;
   launch_wait_settings(&pr.wait_ns, &pr.withhold);
-  // split-K: ranges of ceil(kblocks / ksplit) blocks, their count recomputed so
-  // that none is empty (an empty range would leave its accumulator unwritten)
-  if (ksplit < 1) ksplit = 1;
-  if (ksplit > pr.kblocks) ksplit = pr.kblocks > 0 ? pr.kblocks : 1;
-  pr.kb_per_split = (pr.kblocks + ksplit - 1) / ksplit;
-  pr.ksplit = pr.kb_per_split > 0 ? (pr.kblocks + pr.kb_per_split - 1) / pr.kb_per_split : 1;
-  if (pr.ksplit < 1) pr.ksplit = 1;
+  set_split(pr, ksplit, kb_range, SUM ? sub_kb : 0);
   const long long total =
       (long long)pr.tiles_p * pr.tiles_q * (NACC == 1 ? nbatch : 1) * pr.ksplit;
   if (total <= 0 || (NACC > 1 && pr.kblocks <= 0)) return B2_OK;
   int grid = (int)(total < sm_count ? total : sm_count);
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  auto kern = umma_gemm_kernel<KIND, BN, STAGES, Epi, NACC>;
+  auto kern = umma_gemm_kernel<KIND, BN, STAGES, Epi, NACC, SUM>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
   if (e != cudaSuccess) return cuda_fail(e, "umma smem attribute");
   B2_PROF(prof_name, s);
-  kern<<<grid, THREADS, L::TOTAL, s>>>(tmX, tmY, pr, epi);
+  kern<<<grid, threads_for(BN, SUM), L::TOTAL, s>>>(tmX, tmY, pr, epi);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, prof_name);
   return B2_OK;
@@ -870,11 +987,12 @@ int launch(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, long lo
 // Pair launch: clusters of 2 CTAs, one pair per two SMs (as many pairs as can
 // be resident at once, queried once per device), tiles of 256 X rows x BN Y
 // rows.  tmX must have a 128-row box and tmY a BN/2-row box.
-template <int KIND, int BN, int STAGES, class Epi>
+template <int KIND, int BN, int STAGES, class Epi, bool SUM = false>
 int launch_pair(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, long long kelems,
                 int nbatch, const Epi &epi, int device, int *derr, cudaStream_t s,
                 const char *prof_name, const int *nbatch_dev = nullptr, int ksplit = 1,
-                int seg_kb = 0, unsigned seg_x = 0, unsigned seg_y = 0) {
+                int seg_kb = 0, unsigned seg_x = 0, unsigned seg_y = 0, int kb_range = 0,
+                int sub_kb = 0) {
   using L = SmemLayout<BN / 2, STAGES>;
   Problem pr;
   pr.P = P;
@@ -885,13 +1003,7 @@ int launch_pair(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, lo
   pr.seg_kb = seg_kb;
   pr.seg_x = seg_x;
   pr.seg_y = seg_y;
-  // split-K exactly as in launch(): ranges of ceil(kblocks / ksplit) blocks,
-  // their count recomputed so that none is empty
-  if (ksplit < 1) ksplit = 1;
-  if (ksplit > pr.kblocks) ksplit = pr.kblocks > 0 ? pr.kblocks : 1;
-  pr.kb_per_split = (pr.kblocks + ksplit - 1) / ksplit;
-  pr.ksplit = pr.kb_per_split > 0 ? (pr.kblocks + pr.kb_per_split - 1) / pr.kb_per_split : 1;
-  if (pr.ksplit < 1) pr.ksplit = 1;
+  set_split(pr, ksplit, kb_range, SUM ? sub_kb : 0);
   pr.tiles_p = (P + PAIR_BM - 1) / PAIR_BM;
   pr.tiles_q = (Q + BN - 1) / BN;
   pr.group = 8;
@@ -899,14 +1011,14 @@ int launch_pair(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, lo
   launch_wait_settings(&pr.wait_ns, &pr.withhold);
   const long long total = (long long)pr.tiles_p * pr.tiles_q * nbatch * pr.ksplit;
   if (total <= 0) return B2_OK;
-  auto kern = umma_gemm_pair_kernel<KIND, BN, STAGES, Epi>;
+  auto kern = umma_gemm_pair_kernel<KIND, BN, STAGES, Epi, SUM>;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  cfg.blockDim = dim3(THREADS);
+  cfg.blockDim = dim3(threads_for(BN, SUM));
   cfg.dynamicSmemBytes = L::TOTAL;
   cfg.stream = s;
   cfg.attrs = attr;
