@@ -79,7 +79,8 @@ int sgemm_simt(char ta, char tb, int m, int n, int k, float alpha, const float *
 int sgemm_split_tf32x3(const float *X, long long sr, long long sk, int R, int K, int kp,
                        float *out, cudaStream_t s);
 // C(m, n) = alpha * sum_ks W[ks * plane + n * ldw + m] + beta C (beta != 1
-// multiplies), the S partials summed in FP64 in K order and rounded once.
+// multiplies), the S partials summed in FP64 in K order and rounded once; W
+// 16-byte aligned, plane and ldw multiples of 4.
 int sgemm_splitk_reduce(const float *W, long long plane, int ldw, int S, int m, int n,
                         float alpha, float beta, float *C, int ldc, cudaStream_t s);
 

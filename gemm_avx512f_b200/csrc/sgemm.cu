@@ -255,7 +255,8 @@ int launch_ffma2(int m, int n, int k, float alpha, const float *A, int lda, cons
   // reduction adding them in K order (FP64 sums, rounded once) into C.
   const int kchunk = (kblocks + S - 1) / S * S2_K;
   const int S_used = (k + kchunk - 1) / kchunk;
-  const long long plane = (long long)n * m;
+  const int ldp = (m + 3) & ~3;
+  const long long plane = (long long)n * ldp;
   float *P = (float *)workspace(cx, WS_MISC, (size_t)plane * S_used * sizeof(float));
   if (!P) return B2_ERR_NOMEM;
   {
@@ -263,10 +264,10 @@ int launch_ffma2(int m, int n, int k, float alpha, const float *A, int lda, cons
         cudaFuncSetAttribute(kern_split, cudaFuncAttributeMaxDynamicSharedMemorySize, S2_SMEM));
     B2_PROF("sgemm_simt", s);
     kern_split<<<dim3(gx, gy, S_used), 256, S2_SMEM, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C,
-                                                           ldc, kchunk, P, plane, m);
+                                                           ldc, kchunk, P, plane, ldp);
     B2_CUDA_TRY(cudaGetLastError());
   }
-  return sgemm_splitk_reduce(P, plane, m, S_used, m, n, alpha, beta, C, ldc, s);
+  return sgemm_splitk_reduce(P, plane, ldp, S_used, m, n, alpha, beta, C, ldc, s);
 }
 
 }  // namespace

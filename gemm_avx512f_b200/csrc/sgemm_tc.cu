@@ -8,13 +8,11 @@
 //                       C = Ab Bb + Ab Bs + As Bb                (kind::tf32)
 //   BF16X3  3 products: A = Ah + Al, B = Bh + Bl (each BF16),
 //                       C = Ah Bh + Ah Bl + Al Bh                (kind::f16, bf16 in)
-// Every method is ONE GEMM over K' = terms * Kp on the engine in umma.cuh;
-// the split/convert kernel is the only extra pass.  For three terms each
-// operand stores two segments, [big | small], each padded with zeros to a
-// 128-byte K block, and the engine's three-term interleave reads K' block j
-// as term j % 3 of K block j / 3: (Bb, Ab), (Bs, Ab), (Bb, As).  The big part
-// used by two terms is written once and read from DRAM once (its second load
-// is an L2 hit a few K' blocks later).
+// Every method is ONE GEMM on the engine in umma.cuh; the split/convert kernel
+// is the only extra pass.  For three terms each operand stores two segments,
+// [big | small], each padded with zeros to a 128-byte K block, and a stage of
+// the engine holds both segments of a K block of A and B: its MMAs add
+// Ab Bb + Ab Bs + As Bb, so every segment is loaded once.
 #include <cuda_bf16.h>
 
 #include <type_traits>
@@ -46,11 +44,14 @@ struct SplitOp {
 // segments of kp elements of type T, zero beyond K: out[r][segs*kp].  One
 // block turns 64 rows x 64 k around in shared memory; blocks that follow each
 // other read neighbouring memory.
-// Bound: HBM, 4 bytes read and segs*sizeof(T) written per element.  FILL
+// Bound: HBM, 4 bytes read and segs*sizeof(T) written per element: 8192x8192
+// to two bfloat16 segments in 83 us, 6.4 TB/s (32x64 blocks with two loads in
+// flight per thread, k blocks first: 125 us).
 template <typename T>
 __global__ void __launch_bounds__(256)
     split_kernel(const SplitOp a, const SplitOp b, unsigned blocks_a, int K, int kp, int segs) {
   __shared__ float tile[64][65];
+  umma::grid_dependency_wait();
   const bool second = blockIdx.x >= blocks_a;
   const float *X = second ? b.X : a.X;
   const long long ld = second ? b.ld : a.ld;
@@ -156,6 +157,15 @@ struct F32Epi {
   int ldc;
   int M, N;
   float alpha, beta;
+  // Brings the warp's 32 rows x 128 columns of C (rows from p0) into L2 while
+  // the product is formed: one line per lane and column.
+  __device__ __forceinline__ void prefetch(int p0, int lane, int q0) const {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int q = q0 + 32 * i + lane;
+      if (p0 < M && q < N) umma::prefetch_l2(C + (long long)q * ldc + p0);
+    }
+  }
   __device__ __forceinline__ void operator()(int, int p, int q0, const float (&v)[16]) const {
     if (p >= M || q0 >= N) return;
     // (the volatile asms keep the compiler from holding the addresses of many
@@ -189,6 +199,7 @@ struct F32PartialEpi {
   long long plane;
   int ldw;
   int M, N;
+  __device__ __forceinline__ void prefetch(int, int, int) const {}
   __device__ __forceinline__ void operator()(int ks, int p, int q0, const float (&v)[16]) const {
     if (p >= M || q0 >= N) return;
     float *w = W + ks * plane + (long long)q0 * ldw + p;
@@ -201,17 +212,48 @@ struct F32PartialEpi {
 
 // C(m, n) = alpha * sum_ks W[ks][n][m] + beta C (beta != 1 multiplies), the
 // partials summed in FP64 in K order and rounded once.
-__global__ void sgemm_splitk_reduce_kernel(const float *__restrict__ W, long long plane, int ldw,
-                                           int S, int M, int N, float alpha, float beta,
-                                           float *__restrict__ C, int ldc) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= M) return;
-  for (int n = blockIdx.y; n < N; n += gridDim.y) {
-    double acc = 0.0;
-    for (int ks = 0; ks < S; ++ks) acc += (double)W[ks * plane + (long long)n * ldw + m];
+// Four rows per thread; launched as a programmatic dependent of the GEMM, whose
+// writes it waits for.  W is 16-byte aligned and ldw a multiple of 4.
+__global__ void __launch_bounds__(256)
+    sgemm_splitk_reduce_kernel(const float *__restrict__ W, long long plane, int ldw, int S, int M,
+                               int N, float alpha, float beta, float *__restrict__ C, int ldc) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const unsigned quads = (unsigned)(M + 3) / 4;
+  const unsigned long long total = (unsigned long long)quads * (unsigned)N;
+  const bool cvec = (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldc & 3) == 0;
+  for (unsigned long long i = blockIdx.x * 256ull + threadIdx.x; i < total;
+       i += gridDim.x * 256ull) {
+    const int n = (int)(i / quads), m = (int)(i - (unsigned long long)n * quads) * 4;
     float *c = C + (long long)n * ldc + m;
-    const float a = (float)acc;
-    *c = (beta == 1.f) ? fmaf(alpha, a, *c) : fmaf(alpha, a, beta * *c);
+    const float *w = W + (long long)n * ldw + m;
+    const int left = M - m;
+    float old[4];
+    if (cvec && left >= 4) {
+      const float4 q = *reinterpret_cast<const float4 *>(c);
+      old[0] = q.x, old[1] = q.y, old[2] = q.z, old[3] = q.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) old[e] = e < left ? c[e] : 0.f;
+    }
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int ks = 0; ks < S; ++ks) {
+      const float4 x = *reinterpret_cast<const float4 *>(w + ks * plane);
+      acc[0] += (double)x.x, acc[1] += (double)x.y, acc[2] += (double)x.z, acc[3] += (double)x.w;
+    }
+    float r[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float a = (float)acc[e];
+      r[e] = (beta == 1.f) ? fmaf(alpha, a, old[e]) : fmaf(alpha, a, beta * old[e]);
+    }
+    if (cvec && left >= 4) {
+      *reinterpret_cast<float4 *>(c) = make_float4(r[0], r[1], r[2], r[3]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (e < left) c[e] = r[e];
+    }
   }
 }
 
@@ -249,7 +291,7 @@ int ranges_per_unit(long long tiles, int S, int kbps, int kblocks, int slots, do
   double best_us = 1e300;
   for (int per = S; per >= 1; --per) {
     const int E = (S + per - 1) / per;
-    if (per < S && (S + per) / (per + 1) == E) continue;  // same E with fewer ranges: no better
+    if (per > 1 && (S + per - 2) / (per - 1) == E) continue;  // more even with per - 1
     const long long waves = (tiles * E + slots - 1) / slots;
     const int kb = per * kbps < kblocks ? per * kbps : kblocks;
     double us = (double)waves * (kb * t_kb + 3.0);
@@ -276,7 +318,16 @@ int run_split(const SplitOp &a, const SplitOp &b, int K, int kp, int segs, cudaS
   const unsigned kt = (unsigned)(kp + 63) / 64;
   const unsigned ba = kt * ((unsigned)(a.R + 63) / 64), bb = kt * ((unsigned)(b.R + 63) / 64);
   B2_PROF("sgemm_split", s);
-  split_kernel<T><<<ba + bb, 256, 0, s>>>(a, b, ba, K, kp, segs);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(ba + bb);
+  lc.blockDim = dim3(256);
+  lc.stream = s;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  B2_CUDA_TRY(cudaLaunchKernelEx(&lc, split_kernel<T>, a, b, ba, K, kp, segs));
   B2_CUDA_TRY(cudaGetLastError());
   return B2_OK;
 }
@@ -330,16 +381,13 @@ int sgemm_tensor_cfg(char ta, char tb, int m, int n, int k, float alpha, const f
   const int terms = (method == B2_METHOD_TF32) ? 1 : 3;
   const int esz = bf16 ? 2 : 4;
   const int kp = (int)round_up(k, 128 / esz);
-  const long long kt = (long long)terms * kp;               // K' of the one GEMM
   const int segs = terms == 3 ? 2 : 1;                      // stored segments per row
   const long long ks_ = (long long)segs * kp;
   void *Xp = workspace(cx, WS_SPLIT_X, (size_t)m * ks_ * esz);
   void *Yp = workspace(cx, WS_SPLIT_Y, (size_t)n * ks_ * esz);
   if (!Yp || !Xp) return B2_ERR_NOMEM;
   // The engine's X (accumulator lanes) is op(A): a warp's 32 lanes are then 32
-  // consecutive rows of a column of C.  Stored segments: [big] or [big, small];
-  // terms read (Ab, Bb), (Ab, Bs), (As, Bb).
-  const unsigned segX = 0x4u, segY = 0x2u;        // term -> segment, A side / B side
+  // consecutive rows of a column of C.  Stored segments: [big] or [big, small].
   const SplitOp oa = split_op(A, asr, ask, m, Xp), ob = split_op(B, bsr, bsk, n, Yp);
   int rc = bf16 ? run_split<__nv_bfloat16>(oa, ob, k, kp, segs, s)
                 : run_split<float>(oa, ob, k, kp, segs, s);
@@ -357,38 +405,48 @@ int sgemm_tensor_cfg(char ta, char tb, int m, int n, int k, float alpha, const f
   if (rc != B2_OK) return rc;
   const int seg_kb = terms == 3 ? (int)((long long)kp * esz / umma::KBLOCK_BYTES) : 0;
   const long long tiles = ((n + tile_q - 1) / tile_q) * (long long)((m + tile_p - 1) / tile_p);
-  const int kblocks = (int)((kt * esz + umma::KBLOCK_BYTES - 1) / umma::KBLOCK_BYTES);
+  const int kblocks = (int)(((long long)kp * esz + umma::KBLOCK_BYTES - 1) / umma::KBLOCK_BYTES);
   const int slots = eng == 2 ? cx->sm_count / 2 : cx->sm_count;
-  // K is accumulated in S ranges of kbps blocks; a unit adds `per` of them
-  int S = cfg.split > 0 ? cfg.split : choose_ksplit(tiles, kblocks, slots);
+  // K is accumulated in S ranges of kbps blocks (of `terms` products each); a
+  // unit adds `per` of them
+  int S = cfg.split > 0 ? cfg.split : choose_ksplit(tiles, terms * kblocks, slots);
   if (S > kblocks) S = kblocks > 0 ? kblocks : 1;
   const int kbps = (kblocks + S - 1) / S;
   S = (kblocks + kbps - 1) / kbps;
-  const int per = ranges_per_unit(tiles, S, kbps, kblocks, slots, eng == 1 ? 0.17 : 0.28, m, n);
+  const int per =
+      ranges_per_unit(tiles, S, kbps, kblocks, slots, terms * (eng == 1 ? 0.17 : 0.28), m, n);
   const int E = (S + per - 1) / per;  // partials per tile
   auto run = [&](auto epi) -> int {
     using Epi = decltype(epi);
     const char *nm = bf16 ? "sgemm_umma_bf16" : "sgemm_umma_tf32";
     const int kbr = per * kbps;
-    auto pair = [&](auto kd) {
-      return umma::launch_pair<decltype(kd)::value, 256, 6, Epi, true>(
-          tmX, tmY, m, n, kt, 1, epi, cx->device, cx->derr, s, nm, nullptr, E, seg_kb, segX, segY,
-          kbr, kbps);
+    // TERMS = 3 stages hold four operand tiles: 64 KB (pair and 128x128), 96 KB
+    auto pair = [&](auto kd, auto t3) {
+      constexpr int T = decltype(t3)::value;
+      return umma::launch_pair<decltype(kd)::value, 256, T == 3 ? 3 : 6, Epi, true, T>(
+          tmX, tmY, m, n, kp, 1, epi, cx->device, cx->derr, s, nm, nullptr, E, seg_kb, kbr, kbps);
     };
-    auto single = [&](auto kd, auto bn, auto st) {
-      return umma::launch<decltype(kd)::value, decltype(bn)::value, decltype(st)::value, Epi, 1,
-                          true>(tmX, tmY, m, n, kt, 1, epi, cx->sm_count, cx->derr, s, nm, 0,
-                                nullptr, E, seg_kb, segX, segY, kbr, kbps);
+    auto single = [&](auto kd, auto bn, auto t3) {
+      constexpr int T = decltype(t3)::value, BN = decltype(bn)::value;
+      constexpr int ST = BN == 256 ? (T == 3 ? 2 : 4) : (T == 3 ? 3 : 6);
+      return umma::launch<decltype(kd)::value, BN, ST, Epi, 1, true, T>(
+          tmX, tmY, m, n, kp, 1, epi, cx->sm_count, cx->derr, s, nm, 0, nullptr, E, seg_kb, 0, 0,
+          kbr, kbps);
     };
     using BF = std::integral_constant<int, umma::KIND_BF16>;
     using TF = std::integral_constant<int, umma::KIND_TF32>;
-    using I4 = std::integral_constant<int, 4>;
-    using I6 = std::integral_constant<int, 6>;
+    using I1 = std::integral_constant<int, 1>;
+    using I3 = std::integral_constant<int, 3>;
     using I128 = std::integral_constant<int, 128>;
     using I256 = std::integral_constant<int, 256>;
-    if (eng == 2) return bf16 ? pair(BF{}) : pair(TF{});
-    if (eng == 1) return bf16 ? single(BF{}, I128{}, I6{}) : single(TF{}, I128{}, I6{});
-    return bf16 ? single(BF{}, I256{}, I4{}) : single(TF{}, I256{}, I4{});
+    if (eng == 2) return bf16 ? pair(BF{}, I3{}) : terms == 3 ? pair(TF{}, I3{}) : pair(TF{}, I1{});
+    if (eng == 1)
+      return bf16         ? single(BF{}, I128{}, I3{})
+             : terms == 3 ? single(TF{}, I128{}, I3{})
+                          : single(TF{}, I128{}, I1{});
+    return bf16         ? single(BF{}, I256{}, I3{})
+           : terms == 3 ? single(TF{}, I256{}, I3{})
+                        : single(TF{}, I256{}, I1{});
   };
   if (E == 1) return run(F32Epi{C, ldc, m, n, alpha, beta});
   // E partial products of K ranges, then one fixed-order reduction.
@@ -403,9 +461,19 @@ int sgemm_tensor_cfg(char ta, char tb, int m, int n, int k, float alpha, const f
 
 int sgemm_splitk_reduce(const float *W, long long plane, int ldw, int S, int m, int n,
                         float alpha, float beta, float *C, int ldc, cudaStream_t s) {
-  dim3 grid((unsigned)((m + 255) / 256), (unsigned)(n < 4096 ? n : 4096));
+  const long long blocks = ((long long)((m + 3) / 4) * n + 255) / 256;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3((unsigned)(blocks < 1184 ? blocks : 1184));  // 8 blocks on each of 148 SMs
+  lc.blockDim = dim3(256);
+  lc.stream = s;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
   B2_PROF("sgemm_splitk_reduce", s);
-  sgemm_splitk_reduce_kernel<<<grid, 256, 0, s>>>(W, plane, ldw, S, m, n, alpha, beta, C, ldc);
+  B2_CUDA_TRY(cudaLaunchKernelEx(&lc, sgemm_splitk_reduce_kernel, W, plane, ldw, S, m, n, alpha,
+                                 beta, C, ldc));
   B2_CUDA_TRY(cudaGetLastError());
   return B2_OK;
 }

@@ -120,6 +120,15 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
+// SUM kernels are launched as programmatic dependents: their set-up overlaps the
+// end of the kernel before them in the stream, whose writes they wait for here.
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void prefetch_l2(const void *p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // Records a timeout in the error word.  A plain store (every writer stores
 // the same value), so the word may live in mapped host memory.
 __device__ __forceinline__ void record_timeout(int *derr) {
@@ -268,7 +277,10 @@ struct Problem {
   int tiles_p, tiles_q;
   int group;       // tile rasterisation: GROUP rows of P tiles share a sweep over Q
   int *derr;       // device error word
-  // Three-term interleave (0 = off): K' block j is term j % 3 of K block j / 3;
+  // TERMS = 3 kernels: a stage holds both segments (big, small) of a K block of
+  // X and Y, the small ones seg_kb K blocks further along K, and its MMAs add
+  // Xb Yb + Xb Ys + Xs Yb, so each segment is loaded once.
+  // TERMS = 1 kernels, three-term interleave (0 = off): K' block j is term j % 3 of K block j / 3;
   // the operands store 2 segments of seg_kb K blocks (0 = big, 1 = small) and
   // bit t of seg_x / seg_y names the segment term t reads.  The big part that
   // two terms share is read from DRAM once: its second load follows the first
@@ -280,11 +292,12 @@ struct Problem {
                      // byte count but issues no copy (the wait for it times out)
 };
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, int TERMS = 1>
 struct SmemLayout {
   static constexpr int X_BYTES = BM * KBLOCK_BYTES;
   static constexpr int Y_BYTES = BN * KBLOCK_BYTES;
-  static constexpr int STAGE_BYTES = X_BYTES + Y_BYTES;
+  static constexpr int HALF_BYTES = X_BYTES + Y_BYTES;  // X and Y of one segment
+  static constexpr int STAGE_BYTES = (TERMS == 3 ? 2 : 1) * HALF_BYTES;
   static constexpr int BAR_OFF = STAGES * STAGE_BYTES;
   // full[S], empty[S], tfull[2], tempty[2], drain, then tmem address (+0),
   // abort flag (+8) and the CTA pair's odd-CTA fill count (+12)
@@ -355,11 +368,11 @@ __device__ __forceinline__ bool sum_epilogue(uint32_t tmem_quarter, int bn, int 
 // operands into NACC accumulators that its epilogue receives together
 // (epi(p, q0, v0, v1, v2) for NACC = 3: the three real products of the 3M
 // method); no split-K.
-template <int KIND, int BN, int STAGES, class Epi, int NACC = 1, bool SUM = false>
+template <int KIND, int BN, int STAGES, class Epi, int NACC = 1, bool SUM = false, int TERMS = 1>
 __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
     umma_gemm_kernel(const __grid_constant__ CUtensorMap tmX,
                      const __grid_constant__ CUtensorMap tmY, const Problem pr, const Epi epi) {
-  using L = SmemLayout<BN, STAGES>;
+  using L = SmemLayout<BN, STAGES, TERMS>;
   // accumulator sets: two (the epilogue of a unit overlaps the next unit's
   // MMAs) when they fit in TMEM's 512 columns, else one
   constexpr int SETS = 2 * NACC * BN <= 512 ? 2 : 1;
@@ -413,6 +426,7 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if constexpr (SUM) grid_dependency_wait();
 
   long issued = 0;  // fills posted by the producer (warp 0, lane 0)
   if (warp == 0) {
@@ -441,7 +455,7 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
           const uint32_t sy = sx + L::X_BYTES;
           mbar_expect_tx(full_bar(stage), L::STAGE_BYTES);
           int kx = kb * kcoord, ky = kx;
-          if (pr.seg_kb) {
+          if (TERMS == 1 && pr.seg_kb) {
             const int kq = kb / 3, tt = kb - 3 * kq;
             kx = ((int)((pr.seg_x >> tt) & 1u) * pr.seg_kb + kq) * kcoord;
             ky = ((int)((pr.seg_y >> tt) & 1u) * pr.seg_kb + kq) * kcoord;
@@ -449,6 +463,11 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
           if (!(pr.withhold && issued == 0)) {
             tma_load_3d(sx, &tmX, full_bar(stage), kx, tp * BM, b);
             tma_load_3d(sy, &tmY, full_bar(stage), ky, tq * BN, b);
+            if constexpr (TERMS == 3) {
+              const int ksm = (kb + pr.seg_kb) * kcoord;
+              tma_load_3d(sx + L::HALF_BYTES, &tmX, full_bar(stage), ksm, tp * BM, b);
+              tma_load_3d(sy + L::HALF_BYTES, &tmY, full_bar(stage), ksm, tq * BN, b);
+            }
           }
           ++issued;
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -487,9 +506,14 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
             const uint32_t sx = base + stage * L::STAGE_BYTES;
             const uint32_t sy = sx + L::X_BYTES;
 #pragma unroll
-            for (int kk = 0; kk < KBLOCK_BYTES / 32; ++kk) {
-              tc_mma<KIND>(d_tmem, sw128_desc(sx + kk * 32), sw128_desc(sy + kk * 32), idesc,
-                           (kb != kr || kk) ? 1u : 0u);
+            for (int tt = 0; tt < TERMS; ++tt) {
+              const uint32_t tx = sx + (tt == 2 ? L::HALF_BYTES : 0);
+              const uint32_t ty = sy + (tt == 1 ? L::HALF_BYTES : 0);
+#pragma unroll
+              for (int kk = 0; kk < KBLOCK_BYTES / 32; ++kk) {
+                tc_mma<KIND>(d_tmem, sw128_desc(tx + kk * 32), sw128_desc(ty + kk * 32), idesc,
+                             (kb != kr || kk || tt) ? 1u : 0u);
+              }
             }
             tc_commit(empty_bar(stage));  // frees the stage once these MMAs have read it
             if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -513,6 +537,7 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
       if constexpr (SUM) {
         const int kb0 = ks * pr.kb_per_split, kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
         const int p = tp * BM + quarter * 32 + lane;
+        epi.prefetch(p - lane, lane, tq * BN + (warp - 2) / 4 * 128);
         if (!sum_epilogue(
                 tmem_base + ((uint32_t)(quarter * 32) << 16), BN, (warp - 2) / 4 * 128,
                 (kb1 - kb0 + pr.sub_kb - 1) / pr.sub_kb, it,
@@ -583,7 +608,7 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
 }
 
 // ------------------------------------------------- CTA-pair (cta_group::2) --
-// The same product (work units of tile x K range, the three-term segment map)
+// The same product (work units of tile x K range, three-term stages)
 // on a cluster of two CTAs that execute one 256 x BN MMA
 // together (tcgen05.mma.cta_group::2): CTA r of the pair stages X rows
 // [256 tp + 128 r, +128) and Y rows [BN tq + (BN/2) r, +BN/2) of every
@@ -691,12 +716,12 @@ __device__ __forceinline__ bool mbar_wait_pair(uint32_t bar, uint32_t parity,
 
 constexpr int PAIR_BM = 2 * BM;  // output rows per pair tile
 
-template <int KIND, int BN, int STAGES, class Epi, bool SUM = false>
+template <int KIND, int BN, int STAGES, class Epi, bool SUM = false, int TERMS = 1>
 __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
     umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX,
                           const __grid_constant__ CUtensorMap tmY, const Problem pr,
                           const Epi epi) {
-  using L = SmemLayout<BN / 2, STAGES>;  // per CTA: 128 X rows + BN/2 Y rows per stage
+  using L = SmemLayout<BN / 2, STAGES, TERMS>;  // per CTA: 128 X rows + BN/2 Y rows per stage
   static_assert(BN % 32 == 0 && BN >= 64 && BN <= 256, "pair MMA N in [64, 256]");
   static_assert(2 * BN <= 512, "two accumulators must fit in TMEM");
   static_assert(!SUM || BN % 128 == 0, "summed epilogue: 128 columns a thread");
@@ -754,6 +779,7 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
   cluster_sync();  // both CTAs hold the accumulator columns before the first MMA
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if constexpr (SUM) grid_dependency_wait();
 
   long issued = 0;  // fills this CTA's producer (warp 0, lane 0) took part in
   if (warp == 0) {
@@ -780,15 +806,15 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
           const uint32_t sy = sx + L::X_BYTES;
           const uint32_t fb = map_rank(full_bar(stage), 0);
           if (leader) mbar_expect_tx(full_bar(stage), 2 * L::STAGE_BYTES);
-          int kx = kb * kcoord, ky = kx;
-          if (pr.seg_kb) {
-            const int kq = kb / 3, tt = kb - 3 * kq;
-            kx = ((int)((pr.seg_x >> tt) & 1u) * pr.seg_kb + kq) * kcoord;
-            ky = ((int)((pr.seg_y >> tt) & 1u) * pr.seg_kb + kq) * kcoord;
-          }
+          const int kx = kb * kcoord;
           if (!(leader && pr.withhold && issued == 0)) {
             tma_load_3d_pair(sx, &tmX, fb, kx, xrow, b);
-            tma_load_3d_pair(sy, &tmY, fb, ky, yrow, b);
+            tma_load_3d_pair(sy, &tmY, fb, kx, yrow, b);
+            if constexpr (TERMS == 3) {
+              const int ksm = (kb + pr.seg_kb) * kcoord;
+              tma_load_3d_pair(sx + L::HALF_BYTES, &tmX, fb, ksm, xrow, b);
+              tma_load_3d_pair(sy + L::HALF_BYTES, &tmY, fb, ksm, yrow, b);
+            }
           }
           ++issued;
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -830,9 +856,14 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
             const uint32_t sx = base + stage * L::STAGE_BYTES;
             const uint32_t sy = sx + L::X_BYTES;
 #pragma unroll
-            for (int kk = 0; kk < KBLOCK_BYTES / 32; ++kk) {
-              tc_mma_pair<KIND>(d_tmem, sw128_desc(sx + kk * 32), sw128_desc(sy + kk * 32), idesc,
-                                (kb != kr || kk) ? 1u : 0u);
+            for (int tt = 0; tt < TERMS; ++tt) {
+              const uint32_t tx = sx + (tt == 2 ? L::HALF_BYTES : 0);
+              const uint32_t ty = sy + (tt == 1 ? L::HALF_BYTES : 0);
+#pragma unroll
+              for (int kk = 0; kk < KBLOCK_BYTES / 32; ++kk) {
+                tc_mma_pair<KIND>(d_tmem, sw128_desc(tx + kk * 32), sw128_desc(ty + kk * 32),
+                                  idesc, (kb != kr || kk || tt) ? 1u : 0u);
+              }
             }
             tc_commit_pair(empty_bar(stage), (uint16_t)3);  // frees the stage in both CTAs
             if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -855,6 +886,7 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
       if constexpr (SUM) {
         const int kb0 = ks * pr.kb_per_split, kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
         const int p = tp * PAIR_BM + (int)rank * BM + quarter * 32 + lane;
+        epi.prefetch(p - lane, lane, tq * BN + (warp - 2) / 4 * 128);
         if (!sum_epilogue(
                 tmem_base + ((uint32_t)(quarter * 32) << 16), BN, (warp - 2) / 4 * 128,
                 (kb1 - kb0 + pr.sub_kb - 1) / pr.sub_kb, it,
@@ -946,14 +978,14 @@ inline void set_split(Problem &pr, int ksplit, int kb_range, int sub_kb) {
   pr.sub_kb = sub_kb > 0 ? sub_kb : (pr.kb_per_split > 0 ? pr.kb_per_split : 1);
 }
 
-template <int KIND, int BN, int STAGES, class Epi, int NACC = 1, bool SUM = false>
+template <int KIND, int BN, int STAGES, class Epi, int NACC = 1, bool SUM = false, int TERMS = 1>
 int launch(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, long long kelems,
            int nbatch, const Epi &epi, int sm_count, int *derr, cudaStream_t s,
            const char *prof_name, int max_ctas = 0, const int *nbatch_dev = nullptr,
            int ksplit = 1, int seg_kb = 0, unsigned seg_x = 0, unsigned seg_y = 0,
            int kb_range = 0, int sub_kb = 0) {
   if (NACC > 1 && (ksplit > 1 || nbatch != NACC || nbatch_dev)) return B2_ERR_ARG;
-  using L = SmemLayout<BN, STAGES>;
+  using L = SmemLayout<BN, STAGES, TERMS>;
   Problem pr;
   pr.P = P;
   pr.Q = Q;
@@ -974,12 +1006,27 @@ int launch(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, long lo
   if (total <= 0 || (NACC > 1 && pr.kblocks <= 0)) return B2_OK;
   int grid = (int)(total < sm_count ? total : sm_count);
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  auto kern = umma_gemm_kernel<KIND, BN, STAGES, Epi, NACC, SUM>;
+  auto kern = umma_gemm_kernel<KIND, BN, STAGES, Epi, NACC, SUM, TERMS>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
   if (e != cudaSuccess) return cuda_fail(e, "umma smem attribute");
   B2_PROF(prof_name, s);
-  kern<<<grid, threads_for(BN, SUM), L::TOTAL, s>>>(tmX, tmY, pr, epi);
-  e = cudaGetLastError();
+  if constexpr (SUM) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(threads_for(BN, SUM));
+    cfg.dynamicSmemBytes = L::TOTAL;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, kern, tmX, tmY, pr, epi);
+    if (e == cudaSuccess) e = cudaGetLastError();
+  } else {
+    kern<<<grid, threads_for(BN, SUM), L::TOTAL, s>>>(tmX, tmY, pr, epi);
+    e = cudaGetLastError();
+  }
   if (e != cudaSuccess) return cuda_fail(e, prof_name);
   return B2_OK;
 }
@@ -987,13 +1034,12 @@ int launch(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, long lo
 // Pair launch: clusters of 2 CTAs, one pair per two SMs (as many pairs as can
 // be resident at once, queried once per device), tiles of 256 X rows x BN Y
 // rows.  tmX must have a 128-row box and tmY a BN/2-row box.
-template <int KIND, int BN, int STAGES, class Epi, bool SUM = false>
+template <int KIND, int BN, int STAGES, class Epi, bool SUM = false, int TERMS = 1>
 int launch_pair(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, long long kelems,
                 int nbatch, const Epi &epi, int device, int *derr, cudaStream_t s,
                 const char *prof_name, const int *nbatch_dev = nullptr, int ksplit = 1,
-                int seg_kb = 0, unsigned seg_x = 0, unsigned seg_y = 0, int kb_range = 0,
-                int sub_kb = 0) {
-  using L = SmemLayout<BN / 2, STAGES>;
+                int seg_kb = 0, int kb_range = 0, int sub_kb = 0) {
+  using L = SmemLayout<BN / 2, STAGES, TERMS>;
   Problem pr;
   pr.P = P;
   pr.Q = Q;
@@ -1001,8 +1047,7 @@ int launch_pair(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, lo
   pr.nbatch = nbatch;
   pr.nbatch_dev = nbatch_dev;
   pr.seg_kb = seg_kb;
-  pr.seg_x = seg_x;
-  pr.seg_y = seg_y;
+  pr.seg_x = pr.seg_y = 0;
   set_split(pr, ksplit, kb_range, SUM ? sub_kb : 0);
   pr.tiles_p = (P + PAIR_BM - 1) / PAIR_BM;
   pr.tiles_q = (Q + BN - 1) / BN;
@@ -1011,9 +1056,9 @@ int launch_pair(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, lo
   launch_wait_settings(&pr.wait_ns, &pr.withhold);
   const long long total = (long long)pr.tiles_p * pr.tiles_q * nbatch * pr.ksplit;
   if (total <= 0) return B2_OK;
-  auto kern = umma_gemm_pair_kernel<KIND, BN, STAGES, Epi, SUM>;
+  auto kern = umma_gemm_pair_kernel<KIND, BN, STAGES, Epi, SUM, TERMS>;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -1021,8 +1066,10 @@ int launch_pair(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, lo
   cfg.blockDim = dim3(threads_for(BN, SUM));
   cfg.dynamicSmemBytes = L::TOTAL;
   cfg.stream = s;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = SUM ? 2 : 1;
   static std::atomic<int> resident_pairs[64];  // per device, filled on first use (0 = unknown)
   const int dslot = device >= 0 && device < 64 ? device : 0;
   if (resident_pairs[dslot].load() == 0) {
