@@ -281,10 +281,13 @@ inline long long round_up(long long x, long long a) { return (x + a - 1) / a * a
 // Work units of a product whose K is accumulated in S ranges of kbps blocks:
 // each unit takes `per` consecutive ranges of its tile (adding them in its
 // epilogue), so that ceil(S / per) partials per tile go through memory.
-// Modelled time (us): waves of units at t_kb per K block (measured MMA rate of
-// the engine) and 3 us of fill and epilogue, plus the partials written and read
-// at about 4 TB/s and a second launch.  2048^3 3xTF32 (64 pair tiles on 74
-// pairs, 8 ranges): one unit per tile instead of 8 partials of 16.8 MB.
+// Modelled time (us): waves of units, each 3 us of fill and final epilogue and,
+// per range, t_kb per K block (measured MMA rate of the engine) but at least
+// the 1.1 us that adding an accumulator to the sums takes (8 ranges of one K
+// block each: 512^3 11.7 us in one unit per tile, 6.6 in several); plus the
+// partials written and read at about 6 TB/s and a second launch.  2048^3
+// 3xTF32 (64 pair tiles on 74 pairs, 8 ranges): one unit per tile instead of 8
+// partials of 16.8 MB.
 int ranges_per_unit(long long tiles, int S, int kbps, int kblocks, int slots, double t_kb, int m,
                     int n) {
   int best = S;
@@ -294,8 +297,9 @@ int ranges_per_unit(long long tiles, int S, int kbps, int kblocks, int slots, do
     if (per > 1 && (S + per - 2) / (per - 1) == E) continue;  // more even with per - 1
     const long long waves = (tiles * E + slots - 1) / slots;
     const int kb = per * kbps < kblocks ? per * kbps : kblocks;
-    double us = (double)waves * (kb * t_kb + 3.0);
-    if (E > 1) us += 3.0 + (double)E * m * n * 8.0 / 4e6;
+    const double work = kb * t_kb, drains = 1.1 * ((kb + kbps - 1) / kbps);
+    double us = (double)waves * ((work > drains ? work : drains) + 3.0);
+    if (E > 1) us += 2.0 + (double)E * m * n * 8.0 / 6e6;
     if (us < best_us) best_us = us, best = per;
   }
   return best;
