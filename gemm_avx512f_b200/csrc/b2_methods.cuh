@@ -84,6 +84,11 @@ int sgemm_split_tf32x3(const float *X, long long sr, long long sk, int R, int K,
 int sgemm_splitk_reduce(const float *W, long long plane, int ldw, int S, int m, int n,
                         float alpha, float beta, float *C, int ldc, cudaStream_t s);
 
+// cgemm3m as one batch of three 3xTF32 products (sgemm_tc.cu).
+int cgemm3m_tensor(char ta, char tb, int m, int n, int k, float ar, float ai, float br, float bi,
+                   const float *A, int lda, const float *B, int ldb, float *C, int ldc,
+                   cudaStream_t s);
+
 // Blocked triangular solve (trsm.cu).
 int dtrsm_device(char side, char uplo, char transa, char diag, int m, int n, double alpha,
                  const double *A, int lda, double *B, int ldb, int method, int block,

@@ -3,8 +3,8 @@
 // zgemm3m runs in ONE fused launch (zgemm3m_dmma_kernel, FP64 DMMA) below 2^35
 // multiply-adds and as three FP64 DMMA GEMMs between a pre-add pass and a
 // combine pass above; cgemm3m runs in one fused FFMA launch below 2^24
-// multiply-adds and otherwise as three 3xTF32 tensor-core GEMMs
-// (gemm3m_three_gemms, at the end).
+// multiply-adds and otherwise as a batch of three 3xTF32 tensor-core products
+// (cgemm3m_tensor, sgemm_tc.cu).
 //
 // Replaces the OpenBLAS gemm3m driver + the reference's 3M kernels
 // (zgemm3m_kernel_2x8_skylakex.c:336-351, zgemm3m_kernel_8x4_skylakex.c:309-334,
@@ -510,14 +510,13 @@ __global__ void combine3m_kernel(const T *__restrict__ P, long long plane, int M
   }
 }
 
-// Products of at least 2^24 multiply-adds: the three real products run as
-// the library's own GEMMs (FP64 DMMA for zgemm3m; 3xTF32 tensor-core SGEMM,
-// FP32-class accuracy, for cgemm3m) between one pre-add pass and one
-// post-combination pass -- both HBM-bound -- instead of the fused tile kernel,
-// whose in-register pre-adds cap it below the plain GEMMs' rate.
-template <typename T>
-int gemm3m_three_gemms(char ta, char tb, int m, int n, int k, T ar, T ai, T br, T bi,
-                       const T *A, int lda, const T *B, int ldb, T *C, int ldc, cudaStream_t s) {
+// Large zgemm3m products: the three real products run as the library's own
+// FP64 DMMA GEMMs between one pre-add pass and one post-combination pass --
+// both HBM-bound.  (cgemm3m: cgemm3m_tensor.)
+int zgemm3m_three_gemms(char ta, char tb, int m, int n, int k, double ar, double ai, double br,
+                        double bi, const double *A, int lda, const double *B, int ldb, double *C,
+                        int ldc, cudaStream_t s) {
+  using T = double;
   Ctx *cx = ctx();
   if (!cx) return B2_ERR_NO_DEVICE;
   const bool tA = !(ta == 'N' || ta == 'n' || ta == 'R' || ta == 'r');
@@ -542,12 +541,8 @@ int gemm3m_three_gemms(char ta, char tb, int m, int n, int k, T ar, T ai, T br, 
   B2_CUDA_TRY(cudaMemsetAsync(P, 0, (size_t)(3 * pc) * sizeof(T), s));
   const T *X[3] = {Ar, Ai, As}, *Y[3] = {Br, Bi, Bs};
   for (int t = 0; t < 3; ++t) {
-    int st;
-    if constexpr (sizeof(T) == 8)
-      st = dgemm_fp64('N', 'N', m, n, k, 1.0, X[t], m, Y[t], k, 0.0, P + t * pc, m, s, nullptr);
-    else
-      st = sgemm_dispatch('N', 'N', m, n, k, 1.0f, X[t], m, Y[t], k, 0.0f, P + t * pc, m,
-                          B2_METHOD_TF32X3, s);
+    const int st =
+        dgemm_fp64('N', 'N', m, n, k, 1.0, X[t], m, Y[t], k, 0.0, P + t * pc, m, s, nullptr);
     if (st != B2_OK) return st;
   }
   B2_PROF("gemm3m_combine", s);
@@ -697,7 +692,10 @@ int gemm3m_device(char ta, char tb, int m, int n, int k, const T *alpha, const T
       if (fused_on && cx && tiles >= cx->sm_count)
         return cgemm3m_fused_tc(ta, tb, m, n, k, ar, ai, br, bi, A, lda, B, ldb, C, ldc, s);
     }
-    return gemm3m_three_gemms<T>(ta, tb, m, n, k, ar, ai, br, bi, A, lda, B, ldb, C, ldc, s);
+    if constexpr (sizeof(T) == 4)
+      return cgemm3m_tensor(ta, tb, m, n, k, ar, ai, br, bi, A, lda, B, ldb, C, ldc, s);
+    else
+      return zgemm3m_three_gemms(ta, tb, m, n, k, ar, ai, br, bi, A, lda, B, ldb, C, ldc, s);
   }
   dim3 grid((m + G_BM - 1) / G_BM, (n + G_BN - 1) / G_BN);
   const int smem = (int)(12 * G_BK * G_LD * sizeof(T));

@@ -305,6 +305,65 @@ int ranges_per_unit(long long tiles, int S, int kbps, int kblocks, int slots, do
   return best;
 }
 
+// Partials per tile, K blocks per unit and K blocks per accumulated range.
+struct Ranges {
+  int E, unit_kb, range_kb;
+};
+
+// One SGEMM product (or nbatch of them) on engine `eng` (see SgCfg).
+template <class Epi>
+int run_engine(int eng, bool bf16, int terms, const CUtensorMap &tmX, const CUtensorMap &tmY, int m,
+               int n, int kp, int nbatch, int seg_kb, const Ranges &rg, const Epi &epi, Ctx *cx,
+               cudaStream_t s) {
+  const char *nm = bf16 ? "sgemm_umma_bf16" : "sgemm_umma_tf32";
+  // TERMS = 3 stages hold four operand tiles: 64 KB (pair and 128x128), 96 KB
+  auto pair = [&](auto kd, auto t3) {
+    constexpr int T = decltype(t3)::value;
+    return umma::launch_pair<decltype(kd)::value, 256, T == 3 ? 3 : 6, Epi, true, T>(
+        tmX, tmY, m, n, kp, nbatch, epi, cx->device, cx->derr, s, nm, nullptr, rg.E, seg_kb,
+        rg.unit_kb, rg.range_kb);
+  };
+  auto single = [&](auto kd, auto bn, auto t3) {
+    constexpr int T = decltype(t3)::value, BN = decltype(bn)::value;
+    constexpr int ST = BN == 256 ? (T == 3 ? 2 : 4) : (T == 3 ? 3 : 6);
+    return umma::launch<decltype(kd)::value, BN, ST, Epi, 1, true, T>(
+        tmX, tmY, m, n, kp, nbatch, epi, cx->sm_count, cx->derr, s, nm, 0, nullptr, rg.E, seg_kb, 0,
+        0, rg.unit_kb, rg.range_kb);
+  };
+  using BF = std::integral_constant<int, umma::KIND_BF16>;
+  using TF = std::integral_constant<int, umma::KIND_TF32>;
+  using I1 = std::integral_constant<int, 1>;
+  using I3 = std::integral_constant<int, 3>;
+  using I128 = std::integral_constant<int, 128>;
+  using I256 = std::integral_constant<int, 256>;
+  if (eng == 2) return bf16 ? pair(BF{}, I3{}) : terms == 3 ? pair(TF{}, I3{}) : pair(TF{}, I1{});
+  if (eng == 1)
+    return bf16         ? single(BF{}, I128{}, I3{})
+           : terms == 3 ? single(TF{}, I128{}, I3{})
+                        : single(TF{}, I128{}, I1{});
+  return bf16         ? single(BF{}, I256{}, I3{})
+         : terms == 3 ? single(TF{}, I256{}, I3{})
+                      : single(TF{}, I256{}, I1{});
+}
+
+// Launch as a programmatic dependent of the kernel before it in the stream
+// (the kernel waits for that one's writes with griddepcontrol.wait).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_dependent(void (*kern)(KArgs...), unsigned blocks, int threads, cudaStream_t s,
+                             Args... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(blocks);
+  lc.blockDim = dim3((unsigned)threads);
+  lc.stream = s;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&lc, kern, args...);
+  return e != cudaSuccess ? e : cudaGetLastError();
+}
+
 SplitOp split_op(const float *X, long long sr, long long sk, int R, void *out) {
   SplitOp o;
   o.X = X;
@@ -322,21 +381,189 @@ int run_split(const SplitOp &a, const SplitOp &b, int K, int kp, int segs, cudaS
   const unsigned kt = (unsigned)(kp + 63) / 64;
   const unsigned ba = kt * ((unsigned)(a.R + 63) / 64), bb = kt * ((unsigned)(b.R + 63) / 64);
   B2_PROF("sgemm_split", s);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3(ba + bb);
-  lc.blockDim = dim3(256);
-  lc.stream = s;
-  lc.attrs = attr;
-  lc.numAttrs = 1;
-  B2_CUDA_TRY(cudaLaunchKernelEx(&lc, split_kernel<T>, a, b, ba, K, kp, segs));
-  B2_CUDA_TRY(cudaGetLastError());
+  B2_CUDA_TRY(launch_dependent(split_kernel<T>, ba + bb, 256, s, a, b, ba, K, kp, segs));
   return B2_OK;
 }
 
+// ------------------------------------------------- complex64 3M products --
+// One complex operand of a 3M product: R rows of K complex elements, element
+// (r, k) at complex index r + k*ld (rowcont) or r*ld + k; sgn = -1 conjugates.
+struct Split3Op {
+  const float *X;
+  long long ld;
+  int R, rowcont, pairs;  // pairs: 8-byte loads are legal
+  float sgn;
+  float *out;
+};
+
+// Writes the real part, the imaginary part and their sum of every row of both
+// operands as [big | small] TF32 segments: out[t][r][2*kp], t = 0, 1, 2 (the
+// operands of P1, P2, P3).  One block turns 64 rows x 32 k around.
+// Bound: HBM, 8 bytes read and 24 written per element.  The pre-adds and the
+// splits were passes of their own (20 + 36 bytes per element): 110 -> 31 us at
+// 1900x1300x2100 on B200, the whole product 367 -> 199.
+__global__ void __launch_bounds__(256)
+    split3m_kernel(const Split3Op a, const Split3Op b, unsigned blocks_a, int K, int kp) {
+  __shared__ float tr[64][33], ti[64][33];
+  umma::grid_dependency_wait();
+  const bool second = blockIdx.x >= blocks_a;
+  const float *X = second ? b.X : a.X;
+  const long long ld = second ? b.ld : a.ld;
+  const int R = second ? b.R : a.R;
+  const bool rowcont = second ? b.rowcont : a.rowcont, pairs = second ? b.pairs : a.pairs;
+  const float sgn = second ? b.sgn : a.sgn;
+  float *out = second ? b.out : a.out;
+  const unsigned id = second ? blockIdx.x - blocks_a : blockIdx.x;
+  const unsigned kt = (unsigned)kp / 32, rt = (unsigned)(R + 63) / 64;
+  const int r0 = (int)(rowcont ? id % rt : id / kt) * 64;
+  const int k0 = (int)(rowcont ? id / rt : id % kt) * 32;
+  const int tid = threadIdx.x;
+  float2 v[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int idx = tid + 256 * e;
+    const int rr = rowcont ? idx & 63 : idx >> 5, kk = rowcont ? idx >> 6 : idx & 31;
+    const int r = r0 + rr, k = k0 + kk;
+    v[e] = make_float2(0.f, 0.f);
+    if (r < R && k < K) {
+      const float *p = X + 2 * (rowcont ? r + k * ld : r * ld + k);
+      if (pairs) v[e] = __ldg(reinterpret_cast<const float2 *>(p));
+      else v[e] = make_float2(__ldg(p), __ldg(p + 1));
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int idx = tid + 256 * e;
+    const int rr = rowcont ? idx & 63 : idx >> 5, kk = rowcont ? idx >> 6 : idx & 31;
+    tr[rr][kk] = v[e].x;
+    ti[rr][kk] = sgn * v[e].y;
+  }
+  __syncthreads();
+  const long long plane = (long long)R * 2 * kp;
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int idx = tid + 256 * e, rr = idx >> 3, kl = (idx & 7) * 4;
+    const int r = r0 + rr;
+    if (r >= R) continue;
+    float *dst = out + (long long)r * 2 * kp + k0 + kl;
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+      float big[4], small[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float re = tr[rr][kl + j], im = ti[rr][kl + j];
+        const float x = t == 0 ? re : t == 1 ? im : re + im;
+        big[j] = tf32_round(x);
+        small[j] = tf32_round(x - big[j]);
+      }
+      *reinterpret_cast<float4 *>(dst + t * plane) = make_float4(big[0], big[1], big[2], big[3]);
+      *reinterpret_cast<float4 *>(dst + t * plane + kp) =
+          make_float4(small[0], small[1], small[2], small[3]);
+    }
+  }
+}
+
+// C = alpha (P1 - P2 + i (P3 - P1 - P2)) + beta C from the E partials of each
+// product (plane t*E + e of W), summed in FP64 and rounded once.
+__global__ void __launch_bounds__(256)
+    combine3m_tc_kernel(const float *__restrict__ W, long long plane, int ldw, int E, int M, int N,
+                        float ar, float ai, float br, float bi, float *__restrict__ C, int ldc) {
+  umma::grid_dependency_wait();
+  const bool beta_one = br == 1.f && bi == 0.f;
+  const unsigned long long total = (unsigned long long)(unsigned)M * (unsigned)N;
+  for (unsigned long long i = blockIdx.x * 256ull + threadIdx.x; i < total;
+       i += gridDim.x * 256ull) {
+    const int n = (int)(i / (unsigned)M), m = (int)(i - (unsigned long long)n * (unsigned)M);
+    const float *w = W + (long long)n * ldw + m;
+    float *c = C + 2 * ((long long)n * ldc + m);
+    float cr = c[0], ci = c[1], p[3];
+    if (E == 1) {
+#pragma unroll
+      for (int t = 0; t < 3; ++t) p[t] = w[t * plane];
+    } else {
+      double acc[3] = {0.0, 0.0, 0.0};
+      for (int e = 0; e < E; ++e)
+#pragma unroll
+        for (int t = 0; t < 3; ++t) acc[t] += (double)w[(t * E + e) * plane];
+#pragma unroll
+      for (int t = 0; t < 3; ++t) p[t] = (float)acc[t];
+    }
+    const float re = p[0] - p[1], im = p[2] - p[0] - p[1];
+    if (!beta_one) {
+      const float tr = br * cr - bi * ci, ti = br * ci + bi * cr;
+      cr = tr;
+      ci = ti;
+    }
+    c[0] = cr + (ar * re - ai * im);
+    c[1] = ci + (ar * im + ai * re);
+  }
+}
+
+Split3Op split3_op(const float *X, int ld, bool rowcont, bool conj, int R, float *out) {
+  return Split3Op{X, ld, R, rowcont ? 1 : 0, ((uintptr_t)X & 7) == 0 ? 1 : 0, conj ? -1.f : 1.f,
+                  out};
+}
+
 }  // namespace
+
+// cgemm3m on the tensor cores in three launches: one pass writes the three
+// products' split operands, one GEMM launch runs P1, P2 and P3 (3xTF32) as a
+// batch, one pass combines them into C.
+int cgemm3m_tensor(char ta, char tb, int m, int n, int k, float ar, float ai, float br, float bi,
+                   const float *A, int lda, const float *B, int ldb, float *C, int ldc,
+                   cudaStream_t s) {
+  Ctx *cx = ctx();
+  if (!cx) return B2_ERR_NO_DEVICE;
+  const bool tA = !(ta == 'N' || ta == 'n' || ta == 'R' || ta == 'r');
+  const bool tB = !(tb == 'N' || tb == 'n' || tb == 'R' || tb == 'r');
+  const bool cA = ta == 'C' || ta == 'c' || ta == 'R' || ta == 'r';
+  const bool cB = tb == 'C' || tb == 'c' || tb == 'R' || tb == 'r';
+  const int kp = (int)round_up(k, 32);
+  const long long ks = 2LL * kp;
+  float *Xp = (float *)workspace(cx, WS_SPLIT_X, (size_t)(3 * m * ks) * sizeof(float));
+  float *Yp = (float *)workspace(cx, WS_SPLIT_Y, (size_t)(3 * n * ks) * sizeof(float));
+  if (!Xp || !Yp) return B2_ERR_NOMEM;
+  {
+    const unsigned kt = (unsigned)kp / 32;
+    const unsigned ba = kt * ((unsigned)(m + 63) / 64), bb = kt * ((unsigned)(n + 63) / 64);
+    B2_PROF("gemm3m_prep", s);
+    B2_CUDA_TRY(launch_dependent(split3m_kernel, ba + bb, 256, s, split3_op(A, lda, !tA, cA, m, Xp),
+                                 split3_op(B, ldb, tB, cB, n, Yp), ba, k, kp));
+  }
+  // engine and K ranges as for one 3xTF32 SGEMM of this shape
+  const SgCfg cfg = sgemm_pick_cfg('N', 'N', m, n, k, 1, B2_METHOD_TF32X3);
+  const int eng = (cfg.engine >= 0 && cfg.engine <= 2) ? cfg.engine : 0;
+  const int tile_p = eng == 2 ? 256 : umma::BM, tile_q = eng == 1 ? 128 : 256;
+  CUtensorMap tmX, tmY;
+  int rc = umma::make_kmajor_map(&tmX, umma::KIND_TF32, Xp, ks, m, 3, ks * 4, (long long)m * ks * 4,
+                                 umma::BM);
+  if (rc == B2_OK)
+    rc = umma::make_kmajor_map(&tmY, umma::KIND_TF32, Yp, ks, n, 3, ks * 4, (long long)n * ks * 4,
+                               eng == 0 ? 256 : 128);
+  if (rc != B2_OK) return rc;
+  const int seg_kb = kp * 4 / umma::KBLOCK_BYTES, kblocks = seg_kb;
+  const long long tiles = ((n + tile_q - 1) / tile_q) * (long long)((m + tile_p - 1) / tile_p);
+  const int slots = eng == 2 ? cx->sm_count / 2 : cx->sm_count;
+  int S = cfg.split > 0 ? cfg.split : choose_ksplit(tiles, 3 * kblocks, slots);
+  if (S > kblocks) S = kblocks;
+  const int kbps = (kblocks + S - 1) / S;
+  S = (kblocks + kbps - 1) / kbps;
+  const int per =
+      ranges_per_unit(3 * tiles, S, kbps, kblocks, slots, 3 * (eng == 1 ? 0.17 : 0.28), m, 3 * n);
+  const int E = (S + per - 1) / per;
+  const int ldw = (int)round_up(m, 32);
+  const long long plane = (long long)n * ldw;
+  float *W = (float *)workspace(cx, WS_3M, (size_t)plane * 3 * E * sizeof(float));
+  if (!W) return B2_ERR_NOMEM;
+  rc = run_engine(eng, false, 3, tmX, tmY, m, n, kp, 3, seg_kb, Ranges{E, per * kbps, kbps},
+                  F32PartialEpi{W, plane, ldw, m, n}, cx, s);
+  if (rc != B2_OK) return rc;
+  const long long blocks = ((long long)m * n + 255) / 256;
+  B2_PROF("gemm3m_combine", s);
+  B2_CUDA_TRY(launch_dependent(combine3m_tc_kernel, (unsigned)(blocks < 2368 ? blocks : 2368), 256,
+                               s, (const float *)W, plane, ldw, E, m, n, ar, ai, br, bi, C, ldc));
+  return B2_OK;
+}
 
 int sgemm_split_tf32x3(const float *X, long long sr, long long sk, int R, int K, int kp,
                        float *out, cudaStream_t s) {
@@ -420,45 +647,17 @@ int sgemm_tensor_cfg(char ta, char tb, int m, int n, int k, float alpha, const f
   const int per =
       ranges_per_unit(tiles, S, kbps, kblocks, slots, terms * (eng == 1 ? 0.17 : 0.28), m, n);
   const int E = (S + per - 1) / per;  // partials per tile
-  auto run = [&](auto epi) -> int {
-    using Epi = decltype(epi);
-    const char *nm = bf16 ? "sgemm_umma_bf16" : "sgemm_umma_tf32";
-    const int kbr = per * kbps;
-    // TERMS = 3 stages hold four operand tiles: 64 KB (pair and 128x128), 96 KB
-    auto pair = [&](auto kd, auto t3) {
-      constexpr int T = decltype(t3)::value;
-      return umma::launch_pair<decltype(kd)::value, 256, T == 3 ? 3 : 6, Epi, true, T>(
-          tmX, tmY, m, n, kp, 1, epi, cx->device, cx->derr, s, nm, nullptr, E, seg_kb, kbr, kbps);
-    };
-    auto single = [&](auto kd, auto bn, auto t3) {
-      constexpr int T = decltype(t3)::value, BN = decltype(bn)::value;
-      constexpr int ST = BN == 256 ? (T == 3 ? 2 : 4) : (T == 3 ? 3 : 6);
-      return umma::launch<decltype(kd)::value, BN, ST, Epi, 1, true, T>(
-          tmX, tmY, m, n, kp, 1, epi, cx->sm_count, cx->derr, s, nm, 0, nullptr, E, seg_kb, 0, 0,
-          kbr, kbps);
-    };
-    using BF = std::integral_constant<int, umma::KIND_BF16>;
-    using TF = std::integral_constant<int, umma::KIND_TF32>;
-    using I1 = std::integral_constant<int, 1>;
-    using I3 = std::integral_constant<int, 3>;
-    using I128 = std::integral_constant<int, 128>;
-    using I256 = std::integral_constant<int, 256>;
-    if (eng == 2) return bf16 ? pair(BF{}, I3{}) : terms == 3 ? pair(TF{}, I3{}) : pair(TF{}, I1{});
-    if (eng == 1)
-      return bf16         ? single(BF{}, I128{}, I3{})
-             : terms == 3 ? single(TF{}, I128{}, I3{})
-                          : single(TF{}, I128{}, I1{});
-    return bf16         ? single(BF{}, I256{}, I3{})
-           : terms == 3 ? single(TF{}, I256{}, I3{})
-                        : single(TF{}, I256{}, I1{});
-  };
-  if (E == 1) return run(F32Epi{C, ldc, m, n, alpha, beta});
+  const Ranges rg{E, per * kbps, kbps};
+  if (E == 1)
+    return run_engine(eng, bf16, terms, tmX, tmY, m, n, kp, 1, seg_kb, rg,
+                      F32Epi{C, ldc, m, n, alpha, beta}, cx, s);
   // E partial products of K ranges, then one fixed-order reduction.
   const int ldw = (int)round_up(m, 32);
   const long long plane = (long long)n * ldw;
   float *W = (float *)workspace(cx, WS_MISC, (size_t)plane * E * sizeof(float));
   if (!W) return B2_ERR_NOMEM;
-  rc = run(F32PartialEpi{W, plane, ldw, m, n});
+  rc = run_engine(eng, bf16, terms, tmX, tmY, m, n, kp, 1, seg_kb, rg,
+                  F32PartialEpi{W, plane, ldw, m, n}, cx, s);
   if (rc != B2_OK) return rc;
   return sgemm_splitk_reduce(W, plane, ldw, E, m, n, alpha, beta, C, ldc, s);
 }
@@ -466,19 +665,10 @@ int sgemm_tensor_cfg(char ta, char tb, int m, int n, int k, float alpha, const f
 int sgemm_splitk_reduce(const float *W, long long plane, int ldw, int S, int m, int n,
                         float alpha, float beta, float *C, int ldc, cudaStream_t s) {
   const long long blocks = ((long long)((m + 3) / 4) * n + 255) / 256;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3((unsigned)(blocks < 1184 ? blocks : 1184));  // 8 blocks on each of 148 SMs
-  lc.blockDim = dim3(256);
-  lc.stream = s;
-  lc.attrs = attr;
-  lc.numAttrs = 1;
   B2_PROF("sgemm_splitk_reduce", s);
-  B2_CUDA_TRY(cudaLaunchKernelEx(&lc, sgemm_splitk_reduce_kernel, W, plane, ldw, S, m, n, alpha,
-                                 beta, C, ldc));
-  B2_CUDA_TRY(cudaGetLastError());
+  // 8 blocks on each of 148 SMs
+  B2_CUDA_TRY(launch_dependent(sgemm_splitk_reduce_kernel, (unsigned)(blocks < 1184 ? blocks : 1184),
+                               256, s, W, plane, ldw, S, m, n, alpha, beta, C, ldc));
   return B2_OK;
 }
 
