@@ -17,8 +17,9 @@ namespace {
 // Paired-FMA FP32 kernel (sm_100 fma.rn.f32x2: two FP32 FMAs per issued
 // instruction, so the FFMA pipe, not instruction issue, is the limit).
 // CTA tile 128 x 128, K blocks of 16, 256 threads of 8 x 8 outputs, K panels
-// staged through registers (16-byte global loads when the layout allows)
-// into double-buffered shared memory.  Thread (tx, ty) owns rows
+// copied by cp.async through a 3-deep ring as [k][m] and [k][n] (16 bytes at a
+// time where the operand is contiguous that way and aligned, else 4: a panel
+// staged through registers needs 16 of the 128, which spilled).  Thread (tx, ty) owns rows
 // 4 tx + {0..3} + 64 h' and columns 4 ty + {0..3} + 64 h (h', h = 0, 1): per
 // K step it reads two 16-byte A vectors and two 16-byte B vectors (64 bytes
 // for 64 FMAs -- the shared-memory rate of 128 bytes per clock per SM then
@@ -31,7 +32,9 @@ namespace {
 constexpr int S2_M = 128, S2_N = 128, S2_K = 16, S2_APAD = 4, S2_BPAD = 4;
 constexpr int S2_ALD = S2_M + S2_APAD;  // floats per k row of the A panel
 constexpr int S2_BLD = S2_N + S2_BPAD;
-constexpr int S2_SMEM = (2 * S2_K * S2_ALD + 2 * S2_K * S2_BLD) * 4;
+constexpr int S2_STAGES = 3;
+constexpr int S2_STAGE = S2_K * (S2_ALD + S2_BLD);  // floats per stage: A panel, B panel
+constexpr int S2_SMEM = S2_STAGES * S2_STAGE * 4;
 
 __device__ __forceinline__ unsigned long long dup2(float a) {
   unsigned long long d;
@@ -44,51 +47,106 @@ __device__ __forceinline__ void ffma2(unsigned long long &c, unsigned long long 
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
 }
 
-// Four consecutive floats starting at p (16-byte aligned when VEC), or fewer
-// at the matrix edge (lim = elements available from p), zero beyond.
-template <bool VEC>
-__device__ __forceinline__ float4 load4(const float *p, int lim) {
-  if (VEC && lim >= 4) return __ldg(reinterpret_cast<const float4 *>(p));
-  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (lim > 0) v.x = p[0];
-  if (lim > 1) v.y = p[1];
-  if (lim > 2) v.z = p[2];
-  if (lim > 3) v.w = p[3];
-  return v;
+// `bytes` (0 .. 4 or 16) of one copy, the rest of it zero.
+__device__ __forceinline__ void copy16(uint32_t dst, const float *src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
+}
+__device__ __forceinline__ void copy4(uint32_t dst, const float *src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
 }
 
-template <bool TA, bool TB, bool VEC, bool SPLIT>
+// Place of element (k, o) of a K-contiguous operand's panel.  From k = 8 on the
+// pairs of a group of four outer indices are swapped: the stores of 16 k x 2 o
+// then fall on 32 different banks (4 k + o repeats from k = 8), and a 16-byte
+// read of a group only has its halves exchanged.
+__device__ __forceinline__ int panel_at(int k, int o) { return k * S2_ALD + (o ^ ((k >> 3) << 1)); }
+
+// One 16 x 128 panel of an operand into shared memory as [k][S2_ALD]: outer
+// index o = o0 .. o0 + 127 (zero from olim on), k = k0 .. k0 + 15 (zero from
+// klim on).  KCONT: element (o, k) at g[o*ld + k] (placed by panel_at), else
+// g[k*ld + o].
+template <bool KCONT, bool VEC>
+__device__ __forceinline__ void load_panel(uint32_t dst, const float *__restrict__ g, int ld,
+                                           int o0, int k0, int olim, int klim, int tid) {
+  if constexpr (KCONT) {
+    // a warp: 16 k of 2 outer indices, stored to 32 banks (see panel_at)
+    const int k = tid & 15, o = tid >> 4;
+    const float *p = g + (size_t)(o0 + o) * ld + (k0 + k);
+    const bool kin = k0 + k < klim;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const bool in = kin && o0 + o + 16 * e < olim;
+      copy4(dst + (uint32_t)panel_at(k, o + 16 * e) * 4u, in ? p + (size_t)(16 * e) * ld : g,
+            in ? 4 : 0);
+    }
+  } else {
+    const int k = tid >> 5, o = (tid & 31) * 4;
+    const float *p = g + (size_t)(k0 + k) * ld + (o0 + o);
+    const int left = olim - (o0 + o);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int have = k0 + k + 8 * h < klim ? left : 0;
+      const uint32_t d = dst + (uint32_t)((k + 8 * h) * S2_ALD + o) * 4u;
+      const float *q = p + (size_t)(8 * h) * ld;
+      if constexpr (VEC) {
+        copy16(d, have > 0 ? q : g, have >= 4 ? 16 : have > 0 ? 4 * have : 0);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) copy4(d + 4u * e, have > e ? q + e : g, have > e ? 4 : 0);
+      }
+    }
+  }
+}
+
+// The same panel when it lies wholly inside the operand: from the thread's
+// running pointer (element (o0 + o, k0 + k) of the map above), `step` = ld times
+// the distance between its copies.
+template <bool KCONT, bool VEC>
+__device__ __forceinline__ void run_panel(uint32_t dst, const float *p, size_t step) {
+  if constexpr (KCONT) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst + 64u * e), "l"(p));
+      p += step;
+    }
+  } else {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t d = dst + (uint32_t)(8 * h * S2_ALD) * 4u;
+      if constexpr (VEC) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(p));
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d + 4u * e), "l"(p + e));
+      }
+      p += step;
+    }
+  }
+}
+
+// MODE 0: tiles [tile0, tile0 + gridDim.x) of C in full; MODE 1: K slice
+// blockIdx.z of a split-K product, its raw sums to P + z*plane (ld ldp); MODE 2:
+// K slice blockIdx.z of tile tile0 + blockIdx.x, the raw sums of its 128 x 128
+// outputs to P + (z*gridDim.x + blockIdx.x)*128*128.  Tiles run down the columns.
+// dependents: the launch after this one (MODE 2, other tiles) may start as these
+// blocks leave.
+template <bool TA, bool TB, bool VEC, int MODE>
 __global__ void __launch_bounds__(256, 2)
     sgemm_ffma2_kernel(int M, int N, int K, float alpha, const float *__restrict__ A, int lda,
                        const float *__restrict__ B, int ldb, float beta, float *__restrict__ C,
-                       int ldc, int kchunk, float *__restrict__ P, long long plane, int ldp) {
-  // Slice blockIdx.z of a split-K launch reads its own K range: either the
-  // operand bases shift to it and K shortens (SHIFT), or K stays and kbeg /
-  // kend bound the range.  The form per transpose pair is the one ptxas
-  // compiles with the fewest spilled registers (NN shifts by 64-bit offsets).
-  constexpr bool SHIFT = SPLIT && (TA || !TB);
-  if (SHIFT) {
-    if (TA) {
-      const int kb = blockIdx.z * kchunk;
-      A += (size_t)kb;
-      B += TB ? (size_t)kb * ldb : (size_t)kb;
-      K = min(kchunk, K - kb);
-    } else {
-      const long long kb = (long long)blockIdx.z * kchunk;
-      A += kb * lda;
-      B += kb;
-      K = min(kchunk, K - (int)kb);
-    }
-  }
-  extern __shared__ __align__(16) float s2mem[];
-  float *As = s2mem;                        // [2][S2_K][S2_ALD]
-  float *Bs = s2mem + 2 * S2_K * S2_ALD;    // [2][S2_K][S2_BLD]
+                       int ldc, int kchunk, float *__restrict__ P, long long plane, int ldp,
+                       int tiles_m, int tile0, int dependents) {
+  constexpr bool SPLIT = MODE != 0;
+  if (dependents) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  extern __shared__ __align__(16) float s2mem[];  // stages of [S2_K][S2_ALD], [S2_K][S2_BLD]
+  const uint32_t smem_u = (uint32_t)__cvta_generic_to_shared(s2mem);
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.x * S2_M, n0 = blockIdx.y * S2_N;
-  // K range of this CTA (kchunk a multiple of S2_K); a split-K slice writes
-  // its raw sums to P + z * plane.
-  const int kbeg = (SPLIT && !SHIFT) ? blockIdx.z * kchunk : 0;
-  const int kend = (SPLIT && !SHIFT) ? min(K, kbeg + kchunk) : K;
+  const int tile = tile0 + (int)blockIdx.x;
+  const int m0 = tile % tiles_m * S2_M, n0 = tile / tiles_m * S2_N;
+  // K range of this CTA (kchunk a multiple of S2_K)
+  const int kbeg = SPLIT ? blockIdx.z * kchunk : 0;
+  const int kend = SPLIT ? min(K, kbeg + kchunk) : K;
 
   unsigned long long acc[8][4];  // row r: 4tx + (r&3) + 64(r>>2); column pair c
 #pragma unroll
@@ -96,81 +154,65 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
     for (int c = 0; c < 4; ++c) acc[r][c] = 0ull;
 
-  // Register staging of one K block: 8 A values and 8 B values per thread.
-  // A: element (m, k) at A[k*lda + m] ('N') or A[m*lda + k] ('T');
-  // B: element (k, n) at B[n*ldb + k] ('N') or B[k*ldb + n] ('T').
-  float4 ra[2], rb[2];
-  auto gload = [&](int k0) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int c = tid + 256 * h;
-      if (!TA) {  // 4 consecutive m of one k
-        const int kk = c >> 5, mm = (c & 31) * 4, gm = m0 + mm, gk = k0 + kk;
-        ra[h] = gk < kend ? load4<VEC>(A + (size_t)gk * lda + gm, M - gm) : make_float4(0.f, 0.f, 0.f, 0.f);
-      } else {    // 4 consecutive k of one m
-        const int mm = c >> 2, kk = (c & 3) * 4, gm = m0 + mm, gk = k0 + kk;
-        ra[h] = gm < M ? load4<VEC>(A + (size_t)gm * lda + gk, kend - gk) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      if (TB) {   // 4 consecutive n of one k
-        const int kk = c >> 5, nn = (c & 31) * 4, gn = n0 + nn, gk = k0 + kk;
-        rb[h] = gk < kend ? load4<VEC>(B + (size_t)gk * ldb + gn, N - gn) : make_float4(0.f, 0.f, 0.f, 0.f);
-      } else {    // 4 consecutive k of one n
-        const int nn = c >> 2, kk = (c & 3) * 4, gn = n0 + nn, gk = k0 + kk;
-        rb[h] = gn < N ? load4<VEC>(B + (size_t)gn * ldb + gk, kend - gk) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
-  };
-  auto sstore = [&](int buf) {
-    float *as = As + buf * S2_K * S2_ALD;
-    float *bs = Bs + buf * S2_K * S2_BLD;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int c = tid + 256 * h;
-      if (!TA) {
-        const int kk = c >> 5, mm = (c & 31) * 4;
-        *reinterpret_cast<float4 *>(as + kk * S2_ALD + mm) = ra[h];
-      } else {
-        const int mm = c >> 2, kk = (c & 3) * 4;
-        const float av[4] = {ra[h].x, ra[h].y, ra[h].z, ra[h].w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) as[(kk + e) * S2_ALD + mm] = av[e];
-      }
-      if (TB) {
-        const int kk = c >> 5, nn = (c & 31) * 4;
-        *reinterpret_cast<float4 *>(bs + kk * S2_BLD + nn) = rb[h];
-      } else {
-        const int nn = c >> 2, kk = (c & 3) * 4;
-        const float bv[4] = {rb[h].x, rb[h].y, rb[h].z, rb[h].w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) bs[(kk + e) * S2_BLD + nn] = bv[e];
-      }
-    }
-  };
-
   const int KT = (kend - kbeg + S2_K - 1) / S2_K;
-  gload(kbeg);
-  sstore(0);
-  __syncthreads();
+  const bool in_a = m0 + S2_M <= M, in_b = n0 + S2_N <= N;
+  constexpr bool KA = TA, KB = !TB;  // K contiguous
+  const float *pa = A + (KA ? (size_t)(m0 + (tid >> 4)) * lda + (kbeg + (tid & 15))
+                            : (size_t)(kbeg + (tid >> 5)) * lda + (m0 + (tid & 31) * 4));
+  const float *pb = B + (KB ? (size_t)(n0 + (tid >> 4)) * ldb + (kbeg + (tid & 15))
+                            : (size_t)(kbeg + (tid >> 5)) * ldb + (n0 + (tid & 31) * 4));
+  const uint32_t da =
+      smem_u + (uint32_t)(KA ? panel_at(tid & 15, tid >> 4) : (tid >> 5) * S2_ALD + (tid & 31) * 4) * 4u;
+  const uint32_t db = smem_u + S2_K * S2_ALD * 4u +
+                      (uint32_t)(KB ? panel_at(tid & 15, tid >> 4)
+                                    : (tid >> 5) * S2_BLD + (tid & 31) * 4) * 4u;
+  // Copies stage kt (called once per kt, in order) into ring slot st.
+  auto load_stage = [&](int st, int kt) {
+    const int k0 = kbeg + kt * S2_K;
+    const bool full = k0 + S2_K <= kend;
+    const uint32_t d = (uint32_t)(st * S2_STAGE) * 4u;
+    if (full && in_a) run_panel<KA, VEC>(da + d, pa, (size_t)(KA ? 16 : 8) * lda);
+    else load_panel<KA, VEC>(smem_u + d, A, lda, m0, k0, M, kend, tid);
+    if (full && in_b) run_panel<KB, VEC>(db + d, pb, (size_t)(KB ? 16 : 8) * ldb);
+    else load_panel<KB, VEC>(smem_u + d + S2_K * S2_ALD * 4u, B, ldb, n0, k0, N, kend, tid);
+    pa += KA ? (size_t)S2_K : (size_t)S2_K * lda;
+    pb += KB ? (size_t)S2_K : (size_t)S2_K * ldb;
+  };
+#pragma unroll
+  for (int i = 0; i < S2_STAGES - 1; ++i) {
+    if (i < KT) load_stage(i, i);
+    asm volatile("cp.async.commit_group;\n" ::);
+  }
+  int st = 0, st_fill = S2_STAGES - 1;
   for (int kt = 0; kt < KT; ++kt) {
-    const int buf = kt & 1;
-    if (kt + 1 < KT) gload(kbeg + (kt + 1) * S2_K);
-    const float *as = As + buf * S2_K * S2_ALD;
-    const float *bs = Bs + buf * S2_K * S2_BLD;
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(S2_STAGES - 2));
+    __syncthreads();  // stage kt is in, and every thread is done with the one refilled here
+    if (kt + S2_STAGES - 1 < KT) load_stage(st_fill, kt + S2_STAGES - 1);
+    asm volatile("cp.async.commit_group;\n" ::);
+    const float *as = s2mem + st * S2_STAGE;
+    const float *bs = as + S2_K * S2_ALD;
+    st = st + 1 == S2_STAGES ? 0 : st + 1;
+    st_fill = st_fill + 1 == S2_STAGES ? 0 : st_fill + 1;
 #pragma unroll
     for (int kk = 0; kk < S2_K; ++kk) {
       float av[8];  // rows 4tx + i + 64h'
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
         const float4 v = *reinterpret_cast<const float4 *>(as + kk * S2_ALD + 64 * hh + 4 * tx);
-        av[4 * hh] = v.x;
-        av[4 * hh + 1] = v.y;
-        av[4 * hh + 2] = v.z;
-        av[4 * hh + 3] = v.w;
+        const int sw = TA && kk >= 8 ? 2 : 0;  // panel_at's order
+        av[4 * hh + sw] = v.x;
+        av[4 * hh + 1 + sw] = v.y;
+        av[4 * hh + (2 ^ sw)] = v.z;
+        av[4 * hh + (3 ^ sw)] = v.w;
       }
       ulonglong2 b2[2];  // columns 64h + 4ty .. 64h + 4ty + 3
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
-        b2[h] = *reinterpret_cast<const ulonglong2 *>(bs + kk * S2_BLD + 64 * h + 4 * ty);
+      for (int h = 0; h < 2; ++h) {
+        const ulonglong2 v =
+            *reinterpret_cast<const ulonglong2 *>(bs + kk * S2_BLD + 64 * h + 4 * ty);
+        const bool sw = !TB && kk >= 8;
+        b2[h] = make_ulonglong2(sw ? v.y : v.x, sw ? v.x : v.y);
+      }
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
         const unsigned long long a = dup2(av[r]);
@@ -181,35 +223,125 @@ __global__ void __launch_bounds__(256, 2)
         }
       }
     }
-    if (kt + 1 < KT) {
-      // the other buffer was last read in the previous iteration, which every
-      // thread finished before that iteration's closing barrier
-      sstore(buf ^ 1);
-      __syncthreads();
-    }
   }
-  const bool beta_one = (beta == 1.f);
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  // Output element (r, c, e): row 4tx + (r & 3) + 64 (r >> 2), column
+  // 64 (c >> 1) + 4ty + 2 (c & 1) + e.
+  auto value = [&](int r, int col) {  // col = 2c + e
+    const float2 v = *reinterpret_cast<const float2 *>(&acc[r][col >> 1]);
+    return (col & 1) ? v.y : v.x;
+  };
+  auto column = [&](int col) { return 64 * (col >> 2) + 4 * ty + (col & 3); };
+  if (MODE == 2) {
+    float *T = P + ((long long)blockIdx.z * gridDim.x + blockIdx.x) * (S2_M * S2_N);
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int m = m0 + 4 * tx + (r & 3) + 64 * (r >> 2);
-    if (m >= M) continue;
+    for (int col = 0; col < 8; ++col)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const float2 v = *reinterpret_cast<const float2 *>(&acc[r][c]);
-      const int nb = n0 + 64 * (c >> 1) + 4 * ty + 2 * (c & 1);
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<float4 *>(T + column(col) * S2_M + 64 * h + 4 * tx) =
+            make_float4(value(4 * h, col), value(4 * h + 1, col), value(4 * h + 2, col),
+                        value(4 * h + 3, col));
+    // this launch ends only after the one it overlaps
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    return;
+  }
+  if (MODE == 1) {
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int n = nb + e;
-        if (n >= N) continue;
-        const float x = e ? v.y : v.x;
-        if (SPLIT) {
-          P[blockIdx.z * plane + (long long)n * ldp + m] = x;
-          continue;
-        }
-        float *p = C + (size_t)n * ldc + m;
-        *p = beta_one ? fmaf(alpha, x, *p) : fmaf(alpha, x, beta * *p);
+    for (int col = 0; col < 8; ++col) {
+      const int n = n0 + column(col);
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const int m = m0 + 4 * tx + (r & 3) + 64 * (r >> 2);
+        if (m < M && n < N) P[blockIdx.z * plane + (long long)n * ldp + m] = value(r, col);
       }
     }
+    return;
+  }
+  // C two columns at a time, all of their reads before their writes (between
+  // two writes each read would wait for the one before it)
+  const bool beta_one = (beta == 1.f);
+  const bool cvec = (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldc & 3) == 0;
+  const bool inside = m0 + S2_M <= M && n0 + S2_N <= N;
+#pragma unroll
+  for (int q = 0; q < 8; q += 2) {
+    float old[2][8];
+    if (cvec && inside) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float4 v = *reinterpret_cast<const float4 *>(
+              C + (size_t)(n0 + column(q + u)) * ldc + m0 + 64 * h + 4 * tx);
+          old[u][4 * h] = v.x, old[u][4 * h + 1] = v.y;
+          old[u][4 * h + 2] = v.z, old[u][4 * h + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int n = n0 + column(q + u);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const int m = m0 + 4 * tx + (r & 3) + 64 * (r >> 2);
+          old[u][r] = (m < M && n < N) ? C[(size_t)n * ldc + m] : 0.f;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const float x = value(r, q + u);
+        old[u][r] = beta_one ? fmaf(alpha, x, old[u][r]) : fmaf(alpha, x, beta * old[u][r]);
+      }
+    if (cvec && inside) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          *reinterpret_cast<float4 *>(C + (size_t)(n0 + column(q + u)) * ldc + m0 + 64 * h +
+                                      4 * tx) =
+              make_float4(old[u][4 * h], old[u][4 * h + 1], old[u][4 * h + 2], old[u][4 * h + 3]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int n = n0 + column(q + u);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const int m = m0 + 4 * tx + (r & 3) + 64 * (r >> 2);
+          if (m < M && n < N) C[(size_t)n * ldc + m] = old[u][r];
+        }
+      }
+    }
+  }
+}
+
+// C = alpha * (sum of the K slices of tiles tile0 .. tile0 + tiles - 1, in FP64
+// and slice order) + beta * C; 16 blocks per tile, four rows per thread.
+__global__ void __launch_bounds__(256)
+    ffma2_tail_reduce_kernel(const float *__restrict__ P, int tiles, int S, int M, int N,
+                             float alpha, float beta, float *__restrict__ C, int ldc, int tiles_m,
+                             int tile0) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int lt = blockIdx.x >> 4, idx = ((blockIdx.x & 15) * 256 + threadIdx.x) * 4;
+  const int tile = tile0 + lt;
+  const int m = tile % tiles_m * S2_M + idx % S2_M, n = tile / tiles_m * S2_N + idx / S2_M;
+  if (m >= M || n >= N) return;
+  const float *p = P + (long long)lt * (S2_M * S2_N) + idx;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+  for (int z = 0; z < S; ++z) {
+    const float4 x =
+        *reinterpret_cast<const float4 *>(p + (long long)z * tiles * (S2_M * S2_N));
+    acc[0] += (double)x.x, acc[1] += (double)x.y, acc[2] += (double)x.z, acc[3] += (double)x.w;
+  }
+  float *c = C + (size_t)n * ldc + m;
+  float old[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) old[e] = m + e < M ? c[e] : 0.f;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float a = (float)acc[e];
+    if (m + e < M) c[e] = (beta == 1.f) ? fmaf(alpha, a, old[e]) : fmaf(alpha, a, beta * old[e]);
   }
 }
 
@@ -236,19 +368,66 @@ int ffma2_ksplit(long long tiles, int kblocks, int sms) {
 template <bool TA, bool TB, bool VEC>
 int launch_ffma2(int m, int n, int k, float alpha, const float *A, int lda, const float *B,
                  int ldb, float beta, float *C, int ldc, cudaStream_t s) {
-  auto kern = sgemm_ffma2_kernel<TA, TB, VEC, false>;
-  auto kern_split = sgemm_ffma2_kernel<TA, TB, VEC, true>;
+  auto kern = sgemm_ffma2_kernel<TA, TB, VEC, 0>;
+  auto kern_split = sgemm_ffma2_kernel<TA, TB, VEC, 1>;
   Ctx *cx = ctx();
   if (!cx) return B2_ERR_NO_DEVICE;
   const int gx = (m + S2_M - 1) / S2_M, gy = (n + S2_N - 1) / S2_N;
+  const long long tiles = (long long)gx * gy, slots = 2ll * cx->sm_count;
+  if (tiles > 0x7fffffffll) return B2_ERR_ARG;
   const int kblocks = (k + S2_K - 1) / S2_K;
-  const int S = ffma2_ksplit((long long)gx * gy, kblocks, cx->sm_count);
+  const int S = ffma2_ksplit(tiles, kblocks, cx->sm_count);
   if (S == 1) {
+    // The tiles of whole waves run in full; the rest, when it would leave half
+    // or more of the CTA slots empty, is cut into K slices that fill them, as a
+    // launch of its own (a programmatic dependent: it starts while the last
+    // whole wave ends).  4096^3: 1024 tiles are 3 waves of 296 and 136 tiles,
+    // 2607 -> 2358 us with the rest in 2 slices and the cp.async ring (B200).
+    const int rest = (int)(tiles % slots);
+    int St = rest > 0 ? (int)(slots / rest) : 1;
+    if (St > 8) St = 8;
+    while (St > 1 && kblocks / St < 16) --St;
+    const bool tail = tiles > slots && tiles < 12 * slots && St >= 2;
+    const int whole = (int)(tail ? tiles - rest : tiles);
+    float *P = nullptr;
+    int kchunk = k;
+    if (tail) {
+      kchunk = (kblocks + St - 1) / St * S2_K;
+      St = (k + kchunk - 1) / kchunk;
+      P = (float *)workspace(cx, WS_MISC, (size_t)St * rest * S2_M * S2_N * sizeof(float));
+      if (!P) return B2_ERR_NOMEM;
+    }
     B2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S2_SMEM));
-    B2_PROF("sgemm_simt", s);
-    kern<<<dim3(gx, gy), 256, S2_SMEM, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, k,
-                                             nullptr, 0, 0);
-    B2_CUDA_TRY(cudaGetLastError());
+    {
+      B2_PROF("sgemm_simt", s);
+      kern<<<whole, 256, S2_SMEM, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, k, nullptr, 0,
+                                       0, gx, 0, tail ? 1 : 0);
+      B2_CUDA_TRY(cudaGetLastError());
+    }
+    if (!tail) return B2_OK;
+    auto kern_tail = sgemm_ffma2_kernel<TA, TB, VEC, 2>;
+    B2_CUDA_TRY(
+        cudaFuncSetAttribute(kern_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, S2_SMEM));
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)rest, 1, (unsigned)St);
+    lc.blockDim = dim3(256);
+    lc.dynamicSmemBytes = S2_SMEM;
+    lc.stream = s;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    {
+      B2_PROF("sgemm_simt", s);
+      B2_CUDA_TRY(cudaLaunchKernelEx(&lc, kern_tail, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc,
+                                     kchunk, P, 0ll, 0, gx, whole, 0));
+    }
+    lc.gridDim = dim3((unsigned)rest * 16);
+    lc.dynamicSmemBytes = 0;
+    B2_PROF("sgemm_splitk_reduce", s);
+    B2_CUDA_TRY(cudaLaunchKernelEx(&lc, ffma2_tail_reduce_kernel, (const float *)P, rest, St, m, n,
+                                   alpha, beta, C, ldc, gx, whole));
     return B2_OK;
   }
   // Split-K: S raw partial products of K ranges (multiples of S2_K), then one
@@ -263,8 +442,8 @@ int launch_ffma2(int m, int n, int k, float alpha, const float *A, int lda, cons
     B2_CUDA_TRY(
         cudaFuncSetAttribute(kern_split, cudaFuncAttributeMaxDynamicSharedMemorySize, S2_SMEM));
     B2_PROF("sgemm_simt", s);
-    kern_split<<<dim3(gx, gy, S_used), 256, S2_SMEM, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C,
-                                                           ldc, kchunk, P, plane, ldp);
+    kern_split<<<dim3((unsigned)tiles, 1, S_used), 256, S2_SMEM, s>>>(
+        m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, kchunk, P, plane, ldp, gx, 0, 0);
     B2_CUDA_TRY(cudaGetLastError());
   }
   return sgemm_splitk_reduce(P, plane, ldp, S_used, m, n, alpha, beta, C, ldc, s);
