@@ -69,6 +69,7 @@ struct Ctx {
   static constexpr size_t BOUNCE_BYTES = 64ull << 20;
   void *bounce[2] = {nullptr, nullptr};
   cudaEvent_t bounce_ev[2] = {nullptr, nullptr};
+  int bounce_next = 0;  // buffer of the next host-to-device chunk
   static constexpr int OZ_EVENTS = 2 * 16 + 3;  // per block: sliced, multiplied; fork, 2 joins (the last two also join the norm passes)
   cudaStream_t oz_gemm = nullptr, oz_aux = nullptr;
   cudaEvent_t oz_ev[OZ_EVENTS] = {};
