@@ -25,12 +25,13 @@
 
 #include "b2_methods.cuh"
 #include "b2_profile.cuh"
+#include "fp32_copy.cuh"
+#include "fp64_copy.cuh"
 
 namespace b2 {
 namespace {
 
 constexpr int GT_M = 64, GT_N = 64, GT_K = 16;
-constexpr int GT_NE = GT_M * GT_K / 256;  // elements of each operand panel per thread
 constexpr int GT_MINB = 3;                 // resident CTAs per SM
 constexpr int GT_LD = GT_M + 4;  // [k][m] stride (68 = 4 mod 16 doubles)
 
@@ -48,110 +49,69 @@ struct GroupDesc {
   int ca, cb;              // complex dtypes: operand conjugated ('C', 'R')
 };
 
-// A GT_K-deep panel: op(A) tile (64 x 16) and op(B) tile (16 x 64), 4
-// elements of each per thread.  load_panel fetches it from global memory into
-// registers (zero outside the problem), store_panel writes it to shared
-// memory as As[k][m] and Bs[k][n] (stride GT_LD).  Tiles double-buffer the
-// panels: the next panel's loads are in flight while the current one is
-// multiplied.
-//
-// Element of a thread's e-th slot (idx = tid + 256 e, lane = idx % 32,
-// w = idx / 32): an operand whose m (or n) index is contiguous in memory
-// takes m = idx % 64, k = idx / 64 (one warp: 32 consecutive m of one k).  An
-// operand whose k is contiguous takes KL consecutive k per row (KL = 4
-// doubles or 8 floats, one 32-byte sector) over 32 / KL rows per warp:
-// k = lane % KL + KL (w % (16 / KL)), m = lane / KL + (32 / KL)(w / (16 / KL)).
-// Its shared-memory stores then hit every bank pair at most twice per warp
-// (stride 68: bank pair (8k + 2m) mod 32 for doubles, bank (4k + m) mod 32
-// for floats), where one k column of 16 k by 2 rows had hit each four times.
-template <typename T, int W = GT_M>
-__device__ __forceinline__ void panel_slot(int idx, bool kcont, int &mn, int &kk) {
-  if (!kcont) {
-    mn = idx % W;
-    kk = idx / W;
-    return;
-  }
-  constexpr int KL = 32 / (int)sizeof(T);  // 4 doubles or 8 floats: one 32-byte sector
-  const int lane = idx & 31, w = idx >> 5;
-  kk = lane % KL + KL * (w % (GT_K / KL));
-  mn = lane / KL + (32 / KL) * (w / (GT_K / KL));
-}
+// Operand panels of a real tile (64 x 16 of op(A), 16 x 64 of op(B)) go through a
+// cp.async ring: FP64 16 bytes at a time in either orientation (fp64_copy.cuh;
+// rows off a 16-byte boundary shifted by one element), FP32 as [k][m] and [k][n]
+// (fp32_copy.cuh).  Tiles inside the operand copy from running pointers; the
+// panels were staged through registers element by element before, and the
+// addresses and bounds checks of that were most of the kernel's instructions:
+// 1024 problems 1392 -> 1128 us on B200 (with C read before it is written).
+constexpr int GT_STAGES = 3;   // FP64 ring: 20 KB a stage, three CTAs per SM
+constexpr int GT_STAGES32 = 4;
+constexpr int GT_ST64 = 64 * (GT_K + 4);  // doubles of one FP64 operand panel (either layout fits)
+constexpr int GT_SMEM = GT_STAGES * 2 * GT_ST64 * (int)sizeof(double);
+static_assert(GT_ST64 >= GT_K * GT_LD, "both layouts fit a panel");
+static_assert(GT_STAGES32 * 2 * GT_K * GT_LD * 4 <= GT_SMEM, "the FP32 ring fits the FP64 one");
 
-template <typename T>
-struct PanelRegs {
-  T a[GT_NE], b[GT_NE];
+// One FP64 operand's side of a tile: AK (K contiguous) fixed, the rest per tile.
+template <bool KC>
+struct Op64 {
+  const double *g, *p;  // operand, running pointer
+  int ld, o0, olim, sh, fs;
+  bool inside, tail, first;
+  __device__ __forceinline__ Op64(const void *base, int ld_, int o0_, int olim_, int frag_row,
+                                  int tid) {
+    using namespace f64copy;
+    g = (const double *)base;
+    ld = ld_, o0 = o0_, olim = olim_;
+    constexpr int CPR = (KC ? GT_K : 64) / 2;
+    sh = row_shift(g, ld, (KC ? o0 : 0) + tid / CPR);
+    fs = row_shift(g, ld, frag_row);
+    tail = tid < (KC ? 64 : GT_K) && row_shift(g, ld, (KC ? o0 : 0) + tid);
+    inside = o0 + 64 <= olim;
+    // the operand's first row starts off a 16-byte boundary, and this tile's
+    // first stage copies from before it
+    first = o0 == 0 && ((uintptr_t)g & 8) != 0;
+    p = g + run_offset<64, GT_K, KC>(o0, 0, ld, tid) - sh;
+  }
+  __device__ __forceinline__ void load(uint32_t dst, int kt, int klim, int tid) {
+    using namespace f64copy;
+    const int k0 = kt * GT_K;
+    if (inside && k0 + GT_K <= klim && !(first && kt == 0)) {
+      const uint32_t d = dst + run_dst<64, GT_K, KC>(tid);
+      const size_t step = run_step<64, GT_K, KC, 256>(ld);
+#pragma unroll
+      for (int c = 0; c < tile_chunks<64, GT_K, 256>(); ++c)
+        cp_async_full<16>(d + c * run_dst_step<64, GT_K, KC, 256>(), p + c * step);
+      if (tail)
+        cp_async<16>(dst + run_tail_dst<64, GT_K, KC>(tid), g + run_tail<64, GT_K, KC>(o0, k0, ld, tid),
+                     (KC ? k0 + GT_K < klim : o0 + 64 < olim) ? 16 : 8);
+    } else {
+#pragma unroll
+      for (int c = 0; c < tile_chunks<64, GT_K, 256>(); ++c)
+        load_chunk<64, GT_K, KC, true, 256>(dst, g, ld, o0, k0, olim, klim, tid, c, sh);
+      load_tails<64, GT_K, KC, 256>(dst, g, ld, o0, k0, olim, klim, tid);
+    }
+    p += KC ? (size_t)GT_K : (size_t)GT_K * ld;
+  }
 };
 
-template <typename T>
-__device__ __forceinline__ void load_panel(const GroupDesc &g, int m0, int n0, int k0,
-                                           PanelRegs<T> &r) {
-  const T *A = (const T *)g.A;
-  const T *B = (const T *)g.B;
-#pragma unroll
-  for (int e = 0; e < GT_NE; ++e) {
-    const int idx = threadIdx.x + 256 * e;
-    int mm, kk;
-    panel_slot<T>(idx, g.ta != 0, mm, kk);
-    const int gm = m0 + mm, gk = k0 + kk;
-    r.a[e] = (gm < g.m && gk < g.k)
-                 ? (g.ta ? A[(long long)gm * g.lda + gk] : A[(long long)gk * g.lda + gm])
-                 : (T)0;
-    int nn, kb;
-    panel_slot<T>(idx, g.tb == 0, nn, kb);
-    const int gn = n0 + nn, gk2 = k0 + kb;
-    r.b[e] = (gn < g.n && gk2 < g.k)
-                 ? (g.tb ? B[(long long)gk2 * g.ldb + gn] : B[(long long)gn * g.ldb + gk2])
-                 : (T)0;
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ void store_panel(const GroupDesc &g, const PanelRegs<T> &r, T *As,
-                                            T *Bs) {
-#pragma unroll
-  for (int e = 0; e < GT_NE; ++e) {
-    const int idx = threadIdx.x + 256 * e;
-    int mm, kk;
-    panel_slot<T>(idx, g.ta != 0, mm, kk);
-    As[kk * GT_LD + mm] = r.a[e];
-    int nn, kb;
-    panel_slot<T>(idx, g.tb == 0, nn, kb);
-    Bs[kb * GT_LD + nn] = r.b[e];
-  }
-}
-
-constexpr int GT_PANEL = GT_K * GT_LD;  // elements of one operand panel
-constexpr int GT_STAGE = 2 * GT_PANEL;  // A and B panels of one stage
-constexpr int GT_SMEM = 2 * GT_STAGE * (int)sizeof(double);
-
-// Runs the K loop of one tile over two shared-memory stages; `mac(As, Bs)`
-// multiplies one resident panel pair.
-template <typename T, class Mac>
-__device__ __forceinline__ void tile_k_loop(const GroupDesc &g, int m0, int n0, T *buf, Mac mac) {
-  const int nk = (g.k + GT_K - 1) / GT_K;
-  PanelRegs<T> r;
-  if (nk > 0) {
-    load_panel<T>(g, m0, n0, 0, r);
-    store_panel<T>(g, r, buf, buf + GT_PANEL);
-  }
-  __syncthreads();
-  for (int it = 0; it < nk; ++it) {
-    T *As = buf + (it & 1) * GT_STAGE;
-    const bool more = it + 1 < nk;
-    if (more) load_panel<T>(g, m0, n0, (it + 1) * GT_K, r);
-    mac(As, As + GT_PANEL);
-    if (more) {
-      T *An = buf + ((it + 1) & 1) * GT_STAGE;
-      store_panel<T>(g, r, An, An + GT_PANEL);
-    }
-    __syncthreads();  // the stage just read is refilled two iterations later
-  }
-}
-
-__device__ void tile_f64(const GroupDesc &g, int m0, int n0, double *sm) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+template <bool AK, bool BK>
+__device__ __forceinline__ void tile_f64(const GroupDesc &g, int m0, int n0, double *sm) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gq = lane >> 2, t = lane & 3;
   const int wm0 = (warp >> 2) * 32, wn0 = (warp & 3) * 16;
+  const uint32_t smu = (uint32_t)__cvta_generic_to_shared(sm);
   double acc[2][2][4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
@@ -161,53 +121,89 @@ __device__ void tile_f64(const GroupDesc &g, int m0, int n0, double *sm) {
       for (int v = 0; v < 4; ++v) acc[i][j][v] = 0.0;
   // A warp whose 32 x 16 block lies wholly outside the problem (edge tiles of
   // small M or N) skips its multiplies: the test depends on the warp and the
-  // tile only, so every lane of the warp takes the same branch.  (Skipping
-  // single 16 x 8 blocks as well spills registers and was slower.)
+  // tile only, so every lane of the warp takes the same branch.
   const bool live = m0 + wm0 < g.m && n0 + wn0 < g.n;
-  // DMMA m16n8k8: A fragment rows g, g+8 x k t, t+4; B fragment k t, t+4 x column g
-  tile_k_loop<double>(g, m0, n0, sm, [&](const double *As, const double *Bs) {
-    if (!live) return;
+  const int K = g.k, KT = (K + GT_K - 1) / GT_K;
+  {
+    Op64<AK> a(g.A, g.lda, m0, g.m, AK ? gq : t, tid);
+    Op64<BK> b(g.B, g.ldb, n0, g.n, BK ? gq : t, tid);
+    auto load_stage = [&](int st, int kt) {
+      const uint32_t d = smu + (uint32_t)(st * 2 * GT_ST64) * 8u;
+      a.load(d, kt, K, tid);
+      b.load(d + GT_ST64 * 8u, kt, K, tid);
+    };
 #pragma unroll
-    for (int kk = 0; kk < GT_K; kk += 8) {
-      double af[2][4], bf[2][2];
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int v1 = 0; v1 < 2; ++v1)
-#pragma unroll
-          for (int v0 = 0; v0 < 2; ++v0)
-            af[i][v0 + 2 * v1] = As[(kk + t + 4 * v1) * GT_LD + wm0 + i * 16 + gq + 8 * v0];
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int v = 0; v < 2; ++v) bf[j][v] = Bs[(kk + t + 4 * v) * GT_LD + wn0 + j * 8 + gq];
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-          asm volatile(
-              "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-              "{%8,%9}, {%0,%1,%2,%3};\n"
-              : "+d"(acc[i][j][0]), "+d"(acc[i][j][1]), "+d"(acc[i][j][2]), "+d"(acc[i][j][3])
-              : "d"(af[i][0]), "d"(af[i][1]), "d"(af[i][2]), "d"(af[i][3]), "d"(bf[j][0]),
-                "d"(bf[j][1]));
+    for (int i = 0; i < GT_STAGES - 1; ++i) {
+      if (i < KT) load_stage(i, i);
+      f64copy::cp_async_commit();
     }
-  });
-  double *C = (double *)g.C;
-  const bool one = (g.beta == 1.0);
+    int st = 0, fill = GT_STAGES - 1;
+    for (int kt = 0; kt < KT; ++kt) {
+      f64copy::cp_async_wait<GT_STAGES - 2>();
+      __syncthreads();  // stage kt is in; every warp is done with the one refilled here
+      if (kt + GT_STAGES - 1 < KT) load_stage(fill, kt + GT_STAGES - 1);
+      f64copy::cp_async_commit();
+      const double *As = sm + st * 2 * GT_ST64 + a.fs, *Bs = sm + st * 2 * GT_ST64 + GT_ST64 + b.fs;
+      st = st + 1 == GT_STAGES ? 0 : st + 1;
+      fill = fill + 1 == GT_STAGES ? 0 : fill + 1;
+      if (!live) continue;
+      // DMMA m16n8k4: A fragment rows gq, gq + 8 x k t; B fragment k t x column gq
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+      for (int kk = 0; kk < GT_K; kk += 4) {
+        double af[2][2], bf[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int v = 0; v < 2; ++v) {
+            const int m = wm0 + i * 16 + gq + 8 * v, k = kk + t;
+            af[i][v] = AK ? As[m * (GT_K + 4) + k] : As[k * GT_LD + m];
+          }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int n = wn0 + j * 8 + gq, k = kk + t;
+          bf[j] = BK ? Bs[n * (GT_K + 4) + k] : Bs[k * GT_LD + n];
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            asm volatile(
+                "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+                "{%0,%1,%2,%3};\n"
+                : "+d"(acc[i][j][0]), "+d"(acc[i][j][1]), "+d"(acc[i][j][2]), "+d"(acc[i][j][3])
+                : "d"(af[i][0]), "d"(af[i][1]), "d"(bf[j]));
+      }
+    }
+  }
+  if (!live) return;
+  // all of C's reads before its writes (between two writes each read would wait
+  // for the one before it)
+  double *C = (double *)g.C;
+  const int ldc = g.ldc;
+  const double alpha = g.alpha, beta = g.beta;
+  const bool one = (beta == 1.0);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    double old[2][4];
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         const int m = m0 + wm0 + i * 16 + gq + 8 * (v >> 1);
         const int n = n0 + wn0 + j * 8 + 2 * t + (v & 1);
-        if (m < g.m && n < g.n) {
-          double *p = C + (long long)n * g.ldc + m;
-          *p = one ? fma(g.alpha, acc[i][j][v], *p) : fma(g.alpha, acc[i][j][v], g.beta * *p);
-        }
+        old[j][v] = (m < g.m && n < g.n) ? C[(long long)n * ldc + m] : 0.0;
       }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const int m = m0 + wm0 + i * 16 + gq + 8 * (v >> 1);
+        const int n = n0 + wn0 + j * 8 + 2 * t + (v & 1);
+        if (m < g.m && n < g.n)
+          C[(long long)n * ldc + m] =
+              one ? fma(alpha, acc[i][j][v], old[j][v]) : fma(alpha, acc[i][j][v], beta * old[j][v]);
+      }
+  }
 }
 
 // Two FP32 FMAs per issued instruction (sm_100 fma.rn.f32x2, each lane
@@ -222,49 +218,113 @@ __device__ __forceinline__ void ffma2(unsigned long long &c, unsigned long long 
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
 }
 
+// One FP32 operand's side of a tile.
+template <bool KC>
+struct Op32 {
+  const float *g, *p;
+  int ld, o0, olim;
+  uint32_t d;
+  bool vec, inside;
+  __device__ __forceinline__ Op32(const void *base, int ld_, int o0_, int olim_, int tid) {
+    using namespace f32copy;
+    g = (const float *)base;
+    ld = ld_, o0 = o0_, olim = olim_;
+    vec = !KC && (ld & 3) == 0 && ((uintptr_t)g & 15) == 0;
+    inside = o0 + 64 <= olim;
+    p = g + (vec ? run_offset<64, KC, true>(o0, 0, ld, tid) : run_offset<64, KC, false>(o0, 0, ld, tid));
+    d = vec ? run_dst<64, GT_LD, KC, true>(tid) : run_dst<64, GT_LD, KC, false>(tid);
+  }
+  __device__ __forceinline__ void load(uint32_t dst, int kt, int klim, int tid) {
+    using namespace f32copy;
+    const int k0 = kt * GT_K;
+    if (inside && k0 + GT_K <= klim) {
+      if (!KC && vec) run_panel<64, GT_LD, KC, true>(dst + d, p, ld);
+      else run_panel<64, GT_LD, KC, false>(dst + d, p, ld);
+    } else {
+      if (!KC && vec) load_panel<64, GT_LD, KC, true>(dst, g, ld, o0, k0, olim, klim, tid);
+      else load_panel<64, GT_LD, KC, false>(dst, g, ld, o0, k0, olim, klim, tid);
+    }
+    p += KC ? (size_t)GT_K : (size_t)GT_K * ld;
+  }
+};
+
 // FP32 tile: 8 warps of 32 x 16 outputs (the FP64 warp grid), each lane 4 x 4
 // of them: rows 32 (warp / 4) + 4 (lane % 8) + i, columns 16 (warp % 4) +
 // 4 (lane / 8) + j, accumulated as column pairs with paired FMAs.  A warp
 // whose block lies wholly outside the problem skips its multiplies.
-__device__ void tile_f32(const GroupDesc &g, int m0, int n0, float *sm) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+template <bool AK, bool BK>
+__device__ __forceinline__ void tile_f32(const GroupDesc &g, int m0, int n0, float *sm) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rm = (warp >> 2) * 32 + (lane & 7) * 4, cn = (warp & 3) * 16 + (lane >> 3) * 4;
   const bool live = m0 + (warp >> 2) * 32 < g.m && n0 + (warp & 3) * 16 < g.n;
+  const uint32_t smu = (uint32_t)__cvta_generic_to_shared(sm);
+  constexpr int PANEL = GT_K * GT_LD;
   unsigned long long acc[4][2];  // row i, columns (2 jp, 2 jp + 1)
 #pragma unroll
   for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0ull;
-  tile_k_loop<float>(g, m0, n0, sm, [&](const float *As, const float *Bs) {
-    if (!live) return;
+  const int K = g.k, KT = (K + GT_K - 1) / GT_K;
+  {
+    Op32<AK> a(g.A, g.lda, m0, g.m, tid);
+    Op32<BK> b(g.B, g.ldb, n0, g.n, tid);
+    auto load_stage = [&](int st, int kt) {
+      const uint32_t d = smu + (uint32_t)(st * 2 * PANEL) * 4u;
+      a.load(d, kt, K, tid);
+      b.load(d + PANEL * 4u, kt, K, tid);
+    };
 #pragma unroll
-    for (int kk = 0; kk < GT_K; ++kk) {
-      const float4 a = *reinterpret_cast<const float4 *>(&As[kk * GT_LD + rm]);
-      const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(&Bs[kk * GT_LD + cn]);
-      const float av[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const unsigned long long ai = dup2(av[i]);
-        ffma2(acc[i][0], ai, b.x);
-        ffma2(acc[i][1], ai, b.y);
-      }
+    for (int i = 0; i < GT_STAGES32 - 1; ++i) {
+      if (i < KT) load_stage(i, i);
+      f64copy::cp_async_commit();
     }
-  });
-  float *C = (float *)g.C;
-  const float al = (float)g.alpha, be = (float)g.beta;
-  const bool one = (be == 1.f);
+    int st = 0, fill = GT_STAGES32 - 1;
+    for (int kt = 0; kt < KT; ++kt) {
+      f64copy::cp_async_wait<GT_STAGES32 - 2>();
+      __syncthreads();
+      if (kt + GT_STAGES32 - 1 < KT) load_stage(fill, kt + GT_STAGES32 - 1);
+      f64copy::cp_async_commit();
+      const float *As = sm + st * 2 * PANEL, *Bs = As + PANEL;
+      st = st + 1 == GT_STAGES32 ? 0 : st + 1;
+      fill = fill + 1 == GT_STAGES32 ? 0 : fill + 1;
+      if (!live) continue;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+      for (int kk = 0; kk < GT_K; ++kk) {
+        const float4 a4 = *reinterpret_cast<const float4 *>(&As[kk * GT_LD + rm]);
+        const ulonglong2 b2 = *reinterpret_cast<const ulonglong2 *>(&Bs[kk * GT_LD + cn]);
+        const bool sa = AK && kk >= 8, sb = BK && kk >= 8;  // panel_at's order
+        const float av[4] = {sa ? a4.z : a4.x, sa ? a4.w : a4.y, sa ? a4.x : a4.z,
+                             sa ? a4.y : a4.w};
+        const unsigned long long bl = sb ? b2.y : b2.x, bh = sb ? b2.x : b2.y;
 #pragma unroll
-    for (int jp = 0; jp < 2; ++jp) {
-      const float2 v = *reinterpret_cast<const float2 *>(&acc[i][jp]);
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int m = m0 + rm + i, n = n0 + cn + 2 * jp + e;
-        if (m < g.m && n < g.n) {
-          float *p = C + (long long)n * g.ldc + m;
-          const float x = e ? v.y : v.x;
-          *p = one ? fmaf(al, x, *p) : fmaf(al, x, be * *p);
+        for (int i = 0; i < 4; ++i) {
+          const unsigned long long ai = dup2(av[i]);
+          ffma2(acc[i][0], ai, bl);
+          ffma2(acc[i][1], ai, bh);
         }
       }
+    }
+  }
+  if (!live) return;
+  float *C = (float *)g.C;
+  const int ldc = g.ldc;
+  const float al = (float)g.alpha, be = (float)g.beta;
+  const bool one = (be == 1.f);
+  float old[4][4];  // all of C's reads before its writes
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int m = m0 + rm + i, n = n0 + cn + j;
+      old[i][j] = (m < g.m && n < g.n) ? C[(long long)n * ldc + m] : 0.f;
+    }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int m = m0 + rm + i, n = n0 + cn + j;
+      const float2 v = *reinterpret_cast<const float2 *>(&acc[i][j >> 1]);
+      const float x = (j & 1) ? v.y : v.x;
+      if (m < g.m && n < g.n)
+        C[(long long)n * ldc + m] = one ? fmaf(al, x, old[i][j]) : fmaf(al, x, be * old[i][j]);
     }
 }
 
@@ -287,7 +347,8 @@ constexpr int Z_LD = Z_T + 4;            // panel row stride (36 = 4 mod 16)
 constexpr int Z_PANEL = GT_K * Z_LD;     // one real panel
 constexpr int Z_STAGE = 4 * Z_PANEL;     // A: re, im; B: re, im
 constexpr int Z_PER = Z_T * GT_K / 256;  // complex elements per thread per operand
-constexpr int GT_SMEM_3M = 2 * Z_STAGE * (int)sizeof(double);
+constexpr int GT_SMEM_3M = GT_SMEM;
+static_assert(2 * Z_STAGE * (int)sizeof(double) <= GT_SMEM, "the 3M stages fit the FP64 ring");
 
 // Slot map of a complex panel (32 wide), in complex elements (16 or 8 bytes).
 // An operand whose m (or n) is contiguous takes m = idx % 32, k = idx / 32.  A
@@ -527,19 +588,37 @@ __global__ void __launch_bounds__(256, GT_MINB)
   // two stages of A and B panels (GT_SMEM; GT_SMEM_3M when the batch has complex problems)
   extern __shared__ __align__(16) double sm[];
   __shared__ long long next_s;
+  __shared__ GroupDesc desc;
   if (threadIdx.x == 0) next_s = (long long)atomicAdd(counter, 1ull);
   __syncthreads();
   long long t = next_s;
   while (t < total_tiles) {
     __syncthreads();  // every thread has read next_s
     if (threadIdx.x == 0) next_s = (long long)atomicAdd(counter, 1ull);
-    const GroupDesc g = d[tile_prob[t]];
+    // the tile's descriptor in shared memory: its fields are read where they are
+    // used instead of holding registers through the tile
+    if (threadIdx.x < sizeof(GroupDesc) / 4)
+      reinterpret_cast<int *>(&desc)[threadIdx.x] =
+          reinterpret_cast<const int *>(d + tile_prob[t])[threadIdx.x];
+    __syncthreads();
+    const GroupDesc &g = desc;
     const int local = (int)(t - g.tile_offset);
     const int tm = local % g.tiles_m, tn = local / g.tiles_m;
     float *smf = reinterpret_cast<float *>(sm);
     if (!CPLX || g.dtype < 2) {
-      if (g.dtype == 0) tile_f64(g, tm * GT_M, tn * GT_N, sm);
-      else tile_f32(g, tm * GT_M, tn * GT_N, smf);
+      // op(A) is K-contiguous when transposed, op(B) when not
+      const int m0 = tm * GT_M, n0 = tn * GT_N, form = (g.ta ? 2 : 0) + (g.tb ? 0 : 1);
+      if (g.dtype == 0) {
+        if (form == 0) tile_f64<false, false>(g, m0, n0, sm);
+        else if (form == 1) tile_f64<false, true>(g, m0, n0, sm);
+        else if (form == 2) tile_f64<true, false>(g, m0, n0, sm);
+        else tile_f64<true, true>(g, m0, n0, sm);
+      } else {
+        if (form == 0) tile_f32<false, false>(g, m0, n0, smf);
+        else if (form == 1) tile_f32<false, true>(g, m0, n0, smf);
+        else if (form == 2) tile_f32<true, false>(g, m0, n0, smf);
+        else tile_f32<true, true>(g, m0, n0, smf);
+      }
     } else {
       if (g.dtype == 2) tile_z3m(g, tm * Z_T, tn * Z_T, sm);
       else tile_c3m(g, tm * Z_T, tn * Z_T, smf);

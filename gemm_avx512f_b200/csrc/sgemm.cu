@@ -9,6 +9,7 @@
 // engine (sgemm_tc.cu).
 #include "b2_methods.cuh"
 #include "b2_profile.cuh"
+#include "fp32_copy.cuh"
 
 namespace b2 {
 namespace {
@@ -47,84 +48,6 @@ __device__ __forceinline__ void ffma2(unsigned long long &c, unsigned long long 
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
 }
 
-// `bytes` (0 .. 4 or 16) of one copy, the rest of it zero.
-__device__ __forceinline__ void copy16(uint32_t dst, const float *src, int bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
-}
-__device__ __forceinline__ void copy4(uint32_t dst, const float *src, int bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
-}
-
-// Place of element (k, o) of a K-contiguous operand's panel.  From k = 8 on the
-// pairs of a group of four outer indices are swapped: the stores of 16 k x 2 o
-// then fall on 32 different banks (4 k + o repeats from k = 8), and a 16-byte
-// read of a group only has its halves exchanged.
-__device__ __forceinline__ int panel_at(int k, int o) { return k * S2_ALD + (o ^ ((k >> 3) << 1)); }
-
-// One 16 x 128 panel of an operand into shared memory as [k][S2_ALD]: outer
-// index o = o0 .. o0 + 127 (zero from olim on), k = k0 .. k0 + 15 (zero from
-// klim on).  KCONT: element (o, k) at g[o*ld + k] (placed by panel_at), else
-// g[k*ld + o].
-template <bool KCONT, bool VEC>
-__device__ __forceinline__ void load_panel(uint32_t dst, const float *__restrict__ g, int ld,
-                                           int o0, int k0, int olim, int klim, int tid) {
-  if constexpr (KCONT) {
-    // a warp: 16 k of 2 outer indices, stored to 32 banks (see panel_at)
-    const int k = tid & 15, o = tid >> 4;
-    const float *p = g + (size_t)(o0 + o) * ld + (k0 + k);
-    const bool kin = k0 + k < klim;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const bool in = kin && o0 + o + 16 * e < olim;
-      copy4(dst + (uint32_t)panel_at(k, o + 16 * e) * 4u, in ? p + (size_t)(16 * e) * ld : g,
-            in ? 4 : 0);
-    }
-  } else {
-    const int k = tid >> 5, o = (tid & 31) * 4;
-    const float *p = g + (size_t)(k0 + k) * ld + (o0 + o);
-    const int left = olim - (o0 + o);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int have = k0 + k + 8 * h < klim ? left : 0;
-      const uint32_t d = dst + (uint32_t)((k + 8 * h) * S2_ALD + o) * 4u;
-      const float *q = p + (size_t)(8 * h) * ld;
-      if constexpr (VEC) {
-        copy16(d, have > 0 ? q : g, have >= 4 ? 16 : have > 0 ? 4 * have : 0);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) copy4(d + 4u * e, have > e ? q + e : g, have > e ? 4 : 0);
-      }
-    }
-  }
-}
-
-// The same panel when it lies wholly inside the operand: from the thread's
-// running pointer (element (o0 + o, k0 + k) of the map above), `step` = ld times
-// the distance between its copies.
-template <bool KCONT, bool VEC>
-__device__ __forceinline__ void run_panel(uint32_t dst, const float *p, size_t step) {
-  if constexpr (KCONT) {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst + 64u * e), "l"(p));
-      p += step;
-    }
-  } else {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const uint32_t d = dst + (uint32_t)(8 * h * S2_ALD) * 4u;
-      if constexpr (VEC) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(p));
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d + 4u * e), "l"(p + e));
-      }
-      p += step;
-    }
-  }
-}
-
 // MODE 0: tiles [tile0, tile0 + gridDim.x) of C in full; MODE 1: K slice
 // blockIdx.z of a split-K product, its raw sums to P + z*plane (ld ldp); MODE 2:
 // K slice blockIdx.z of tile tile0 + blockIdx.x, the raw sums of its 128 x 128
@@ -157,24 +80,21 @@ __global__ void __launch_bounds__(256, 2)
   const int KT = (kend - kbeg + S2_K - 1) / S2_K;
   const bool in_a = m0 + S2_M <= M, in_b = n0 + S2_N <= N;
   constexpr bool KA = TA, KB = !TB;  // K contiguous
-  const float *pa = A + (KA ? (size_t)(m0 + (tid >> 4)) * lda + (kbeg + (tid & 15))
-                            : (size_t)(kbeg + (tid >> 5)) * lda + (m0 + (tid & 31) * 4));
-  const float *pb = B + (KB ? (size_t)(n0 + (tid >> 4)) * ldb + (kbeg + (tid & 15))
-                            : (size_t)(kbeg + (tid >> 5)) * ldb + (n0 + (tid & 31) * 4));
-  const uint32_t da =
-      smem_u + (uint32_t)(KA ? panel_at(tid & 15, tid >> 4) : (tid >> 5) * S2_ALD + (tid & 31) * 4) * 4u;
-  const uint32_t db = smem_u + S2_K * S2_ALD * 4u +
-                      (uint32_t)(KB ? panel_at(tid & 15, tid >> 4)
-                                    : (tid >> 5) * S2_BLD + (tid & 31) * 4) * 4u;
+  const float *pa = A + f32copy::run_offset<S2_M, KA, VEC>(m0, kbeg, lda, tid);
+  const float *pb = B + f32copy::run_offset<S2_N, KB, VEC>(n0, kbeg, ldb, tid);
+  const uint32_t da = smem_u + f32copy::run_dst<S2_M, S2_ALD, KA, VEC>(tid);
+  const uint32_t db = smem_u + S2_K * S2_ALD * 4u + f32copy::run_dst<S2_N, S2_BLD, KB, VEC>(tid);
   // Copies stage kt (called once per kt, in order) into ring slot st.
   auto load_stage = [&](int st, int kt) {
     const int k0 = kbeg + kt * S2_K;
     const bool full = k0 + S2_K <= kend;
     const uint32_t d = (uint32_t)(st * S2_STAGE) * 4u;
-    if (full && in_a) run_panel<KA, VEC>(da + d, pa, (size_t)(KA ? 16 : 8) * lda);
-    else load_panel<KA, VEC>(smem_u + d, A, lda, m0, k0, M, kend, tid);
-    if (full && in_b) run_panel<KB, VEC>(db + d, pb, (size_t)(KB ? 16 : 8) * ldb);
-    else load_panel<KB, VEC>(smem_u + d + S2_K * S2_ALD * 4u, B, ldb, n0, k0, N, kend, tid);
+    if (full && in_a) f32copy::run_panel<S2_M, S2_ALD, KA, VEC>(da + d, pa, lda);
+    else f32copy::load_panel<S2_M, S2_ALD, KA, VEC>(smem_u + d, A, lda, m0, k0, M, kend, tid);
+    if (full && in_b) f32copy::run_panel<S2_N, S2_BLD, KB, VEC>(db + d, pb, ldb);
+    else
+      f32copy::load_panel<S2_N, S2_BLD, KB, VEC>(smem_u + d + S2_K * S2_ALD * 4u, B, ldb, n0, k0, N,
+                                                 kend, tid);
     pa += KA ? (size_t)S2_K : (size_t)S2_K * lda;
     pb += KB ? (size_t)S2_K : (size_t)S2_K * ldb;
   };
