@@ -75,6 +75,7 @@ __global__ void __launch_bounds__(WM *WN * 32, BM * BN <= 64 * 64 && MMAK == 4 ?
   extern __shared__ __align__(16) double smem[];
   double *sA = smem;
   double *sB = smem + STAGES * A_ST;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t sA_u = (uint32_t)__cvta_generic_to_shared(sA);
   const uint32_t sB_u = (uint32_t)__cvta_generic_to_shared(sB);
 
@@ -347,10 +348,23 @@ cudaError_t launch_one(const LaunchArgs &a, cudaStream_t s) {
                                        (int)SMEM);
   if (e != cudaSuccess) return e;
   dim3 grid((a.M + BM - 1) / BM, (a.N + BN - 1) / BN, a.splits);
+  // A programmatic dependent: it is set up while the kernel before it ends and
+  // waits for that one's writes before it touches memory (48x40x64 in a row of
+  // calls 8.5 -> 7.9 us, 1024^3 79.9 -> 77.8).
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = grid;
+  lc.blockDim = dim3(WM * WN * 32);
+  lc.dynamicSmemBytes = SMEM;
+  lc.stream = s;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
   B2_PROF("dgemm_dmma", s);
-  kern<<<grid, WM * WN * 32, SMEM, s>>>(a.M, a.N, a.K, a.kchunk, a.alpha, a.A, a.lda, a.B, a.ldb,
-                                        a.beta, a.C, a.ldc, a.P, a.ldp);
-  return cudaGetLastError();
+  e = cudaLaunchKernelEx(&lc, kern, a.M, a.N, a.K, a.kchunk, a.alpha, a.A, a.lda,
+                                           a.B, a.ldb, a.beta, a.C, a.ldc, a.P, a.ldp);
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 template <int BM, int BN, int WM, int WN, int STAGES, int MMAK, bool SH>
@@ -384,8 +398,10 @@ Fp64Cfg fp64_default_cfg(int m, int n, int k, int sm_count) {
   // q = work units (tiles x slices) per SM, each of `kit` K blocks of 16 that
   // take the FP64 pipe 0.53 us; a lone CTA per SM reaches 74 % of that rate,
   // two 91 %; 3 us to fill and drain, 1 us per further wave of three; a split
-  // adds a second launch and 64 KB of partials per unit, written and read at
-  // about 8 TB/s (they stay in L2).  Measured (B200, us, graph replays):
+  // adds a second launch (1.5 us on the device and 2 on the host, which bounds a
+  // run of small calls: 128x128x128 11.2 us a call in two launches, 9.1 in one) and
+  // 64 KB of partials per unit, written and read at about 8 TB/s (they stay in
+  // L2).  Measured (B200, us, graph replays):
   //   128x4096x128   S=1 9.7  2 11.7  4 12.7  8 15.4     512^3  28.3 17.6 15.5 17.5
   //   512x1024x512   28.4 26.1 27.6 27.4     256^3  15.7 10.5 7.4 6.2
   // (one fixed rule, 8 slices up to 1024 units, took the last column of the
@@ -403,7 +419,7 @@ Fp64Cfg fp64_default_cfg(int m, int n, int k, int sm_count) {
     const int kit = ((k + s - 1) / s + 15) / 16;
     const double rate = q == 1 ? 0.74 : q == 2 ? 0.91 : 0.98;
     double us = (double)q * kit * 0.53 / rate + 3.0 + (double)((q + 2) / 3 - 1);
-    if (s > 1) us += 2.0 + units * 65536.0 / 8e6;
+    if (s > 1) us += 3.5 + units * 65536.0 / 8e6;
     if (us < best) best = us, sk = s;
   }
   c.split_k = sk;
