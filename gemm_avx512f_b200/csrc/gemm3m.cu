@@ -19,7 +19,8 @@
 // complex alpha/beta happen in the epilogue.  beta follows the reference
 // drivers (C scaled whenever beta != 1, src/gemm_driver.c:131).
 //   zgemm3m: FP64 DMMA (mma.sync.m16n8k4.f64), 64x32 tile, 8 warps of 16x16.
-//   cgemm3m: FP32 FFMA, 64x64 tile, 256 threads of 4x4 outputs.
+//   cgemm3m: FP32 FFMA, 32x32 tile, four groups of 64 threads of 4x4 outputs
+//   splitting each panel's k.
 #include <stdlib.h>
 
 #include "b2_methods.cuh"
@@ -32,10 +33,10 @@ namespace {
 constexpr int G_BM = 64, G_BN = 64, G_BK = 16, G_PAD = 4;
 constexpr int G_LD = G_BM + G_PAD;  // [k][m] / [k][n] row stride (68 = 4 mod 16 doubles)
 
-__device__ __forceinline__ bool tr_is_t(char c) {
+__host__ __device__ __forceinline__ bool tr_is_t(char c) {
   return !(c == 'N' || c == 'n' || c == 'R' || c == 'r');
 }
-__device__ __forceinline__ bool tr_is_conj(char c) {
+__host__ __device__ __forceinline__ bool tr_is_conj(char c) {
   return c == 'C' || c == 'c' || c == 'R' || c == 'r';
 }
 
@@ -189,17 +190,62 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------------------------------------------- cgemm3m: FP32 FFMA --
+// Products below 2^24 multiply-adds: a few CTAs, so what bounds them is the
+// chain of K panels of one CTA.  CTA tile 32 x 32 complex outputs, 256 threads:
+// four groups of 64 take every fourth k of a panel of 16, each thread 4 x 4
+// outputs (rows 2 tx + {0, 1} and 16 further, columns likewise with ty) of the
+// three products; the groups' sums meet in shared memory at the end, each group
+// storing one of a thread's four rows.  The complex panels go through a
+// four-stage cp.async ring as they are, the pre-adds are made in registers.
+// With 64 x 64 tiles, panels of three real planes staged through registers and
+// no split, B200 us: 64^3 17.9, 200x100x300 70.1, 255^3 60.4, 2000x1000x8 28.0;
+// this way 4.8, 15.6, 13.6 and 19.7.  (From 2^24 multiply-adds on the
+// tensor-core products, 3xTF32, take over: their rounding differs, so the line
+// stays where it was.)
+constexpr int C_T = 32, C_K = 16, C_LD = 34;  // tile edge, k per panel, [k][.] pitch
+constexpr int C_STAGES = 4;
+constexpr int C_PANEL = C_K * C_LD;  // complex elements of one operand's panel
+constexpr int C_SMEM = 4 * 48 * 64 * 4;  // the groups' sums
+static_assert(C_STAGES * 2 * C_PANEL * 8 <= C_SMEM, "the ring fits where the sums go");
+
+// Panel of 32 outer indices x 16 k at [k][C_LD], two elements per thread, as 8
+// bytes or (operand off an 8-byte boundary) 4 + 4.  KC: K is contiguous in
+// memory; a half-warp then stores 8 k x 2 outer indices, 32 different banks.
+template <bool KC>
+__device__ __forceinline__ void c3m_copy(uint32_t dst, const float2 *__restrict__ g, int ld, int o0,
+                                         int k0, int olim, int K, bool al8, int tid) {
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int o = KC ? tid >> 3 : tid & 31, k = (KC ? tid & 7 : tid >> 5) + 8 * e;
+    const bool in = o0 + o < olim && k0 + k < K;
+    const float2 *p = in ? g + (KC ? (long long)(o0 + o) * ld + (k0 + k)
+                                   : (long long)(k0 + k) * ld + (o0 + o))
+                         : g;
+    const uint32_t d = dst + (uint32_t)(k * C_LD + o) * 8u;
+    if (al8) {
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(p),
+                   "r"(in ? 8 : 0));
+    } else {
+      const float *q = reinterpret_cast<const float *>(p);
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d + 4 * h),
+                     "l"(q + h), "r"(in ? 4 : 0));
+    }
+  }
+}
+
+template <bool AK, bool BK>
 __global__ void __launch_bounds__(256)
-    cgemm3m_kernel(int M, int N, int K, const float *__restrict__ A, int lda,
-                   const float *__restrict__ B, int ldb, float *__restrict__ C, int ldc,
-                   float ar, float ai, float br, float bi, char transa, char transb) {
-  extern __shared__ __align__(16) float csm[];
-  float *sA[2] = {csm, csm + 3 * G_BK * G_LD};
-  float *sB[2] = {csm + 6 * G_BK * G_LD, csm + 9 * G_BK * G_LD};
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.x * G_BM, n0 = blockIdx.y * G_BN;
-  const bool tA = tr_is_t(transa), tB = tr_is_t(transb);
-  const float sa = tr_is_conj(transa) ? -1.f : 1.f, sb = tr_is_conj(transb) ? -1.f : 1.f;
+    cgemm3m_kernel(int M, int N, int K, const float2 *__restrict__ A, int lda,
+                   const float2 *__restrict__ B, int ldb, float *__restrict__ C, int ldc, float ar,
+                   float ai, float br, float bi, float sa, float sb, int tiles_m, bool al8a,
+                   bool al8b) {
+  extern __shared__ __align__(16) float2 csm[];
+  const int tid = threadIdx.x, lane = tid & 31, grp = tid >> 6, t64 = tid & 63;
+  const int tx = lane & 7, ty = t64 >> 3;
+  const int m0 = (int)(blockIdx.x % tiles_m) * C_T, n0 = (int)(blockIdx.x / tiles_m) * C_T;
+  const uint32_t smu = (uint32_t)__cvta_generic_to_shared(csm);
   float acc[3][4][4];
 #pragma unroll
   for (int p = 0; p < 3; ++p)
@@ -207,41 +253,105 @@ __global__ void __launch_bounds__(256)
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[p][i][j] = 0.f;
-  Stage3M<float, 256> st;
-  const int KT = (K + G_BK - 1) / G_BK;
-  st.load(A, lda, B, ldb, M, N, K, m0, n0, 0, tA, tB, sa, sb, tid);
-  st.store(sA[0], sB[0], tA, tB, tid);
-  __syncthreads();
+  const int KT = (K + C_K - 1) / C_K;
+  auto load_stage = [&](int st, int kt) {
+    const uint32_t d = smu + (uint32_t)(st * 2 * C_PANEL) * 8u;
+    c3m_copy<AK>(d, A, lda, m0, kt * C_K, M, K, al8a, tid);
+    c3m_copy<BK>(d + C_PANEL * 8u, B, ldb, n0, kt * C_K, N, K, al8b, tid);
+  };
+#pragma unroll
+  for (int i = 0; i < C_STAGES - 1; ++i) {
+    if (i < KT) load_stage(i, i);
+    asm volatile("cp.async.commit_group;\n" ::);
+  }
+  int st = 0, fill = C_STAGES - 1;
   for (int kt = 0; kt < KT; ++kt) {
-    const int buf = kt & 1;
-    if (kt + 1 < KT) st.load(A, lda, B, ldb, M, N, K, m0, n0, (kt + 1) * G_BK, tA, tB, sa, sb, tid);
-    const float *As = sA[buf], *Bs = sB[buf];
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(C_STAGES - 2));
+    __syncthreads();  // panel kt is in; every thread is done with the one refilled here
+    if (kt + C_STAGES - 1 < KT) load_stage(fill, kt + C_STAGES - 1);
+    asm volatile("cp.async.commit_group;\n" ::);
+    const float2 *As = csm + st * 2 * C_PANEL + 2 * tx, *Bs = csm + st * 2 * C_PANEL + C_PANEL + 2 * ty;
+    st = st + 1 == C_STAGES ? 0 : st + 1;
+    fill = fill + 1 == C_STAGES ? 0 : fill + 1;
 #pragma unroll
-    for (int kk = 0; kk < G_BK; ++kk) {
+    for (int kq = 0; kq < C_K / 4; ++kq) {
+      const int kk = (kq * 4 + grp) * C_LD;
+      float a[3][4], b[3][4];  // re, im, re + im (conjugated: im negated)
 #pragma unroll
-      for (int p = 0; p < 3; ++p) {
-        const float4 a = *reinterpret_cast<const float4 *>(&As[(p * G_BK + kk) * G_LD + tx * 4]);
-        const float4 b = *reinterpret_cast<const float4 *>(&Bs[(p * G_BK + kk) * G_LD + ty * 4]);
-        const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+      for (int h = 0; h < 2; ++h) {
+        const float4 u = *reinterpret_cast<const float4 *>(As + kk + 16 * h);
+        const float4 v = *reinterpret_cast<const float4 *>(Bs + kk + 16 * h);
+        a[0][2 * h] = u.x, a[1][2 * h] = sa * u.y, a[0][2 * h + 1] = u.z, a[1][2 * h + 1] = sa * u.w;
+        b[0][2 * h] = v.x, b[1][2 * h] = sb * v.y, b[0][2 * h + 1] = v.z, b[1][2 * h + 1] = sb * v.w;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a[2][i] = a[0][i] + a[1][i];
+        b[2][i] = b[0][i] + b[1][i];
+      }
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) acc[p][i][j] = fmaf(av[i], bv[j], acc[p][i][j]);
-      }
-    }
-    if (kt + 1 < KT) {
-      st.store(sA[buf ^ 1], sB[buf ^ 1], tA, tB, tid);
-      __syncthreads();
+          for (int j = 0; j < 4; ++j) acc[p][i][j] = fmaf(a[p][i], b[p][j], acc[p][i][j]);
     }
   }
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  // group g finishes row g of each thread's four; C's reads before its writes
+  const int m = m0 + 2 * tx + (grp & 1) + 16 * (grp >> 1);
+  float *c[4];
+  float old[4][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int j = 0; j < 4; ++j) {
+    const int n = n0 + 2 * ty + (j & 1) + 16 * (j >> 1);
+    const bool in = m < M && n < N;
+    c[j] = in ? C + 2 * ((long long)n * ldc + m) : nullptr;
+    old[j][0] = in ? c[j][0] : 0.f;
+    old[j][1] = in ? c[j][1] : 0.f;
+  }
+  float *red = reinterpret_cast<float *>(csm);  // [p][i][j][group][64]
+  __syncthreads();  // every thread is done with the last panel
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int m = m0 + tx * 4 + i, n = n0 + ty * 4 + j;
-      if (m < M && n < N)
-        epilogue3m<float>(C, ldc, m, n, acc[0][i][j], acc[1][i][j], acc[2][i][j], ar, ai, br, bi);
+  for (int p = 0; p < 3; ++p)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) red[((p * 4 + i) * 4 + j) * 256 + tid] = acc[p][i][j];
+  __syncthreads();
+  const bool one = br == 1.f && bi == 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float s[3];
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      const float *r = red + ((p * 4 + grp) * 4 + j) * 256 + t64;
+      s[p] = (r[0] + r[64]) + (r[128] + r[192]);
     }
+    if (c[j] == nullptr) continue;
+    const float re = s[0] - s[1], im = s[2] - s[0] - s[1];
+    float cr = old[j][0], ci = old[j][1];
+    if (!one) {
+      const float tr = br * cr - bi * ci, ti = br * ci + bi * cr;
+      cr = tr;
+      ci = ti;
+    }
+    c[j][0] = cr + (ar * re - ai * im);
+    c[j][1] = ci + (ar * im + ai * re);
+  }
+}
+
+template <bool AK, bool BK>
+int launch_cgemm3m(int m, int n, int k, const float *A, int lda, const float *B, int ldb, float *C,
+                   int ldc, float ar, float ai, float br, float bi, float sa, float sb,
+                   cudaStream_t s) {
+  const int tm = (m + C_T - 1) / C_T, tn = (n + C_T - 1) / C_T;
+  B2_PROF("cgemm3m_fused", s);
+  cgemm3m_kernel<AK, BK><<<(unsigned)tm * (unsigned)tn, 256, C_SMEM, s>>>(
+      m, n, k, reinterpret_cast<const float2 *>(A), lda, reinterpret_cast<const float2 *>(B), ldb,
+      C, ldc, ar, ai, br, bi, sa, sb, tm, ((uintptr_t)A & 7) == 0, ((uintptr_t)B & 7) == 0);
+  B2_CUDA_TRY(cudaGetLastError());
+  return B2_OK;
 }
 
 // --------------------------------------- zgemm3m: one-launch FP64 DMMA --
@@ -697,19 +807,25 @@ int gemm3m_device(char ta, char tb, int m, int n, int k, const T *alpha, const T
     else
       return zgemm3m_three_gemms(ta, tb, m, n, k, ar, ai, br, bi, A, lda, B, ldb, C, ldc, s);
   }
-  dim3 grid((m + G_BM - 1) / G_BM, (n + G_BN - 1) / G_BN);
-  const int smem = (int)(12 * G_BK * G_LD * sizeof(T));
   if constexpr (sizeof(T) == 8) {
+    dim3 grid((m + G_BM - 1) / G_BM, (n + G_BN - 1) / G_BN);
+    const int smem = (int)(12 * G_BK * G_LD * sizeof(T));
     B2_CUDA_TRY(cudaFuncSetAttribute(zgemm3m_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     B2_PROF("zgemm3m_fused", s);
     zgemm3m_kernel<<<grid, 256, smem, s>>>(m, n, k, A, lda, B, ldb, C, ldc, ar, ai, br, bi, ta, tb);
+    B2_CUDA_TRY(cudaGetLastError());
+    return B2_OK;
   } else {
-    B2_CUDA_TRY(cudaFuncSetAttribute(cgemm3m_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    B2_PROF("cgemm3m_fused", s);
-    cgemm3m_kernel<<<grid, 256, smem, s>>>(m, n, k, A, lda, B, ldb, C, ldc, ar, ai, br, bi, ta, tb);
+    const bool ak = tr_is_t(ta), bk = !tr_is_t(tb);  // K contiguous in memory
+    const float sa = tr_is_conj(ta) ? -1.f : 1.f, sb = tr_is_conj(tb) ? -1.f : 1.f;
+    if (ak && bk)
+      return launch_cgemm3m<true, true>(m, n, k, A, lda, B, ldb, C, ldc, ar, ai, br, bi, sa, sb, s);
+    if (ak)
+      return launch_cgemm3m<true, false>(m, n, k, A, lda, B, ldb, C, ldc, ar, ai, br, bi, sa, sb, s);
+    if (bk)
+      return launch_cgemm3m<false, true>(m, n, k, A, lda, B, ldb, C, ldc, ar, ai, br, bi, sa, sb, s);
+    return launch_cgemm3m<false, false>(m, n, k, A, lda, B, ldb, C, ldc, ar, ai, br, bi, sa, sb, s);
   }
-  B2_CUDA_TRY(cudaGetLastError());
-  return B2_OK;
 }
 
 template int gemm3m_device<double>(char, char, int, int, int, const double *, const double *, int,
