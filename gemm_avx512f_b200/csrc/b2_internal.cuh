@@ -105,7 +105,7 @@ cudaStream_t pick_stream(Ctx *c, void *user_stream);
 
 // Plain FP64 GEMM on the DMMA tensor-core path (dgemm_fp64.cu).
 struct Fp64Cfg {
-  int tile = 0;    // 0: 128x128, 1: 128x64, 2: 64x64
+  int tile = 0;    // 0: 128x128, 1: 128x64, 2: 64x64, 3: 32x32 (DMMA K 4 only)
   int mmak = 4;    // DMMA K shape: 4, 8 or 16
   int split_k = 1; // >1: K split across CTAs, reduced in FP64 workspace
 };

@@ -7,7 +7,8 @@
 // mma.sync.aligned.m16n8k{4,8,16}.row.col.f64 with accumulators in registers.
 //
 // Design:
-//  * CTA tile BM x BN (128x128 / 128x64 / 64x64), warp tile 64x32 or 32x32;
+//  * CTA tile BM x BN (128x128 / 128x64 / 64x64 / 32x32), warp tile 64x32,
+//    32x32 or 16x16;
 //    fragments double-buffered in registers (DMMA K 4 and 8).
 //  * op(A)/op(B) tiles streamed global->shared with 16-byte cp.async (rows off
 //    a 16-byte boundary shifted by one element) through a STAGES-deep ring;
@@ -132,6 +133,12 @@ __global__ void __launch_bounds__(WM *WN * 32, BM * BN <= 64 * 64 && MMAK == 4 ?
         cp_async<16>(sA_u + st * (A_ST * 8) + run_tail_dst<BM, BK, A_KCONT>(tid),
                      A + run_tail<BM, BK, A_KCONT>(m0, k0, lda, tid),
                      (A_KCONT ? k0 + BK < kend : m0 + BM < M) ? 16 : 8);
+    } else if (full && !(a_first && kt == 0)) {
+#pragma unroll
+      for (int c = 0; c < A_CH; ++c)
+        cp_async_edge(da + st * (A_ST * 8) + c * run_dst_step<BM, BK, A_KCONT, NT>(),
+                      pa + c * ia, A, edge_bytes<BM, BK, A_KCONT, NT>(m0, M, tid, sha, c));
+      if (SH) load_tails<BM, BK, A_KCONT, NT>(sA_u + st * A_ST * 8, A, lda, m0, k0, M, kend, tid);
     } else {
 #pragma unroll
       for (int c = 0; c < A_CH; ++c)
@@ -148,6 +155,12 @@ __global__ void __launch_bounds__(WM *WN * 32, BM * BN <= 64 * 64 && MMAK == 4 ?
         cp_async<16>(sB_u + st * (B_ST * 8) + run_tail_dst<BN, BK, B_KCONT>(tid),
                      B + run_tail<BN, BK, B_KCONT>(n0, k0, ldb, tid),
                      (B_KCONT ? k0 + BK < kend : n0 + BN < N) ? 16 : 8);
+    } else if (full && !(b_first && kt == 0)) {
+#pragma unroll
+      for (int c = 0; c < B_CH; ++c)
+        cp_async_edge(db + st * (B_ST * 8) + c * run_dst_step<BN, BK, B_KCONT, NT>(),
+                      pb + c * ib, B, edge_bytes<BN, BK, B_KCONT, NT>(n0, N, tid, shb, c));
+      if (SH) load_tails<BN, BK, B_KCONT, NT>(sB_u + st * B_ST * 8, B, ldb, n0, k0, N, kend, tid);
     } else {
 #pragma unroll
       for (int c = 0; c < B_CH; ++c)
@@ -172,6 +185,8 @@ __global__ void __launch_bounds__(WM *WN * 32, BM * BN <= 64 * 64 && MMAK == 4 ?
   // running copy pointers and DMMA K 4 (whose fragments leave three CTAs per
   // SM) a block takes 0.553 us where it took 0.597 (K = 4096, 10 tiles per SM;
   // 4096^3 4228 -> 3886 us); one CTA alone on an SM 0.72 instead of 1.0.
+  // Edge tiles copy from running pointers too (bounds checked element by element
+  // they cost a lone CTA 1.34 us a block, now 0.90: 424x39x1600 21.3 -> 16.0 us).
   // Copies placed one by one between the DMMAs were slower (0.70).
   constexpr int KS = BK / MMAK;
   // (DMMA K 16 has one step per stage and twice the fragments: single-buffered.)
@@ -383,6 +398,9 @@ cudaError_t launch_tile(int tile, bool ak, bool bk, const LaunchArgs &a, cudaStr
   switch (tile) {
     case 0: return launch_layout<128, 128, 2, 4, 4, MMAK, SH>(ak, bk, a, s);
     case 1: return launch_layout<128, 64, 2, 2, 4, MMAK, SH>(ak, bk, a, s);
+    case 3:  // fp64_call_cfg's, DMMA K 4 only
+      if constexpr (MMAK == 4) return launch_layout<32, 32, 2, 2, 4, 4, SH>(ak, bk, a, s);
+      else return cudaErrorInvalidValue;
     default: return launch_layout<64, 64, 2, 2, 4, MMAK, SH>(ak, bk, a, s);
   }
 }
@@ -391,38 +409,88 @@ inline bool is_notrans(char c) { return c == 'N' || c == 'n'; }
 
 }  // namespace
 
+namespace {
+
+// Model of the 64x64 tile's time in us over S = 1, 2, 4, 8 slices of K; the best S
+// in *sk.  q = work units (tiles x slices) per SM, each of `kit` K blocks of 16
+// that take the FP64 pipe 0.53 us; a lone CTA per SM reaches 74 % of that rate,
+// up to four 91 %, more 95 %; 3 us to fill and drain, 1 us per further wave of
+// three; rows off a 16-byte boundary cost 9 % (shared-memory conflicts).  A
+// split adds a second launch (1.5 us on the device and 2 on the host, which
+// bounds a run of small calls: 128x128x128 8.2 us a call in two launches, 6.0
+// in one) and 64 KB of partials per unit, written and read at about 8 TB/s
+// (they stay in L2).  Measured (B200, us, graph replays):
+//   128x4096x128   S=1 9.2  2 12.4  4 13.0  8 16.2     512^3  26.4 17.1 15.7 17.6
+//   512x1024x512   26.6 26.6 27.3 27.3     2048^3  504 541 551 588
+// (one fixed rule, 8 slices up to 1024 units, took the last column of the
+// first three).
+double model64(int m, int n, int k, int sms, bool shifted, int *sk) {
+  const long long tiles = (long long)((m + 63) / 64) * ((n + 63) / 64);
+  double best = 1e300;
+  for (int s = 1; s <= 8 && (s == 1 || tiles < 8192); s *= 2) {
+    if (s > 1 && k < 8 * s) break;
+    const long long units = tiles * s, q = (units + sms - 1) / sms;
+    const int kit = ((k + s - 1) / s + 15) / 16;
+    const double rate = q == 1 ? 0.74 : q <= 4 ? 0.91 : 0.95;
+    double us = (double)q * kit * 0.53 / rate * (shifted ? 1.09 : 1.0) + 3.0 +
+                (double)((q + 2) / 3 - 1);
+    if (s > 1) us += 3.5 + (double)units * 65536.0 / 8e6;
+    if (us < best) best = us, *sk = s;
+  }
+  return best;
+}
+
+// The same for the 32x32 tile: up to five CTAs per SM, 0.24 us per K block for
+// one CTA alone on an SM, 0.33 for two, 0.148 each from three on (0.139 a
+// quarter of a 64x64 tile), 0.8 us per further wave of five, 16 KB of partials
+// per unit; 5 % for tiles past an edge, 20 % for shifted rows (40 % for a lone
+// CTA, whose copies are on its critical path).
+double model32(int m, int n, int k, int sms, bool shifted, int *sk) {
+  const long long tm = (m + 31) / 32, tn = (n + 31) / 32;
+  double best = 1e300;
+  for (int s = 1; s <= 8 && tn <= 65535; s *= 2) {
+    if (s > 1 && (k < 8 * s || tm * tn >= 8192)) break;
+    const long long units = tm * tn * s, qc = (units + sms - 1) / sms;
+    const double q = qc <= 6 ? (double)qc : (double)units / sms;
+    const int kit = ((k + s - 1) / s + 15) / 16;
+    const double block = qc == 1 ? 0.24 : qc == 2 ? 0.33 : 0.148 * q;
+    double us = kit * block * (!shifted ? 1.0 : qc == 1 ? 1.4 : 1.2) *
+                    (m % 32 || n % 32 ? 1.05 : 1.0) + 2.2 +
+                0.8 * (double)((qc + 4) / 5 - 1);
+    if (s > 1) us += 3.5 + (double)units * 16384.0 / 8e6;
+    if (us < best) best = us, *sk = s;
+  }
+  return best;
+}
+
+}  // namespace
+
+// The 64x64 tile (three CTAs per SM) is the best of the three tiles of the
+// tuner's list from 1024^3 to 8192^3 and in the exhaustive sweep over M, N, K in
+// [16, 1024]; K in the slices that its model likes best.
 Fp64Cfg fp64_default_cfg(int m, int n, int k, int sm_count) {
-  // The 64x64 tile (three CTAs per SM) is the best of the three tiles from
-  // 1024^3 to 8192^3 and in the exhaustive sweep over M, N, K in [16, 1024].
-  // The K split is the one of 1, 2, 4, 8 with the smallest modelled time:
-  // q = work units (tiles x slices) per SM, each of `kit` K blocks of 16 that
-  // take the FP64 pipe 0.53 us; a lone CTA per SM reaches 74 % of that rate,
-  // two 91 %; 3 us to fill and drain, 1 us per further wave of three; a split
-  // adds a second launch (1.5 us on the device and 2 on the host, which bounds a
-  // run of small calls: 128x128x128 11.2 us a call in two launches, 9.1 in one) and
-  // 64 KB of partials per unit, written and read at about 8 TB/s (they stay in
-  // L2).  Measured (B200, us, graph replays):
-  //   128x4096x128   S=1 9.7  2 11.7  4 12.7  8 15.4     512^3  28.3 17.6 15.5 17.5
-  //   512x1024x512   28.4 26.1 27.6 27.4     256^3  15.7 10.5 7.4 6.2
-  // (one fixed rule, 8 slices up to 1024 units, took the last column of the
-  // first three).
   Fp64Cfg c;
   c.tile = 2;
   c.mmak = 4;
-  const long long t64 = (long long)((m + 63) / 64) * ((n + 63) / 64);
+  model64(m, n, k, sm_count > 0 ? sm_count : 148, false, &c.split_k);
+  return c;
+}
+
+// A call's own choice (no configuration asked for): the 32x32 tile where the
+// models find it faster.  Four times the tiles fill the SMs where 64x64 ones
+// leave them one chain of K blocks or an uneven last wave; from about 2048^3 on
+// its extra shared reads lose.  B200, us, the better S of each, 64x64 / 32x32:
+//   48x40x64 3.8 / 2.8     256^3 5.9 / 5.1        424x39x1600 16.0 / 10.3
+//   512^3 15.7 / 12.8      900^3 65.3 / 58.3      1024^3 76.3 / 70.8
+//   1536x1024x2048 217 / 211    2048^3 504 / 525  4096^3 3896 / 4083
+static Fp64Cfg fp64_call_cfg(int m, int n, int k, int sm_count, bool shifted) {
   const int sms = sm_count > 0 ? sm_count : 148;
-  int sk = 1;
-  double best = 1e300;
-  for (int s = 1; s <= 8 && t64 < 8192; s *= 2) {
-    if (s > 1 && k < 8 * s) break;
-    const long long units = t64 * s, q = (units + sms - 1) / sms;
-    const int kit = ((k + s - 1) / s + 15) / 16;
-    const double rate = q == 1 ? 0.74 : q == 2 ? 0.91 : 0.98;
-    double us = (double)q * kit * 0.53 / rate + 3.0 + (double)((q + 2) / 3 - 1);
-    if (s > 1) us += 3.5 + units * 65536.0 / 8e6;
-    if (us < best) best = us, sk = s;
-  }
-  c.split_k = sk;
+  Fp64Cfg c;
+  c.mmak = 4;
+  int s64 = 1, s32 = 1;
+  const bool small = model32(m, n, k, sms, shifted, &s32) < model64(m, n, k, sms, shifted, &s64);
+  c.tile = small ? 3 : 2;
+  c.split_k = small ? s32 : s64;
   return c;
 }
 
@@ -458,13 +526,13 @@ int dgemm_fp64(char ta, char tb, int m, int n, int k, double alpha, const double
   Ctx *cx = ctx();
   if (!cx) return B2_ERR_NO_DEVICE;
   if (k <= 0 || alpha == 0.0) return beta == 1.0 ? B2_OK : scale_matrix_d(m, n, beta, C, ldc, s);
-  Fp64Cfg cfg = cfg_in            ? *cfg_in
-                : cx->fp64_override ? fp64_override_cfg()
-                                    : fp64_default_cfg(m, n, k, cx->sm_count);
   const bool ak = !is_notrans(ta);  // transposed A: k contiguous
   const bool bk = is_notrans(tb);   // plain B: k contiguous
   const bool vec2 = (lda % 2 == 0) && (ldb % 2 == 0) && (((uintptr_t)A & 15) == 0) &&
                     (((uintptr_t)B & 15) == 0);
+  Fp64Cfg cfg = cfg_in            ? *cfg_in
+                : cx->fp64_override ? fp64_override_cfg()
+                                    : fp64_call_cfg(m, n, k, cx->sm_count, !vec2);
   LaunchArgs a{m, n, k, k, alpha, A, lda, B, ldb, beta, C, ldc, nullptr, 0, 1};
   int splits = cfg.split_k < 1 ? 1 : cfg.split_k;
   if (splits > 1) {

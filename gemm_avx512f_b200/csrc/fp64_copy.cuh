@@ -116,6 +116,23 @@ __host__ __device__ constexpr uint32_t run_dst_step() {
   return (uint32_t)(NT / ((KCONT ? BK : OUTER) / 2) * (KCONT ? BK + 4 : OUTER + 4)) * 8u;
 }
 
+// A tile that reaches past the operand's outer limit, K block inside: a chunk's
+// copies from the same running pointers need only its byte count, from the
+// thread's rows left (KCONT) or its pair's place on the row.
+template <int OUTER, int BK, bool KCONT, int NT>
+__device__ __forceinline__ int edge_bytes(int o0, int olim, int tid, int sh, int c) {
+  constexpr int CPR = (KCONT ? BK : OUTER) / 2;
+  if (KCONT) return c * (NT / CPR) < olim - o0 - tid / CPR ? 16 : 0;
+  const int have = olim - (o0 + (tid % CPR) * 2 - sh);
+  return have >= 2 ? 16 : have == 1 ? 8 : 0;
+}
+__device__ __forceinline__ void cp_async_edge(uint32_t dst, const double *src, const double *g,
+                                              int bytes) {
+  const double *none = reinterpret_cast<const double *>(reinterpret_cast<uintptr_t>(g) &
+                                                        ~(uintptr_t)15);
+  cp_async<16>(dst, bytes ? src : none, bytes);
+}
+
 // Operand offset and shared byte offset of the chunk past the end of row tid.
 template <int OUTER, int BK, bool KCONT>
 __device__ __forceinline__ size_t run_tail(int o0, int k0, int ld, int tid) {

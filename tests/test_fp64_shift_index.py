@@ -26,7 +26,8 @@ def _stage(mem, base, ld, kcont, outer, o0, k0, olim, klim, kbeg, kt):
     r0, c0 = (o0, k0) if kcont else (k0, o0)
     rlim, clim = (olim, klim) if kcont else (klim, olim)
     first = (o0 if kcont else kbeg) == 0
-    inside = o0 + outer <= olim and k0 + BK <= klim and not (kt == 0 and first)
+    run = k0 + BK <= klim and not (kt == 0 and first)  # from running pointers
+    inside = run and o0 + outer <= olim
     cpr = length // 2
     for tid in range(NT):
         sh = (base + (r0 + tid // cpr) * ld) & 1
@@ -39,6 +40,16 @@ def _stage(mem, base, ld, kcont, outer, o0, k0, olim, klim, kbeg, kt):
                 assert a % 2 == 0 and a >= base
                 for j in range(2):
                     sm[hi * pitch + lo + j] = mem[a + j]
+            elif run:  # past the outer limit: edge_bytes
+                if kcont:
+                    valid = 2 if i * (NT // cpr) < olim - o0 - tid // cpr else 0
+                else:
+                    valid = max(0, min(2, olim - (o0 + (tid % cpr) * 2 - sh)))
+                a = base + (r0 + hi) * ld + c0 + lo - sh
+                if valid:
+                    assert a % 2 == 0 and a >= base
+                for j in range(2):
+                    sm[hi * pitch + lo + j] = mem[a + j] if j < valid else 0
             else:
                 _copy_pair(mem, sm, hi * pitch + lo, base, ld, r0 + hi, rlim, c0 + lo - sh, clim,
                            True)
@@ -56,10 +67,10 @@ class _Mem(dict):
 
 @pytest.mark.parametrize("kcont", [True, False])
 @pytest.mark.parametrize("base", [0, 1])
+@pytest.mark.parametrize("outer", [64, 32])
 @pytest.mark.parametrize("outer_n,kn,pad", [(64, 16, 1), (65, 33, 0), (130, 47, 1), (63, 15, 2),
                                             (129, 32, 0), (1, 1, 0)])
-def test_shifted_rows_hold_what_the_fragments_read(kcont, base, outer_n, kn, pad):
-    outer = 64
+def test_shifted_rows_hold_what_the_fragments_read(kcont, base, outer, outer_n, kn, pad):
     ld = (kn if kcont else outer_n) + pad
     nrows = outer_n if kcont else kn
     last = base + (nrows - 1) * ld + (kn if kcont else outer_n)

@@ -1,5 +1,5 @@
-"""GPU tests of the FP64 split-K forms (csrc/dgemm_fp64.cu): up to 8 slices
-meet in one thread-block cluster, more write partials to workspace.
+"""GPU tests of the FP64 split-K forms and of operand copies off a 16-byte
+boundary (csrc/dgemm_fp64.cu).
 
 Tile edges, slice counts that are not powers of two, a last slice shorter than
 the others, odd leading dimensions (8-byte copies, scalar C) and padding rows
@@ -73,10 +73,11 @@ def test_operands_off_a_16_byte_boundary(cuda, ta, tb, offs):
             t[off:off + x.size] = torch.from_numpy(x.T.copy().reshape(-1)).to(cuda)
             return t[off:]
 
-        for tile in (0, 1, 2):
+        for tile in (0, 1, 2, None):  # None: the call's own choice, 32x32 at these sizes
             da, db, dc = up(a, offs[0]), up(b, offs[1]), up(c, 1)
             torch.cuda.synchronize()
-            assert _lib.lib().b2_set_fp64_config(tile, 4, 1) == 0
+            if tile is not None:
+                assert _lib.lib().b2_set_fp64_config(tile, 4, 1) == 0
             try:
                 blas.dgemm_device(ta, tb, m, n, k, 1.0, da, a.shape[0], db, b.shape[0], 0.5, dc,
                                   m + 1)
@@ -86,3 +87,29 @@ def test_operands_off_a_16_byte_boundary(cuda, ta, tb, offs):
             got = dc[:c.size].cpu().numpy().reshape(n, m + 1).T
             assert np.array_equal(got[m:], c[m:])
             assert normalized(got[:m], ref, k, opa, opb, U) <= 8, (m, n, k, tile)
+
+
+@pytest.mark.parametrize("ta,tb", [("N", "N"), ("N", "T"), ("T", "N"), ("T", "T")])
+def test_small_tile_edges(cuda, ta, tb):
+    """Sizes for which a call takes 32x32 tiles, in one slice and in several:
+    around the tile's edges and the K block of 16, long K on one tile, padding."""
+    import torch
+
+    rng = np.random.default_rng(29)
+    for m, n, k, pad in ((1, 1, 1, 0), (31, 33, 15, 0), (32, 32, 16, 2), (33, 31, 17, 1),
+                         (64, 65, 48, 0), (65, 96, 130, 3), (40, 24, 4099, 0), (300, 65, 1000, 0),
+                         (130, 1000, 64, 1)):
+        a = fmat(rng, *((m, k) if ta == "N" else (k, m)), pad=pad)
+        b = fmat(rng, *((k, n) if tb == "N" else (n, k)), pad=pad)
+        c = fmat(rng, m, n, pad=pad)
+        opa = a[:m] if ta == "N" else a[:k].T
+        opb = b[:k] if tb == "N" else b[:n].T
+        ref = (1.25 * (opa.astype(np.longdouble) @ opb.astype(np.longdouble))
+               - 0.5 * c[:m].astype(np.longdouble)).astype(np.float64)
+        da, db, dc = (torch.from_numpy(x.T.copy()).to(cuda) for x in (a, b, c))
+        torch.cuda.synchronize()
+        blas.dgemm_device(ta, tb, m, n, k, 1.25, da, a.shape[0], db, b.shape[0], -0.5, dc, m + pad)
+        torch.cuda.synchronize()
+        got = dc.cpu().numpy().T
+        assert np.array_equal(got[m:], c[m:]), "padding rows of C were written"
+        assert normalized(got[:m], ref, k, opa, opb, U) <= 8, (m, n, k)
