@@ -18,7 +18,7 @@
 // tiles are de-interleaved into shared memory; the post-additions and the
 // complex alpha/beta happen in the epilogue.  beta follows the reference
 // drivers (C scaled whenever beta != 1, src/gemm_driver.c:131).
-//   zgemm3m: FP64 DMMA (mma.sync.m16n8k4.f64), 64x32 tile, 8 warps of 16x16.
+//   zgemm3m: FP64 DMMA (mma.sync.m16n8k4.f64), 32x32 tile, 4 warps of 16x16.
 //   cgemm3m: FP32 FFMA, 32x32 tile, four groups of 64 threads of 4x4 outputs
 //   splitting each panel's k.
 #include <stdlib.h>
@@ -356,8 +356,8 @@ int launch_cgemm3m(int m, int n, int k, const float *A, int lda, const float *B,
 
 // --------------------------------------- zgemm3m: one-launch FP64 DMMA --
 // The fused 3M product for complex128 at any size, on the FP64 tensor path
-// (mma.sync.m16n8k4.f64; tcgen05 has no f64 kind).  CTA tile 64 x 32 complex
-// outputs, 8 warps of 16 x 16, two CTAs per SM; K in blocks of 16 complex
+// (mma.sync.m16n8k4.f64; tcgen05 has no f64 kind).  CTA tile 32 x 32 complex
+// outputs, 4 warps of 16 x 16, three CTAs per SM; K in blocks of 16 complex
 // elements streamed global -> shared by cp.async (one 16-byte complex element
 // per copy, zero filled outside the matrix) through a 3-deep ring.  The smem
 // tile keeps the interleaved (re, im) pairs, so one 16-byte shared load gives a
@@ -374,8 +374,11 @@ int launch_cgemm3m(int m, int n, int k, const float *A, int lda, const float *B,
 // fragments are loaded, across a stage's edge too, before the current step's
 // DMMAs issue, and tiles inside the matrices copy from running pointers.  The
 // earlier form (one 512-thread CTA of 64 x 64 per SM, fragments loaded at
-// their use) kept the pipe 75 % busy: 2048^3 1886 -> 1682 us on B200 (84 % busy).
-constexpr int Z_BM = 64, Z_BN = 32, Z_BK = 16, Z_WM = 4, Z_WN = 2, Z_STAGES = 3;
+// their use) kept the pipe 75 % busy: 2048^3 1886 -> 1680 us on B200 (84 % busy).
+// A 64 x 32 tile (two CTAs per SM) is no faster there and leaves small products
+// with few CTAs and uneven last waves: 48^3 6.5 us against 4.6, 255^3 23.9 / 16.0,
+// 1000^3 257 / 225, 1500^3 732 / 682, 2048^3 1679 / 1678.
+constexpr int Z_BM = 32, Z_BN = 32, Z_BK = 16, Z_WM = 2, Z_WN = 2, Z_STAGES = 3;
 constexpr int Z_NT = Z_WM * Z_WN * 32;
 
 template <bool KC>
@@ -412,7 +415,7 @@ __device__ __forceinline__ void z_mma(double (&c)[4], double a0, double a1, doub
 }
 
 template <bool A_KC, bool B_KC>
-__global__ void __launch_bounds__(Z_NT, 2)
+__global__ void __launch_bounds__(Z_NT, 3)
     zgemm3m_dmma_kernel(int M, int N, int K, const double2 *__restrict__ A, int lda,
                         const double2 *__restrict__ B, int ldb, double2 *__restrict__ C, int ldc,
                         double ar, double ai, double br, double bi, double sa, double sb) {
