@@ -4,8 +4,8 @@
 // built without -DDOUBLE driving the 48x8 tile of src/kernel/gemm_kernel.S,
 // and the m16 x n24 tiles of OpenBLAS-like_implementation/sgemm.c:366-412):
 // a CUDA-core kernel of paired FP32 FMAs (fma.rn.f32x2) with a 128x128 CTA
-// tile, 8x8 outputs per thread in registers, double-buffered shared-memory K
-// panels.  The tensor-core forms (TF32, 3xTF32, 3xBF16) run on the tcgen05
+// tile, 8x8 outputs per thread in registers, K panels in a cp.async ring, and a
+// 64x64 form for products that leave SMs idle.  The tensor-core forms (TF32, 3xTF32, 3xBF16) run on the tcgen05
 // engine (sgemm_tc.cu).
 #include "b2_methods.cuh"
 #include "b2_profile.cuh"
@@ -285,6 +285,193 @@ int ffma2_ksplit(long long tiles, int kblocks, int sms) {
   return best;
 }
 
+// ----------------------------------------------------------------------
+// Small products: 64 x 64 tiles, so that four times the CTAs share them, and
+// four groups of 64 threads of 8 x 8 outputs that take every fourth k of a panel
+// (a chain of K panels bounds a call that leaves SMs idle, and a panel is 0.4 us
+// here against 1.7 for a lone 128 x 128 CTA).  Shared reads and paired FMAs are
+// in the big tile's proportion.  The groups exchange column pairs of their sums
+// through shared memory; group g finishes pair g of each thread's four.
+// Slices of K (blockIdx.z) write their raw sums to P (plane, ldp); else C.
+constexpr int S4_T = 64, S4_K = 16, S4_LD = S4_T + 4, S4_STAGES = 4;
+constexpr int S4_PANEL = S4_K * S4_LD;
+constexpr int S4_SMEM = 3 * 16 * 256 * 4;  // the exchange; 48 KB
+static_assert(S4_STAGES * 2 * S4_PANEL * 4 <= S4_SMEM, "the ring fits where the exchange goes");
+
+template <bool TA, bool TB, bool VEC>
+__global__ void __launch_bounds__(256, 2)
+    sgemm_small_kernel(int M, int N, int K, float alpha, const float *__restrict__ A, int lda,
+                       const float *__restrict__ B, int ldb, float beta, float *__restrict__ C,
+                       int ldc, int kchunk, float *__restrict__ P, long long plane, int ldp,
+                       int tiles_m) {
+  constexpr bool KA = TA, KB = !TB;  // K contiguous in memory
+  constexpr bool VA = VEC && !KA, VB = VEC && !KB;
+  extern __shared__ __align__(16) float s4m[];
+  const uint32_t smu = (uint32_t)__cvta_generic_to_shared(s4m);
+  const int tid = threadIdx.x, lane = tid & 31, grp = tid >> 6, t64 = tid & 63;
+  const int rm = (lane & 7) * 4, cn = (t64 >> 3) * 4;
+  const int m0 = (int)(blockIdx.x % tiles_m) * S4_T, n0 = (int)(blockIdx.x / tiles_m) * S4_T;
+  const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
+  const int KT = (kend - kbeg + S4_K - 1) / S4_K;
+  unsigned long long acc[8][4];  // row 4 tx + i (+ 32 from i = 4), column pairs
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+  const bool in_a = m0 + S4_T <= M, in_b = n0 + S4_T <= N;
+  const float *pa = A + f32copy::run_offset<S4_T, KA, VA>(m0, kbeg, lda, tid);
+  const float *pb = B + f32copy::run_offset<S4_T, KB, VB>(n0, kbeg, ldb, tid);
+  const uint32_t da = f32copy::run_dst<S4_T, S4_LD, KA, VA>(tid);
+  const uint32_t db = f32copy::run_dst<S4_T, S4_LD, KB, VB>(tid) + S4_PANEL * 4u;
+  auto load_stage = [&](int st, int kt) {
+    const int k0 = kbeg + kt * S4_K;
+    const uint32_t d = smu + (uint32_t)(st * 2 * S4_PANEL) * 4u;
+    const bool full = k0 + S4_K <= kend;
+    if (full && in_a) f32copy::run_panel<S4_T, S4_LD, KA, VA>(d + da, pa, lda);
+    else f32copy::load_panel<S4_T, S4_LD, KA, VA>(d, A, lda, m0, k0, M, kend, tid);
+    if (full && in_b) f32copy::run_panel<S4_T, S4_LD, KB, VB>(d + db, pb, ldb);
+    else f32copy::load_panel<S4_T, S4_LD, KB, VB>(d + S4_PANEL * 4u, B, ldb, n0, k0, N, kend, tid);
+    pa += KA ? (size_t)S4_K : (size_t)S4_K * lda;
+    pb += KB ? (size_t)S4_K : (size_t)S4_K * ldb;
+  };
+#pragma unroll
+  for (int i = 0; i < S4_STAGES - 1; ++i) {
+    if (i < KT) load_stage(i, i);
+    asm volatile("cp.async.commit_group;\n" ::);
+  }
+  int st = 0, fill = S4_STAGES - 1;
+  for (int kt = 0; kt < KT; ++kt) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(S4_STAGES - 2));
+    __syncthreads();  // panel kt is in; every thread is done with the one refilled here
+    if (kt + S4_STAGES - 1 < KT) load_stage(fill, kt + S4_STAGES - 1);
+    asm volatile("cp.async.commit_group;\n" ::);
+    const float *As = s4m + st * 2 * S4_PANEL + grp * S4_LD + rm;
+    const float *Bs = s4m + st * 2 * S4_PANEL + S4_PANEL + grp * S4_LD + cn;
+    st = st + 1 == S4_STAGES ? 0 : st + 1;
+    fill = fill + 1 == S4_STAGES ? 0 : fill + 1;
+#pragma unroll
+    for (int kq = 0; kq < S4_K / 4; ++kq) {  // k = 4 kq + grp
+      const bool sa = KA && kq >= 2, sb = KB && kq >= 2;  // panel_at's order
+      unsigned long long bv[4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const ulonglong2 b2 = *reinterpret_cast<const ulonglong2 *>(&Bs[4 * kq * S4_LD + 32 * h]);
+        bv[2 * h] = sb ? b2.y : b2.x;
+        bv[2 * h + 1] = sb ? b2.x : b2.y;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float4 a4 = *reinterpret_cast<const float4 *>(&As[4 * kq * S4_LD + 32 * h]);
+        const float av[4] = {sa ? a4.z : a4.x, sa ? a4.w : a4.y, sa ? a4.x : a4.z,
+                             sa ? a4.y : a4.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const unsigned long long ai = dup2(av[i]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) ffma2(acc[4 * h + i][j], ai, bv[j]);
+        }
+      }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  __syncthreads();  // every thread is done with the last panel
+  unsigned long long *xch = reinterpret_cast<unsigned long long *>(s4m);  // [3][8][256]
+#pragma unroll
+  for (int r = 1; r < 4; ++r) {
+    const int q = (grp + r) & 3;  // the group that finishes pair q
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      xch[((r - 1) * 8 + i) * 256 + tid] = q == 0   ? acc[i][0]
+                                           : q == 1 ? acc[i][1]
+                                           : q == 2 ? acc[i][2]
+                                                    : acc[i][3];
+  }
+  const int n = n0 + cn + (grp >> 1) * 32 + (grp & 1) * 2;
+  float old[8][2];  // all of C's reads before its writes
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int m = m0 + rm + i + (i >> 2) * 28;
+      old[i][j] = (P == nullptr && m < M && n + j < N) ? C[(size_t)(n + j) * ldc + m] : 0.f;
+    }
+  __syncthreads();
+  const bool one = beta == 1.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const unsigned long long mine = grp == 0   ? acc[i][0]
+                                    : grp == 1 ? acc[i][1]
+                                    : grp == 2 ? acc[i][2]
+                                               : acc[i][3];
+    float2 v = *reinterpret_cast<const float2 *>(&mine);
+#pragma unroll
+    for (int r = 1; r < 4; ++r) {
+      const unsigned long long o = xch[((r - 1) * 8 + i) * 256 + ((grp - r) & 3) * 64 + t64];
+      const float2 w = *reinterpret_cast<const float2 *>(&o);
+      v.x += w.x;
+      v.y += w.y;
+    }
+    const int m = m0 + rm + i + (i >> 2) * 28;
+    const float x[2] = {v.x, v.y};
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      if (m >= M || n + j >= N) continue;
+      if (P != nullptr) P[blockIdx.z * plane + (size_t)(n + j) * ldp + m] = x[j];
+      else
+        C[(size_t)(n + j) * ldc + m] =
+            one ? fmaf(alpha, x[j], old[i][j]) : fmaf(alpha, x[j], beta * old[i][j]);
+    }
+  }
+}
+
+template <bool TA, bool TB, bool VEC>
+int launch_small(int m, int n, int k, float alpha, const float *A, int lda, const float *B,
+                 int ldb, float beta, float *C, int ldc, int S, Ctx *cx, cudaStream_t s) {
+  const int tm = (m + S4_T - 1) / S4_T, tn = (n + S4_T - 1) / S4_T;
+  const int kblocks = (k + S4_K - 1) / S4_K, ldp = (m + 3) & ~3;
+  const long long plane = (long long)n * ldp;
+  int kchunk = (kblocks + S - 1) / S * S4_K;
+  S = (k + kchunk - 1) / kchunk;
+  float *P = S > 1 ? (float *)workspace(cx, WS_MISC, (size_t)plane * S * sizeof(float)) : nullptr;
+  if (P == nullptr) S = 1, kchunk = k;  // no scratch for the slices: one
+  {
+    B2_PROF("sgemm_simt", s);
+    sgemm_small_kernel<TA, TB, VEC><<<dim3((unsigned)tm * (unsigned)tn, 1, S), 256, S4_SMEM, s>>>(
+        m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, kchunk, P, plane, ldp, tm);
+    B2_CUDA_TRY(cudaGetLastError());
+  }
+  if (S == 1) return B2_OK;
+  return sgemm_splitk_reduce(P, plane, ldp, S, m, n, alpha, beta, C, ldc, s);
+}
+
+// K slices of the small-tile kernel for a product whose 128 x 128 tiles leave
+// slots empty, or 0 where those (in S slices) are modelled faster.  Both models:
+// K panels of 16 in a row times a panel's time at q work units per SM, the ends,
+// and for slices a second launch (1.5 us on the device, 2 on the host) and the
+// partials at 8 TB/s.  128 x 128: 1.47 us a panel alone on an SM, 1.37 a unit
+// from two on (4-byte copies 12 % more); 64 x 64: 0.46 and 0.43 (20 %).  B200, us,
+// 128 x 128 / 64 x 64: 128^3 15.3 / 7.0, 256^3 27.0 / 8.0, 512^3 47.3 / 13.4, 700^3
+// 74.3 / 27.8, 384x240x848 90.8 / 12.4, 128x128x8192 115 / 24.9; 1024^3 54.3 / 60.7,
+// 1500^3 145 / 173, 2048x1024x512 50.7 / 62.3.
+int small_slices(int m, int n, int kblocks, long long tiles, int S, bool vec, int sms) {
+  const auto ends = [](int s, long long units, double bytes) {
+    return s > 1 ? 3.5 + (double)units * bytes / 8e6 : 0.0;
+  };
+  const long long ub = tiles * S, qb = (ub + sms - 1) / sms;
+  double best = 3.5 + (kblocks + S - 1) / S * (qb == 1 ? 1.47 : 1.37 * qb) * (vec ? 1.0 : 1.12) +
+                ends(S, ub, 131072.0);
+  int pick = 0;
+  const long long t64 = (long long)((m + S4_T - 1) / S4_T) * ((n + S4_T - 1) / S4_T);
+  for (const int s : {1, 2, 3, 4, 6, 8, 16}) {
+    if (s > 1 && kblocks < 4 * s) break;
+    const long long u = t64 * s, q = (u + sms - 1) / sms;
+    const double us = 4.4 + (kblocks + s - 1) / s * (q == 1 ? 0.46 : 0.43 * q) * (vec ? 1.0 : 1.2) +
+                      ends(s, u, 32768.0);
+    if (us < best) best = us, pick = s;
+  }
+  return pick;
+}
+
 template <bool TA, bool TB, bool VEC>
 int launch_ffma2(int m, int n, int k, float alpha, const float *A, int lda, const float *B,
                  int ldb, float beta, float *C, int ldc, cudaStream_t s) {
@@ -297,6 +484,11 @@ int launch_ffma2(int m, int n, int k, float alpha, const float *A, int lda, cons
   if (tiles > 0x7fffffffll) return B2_ERR_ARG;
   const int kblocks = (k + S2_K - 1) / S2_K;
   const int S = ffma2_ksplit(tiles, kblocks, cx->sm_count);
+  if (tiles < slots) {
+    const int Ss = small_slices(m, n, kblocks, tiles, S, VEC, cx->sm_count);
+    if (Ss > 0)
+      return launch_small<TA, TB, VEC>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, Ss, cx, s);
+  }
   if (S == 1) {
     // The tiles of whole waves run in full; the rest, when it would leave half
     // or more of the CTA slots empty, is cut into K slices that fill them, as a
