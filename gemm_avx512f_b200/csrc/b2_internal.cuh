@@ -34,6 +34,7 @@ enum WsSlot {
   WS_TRSM, WS_TRSM_INV, WS_3M, WS_GROUP, WS_ERR, WS_MISC,
   WS_KABI_A, WS_KABI_B, WS_KABI_D,         // kernel-ABI unpacked panels / 3M product
   WS_GROUP2,                                // second descriptor slot of one-shot grouped calls
+  WS_F32,                                   // FP32 products' K slices, never used by captured calls
   WS_COUNT
 };
 

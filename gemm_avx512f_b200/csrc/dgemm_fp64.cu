@@ -427,8 +427,8 @@ namespace {
 double model64(int m, int n, int k, int sms, bool shifted, int *sk) {
   const long long tiles = (long long)((m + 63) / 64) * ((n + 63) / 64);
   double best = 1e300;
-  for (int s = 1; s <= 8 && (s == 1 || tiles < 8192); s *= 2) {
-    if (s > 1 && k < 8 * s) break;
+  for (int s = 1; s <= 8; s *= 2) {
+    if (s > 1 && (k < 8 * s || tiles * s > 1024)) break;  // at most 32 MB of partials
     const long long units = tiles * s, q = (units + sms - 1) / sms;
     const int kit = ((k + s - 1) / s + 15) / 16;
     const double rate = q == 1 ? 0.74 : q <= 4 ? 0.91 : 0.95;
@@ -449,7 +449,7 @@ double model32(int m, int n, int k, int sms, bool shifted, int *sk) {
   const long long tm = (m + 31) / 32, tn = (n + 31) / 32;
   double best = 1e300;
   for (int s = 1; s <= 8 && tn <= 65535; s *= 2) {
-    if (s > 1 && (k < 8 * s || tm * tn >= 8192)) break;
+    if (s > 1 && (k < 8 * s || ((tm + 1) / 2) * ((tn + 1) / 2) * s > 1024)) break;  // as model64
     const long long units = tm * tn * s, qc = (units + sms - 1) / sms;
     const double q = qc <= 6 ? (double)qc : (double)units / sms;
     const int kit = ((k + s - 1) / s + 15) / 16;

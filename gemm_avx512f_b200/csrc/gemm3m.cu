@@ -14,8 +14,9 @@
 // of C and forms all three real products from the same staged tiles:
 //     P1 = Ar Br,  P2 = Ai Bi,  P3 = (Ar + Ai)(Br + Bi)
 //     Re(AB) = P1 - P2,  Im(AB) = P3 - P1 - P2
-// The pre-additions (and conjugation for 'C'/'R') happen while the complex
-// tiles are de-interleaved into shared memory; the post-additions and the
+// The pre-additions (and conjugation for 'C'/'R') are made on operand fragments
+// in registers (zgemm3m_kernel, for operands off a 16-byte boundary: while its
+// tiles are de-interleaved into shared memory); the post-additions and the
 // complex alpha/beta happen in the epilogue.  beta follows the reference
 // drivers (C scaled whenever beta != 1, src/gemm_driver.c:131).
 //   zgemm3m: FP64 DMMA (mma.sync.m16n8k4.f64), 32x32 tile, 4 warps of 16x16.

@@ -9,7 +9,7 @@
 // persistent grid pulls tile indices from a device-side atomic counter, finds
 // the owning problem through a tile -> problem map and runs the tile with the
 // problem's own dtype, transposes, strides and alpha/beta:
-//   FP64 tiles: DMMA mma.sync.m16n8k8.f64, 8 warps of 32 x 16;
+//   FP64 tiles: DMMA mma.sync.m16n8k4.f64, 8 warps of 32 x 16;
 //   FP32 tiles: paired FMAs (fma.rn.f32x2), 8 warps of 32 x 16, each lane 4 x 4;
 //   complex tiles (zgemm3m_ / cgemm3m_ problems): 32 x 32, the three real
 //   products of the 3M method on DMMA (complex128) or FFMA (complex64);
@@ -585,7 +585,7 @@ template <bool CPLX>
 __global__ void __launch_bounds__(256, GT_MINB)
     grouped_kernel(const GroupDesc *__restrict__ d, const int *__restrict__ tile_prob,
                    long long total_tiles, unsigned long long *counter) {
-  // two stages of A and B panels (GT_SMEM; GT_SMEM_3M when the batch has complex problems)
+  // the ring of A and B panels (GT_SMEM; GT_SMEM_3M when the batch has complex problems)
   extern __shared__ __align__(16) double sm[];
   __shared__ long long next_s;
   __shared__ GroupDesc desc;

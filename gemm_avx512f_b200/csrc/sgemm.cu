@@ -432,7 +432,7 @@ int launch_small(int m, int n, int k, float alpha, const float *A, int lda, cons
   const long long plane = (long long)n * ldp;
   int kchunk = (kblocks + S - 1) / S * S4_K;
   S = (k + kchunk - 1) / kchunk;
-  float *P = S > 1 ? (float *)workspace(cx, WS_MISC, (size_t)plane * S * sizeof(float)) : nullptr;
+  float *P = S > 1 ? (float *)workspace(cx, WS_F32, (size_t)plane * S * sizeof(float)) : nullptr;
   if (P == nullptr) S = 1, kchunk = k;  // no scratch for the slices: one
   {
     B2_PROF("sgemm_simt", s);
@@ -453,7 +453,8 @@ int launch_small(int m, int n, int k, float alpha, const float *A, int lda, cons
 // 128 x 128 / 64 x 64: 128^3 15.3 / 7.0, 256^3 27.0 / 8.0, 512^3 47.3 / 13.4, 700^3
 // 74.3 / 27.8, 384x240x848 90.8 / 12.4, 128x128x8192 115 / 24.9; 1024^3 54.3 / 60.7,
 // 1500^3 145 / 173, 2048x1024x512 50.7 / 62.3.
-int small_slices(int m, int n, int kblocks, long long tiles, int S, bool vec, int sms) {
+int small_slices(int m, int n, int kblocks, long long tiles, int S, bool vec, int sms,
+                 bool slices) {
   const auto ends = [](int s, long long units, double bytes) {
     return s > 1 ? 3.5 + (double)units * bytes / 8e6 : 0.0;
   };
@@ -463,7 +464,7 @@ int small_slices(int m, int n, int kblocks, long long tiles, int S, bool vec, in
   int pick = 0;
   const long long t64 = (long long)((m + S4_T - 1) / S4_T) * ((n + S4_T - 1) / S4_T);
   for (const int s : {1, 2, 3, 4, 6, 8, 16}) {
-    if (s > 1 && kblocks < 4 * s) break;
+    if (s > 1 && (!slices || kblocks < 4 * s)) break;
     const long long u = t64 * s, q = (u + sms - 1) / sms;
     const double us = 4.4 + (kblocks + s - 1) / s * (q == 1 ? 0.46 : 0.43 * q) * (vec ? 1.0 : 1.2) +
                       ends(s, u, 32768.0);
@@ -484,8 +485,13 @@ int launch_ffma2(int m, int n, int k, float alpha, const float *A, int lda, cons
   if (tiles > 0x7fffffffll) return B2_ERR_ARG;
   const int kblocks = (k + S2_K - 1) / S2_K;
   const int S = ffma2_ksplit(tiles, kblocks, cx->sm_count);
+  // Slices of the 64 x 64 form and of the last wave are for calls that run now: a
+  // captured one would hold scratch that a larger call may replace.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) (void)cudaGetLastError();
+  const bool capturing = cap != cudaStreamCaptureStatusNone;
   if (tiles < slots) {
-    const int Ss = small_slices(m, n, kblocks, tiles, S, VEC, cx->sm_count);
+    const int Ss = small_slices(m, n, kblocks, tiles, S, VEC, cx->sm_count, !capturing);
     if (Ss > 0)
       return launch_small<TA, TB, VEC>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, Ss, cx, s);
   }
@@ -499,16 +505,16 @@ int launch_ffma2(int m, int n, int k, float alpha, const float *A, int lda, cons
     int St = rest > 0 ? (int)(slots / rest) : 1;
     if (St > 8) St = 8;
     while (St > 1 && kblocks / St < 16) --St;
-    const bool tail = tiles > slots && tiles < 12 * slots && St >= 2;
-    const int whole = (int)(tail ? tiles - rest : tiles);
+    bool tail = !capturing && tiles > slots && tiles < 12 * slots && St >= 2;
     float *P = nullptr;
     int kchunk = k;
     if (tail) {
       kchunk = (kblocks + St - 1) / St * S2_K;
       St = (k + kchunk - 1) / kchunk;
-      P = (float *)workspace(cx, WS_MISC, (size_t)St * rest * S2_M * S2_N * sizeof(float));
-      if (!P) return B2_ERR_NOMEM;
+      P = (float *)workspace(cx, WS_F32, (size_t)St * rest * S2_M * S2_N * sizeof(float));
+      if (!P) tail = false;  // no scratch: the last wave in full
     }
+    const int whole = (int)(tail ? tiles - rest : tiles);
     B2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S2_SMEM));
     {
       B2_PROF("sgemm_simt", s);

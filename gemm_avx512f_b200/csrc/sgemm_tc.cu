@@ -520,27 +520,10 @@ int cgemm3m_tensor(char ta, char tb, int m, int n, int k, float ar, float ai, fl
   const bool cB = tb == 'C' || tb == 'c' || tb == 'R' || tb == 'r';
   const int kp = (int)round_up(k, 32);
   const long long ks = 2LL * kp;
-  float *Xp = (float *)workspace(cx, WS_SPLIT_X, (size_t)(3 * m * ks) * sizeof(float));
-  float *Yp = (float *)workspace(cx, WS_SPLIT_Y, (size_t)(3 * n * ks) * sizeof(float));
-  if (!Xp || !Yp) return B2_ERR_NOMEM;
-  {
-    const unsigned kt = (unsigned)kp / 32;
-    const unsigned ba = kt * ((unsigned)(m + 63) / 64), bb = kt * ((unsigned)(n + 63) / 64);
-    B2_PROF("gemm3m_prep", s);
-    B2_CUDA_TRY(launch_dependent(split3m_kernel, ba + bb, 256, s, split3_op(A, lda, !tA, cA, m, Xp),
-                                 split3_op(B, ldb, tB, cB, n, Yp), ba, k, kp));
-  }
   // engine and K ranges as for one 3xTF32 SGEMM of this shape
   const SgCfg cfg = sgemm_pick_cfg('N', 'N', m, n, k, 1, B2_METHOD_TF32X3);
   const int eng = (cfg.engine >= 0 && cfg.engine <= 2) ? cfg.engine : 0;
   const int tile_p = eng == 2 ? 256 : umma::BM, tile_q = eng == 1 ? 128 : 256;
-  CUtensorMap tmX, tmY;
-  int rc = umma::make_kmajor_map(&tmX, umma::KIND_TF32, Xp, ks, m, 3, ks * 4, (long long)m * ks * 4,
-                                 umma::BM);
-  if (rc == B2_OK)
-    rc = umma::make_kmajor_map(&tmY, umma::KIND_TF32, Yp, ks, n, 3, ks * 4, (long long)n * ks * 4,
-                               eng == 0 ? 256 : 128);
-  if (rc != B2_OK) return rc;
   const int seg_kb = kp * 4 / umma::KBLOCK_BYTES, kblocks = seg_kb;
   const long long tiles = ((n + tile_q - 1) / tile_q) * (long long)((m + tile_p - 1) / tile_p);
   const int slots = eng == 2 ? cx->sm_count / 2 : cx->sm_count;
@@ -553,8 +536,25 @@ int cgemm3m_tensor(char ta, char tb, int m, int n, int k, float ar, float ai, fl
   const int E = (S + per - 1) / per;
   const int ldw = (int)round_up(m, 32);
   const long long plane = (long long)n * ldw;
-  float *W = (float *)workspace(cx, WS_3M, (size_t)plane * 3 * E * sizeof(float));
-  if (!W) return B2_ERR_NOMEM;
+  // the split segments of both operands, then the products' sums
+  float *Xp = (float *)workspace(
+      cx, WS_3M, (size_t)(3 * (m + (long long)n) * ks + plane * 3 * E) * sizeof(float));
+  if (!Xp) return B2_ERR_NOMEM;
+  float *Yp = Xp + 3 * m * ks, *W = Yp + 3 * n * ks;
+  {
+    const unsigned kt = (unsigned)kp / 32;
+    const unsigned ba = kt * ((unsigned)(m + 63) / 64), bb = kt * ((unsigned)(n + 63) / 64);
+    B2_PROF("gemm3m_prep", s);
+    B2_CUDA_TRY(launch_dependent(split3m_kernel, ba + bb, 256, s, split3_op(A, lda, !tA, cA, m, Xp),
+                                 split3_op(B, ldb, tB, cB, n, Yp), ba, k, kp));
+  }
+  CUtensorMap tmX, tmY;
+  int rc = umma::make_kmajor_map(&tmX, umma::KIND_TF32, Xp, ks, m, 3, ks * 4, (long long)m * ks * 4,
+                                 umma::BM);
+  if (rc == B2_OK)
+    rc = umma::make_kmajor_map(&tmY, umma::KIND_TF32, Yp, ks, n, 3, ks * 4, (long long)n * ks * 4,
+                               eng == 0 ? 256 : 128);
+  if (rc != B2_OK) return rc;
   rc = run_engine(eng, false, 3, tmX, tmY, m, n, kp, 3, seg_kb, Ranges{E, per * kbps, kbps},
                   F32PartialEpi{W, plane, ldw, m, n}, cx, s);
   if (rc != B2_OK) return rc;

@@ -123,9 +123,9 @@ B2_API void dtrsm_(const char *side, const char *uplo, const char *transa, const
  * cgemm3m_kernel_16x4_skylakex.c:415-440.  zgemm3m products below 2^35
  * multiply-adds (2048^3 included) and cgemm3m products below 2^24 run all
  * three real products and the pre/post additions in one fused launch;
- * larger ones run the three real products as FP64 DMMA GEMMs (zgemm3m) or
- * 3xTF32 tensor-core GEMMs (cgemm3m, FP32-class accuracy) between a pre-add
- * pass and a combine pass. */
+ * larger ones run the three real products as FP64 DMMA GEMMs between a pre-add
+ * pass and a combine pass (zgemm3m), or as one batched 3xTF32 tensor-core GEMM
+ * between a split pass and a combine pass (cgemm3m, FP32-class accuracy). */
 B2_API void zgemm3m_(const char *transa, const char *transb, const int *m, const int *n, const int *k,
               const double *alpha, const double *a, const int *lda, const double *b,
               const int *ldb, const double *beta, double *c, const int *ldc);

@@ -46,3 +46,33 @@ def test_small_products(cuda, m, n, k, off, pad):
             bound = (k + 4) * 2.0 ** -24 * (1.25 * (np.abs(oa) @ np.abs(ob)) + np.abs(c))
             err = np.abs(got[:, :m].T.astype(np.float64) - (1.25 * (oa @ ob) - 0.5 * c))
             assert (err <= bound).all(), (ta, tb)
+
+
+@pytest.mark.parametrize("m,n,k", [(384, 240, 848), (3072, 3072, 512)])
+def test_captured_calls_hold_no_scratch(cuda, m, n, k):
+    """A captured call allocates nothing, and its graph stays right after a
+    larger call has replaced the scratch that running calls slice K with."""
+    import torch
+
+    def product(rows, cols, inner, st):
+        a, b = (torch.rand(x, device=cuda) for x in (rows * inner, inner * cols))
+        c = torch.zeros(rows * cols, device=cuda)
+        call = lambda: blas.sgemm_device("N", "N", rows, cols, inner, 1.0, a, rows, b, inner, 0.0, c,  # noqa: E731
+                                         rows, method="fp32", stream=st)
+        return a, b, c, call
+
+    st = torch.cuda.Stream()
+    a, b, c, call = product(m, n, k, st)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(st):
+        with torch.cuda.graph(graph, stream=st):
+            call()
+    big = product(4096, 4096, 1024, st)
+    torch.cuda.synchronize()
+    big[3]()
+    graph.replay()
+    torch.cuda.synchronize()
+    ref = a.view(k, m).double().T @ b.view(n, k).double().T
+    err = (c.view(n, m).T.double() - ref).abs().max()
+    assert err <= (k + 4) * 2.0 ** -24 * ref.max()  # all operands are positive
