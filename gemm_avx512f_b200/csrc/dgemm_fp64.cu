@@ -416,15 +416,15 @@ namespace {
 // that take the FP64 pipe 0.53 us; a lone CTA per SM reaches 74 % of that rate,
 // up to four 91 %, more 95 %; 3 us to fill and drain, 1 us per further wave of
 // three; rows off a 16-byte boundary cost 9 % (shared-memory conflicts).  A
-// split adds a second launch (1.5 us on the device and 2 on the host, which
-// bounds a run of small calls: 128x128x128 8.2 us a call in two launches, 6.0
+// split adds a second launch (split_us; 1.5 us on the device and 2 on the host,
+// which bounds a run of small calls: 128x128x128 8.2 us a call in two launches, 6.0
 // in one) and 64 KB of partials per unit, written and read at about 8 TB/s
 // (they stay in L2).  Measured (B200, us, graph replays):
 //   128x4096x128   S=1 9.2  2 12.4  4 13.0  8 16.2     512^3  26.4 17.1 15.7 17.6
 //   512x1024x512   26.6 26.6 27.3 27.3     2048^3  504 541 551 588
 // (one fixed rule, 8 slices up to 1024 units, took the last column of the
 // first three).
-double model64(int m, int n, int k, int sms, bool shifted, int *sk) {
+double model64(int m, int n, int k, int sms, bool shifted, double split_us, int *sk) {
   const long long tiles = (long long)((m + 63) / 64) * ((n + 63) / 64);
   double best = 1e300;
   for (int s = 1; s <= 8; s *= 2) {
@@ -434,7 +434,7 @@ double model64(int m, int n, int k, int sms, bool shifted, int *sk) {
     const double rate = q == 1 ? 0.74 : q <= 4 ? 0.91 : 0.95;
     double us = (double)q * kit * 0.53 / rate * (shifted ? 1.09 : 1.0) + 3.0 +
                 (double)((q + 2) / 3 - 1);
-    if (s > 1) us += 3.5 + (double)units * 65536.0 / 8e6;
+    if (s > 1) us += split_us + (double)units * 65536.0 / 8e6;
     if (us < best) best = us, *sk = s;
   }
   return best;
@@ -467,12 +467,13 @@ double model32(int m, int n, int k, int sms, bool shifted, int *sk) {
 
 // The 64x64 tile (three CTAs per SM) is the best of the three tiles of the
 // tuner's list from 1024^3 to 8192^3 and in the exhaustive sweep over M, N, K in
-// [16, 1024]; K in the slices that its model likes best.
+// [16, 1024]; K in the slices that its model likes best on the device (2 us a
+// second launch: the tuner's configurations are compared by their device time).
 Fp64Cfg fp64_default_cfg(int m, int n, int k, int sm_count) {
   Fp64Cfg c;
   c.tile = 2;
   c.mmak = 4;
-  model64(m, n, k, sm_count > 0 ? sm_count : 148, false, &c.split_k);
+  model64(m, n, k, sm_count > 0 ? sm_count : 148, false, 2.0, &c.split_k);
   return c;
 }
 
@@ -488,7 +489,8 @@ static Fp64Cfg fp64_call_cfg(int m, int n, int k, int sm_count, bool shifted) {
   Fp64Cfg c;
   c.mmak = 4;
   int s64 = 1, s32 = 1;
-  const bool small = model32(m, n, k, sms, shifted, &s32) < model64(m, n, k, sms, shifted, &s64);
+  const bool small = model32(m, n, k, sms, shifted, &s32) <
+                     model64(m, n, k, sms, shifted, 3.5, &s64);
   c.tile = small ? 3 : 2;
   c.split_k = small ? s32 : s64;
   return c;
