@@ -32,11 +32,11 @@ _ref = {}
 
 def reference_dir() -> str | None:
     """The reference's source tree: $B2_REFERENCE_DIR, else a directory named
-    ``reference`` beside this repository's root, when it exists; None
+    ``reference`` beside this repository's root, when it holds the sources; None
     otherwise (then only the prebuilt _ref/ files, if any, are used)."""
     cand = os.environ.get("B2_REFERENCE_DIR") or os.path.join(
         os.path.dirname(os.path.dirname(HERE)), "reference")
-    return cand if os.path.isdir(cand) else None
+    return cand if os.path.isfile(os.path.join(cand, "src", "gemm_driver.c")) else None
 
 
 def build(reference: str | None = None, quiet: bool = True) -> None:
