@@ -28,62 +28,37 @@ namespace b2 {
 namespace {
 
 constexpr int TB = 128;        // diagonal block order
-constexpr int TB_LD = TB + 1;  // shared row stride
-constexpr int TI_NT = 256;     // threads of the inversion
+constexpr int TB_LD = TB + 2;  // shared column stride (2-way conflicts at most for all reads of it)
+constexpr int TI_NT = 512;     // threads of the inversion
+constexpr int TI_K = 16;       // rows it solves at a time
+constexpr int TI_PLD = TB + 4; // stride of the copied columns (conflict-free DMMA fragments)
 
 // Invert every diagonal block T_b = T[kb:kb+bs, kb:kb+bs] (lower or upper, unit
 // or not); block b goes to Tinv + b*TB*TB (column-major, ld TB, zero outside the
 // triangle and beyond bs).  An upper block is inverted as the lower one it is
-// with both indices reversed.  In shared memory, in place: the eight 16x16
-// diagonal blocks by substitution against the identity (one thread per column),
-// then three doublings, M21 <- -inv(M22) M21 inv(M11) for every pair of
-// s x s blocks, s = 16, 32, 64, as two register-tiled products.
-// Bound: FP64 latency of one CTA per block; one thread per column of the whole
-// block (8192 dependent FMAs) took 232 us at order 4096, this 28 us (B200).
+// with both indices reversed.  Substitution against the identity in shared
+// memory, in place, 16 columns of T at a time (copied aside as [k][row]): the 16
+// rows of their diagonal block are solved, one thread per column, and taken off
+// the sums of all later rows, which replace T as its columns are used up.
+// Each element is the same chain as plain substitution column by column, k
+// ascending from the column's own index: a zero of the triangle is never
+// multiplied (it would turn an infinity or a NaN of T into NaN in columns that
+// do not depend on it), and nothing is lost to products of inverses (inversion
+// by doubling: 1.5-2x the backward error on LU factors).
+// Bound: FP64 latency of one CTA per block, about 2.3 us for 16 rows.  A solve of
+// order 128 for 8 right-hand sides takes 31 us, with inversion by doubling 28, with
+// one thread per column of the block 198; of order 16, 11 against 24 and 24 (B200).
+using Yes = std::integral_constant<bool, true>;
+using No = std::integral_constant<bool, false>;
 __device__ __forceinline__ double &tel(double *T, int i, int j) { return T[j * TB_LD + i]; }
-
-template <int S>
-__device__ __forceinline__ void trtri_double(double *T, double *tmp, int tid) {
-  // pairs p: M11 at 2Sp, M22 at 2Sp + S; outputs per pair S x S, all pairs: 64 S.
-  // Each thread: CELLS consecutive columns of one row.
-  constexpr int PAIRS = TB / (2 * S), CELLS = PAIRS * S * S / TI_NT;
-  const int row = tid % S, cg = (tid / S) % (S / CELLS), pair = tid / (S * (S / CELLS));
-  const int o1 = 2 * S * pair, o2 = o1 + S, c0 = cg * CELLS;
-  double acc[CELLS];
-  // tmp = M21 inv(M11): columns c of inv(M11) are zero above c
-#pragma unroll
-  for (int c = 0; c < CELLS; ++c) acc[c] = 0.0;
-#pragma unroll 4
-  for (int k = c0; k < S; ++k) {
-    const double a = tel(T, o2 + row, o1 + k);
-#pragma unroll
-    for (int c = 0; c < CELLS; ++c)  // inv(M11)(k, c0 + c): the upper part holds zeros
-      acc[c] = fma(a, tel(T, o1 + k, o1 + c0 + c), acc[c]);
-  }
-#pragma unroll
-  for (int c = 0; c < CELLS; ++c) tmp[(c0 + c) * (TB / 2 + 1) + pair * S + row] = acc[c];
-  __syncthreads();
-  // M21 = -inv(M22) tmp
-#pragma unroll
-  for (int c = 0; c < CELLS; ++c) acc[c] = 0.0;
-#pragma unroll 4
-  for (int k = 0; k < S; ++k) {  // (zero beyond the row)
-    const double a = tel(T, o2 + row, o2 + k);
-#pragma unroll
-    for (int c = 0; c < CELLS; ++c)
-      acc[c] = fma(a, tmp[(c0 + c) * (TB / 2 + 1) + pair * S + k], acc[c]);
-  }
-#pragma unroll
-  for (int c = 0; c < CELLS; ++c) tel(T, o2 + row, o1 + c0 + c) = -acc[c];
-  __syncthreads();
-}
 
 __global__ void __launch_bounds__(TI_NT)
     trtri_batched_kernel(const double *__restrict__ A, long long rs, long long cs, int n, int lower,
                          int unit, double *__restrict__ Tinv) {
-  extern __shared__ double tsm[];
-  double *T = tsm;                  // T(i, j) at [j*TB_LD + i]
-  double *tmp = tsm + TB * TB_LD;   // up to 64 columns x 64 rows
+  extern __shared__ __align__(16) double tsm[];
+  double *T = tsm;                      // T(i, j) at [j*TB_LD + i], then sums, then the inverse
+  double *pan = tsm + TB * TB_LD;       // 16 columns of T, [k][row], this step's and the next's
+  double *inv = pan + 2 * TI_K * TI_PLD;  // inverted diagonal
   const int kb = blockIdx.x * TB, bs = min(TB, n - kb), tid = threadIdx.x;
   // lower triangle of the (index-reversed if upper) block, identity beyond bs,
   // zeros above the diagonal
@@ -107,28 +82,99 @@ __global__ void __launch_bounds__(TI_NT)
     }
   }
   __syncthreads();
-  double *inv = tmp;  // inverted diagonal
-  if (tid < TB) inv[tid] = 1.0 / tel(T, tid, tid);
-  __syncthreads();
-  // 16x16 diagonal blocks: thread 16 b + j forms column j of block b's inverse
-  if (tid < TB) {
-    const int o = tid & ~15, j = tid & 15;
-    double x[16];
+  const int rows = (bs + TI_K - 1) / TI_K * TI_K;  // those beyond bs are the identity's
+  const int lane = tid & 31, warp = tid >> 5;
+  auto panel = [&](int k0) { return pan + (k0 / TI_K & 1) * TI_K * TI_PLD; };
+  auto copy_panel = [&](int k0, int t0, int nt) {
+    double *p = panel(k0);
+    for (int idx = t0; idx < TI_K * TB; idx += nt)
+      if (idx % TB >= k0) p[idx / TB * TI_PLD + idx % TB] = tel(T, idx % TB, k0 + idx / TB);
+  };
+  // rows k0 .. k0 + 15 of column tid < k0 + 16 (the columns after it are zero);
+  // EDGE: the warp has columns of the diagonal 16 x 16
+  auto solve = [&](auto edge, int k0) {
+    constexpr bool EDGE = decltype(edge)::value;
+    const double *p = panel(k0);
+    double x[TI_K];
+    const int own = tid - k0;  // of the diagonal 16 x 16: the rows before it are zero
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      double acc = i == j ? 1.0 : 0.0;
+    for (int r = 0; r < TI_K; ++r)
+      x[r] = !EDGE || own < 0 ? tel(T, k0 + r, tid) : r == own ? 1.0 : 0.0;
 #pragma unroll
-      for (int k = 0; k < i; ++k) acc = fma(-tel(T, o + i, o + k), x[k], acc);
-      x[i] = i < j ? 0.0 : acc * inv[o + i];
+    for (int r = 0; r < TI_K; ++r) {
+      if (!EDGE || r >= own) {
+        x[r] *= inv[k0 + r];
+#pragma unroll
+        for (int q = r + 1; q < TI_K; ++q) x[q] = fma(-p[r * TI_PLD + k0 + q], x[r], x[q]);
+      }
     }
-    __syncwarp();  // a half-warp owns a block: all of it is read before it is written
 #pragma unroll
-    for (int i = 0; i < 16; ++i) tel(T, o + i, o + j) = x[i];
-  }
+    for (int r = 0; r < TI_K; ++r) tel(T, k0 + r, tid) = x[r];
+  };
+  // takes rows k0 .. k0 + 15 off the sums of rows [r0, r1), warps w0 to the last:
+  // 16 x 8 outputs at a time on DMMA (a chain of multiply-adds, k ascending), the
+  // columns of the diagonal 16 x 16, whose first sums start at their own index, one
+  // column and 8 rows per lane
+  auto update = [&](int k0, int r0, int r1, int w0) {
+    const double *p = panel(k0);
+    const int rblocks = (r1 - r0) / 16, items = rblocks * (k0 / 8 + 1);
+    for (int it = warp - w0; it < items; it += TI_NT / 32 - w0) {
+      const int i0 = r0 + it % rblocks * 16, c = it / rblocks;
+      if (c == 0) {
+        const int i = i0 + (lane >> 4) * 8, j = k0 + (lane & 15);
+        double acc[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) acc[r] = 0.0;
+#pragma unroll
+        for (int k = 0; k < TI_K; ++k) {
+          const double x = tel(T, k0 + k, j);
+          const double2 *t2 = reinterpret_cast<const double2 *>(p + k * TI_PLD + i);
+          if (k0 + k >= j) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+              const double2 t = t2[r];
+              acc[2 * r] = fma(-t.x, x, acc[2 * r]);
+              acc[2 * r + 1] = fma(-t.y, x, acc[2 * r + 1]);
+            }
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) tel(T, i + r, j) = acc[r];
+      } else {
+        const int g = lane >> 2, t = lane & 3, j0 = (c - 1) * 8;
+        double acc[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) acc[v] = tel(T, i0 + g + 8 * (v >> 1), j0 + 2 * t + (v & 1));
+#pragma unroll
+        for (int k = 0; k < TI_K; k += 4) {
+          const double a0 = -p[(k + t) * TI_PLD + i0 + g], a1 = -p[(k + t) * TI_PLD + i0 + g + 8];
+          const double b = tel(T, k0 + k + t, j0 + g);
+          asm volatile(
+              "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+              "{%0,%1,%2,%3};\n"
+              : "+d"(acc[0]), "+d"(acc[1]), "+d"(acc[2]), "+d"(acc[3])
+              : "d"(a0), "d"(a1), "d"(b));
+        }
+#pragma unroll
+        for (int v = 0; v < 4; ++v) tel(T, i0 + g + 8 * (v >> 1), j0 + 2 * t + (v & 1)) = acc[v];
+      }
+    }
+  };
+  if (tid < TB) inv[tid] = 1.0 / tel(T, tid, tid);
+  copy_panel(0, tid, TI_NT);
   __syncthreads();
-  trtri_double<16>(T, tmp, tid);
-  trtri_double<32>(T, tmp, tid);
-  trtri_double<64>(T, tmp, tid);
+  if (tid < TI_K) solve(Yes{}, 0);
+  __syncthreads();
+  // the next 16 rows' sums, then those rows beside the sums of the rows after them
+  for (int k0 = 0, k1 = TI_K; k1 < rows; k0 = k1, k1 += TI_K) {
+    update(k0, k1, k1 + TI_K, 0);
+    copy_panel(k1, tid, TI_NT);
+    __syncthreads();
+    if (tid >= TB) update(k0, k1 + TI_K, rows, 4);
+    else if (warp * 32 + 32 <= k1) solve(No{}, k1);
+    else if (tid < k1 + TI_K) solve(Yes{}, k1);
+    __syncthreads();
+  }
   double *out = Tinv + (long long)blockIdx.x * TB * TB;
   for (int idx = tid; idx < TB * TB; idx += TI_NT) {
     const int i = idx % TB, j = idx / TB;  // element (i, j) of the stored inverse
@@ -222,8 +268,6 @@ __global__ void __launch_bounds__(256, 1)
       }
     }
   };
-  using Yes = std::integral_constant<bool, true>;
-  using No = std::integral_constant<bool, false>;
   auto copy_stage = [&]() {
     if (issued < stages) {
       const int k = forward ? pk : nb - 1 - pk, j = forward ? pj : nb - 1 - pj;
@@ -497,7 +541,7 @@ int dtrsm_device(char side, char uplo, char transa, char diag, int m, int n, dou
   p.tinv = (double *)workspace(cx, WS_TRSM_INV, (size_t)nblk * TB * TB * sizeof(double));
   if (!p.tinv) return B2_ERR_NOMEM;
   {
-    const int smem = (TB * TB_LD + (TB / 2) * (TB / 2 + 1)) * (int)sizeof(double);
+    const int smem = (TB * TB_LD + 2 * TI_K * TI_PLD + TB) * (int)sizeof(double);
     B2_CUDA_TRY(cudaFuncSetAttribute(trtri_batched_kernel,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     B2_PROF("trsm_trtri", s);
