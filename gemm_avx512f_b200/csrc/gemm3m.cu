@@ -356,7 +356,7 @@ int launch_cgemm3m(int m, int n, int k, const float *A, int lda, const float *B,
 }
 
 // --------------------------------------- zgemm3m: one-launch FP64 DMMA --
-// The fused 3M product for complex128 at any size, on the FP64 tensor path
+// The fused 3M product for complex128, on the FP64 tensor path
 // (mma.sync.m16n8k4.f64; tcgen05 has no f64 kind).  CTA tile 32 x 32 complex
 // outputs, 4 warps of 16 x 16, three CTAs per SM; K in blocks of 16 complex
 // elements streamed global -> shared by cp.async (one 16-byte complex element
@@ -430,7 +430,9 @@ __global__ void __launch_bounds__(Z_NT, 3)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int wm0 = (warp / Z_WN) * 16, wn0 = (warp % Z_WN) * 16;
-  const int m0 = blockIdx.x * Z_BM, n0 = blockIdx.y * Z_BN;
+  const unsigned col0 = (blockIdx.z * gridDim.y + blockIdx.y) * Z_BN;
+  if (col0 >= (unsigned)N) return;  // past the last tile, where column tiles fill several planes
+  const int m0 = blockIdx.x * Z_BM, n0 = (int)col0;
   const int KT = (K + Z_BK - 1) / Z_BK;
 
   double acc[3][2][4];
@@ -568,7 +570,10 @@ int launch_zgemm3m_dmma(int m, int n, int k, const double *A, int lda, const dou
       (size_t)Z_STAGES * (z_stage_elems<AK>(Z_BM) + z_stage_elems<BKc>(Z_BN)) * 16;
   auto kern = zgemm3m_dmma_kernel<AK, BKc>;
   B2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM));
-  dim3 grid((unsigned)((m + Z_BM - 1) / Z_BM), (unsigned)((n + Z_BN - 1) / Z_BN));
+  // Column tiles over y and, from N = 2097121 on, z: y ends at 65535.  (One flat
+  // dimension divided by the row tiles in the kernel: 2048^3 1679 -> 1692 us on B200.)
+  const unsigned tn = (unsigned)((n + Z_BN - 1) / Z_BN), planes = (tn + 65534) / 65535;
+  dim3 grid((unsigned)((m + Z_BM - 1) / Z_BM), (tn + planes - 1) / planes, planes);
   B2_PROF("zgemm3m_dmma", s);
   kern<<<grid, Z_NT, SMEM, s>>>(m, n, k, reinterpret_cast<const double2 *>(A), lda,
                                 reinterpret_cast<const double2 *>(B), ldb,
