@@ -485,23 +485,18 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
       for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
         const int ks = u % pr.ksplit;
         const int kb0 = ks * pr.kb_per_split, kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
-        for (int kr = kb0; kr < kb1 && ok; kr += pr.sub_kb, ++it) {
-          const int ke = min(kb1, kr + pr.sub_kb);
+        // K blocks [kr, ke) of the unit into accumulator set it % SETS
+        auto accumulate = [&](int kr, int ke) {
           const int acc = it % SETS;
           const uint32_t acc_phase = (uint32_t)((it / SETS) & 1);
-          if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, pr.derr, pr.wait_ns)) {
-            ok = false;
-            break;
-          }
+          if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, pr.derr, pr.wait_ns))
+            return false;
           tc_fence_after();
           for (int kbb = kr; kbb < kr + NACC * (ke - kr); ++kbb) {
             const int bi = NACC > 1 ? (kbb - kr) % NACC : 0;
             const int kb = NACC > 1 ? kr + (kbb - kr) / NACC : kbb;
             const uint32_t d_tmem = tmem_base + (uint32_t)((acc * NACC + bi) * BN);
-            if (!mbar_wait(full_bar(stage), phase, abort_flag, pr.derr, pr.wait_ns)) {
-              ok = false;
-              break;
-            }
+            if (!mbar_wait(full_bar(stage), phase, abort_flag, pr.derr, pr.wait_ns)) return false;
             tc_fence_after();
             const uint32_t sx = base + stage * L::STAGE_BYTES;
             const uint32_t sy = sx + L::X_BYTES;
@@ -518,8 +513,15 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
             tc_commit(empty_bar(stage));  // frees the stage once these MMAs have read it
             if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           }
-          if (!ok) break;
           tc_commit(tfull_bar(acc));
+          ++it;
+          return true;
+        };
+        if constexpr (SUM) {
+          for (int kr = kb0; kr < kb1 && ok; kr += pr.sub_kb)
+            ok = accumulate(kr, min(kb1, kr + pr.sub_kb));
+        } else {
+          ok = accumulate(kb0, kb1);
         }
       }
       // All MMAs issued so far complete before the drain barrier flips.
@@ -835,23 +837,18 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
       for (int u = pair; u < total_units && ok; u += npairs) {
         const int ks = u % pr.ksplit;
         const int kb0 = ks * pr.kb_per_split, kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
-        for (int kr = kb0; kr < kb1 && ok; kr += pr.sub_kb, ++it) {
-          const int ke = min(kb1, kr + pr.sub_kb);
+        auto accumulate = [&](int kr, int ke) {  // as in the single-CTA engine
           const int acc = it & 1;
           const uint32_t acc_phase = (uint32_t)((it >> 1) & 1);
           if (!mbar_wait_pair(tempty_bar(acc), acc_phase ^ 1u, abort_flag, peer_abort, pr.derr,
-                              pr.wait_ns)) {
-            ok = false;
-            break;
-          }
+                              pr.wait_ns))
+            return false;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
           for (int kb = kr; kb < ke; ++kb) {
             if (!mbar_wait_pair(full_bar(stage), phase, abort_flag, peer_abort, pr.derr,
-                                pr.wait_ns)) {
-              ok = false;
-              break;
-            }
+                                pr.wait_ns))
+              return false;
             tc_fence_after();
             const uint32_t sx = base + stage * L::STAGE_BYTES;
             const uint32_t sy = sx + L::X_BYTES;
@@ -868,8 +865,15 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
             tc_commit_pair(empty_bar(stage), (uint16_t)3);  // frees the stage in both CTAs
             if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           }
-          if (!ok) break;
           tc_commit_pair(tfull_bar(acc), (uint16_t)3);
+          ++it;
+          return true;
+        };
+        if constexpr (SUM) {
+          for (int kr = kb0; kr < kb1 && ok; kr += pr.sub_kb)
+            ok = accumulate(kr, min(kb1, kr + pr.sub_kb));
+        } else {
+          ok = accumulate(kb0, kb1);
         }
       }
       tc_commit_pair(drain_bar, (uint16_t)1);
