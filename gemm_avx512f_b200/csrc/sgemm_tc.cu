@@ -278,17 +278,21 @@ int choose_ksplit(long long tiles, int kblocks, int sms) {
 
 inline long long round_up(long long x, long long a) { return (x + a - 1) / a * a; }
 
-// Work units of a product whose K is accumulated in S ranges of kbps blocks:
-// each unit takes `per` consecutive ranges of its tile (adding them in its
-// epilogue), so that ceil(S / per) partials per tile go through memory.
+// Work units of a product whose K is accumulated in S ranges of tbs term blocks (a
+// K block of a three-term product is three: its MMAs add Ab Bb, Ab Bs and As Bb in
+// turn): each unit takes `per` consecutive ranges of its tile (adding them in its
+// epilogue), so that ceil(S / per) partials per tile go through memory.  Ranges are
+// as short as separate launches per range would have them: the tensor core's
+// accumulation error grows with a chain's length (ranges of whole K blocks, 3xTF32
+// with K = 64: 3.8e-7 instead of 1.1e-7).
 // Modelled time (us): waves of units, each 3 us of fill and final epilogue and,
-// per range, t_kb per K block (measured MMA rate of the engine) but at least
+// per range, t_tb per term block (measured MMA rate of the engine) but at least
 // the 1.1 us that adding an accumulator to the sums takes (8 ranges of one K
 // block each: 512^3 11.7 us in one unit per tile, 6.6 in several); plus the
 // partials written and read at about 6 TB/s and a second launch.  2048^3
 // 3xTF32 (64 pair tiles on 74 pairs, 8 ranges): one unit per tile instead of 8
 // partials of 16.8 MB.
-int ranges_per_unit(long long tiles, int S, int kbps, int kblocks, int slots, double t_kb, int m,
+int ranges_per_unit(long long tiles, int S, int tbs, int tblocks, int slots, double t_tb, int m,
                     int n) {
   int best = S;
   double best_us = 1e300;
@@ -296,8 +300,8 @@ int ranges_per_unit(long long tiles, int S, int kbps, int kblocks, int slots, do
     const int E = (S + per - 1) / per;
     if (per > 1 && (S + per - 2) / (per - 1) == E) continue;  // more even with per - 1
     const long long waves = (tiles * E + slots - 1) / slots;
-    const int kb = per * kbps < kblocks ? per * kbps : kblocks;
-    const double work = kb * t_kb, drains = 1.1 * ((kb + kbps - 1) / kbps);
+    const int tb = per * tbs < tblocks ? per * tbs : tblocks;
+    const double work = tb * t_tb, drains = 1.1 * ((tb + tbs - 1) / tbs);
     double us = (double)waves * ((work > drains ? work : drains) + 3.0);
     if (E > 1) us += 2.0 + (double)E * m * n * 8.0 / 6e6;
     if (us < best_us) best_us = us, best = per;
@@ -305,10 +309,23 @@ int ranges_per_unit(long long tiles, int S, int kbps, int kblocks, int slots, do
   return best;
 }
 
-// Partials per tile, K blocks per unit and K blocks per accumulated range.
+// Partials per tile, term blocks per unit and per accumulated range.
 struct Ranges {
-  int E, unit_kb, range_kb;
+  int E, unit_tb, range_tb;
 };
+
+// The ranges of a product of `tblocks` term blocks: `split` of them (0: chosen for
+// `tiles` tiles on `slots` engines), dealt to units.  nprod: products of that shape
+// in one launch.
+Ranges choose_ranges(int split, int tblocks, long long tiles, int slots, int nprod, double t_tb,
+                     int m, int n) {
+  int S = split > 0 ? split : choose_ksplit(tiles, tblocks, slots);
+  if (S > tblocks) S = tblocks > 0 ? tblocks : 1;
+  const int tbs = (tblocks + S - 1) / S;
+  S = (tblocks + tbs - 1) / tbs;
+  const int per = ranges_per_unit(nprod * tiles, S, tbs, tblocks, slots, t_tb, m, nprod * n);
+  return Ranges{(S + per - 1) / per, per * tbs, tbs};
+}
 
 // One SGEMM product (or nbatch of them) on engine `eng` (see SgCfg).
 template <class Epi>
@@ -321,14 +338,14 @@ int run_engine(int eng, bool bf16, int terms, const CUtensorMap &tmX, const CUte
     constexpr int T = decltype(t3)::value;
     return umma::launch_pair<decltype(kd)::value, 256, T == 3 ? 3 : 6, Epi, true, T>(
         tmX, tmY, m, n, kp, nbatch, epi, cx->device, cx->derr, s, nm, nullptr, rg.E, seg_kb,
-        rg.unit_kb, rg.range_kb);
+        rg.unit_tb, rg.range_tb);
   };
   auto single = [&](auto kd, auto bn, auto t3) {
     constexpr int T = decltype(t3)::value, BN = decltype(bn)::value;
     constexpr int ST = BN == 256 ? (T == 3 ? 2 : 4) : (T == 3 ? 3 : 6);
     return umma::launch<decltype(kd)::value, BN, ST, Epi, 1, true, T>(
         tmX, tmY, m, n, kp, nbatch, epi, cx->sm_count, cx->derr, s, nm, 0, nullptr, rg.E, seg_kb, 0,
-        0, rg.unit_kb, rg.range_kb);
+        0, rg.unit_tb, rg.range_tb);
   };
   using BF = std::integral_constant<int, umma::KIND_BF16>;
   using TF = std::integral_constant<int, umma::KIND_TF32>;
@@ -527,13 +544,9 @@ int cgemm3m_tensor(char ta, char tb, int m, int n, int k, float ar, float ai, fl
   const int seg_kb = kp * 4 / umma::KBLOCK_BYTES, kblocks = seg_kb;
   const long long tiles = ((n + tile_q - 1) / tile_q) * (long long)((m + tile_p - 1) / tile_p);
   const int slots = eng == 2 ? cx->sm_count / 2 : cx->sm_count;
-  int S = cfg.split > 0 ? cfg.split : choose_ksplit(tiles, 3 * kblocks, slots);
-  if (S > kblocks) S = kblocks;
-  const int kbps = (kblocks + S - 1) / S;
-  S = (kblocks + kbps - 1) / kbps;
-  const int per =
-      ranges_per_unit(3 * tiles, S, kbps, kblocks, slots, 3 * (eng == 1 ? 0.17 : 0.28), m, 3 * n);
-  const int E = (S + per - 1) / per;
+  const Ranges rg =
+      choose_ranges(cfg.split, 3 * kblocks, tiles, slots, 3, eng == 1 ? 0.17 : 0.28, m, n);
+  const int E = rg.E;
   const int ldw = (int)round_up(m, 32);
   const long long plane = (long long)n * ldw;
   // the split segments of both operands, then the products' sums
@@ -555,7 +568,7 @@ int cgemm3m_tensor(char ta, char tb, int m, int n, int k, float ar, float ai, fl
     rc = umma::make_kmajor_map(&tmY, umma::KIND_TF32, Yp, ks, n, 3, ks * 4, (long long)n * ks * 4,
                                eng == 0 ? 256 : 128);
   if (rc != B2_OK) return rc;
-  rc = run_engine(eng, false, 3, tmX, tmY, m, n, kp, 3, seg_kb, Ranges{E, per * kbps, kbps},
+  rc = run_engine(eng, false, 3, tmX, tmY, m, n, kp, 3, seg_kb, rg,
                   F32PartialEpi{W, plane, ldw, m, n}, cx, s);
   if (rc != B2_OK) return rc;
   const long long blocks = ((long long)m * n + 255) / 256;
@@ -638,16 +651,9 @@ int sgemm_tensor_cfg(char ta, char tb, int m, int n, int k, float alpha, const f
   const long long tiles = ((n + tile_q - 1) / tile_q) * (long long)((m + tile_p - 1) / tile_p);
   const int kblocks = (int)(((long long)kp * esz + umma::KBLOCK_BYTES - 1) / umma::KBLOCK_BYTES);
   const int slots = eng == 2 ? cx->sm_count / 2 : cx->sm_count;
-  // K is accumulated in S ranges of kbps blocks (of `terms` products each); a
-  // unit adds `per` of them
-  int S = cfg.split > 0 ? cfg.split : choose_ksplit(tiles, terms * kblocks, slots);
-  if (S > kblocks) S = kblocks > 0 ? kblocks : 1;
-  const int kbps = (kblocks + S - 1) / S;
-  S = (kblocks + kbps - 1) / kbps;
-  const int per =
-      ranges_per_unit(tiles, S, kbps, kblocks, slots, terms * (eng == 1 ? 0.17 : 0.28), m, n);
-  const int E = (S + per - 1) / per;  // partials per tile
-  const Ranges rg{E, per * kbps, kbps};
+  const Ranges rg =
+      choose_ranges(cfg.split, terms * kblocks, tiles, slots, 1, eng == 1 ? 0.17 : 0.28, m, n);
+  const int E = rg.E;  // partials per tile
   if (E == 1)
     return run_engine(eng, bf16, terms, tmX, tmY, m, n, kp, 1, seg_kb, rg,
                       F32Epi{C, ldc, m, n, alpha, beta}, cx, s);

@@ -17,10 +17,10 @@
 //               accumulator, then the functor.
 // TMEM holds two accumulators (2 x BN columns) so the epilogue of tile i
 // overlaps the MMAs of tile i+1.
-// SUM kernels cut a unit's K range into sub-ranges that go through the two
-// accumulators in turn; the epilogue adds each to FP32 sums in its registers
-// (128 columns a thread: 8 epilogue warps for BN = 256) while the next one is
-// multiplied.  The tensor core's accumulation error grows with the length of a
+// SUM kernels cut a unit's K range into sub-ranges, of term blocks (a K block of a
+// three-term product has three), that go through the two accumulators in turn;
+// the epilogue adds each to FP32 sums in its registers (128 columns a thread: 8
+// epilogue warps for BN = 256) while the next one is multiplied.  The tensor core's accumulation error grows with the length of a
 // chain, so the split forms of SGEMM keep chains short; this keeps them short
 // without writing the partial products to memory.
 //
@@ -270,8 +270,9 @@ struct Problem {
   int kblocks;     // K extent in 128-byte blocks
   int ksplit;      // K ranges per output tile (split-K; 1 = whole K in one accumulator)
   int kb_per_split;  // K blocks per range (every range is non-empty)
-  int sub_kb;        // K blocks accumulated at a time within a unit's range (kernels
-                     // with SUM add the sub-ranges in registers; else the whole range)
+  // SUM kernels count K in term blocks (a K block has TERMS of them, one per
+  // product): a unit's part, and what of it is accumulated at a time
+  int tb_unit, tb_sub;
   int nbatch;      // independent products (3-D tensor maps, batch = outer coordinate)
   const int *nbatch_dev;  // if set: the batch count actually run (<= nbatch), read on the device
   int tiles_p, tiles_q;
@@ -363,6 +364,21 @@ __device__ __forceinline__ bool sum_epilogue(uint32_t tmem_quarter, int bn, int 
   return true;
 }
 
+// Term blocks [t0, t1) and the K blocks [kb0, kb1) that hold them, of K range ks.
+template <bool SUM, int TERMS>
+__device__ __forceinline__ void unit_range(const Problem &pr, int ks, int &t0, int &t1, int &kb0,
+                                           int &kb1) {
+  if constexpr (SUM) {
+    t0 = ks * pr.tb_unit;
+    t1 = min(TERMS * pr.kblocks, t0 + pr.tb_unit);
+    kb0 = t0 / TERMS;
+    kb1 = (t1 + TERMS - 1) / TERMS;
+  } else {
+    t0 = kb0 = ks * pr.kb_per_split;
+    t1 = kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
+  }
+}
+
 // NACC = 1: every (batch, tile, K range) is its own work unit.  NACC > 1: a
 // work unit is a tile, and the unit multiplies batches 0 .. NACC-1 of the
 // operands into NACC accumulators that its epilogue receives together
@@ -440,7 +456,8 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
         const int t = u / pr.ksplit, ks = u - t * pr.ksplit;
         int b, tp, tq;
         tile_coords(pr, t, b, tp, tq);
-        const int kb0 = ks * pr.kb_per_split, kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
+        int t0, t1, kb0, kb1;
+        unit_range<SUM, TERMS>(pr, ks, t0, t1, kb0, kb1);
         // NACC > 1: the unit's batches interleaved per K block (the three
         // products of a K block back to back, so the operand panels of all
         // batches stay in L2 together)
@@ -484,44 +501,91 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
       bool ok = true;
       for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
         const int ks = u % pr.ksplit;
-        const int kb0 = ks * pr.kb_per_split, kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
-        // K blocks [kr, ke) of the unit into accumulator set it % SETS
-        auto accumulate = [&](int kr, int ke) {
+        int t0, t1, kb0, kb1;
+        unit_range<SUM, TERMS>(pr, ks, t0, t1, kb0, kb1);
+        if constexpr (SUM) {
+          int tt = t0 % TERMS;  // next term of the K block in `stage`
+          bool fresh = true;    // its copies have not been waited for
+          for (int j = t0; j < t1 && ok; j += pr.tb_sub) {  // sub-range [j, j + left)
+            int left = min(pr.tb_sub, t1 - j);
+            ok = mbar_wait(tempty_bar(it & 1), (uint32_t)((it >> 1) & 1) ^ 1u, abort_flag, pr.derr,
+                           pr.wait_ns);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_base + (uint32_t)((it & 1) * BN);
+            uint32_t add = 0;  // the first MMA overwrites
+            auto issue = [&](int term) {
+              const uint32_t sx = base + stage * L::STAGE_BYTES;
+              const uint32_t tx = sx + (term == 2 ? L::HALF_BYTES : 0);
+              const uint32_t ty = sx + L::X_BYTES + (term == 1 ? L::HALF_BYTES : 0);
+#pragma unroll
+              for (int kk = 0; kk < KBLOCK_BYTES / 32; ++kk) {
+                tc_mma<KIND>(d_tmem, sw128_desc(tx + kk * 32), sw128_desc(ty + kk * 32), idesc,
+                             add);
+                add = 1;
+              }
+            };
+            while (left > 0) {
+              if (fresh) {
+                ok = mbar_wait(full_bar(stage), phase, abort_flag, pr.derr, pr.wait_ns);
+                if (!ok) break;
+                tc_fence_after();
+                fresh = false;
+              }
+              if (TERMS == 1 || (tt == 0 && left >= TERMS)) {  // the whole K block
+#pragma unroll
+                for (int term = 0; term < TERMS; ++term) issue(term);
+                left -= TERMS;
+                tt = TERMS;
+              } else {
+                issue(tt);
+                --left;
+                ++tt;
+              }
+              if (tt == TERMS) {
+                tc_commit(empty_bar(stage));  // frees the stage once these MMAs have read it
+                if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+                tt = 0;
+                fresh = true;
+              }
+            }
+            if (!ok) break;
+            tc_commit(tfull_bar(it & 1));
+            ++it;
+          }
+          if (ok && tt != 0) {  // the unit ends inside a K block
+            tc_commit(empty_bar(stage));
+            if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          }
+        } else {
           const int acc = it % SETS;
           const uint32_t acc_phase = (uint32_t)((it / SETS) & 1);
-          if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, pr.derr, pr.wait_ns))
-            return false;
+          if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, pr.derr, pr.wait_ns)) {
+            ok = false;
+            break;
+          }
           tc_fence_after();
-          for (int kbb = kr; kbb < kr + NACC * (ke - kr); ++kbb) {
-            const int bi = NACC > 1 ? (kbb - kr) % NACC : 0;
-            const int kb = NACC > 1 ? kr + (kbb - kr) / NACC : kbb;
+          for (int kbb = kb0; kbb < kb0 + NACC * (kb1 - kb0); ++kbb) {
+            const int bi = NACC > 1 ? (kbb - kb0) % NACC : 0;
+            const int kb = NACC > 1 ? kb0 + (kbb - kb0) / NACC : kbb;
             const uint32_t d_tmem = tmem_base + (uint32_t)((acc * NACC + bi) * BN);
-            if (!mbar_wait(full_bar(stage), phase, abort_flag, pr.derr, pr.wait_ns)) return false;
+            if (!mbar_wait(full_bar(stage), phase, abort_flag, pr.derr, pr.wait_ns)) {
+              ok = false;
+              break;
+            }
             tc_fence_after();
             const uint32_t sx = base + stage * L::STAGE_BYTES;
             const uint32_t sy = sx + L::X_BYTES;
 #pragma unroll
-            for (int tt = 0; tt < TERMS; ++tt) {
-              const uint32_t tx = sx + (tt == 2 ? L::HALF_BYTES : 0);
-              const uint32_t ty = sy + (tt == 1 ? L::HALF_BYTES : 0);
-#pragma unroll
-              for (int kk = 0; kk < KBLOCK_BYTES / 32; ++kk) {
-                tc_mma<KIND>(d_tmem, sw128_desc(tx + kk * 32), sw128_desc(ty + kk * 32), idesc,
-                             (kb != kr || kk || tt) ? 1u : 0u);
-              }
-            }
+            for (int kk = 0; kk < KBLOCK_BYTES / 32; ++kk)
+              tc_mma<KIND>(d_tmem, sw128_desc(sx + kk * 32), sw128_desc(sy + kk * 32), idesc,
+                           (kb != kb0 || kk) ? 1u : 0u);
             tc_commit(empty_bar(stage));  // frees the stage once these MMAs have read it
             if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           }
+          if (!ok) break;
           tc_commit(tfull_bar(acc));
           ++it;
-          return true;
-        };
-        if constexpr (SUM) {
-          for (int kr = kb0; kr < kb1 && ok; kr += pr.sub_kb)
-            ok = accumulate(kr, min(kb1, kr + pr.sub_kb));
-        } else {
-          ok = accumulate(kb0, kb1);
         }
       }
       // All MMAs issued so far complete before the drain barrier flips.
@@ -537,12 +601,13 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
       int b, tp, tq;
       tile_coords(pr, t, b, tp, tq);
       if constexpr (SUM) {
-        const int kb0 = ks * pr.kb_per_split, kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
+        int t0, t1, kb0, kb1;
+        unit_range<SUM, TERMS>(pr, ks, t0, t1, kb0, kb1);
         const int p = tp * BM + quarter * 32 + lane;
         epi.prefetch(p - lane, lane, tq * BN + (warp - 2) / 4 * 128);
         if (!sum_epilogue(
                 tmem_base + ((uint32_t)(quarter * 32) << 16), BN, (warp - 2) / 4 * 128,
-                (kb1 - kb0 + pr.sub_kb - 1) / pr.sub_kb, it,
+                (t1 - t0 + pr.tb_sub - 1) / pr.tb_sub, it,
                 [&](int i) {
                   return mbar_wait(tfull_bar(i & 1), (uint32_t)((i >> 1) & 1), abort_flag, pr.derr,
                                    pr.wait_ns);
@@ -797,7 +862,8 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
         tile_coords(pr, t, b, tp, tq);
         const int xrow = tp * PAIR_BM + (int)rank * BM;
         const int yrow = tq * BN + (int)rank * (BN / 2);
-        const int kb0 = ks * pr.kb_per_split, kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
+        int t0, t1, kb0, kb1;
+        unit_range<SUM, TERMS>(pr, ks, t0, t1, kb0, kb1);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait_pair(empty_bar(stage), phase ^ 1u, abort_flag, peer_abort, pr.derr,
                               pr.wait_ns)) {
@@ -836,44 +902,92 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
       bool ok = true;
       for (int u = pair; u < total_units && ok; u += npairs) {
         const int ks = u % pr.ksplit;
-        const int kb0 = ks * pr.kb_per_split, kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
-        auto accumulate = [&](int kr, int ke) {  // as in the single-CTA engine
+        int t0, t1, kb0, kb1;
+        unit_range<SUM, TERMS>(pr, ks, t0, t1, kb0, kb1);
+        if constexpr (SUM) {  // as in the single-CTA engine
+          int tt = t0 % TERMS;  // next term of the K block in `stage`
+          bool fresh = true;    // its copies have not been waited for
+          for (int j = t0; j < t1 && ok; j += pr.tb_sub) {  // sub-range [j, j + left)
+            int left = min(pr.tb_sub, t1 - j);
+            ok = mbar_wait_pair(tempty_bar(it & 1), (uint32_t)((it >> 1) & 1) ^ 1u, abort_flag,
+                                peer_abort, pr.derr, pr.wait_ns);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_base + (uint32_t)((it & 1) * BN);
+            uint32_t add = 0;  // the first MMA overwrites
+            auto issue = [&](int term) {
+              const uint32_t sx = base + stage * L::STAGE_BYTES;
+              const uint32_t tx = sx + (term == 2 ? L::HALF_BYTES : 0);
+              const uint32_t ty = sx + L::X_BYTES + (term == 1 ? L::HALF_BYTES : 0);
+#pragma unroll
+              for (int kk = 0; kk < KBLOCK_BYTES / 32; ++kk) {
+                tc_mma_pair<KIND>(d_tmem, sw128_desc(tx + kk * 32), sw128_desc(ty + kk * 32), idesc,
+                                  add);
+                add = 1;
+              }
+            };
+            while (left > 0) {
+              if (fresh) {
+                ok = mbar_wait_pair(full_bar(stage), phase, abort_flag, peer_abort, pr.derr,
+                                    pr.wait_ns);
+                if (!ok) break;
+                tc_fence_after();
+                fresh = false;
+              }
+              if (TERMS == 1 || (tt == 0 && left >= TERMS)) {  // the whole K block
+#pragma unroll
+                for (int term = 0; term < TERMS; ++term) issue(term);
+                left -= TERMS;
+                tt = TERMS;
+              } else {
+                issue(tt);
+                --left;
+                ++tt;
+              }
+              if (tt == TERMS) {
+                tc_commit_pair(empty_bar(stage), (uint16_t)3);  // frees the stage in both CTAs
+                if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+                tt = 0;
+                fresh = true;
+              }
+            }
+            if (!ok) break;
+            tc_commit_pair(tfull_bar(it & 1), (uint16_t)3);
+            ++it;
+          }
+          if (ok && tt != 0) {  // the unit ends inside a K block
+            tc_commit_pair(empty_bar(stage), (uint16_t)3);
+            if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          }
+        } else {
           const int acc = it & 1;
           const uint32_t acc_phase = (uint32_t)((it >> 1) & 1);
           if (!mbar_wait_pair(tempty_bar(acc), acc_phase ^ 1u, abort_flag, peer_abort, pr.derr,
-                              pr.wait_ns))
-            return false;
+                              pr.wait_ns)) {
+            ok = false;
+            break;
+          }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
-          for (int kb = kr; kb < ke; ++kb) {
+          for (int kb = kb0; kb < kb1; ++kb) {
             if (!mbar_wait_pair(full_bar(stage), phase, abort_flag, peer_abort, pr.derr,
-                                pr.wait_ns))
-              return false;
+                                pr.wait_ns)) {
+              ok = false;
+              break;
+            }
             tc_fence_after();
             const uint32_t sx = base + stage * L::STAGE_BYTES;
             const uint32_t sy = sx + L::X_BYTES;
 #pragma unroll
-            for (int tt = 0; tt < TERMS; ++tt) {
-              const uint32_t tx = sx + (tt == 2 ? L::HALF_BYTES : 0);
-              const uint32_t ty = sy + (tt == 1 ? L::HALF_BYTES : 0);
-#pragma unroll
-              for (int kk = 0; kk < KBLOCK_BYTES / 32; ++kk) {
-                tc_mma_pair<KIND>(d_tmem, sw128_desc(tx + kk * 32), sw128_desc(ty + kk * 32),
-                                  idesc, (kb != kr || kk || tt) ? 1u : 0u);
-              }
-            }
+            for (int kk = 0; kk < KBLOCK_BYTES / 32; ++kk)
+              tc_mma_pair<KIND>(d_tmem, sw128_desc(sx + kk * 32), sw128_desc(sy + kk * 32), idesc,
+                                (kb != kb0 || kk) ? 1u : 0u);
             tc_commit_pair(empty_bar(stage), (uint16_t)3);  // frees the stage in both CTAs
             if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           }
+          if (!ok) break;
           tc_commit_pair(tfull_bar(acc), (uint16_t)3);
           ++it;
-          return true;
-        };
-        if constexpr (SUM) {
-          for (int kr = kb0; kr < kb1 && ok; kr += pr.sub_kb)
-            ok = accumulate(kr, min(kb1, kr + pr.sub_kb));
-        } else {
-          ok = accumulate(kb0, kb1);
         }
       }
       tc_commit_pair(drain_bar, (uint16_t)1);
@@ -888,12 +1002,13 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
       int b, tp, tq;
       tile_coords(pr, t, b, tp, tq);
       if constexpr (SUM) {
-        const int kb0 = ks * pr.kb_per_split, kb1 = min(pr.kblocks, kb0 + pr.kb_per_split);
+        int t0, t1, kb0, kb1;
+        unit_range<SUM, TERMS>(pr, ks, t0, t1, kb0, kb1);
         const int p = tp * PAIR_BM + (int)rank * BM + quarter * 32 + lane;
         epi.prefetch(p - lane, lane, tq * BN + (warp - 2) / 4 * 128);
         if (!sum_epilogue(
                 tmem_base + ((uint32_t)(quarter * 32) << 16), BN, (warp - 2) / 4 * 128,
-                (kb1 - kb0 + pr.sub_kb - 1) / pr.sub_kb, it,
+                (t1 - t0 + pr.tb_sub - 1) / pr.tb_sub, it,
                 [&](int i) {
                   return mbar_wait_pair(tfull_bar(i & 1), (uint32_t)((i >> 1) & 1), abort_flag,
                                         peer_abort, pr.derr, pr.wait_ns);
@@ -971,15 +1086,22 @@ int make_kmajor_map(CUtensorMap *map, int kind, const void *base, long long kele
 
 // K ranges of a launch: `ksplit` of ceil(kblocks / ksplit) blocks, their count
 // recomputed so that none is empty (an empty range would leave its accumulator
-// unwritten); or, with kb_range, ranges of kb_range blocks.  sub_kb: the part
-// of a range accumulated at a time (0: all of it).
-inline void set_split(Problem &pr, int ksplit, int kb_range, int sub_kb) {
+// unwritten).  SUM kernels: units of tb_unit term blocks, tb_sub accumulated at a
+// time; ksplit is then their count.
+inline void set_split(Problem &pr, int ksplit, int terms, int tb_unit, int tb_sub) {
+  if (tb_unit > 0) {
+    pr.tb_unit = tb_unit;
+    pr.tb_sub = tb_sub;
+    pr.kb_per_split = 0;
+    pr.ksplit = pr.kblocks > 0 ? (terms * pr.kblocks + tb_unit - 1) / tb_unit : 1;
+    return;
+  }
+  pr.tb_unit = pr.tb_sub = 0;
   if (ksplit < 1) ksplit = 1;
   if (ksplit > pr.kblocks) ksplit = pr.kblocks > 0 ? pr.kblocks : 1;
-  pr.kb_per_split = kb_range > 0 ? kb_range : (pr.kblocks + ksplit - 1) / ksplit;
+  pr.kb_per_split = (pr.kblocks + ksplit - 1) / ksplit;
   pr.ksplit = pr.kb_per_split > 0 ? (pr.kblocks + pr.kb_per_split - 1) / pr.kb_per_split : 1;
   if (pr.ksplit < 1) pr.ksplit = 1;
-  pr.sub_kb = sub_kb > 0 ? sub_kb : (pr.kb_per_split > 0 ? pr.kb_per_split : 1);
 }
 
 template <int KIND, int BN, int STAGES, class Epi, int NACC = 1, bool SUM = false, int TERMS = 1>
@@ -987,7 +1109,8 @@ int launch(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, long lo
            int nbatch, const Epi &epi, int sm_count, int *derr, cudaStream_t s,
            const char *prof_name, int max_ctas = 0, const int *nbatch_dev = nullptr,
            int ksplit = 1, int seg_kb = 0, unsigned seg_x = 0, unsigned seg_y = 0,
-           int kb_range = 0, int sub_kb = 0) {
+           int tb_unit = 0, int tb_sub = 0) {
+  if (SUM && (tb_unit < 1 || tb_sub < 1)) return B2_ERR_ARG;
   if (NACC > 1 && (ksplit > 1 || nbatch != NACC || nbatch_dev)) return B2_ERR_ARG;
   using L = SmemLayout<BN, STAGES, TERMS>;
   Problem pr;
@@ -1004,7 +1127,7 @@ int launch(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, long lo
   pr.group = 8;
   pr.derr = derr;
   launch_wait_settings(&pr.wait_ns, &pr.withhold);
-  set_split(pr, ksplit, kb_range, SUM ? sub_kb : 0);
+  set_split(pr, ksplit, TERMS, SUM ? tb_unit : 0, tb_sub);
   const long long total =
       (long long)pr.tiles_p * pr.tiles_q * (NACC == 1 ? nbatch : 1) * pr.ksplit;
   if (total <= 0 || (NACC > 1 && pr.kblocks <= 0)) return B2_OK;
@@ -1042,7 +1165,8 @@ template <int KIND, int BN, int STAGES, class Epi, bool SUM = false, int TERMS =
 int launch_pair(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, long long kelems,
                 int nbatch, const Epi &epi, int device, int *derr, cudaStream_t s,
                 const char *prof_name, const int *nbatch_dev = nullptr, int ksplit = 1,
-                int seg_kb = 0, int kb_range = 0, int sub_kb = 0) {
+                int seg_kb = 0, int tb_unit = 0, int tb_sub = 0) {
+  if (SUM && (tb_unit < 1 || tb_sub < 1)) return B2_ERR_ARG;
   using L = SmemLayout<BN / 2, STAGES, TERMS>;
   Problem pr;
   pr.P = P;
@@ -1052,7 +1176,7 @@ int launch_pair(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, lo
   pr.nbatch_dev = nbatch_dev;
   pr.seg_kb = seg_kb;
   pr.seg_x = pr.seg_y = 0;
-  set_split(pr, ksplit, kb_range, SUM ? sub_kb : 0);
+  set_split(pr, ksplit, TERMS, SUM ? tb_unit : 0, tb_sub);
   pr.tiles_p = (P + PAIR_BM - 1) / PAIR_BM;
   pr.tiles_q = (Q + BN - 1) / BN;
   pr.group = 8;
