@@ -157,11 +157,14 @@ struct F32Epi {
   int ldc;
   int M, N;
   float alpha, beta;
-  // Brings the warp's 32 rows x 128 columns of C (rows from p0) into L2 while
+  static constexpr bool PARTIAL = false;
+  __device__ __forceinline__ bool wide() const { return false; }
+  // Brings the warp's 32 rows x NC columns of C (rows from p0) into L2 while
   // the product is formed: one line per lane and column.
+  template <int NC>
   __device__ __forceinline__ void prefetch(int p0, int lane, int q0) const {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < NC / 32; ++i) {
       const int q = q0 + 32 * i + lane;
       if (p0 < M && q < N) umma::prefetch_l2(C + (long long)q * ldc + p0);
     }
@@ -191,18 +194,23 @@ struct F32Epi {
   }
 };
 
-// Split-K epilogue: the raw FP32 partial of K range ks (the engine's batch
-// index) to W[ks][n][ldw]; sgemm_splitk_reduce_kernel adds the ranges in a
-// fixed order.
-struct F32PartialEpi {
-  float *W;
+// Split-K epilogue: the partial of unit ks (the engine's batch index) to
+// W[ks][n][ldw]: one accumulator, FP32, or (pairs) the sum of several with its rounding
+// error, both at 1/16; sgemm_splitk_reduce_kernel adds the units in a fixed order.
+struct PartialEpi {
+  void *W;
   long long plane;
   int ldw;
   int M, N;
+  bool pairs;
+  static constexpr bool PARTIAL = true;
+  __device__ __forceinline__ bool wide() const { return pairs; }
+  template <int NC>
   __device__ __forceinline__ void prefetch(int, int, int) const {}
-  __device__ __forceinline__ void operator()(int ks, int p, int q0, const float (&v)[16]) const {
+  template <typename T>  // float or float2
+  __device__ __forceinline__ void operator()(int ks, int p, int q0, const T (&v)[16]) const {
     if (p >= M || q0 >= N) return;
-    float *w = W + ks * plane + (long long)q0 * ldw + p;
+    T *w = (T *)W + ks * plane + (long long)q0 * ldw + p;
     const int nq = min(16, N - q0);
 #pragma unroll
     for (int j = 0; j < 16; ++j)
@@ -210,12 +218,30 @@ struct F32PartialEpi {
   }
 };
 
+// One partial in FP64 (an infinity's error is a NaN: it is itself).
+__device__ __forceinline__ double partial(float x) { return (double)x; }
+__device__ __forceinline__ double partial(float2 x) {
+  const double s = (double)x.x, r = s + (double)x.y;
+  return 16.0 * (r == r ? r : s);
+}
+__device__ __forceinline__ void add4(double (&acc)[4], const float *w) {
+  const float4 x = *reinterpret_cast<const float4 *>(w);
+  acc[0] += (double)x.x, acc[1] += (double)x.y, acc[2] += (double)x.z, acc[3] += (double)x.w;
+}
+__device__ __forceinline__ void add4(double (&acc)[4], const float2 *w) {
+  const float4 x = *reinterpret_cast<const float4 *>(w);
+  const float4 y = *reinterpret_cast<const float4 *>(w + 2);
+  acc[0] += partial(make_float2(x.x, x.y)), acc[1] += partial(make_float2(x.z, x.w));
+  acc[2] += partial(make_float2(y.x, y.y)), acc[3] += partial(make_float2(y.z, y.w));
+}
+
 // C(m, n) = alpha * sum_ks W[ks][n][m] + beta C (beta != 1 multiplies), the
 // partials summed in FP64 in K order and rounded once.
 // Four rows per thread; launched as a programmatic dependent of the GEMM, whose
 // writes it waits for.  W is 16-byte aligned and ldw a multiple of 4.
+template <typename T>
 __global__ void __launch_bounds__(256)
-    sgemm_splitk_reduce_kernel(const float *__restrict__ W, long long plane, int ldw, int S, int M,
+    sgemm_splitk_reduce_kernel(const T *__restrict__ W, long long plane, int ldw, int S, int M,
                                int N, float alpha, float beta, float *__restrict__ C, int ldc) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const unsigned quads = (unsigned)(M + 3) / 4;
@@ -225,7 +251,7 @@ __global__ void __launch_bounds__(256)
        i += gridDim.x * 256ull) {
     const int n = (int)(i / quads), m = (int)(i - (unsigned long long)n * quads) * 4;
     float *c = C + (long long)n * ldc + m;
-    const float *w = W + (long long)n * ldw + m;
+    const T *w = W + (long long)n * ldw + m;
     const int left = M - m;
     float old[4];
     if (cvec && left >= 4) {
@@ -237,10 +263,7 @@ __global__ void __launch_bounds__(256)
     }
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 4
-    for (int ks = 0; ks < S; ++ks) {
-      const float4 x = *reinterpret_cast<const float4 *>(w + ks * plane);
-      acc[0] += (double)x.x, acc[1] += (double)x.y, acc[2] += (double)x.z, acc[3] += (double)x.w;
-    }
+    for (int ks = 0; ks < S; ++ks) add4(acc, w + ks * plane);
     float r[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -278,58 +301,81 @@ int choose_ksplit(long long tiles, int kblocks, int sms) {
 
 inline long long round_up(long long x, long long a) { return (x + a - 1) / a * a; }
 
-// Work units of a product whose K is accumulated in S ranges of tbs term blocks (a
-// K block of a three-term product is three: its MMAs add Ab Bb, Ab Bs and As Bb in
-// turn): each unit takes `per` consecutive ranges of its tile (adding them in its
-// epilogue), so that ceil(S / per) partials per tile go through memory.  Ranges are
-// as short as separate launches per range would have them: the tensor core's
-// accumulation error grows with a chain's length (ranges of whole K blocks, 3xTF32
-// with K = 64: 3.8e-7 instead of 1.1e-7).
-// Modelled time (us): waves of units, each 3 us of fill and final epilogue and,
-// per range, t_tb per term block (measured MMA rate of the engine) but at least
-// the 1.1 us that adding an accumulator to the sums takes (8 ranges of one K
-// block each: 512^3 11.7 us in one unit per tile, 6.6 in several); plus the
-// partials written and read at about 6 TB/s and a second launch.  2048^3
-// 3xTF32 (64 pair tiles on 74 pairs, 8 ranges): one unit per tile instead of 8
-// partials of 16.8 MB.
-int ranges_per_unit(long long tiles, int S, int tbs, int tblocks, int slots, double t_tb, int m,
-                    int n) {
-  int best = S;
+// Tile of an engine (rows m x columns n), CTAs or pairs that run at once, and time of
+// a term block (us: measured; with one term a 128 x 128 tile waits for its copies).
+struct Engine {
+  int tile_p, tile_q, slots;
+  double t_tb;
+};
+Engine engine(int eng, int terms, int sms) {  // of SgCfg
+  switch (eng) {
+    case 1: return Engine{umma::BM, 128, sms, terms == 1 ? 0.31 : 0.21};
+    case 2: return Engine{256, 256, sms / 2, 0.28};
+    default: return Engine{umma::BM, 256, sms, 0.28};
+  }
+}
+
+// How a product is run: engine, partials per tile, term blocks per unit and per
+// accumulated range; pairs: the partials are sums with their errors.
+struct Ranges {
+  int eng, E, unit_tb, range_tb;
+  bool pairs;
+  size_t bytes() const { return pairs ? sizeof(float2) : sizeof(float); }  // of a partial
+};
+
+// K is accumulated in S ranges of tbs term blocks (a K block of a three-term product is
+// three: its MMAs add Ab Bb, Ab Bs and As Bb in turn): `split` of them (0: chosen for
+// the engine's tiles).  Ranges are as short as separate launches per range would have
+// them: the tensor core's accumulation error grows with a chain's length (ranges of
+// whole K blocks, 3xTF32 with K = 64: 3.8e-7 instead of 1.1e-7).  Either each range is
+// a unit of its own, on engine `eng`, and S partials per tile go through memory; or a
+// unit takes `per` consecutive ranges of its tile and adds them in its epilogue, on
+// engine 1: 64 sums and their rounding errors are what a thread has registers for.
+// (128 of them, for tiles of 256 columns, spill, and the spills leave for L2: 12 us a
+// launch.  A pair's tile of 256 x 128 takes 0.23 us a term block, limited by its
+// copies, against 0.21 for half of it on engine 1.)
+// Modelled time (us): waves of units, each t_tb per term block but at least 1 us a
+// range, which is what adding an accumulator to the sums takes; fill, drain and the
+// gaps between waves; partials written and read, in L2 below 64 MB, and a second
+// launch.  nprod: products of that shape in one launch.  Measured (B200, us, whole
+// calls, partials of each range / the best sums): 3xTF32 512^3 11.9 / 12.9, 1024^3
+// 26.7 / 24.5 (4 ranges a unit), 2048^3 117 / 100, 8192x256x8192 272 / 291; 3xBF16
+// 2048^3 89.6 / 61.4; cgemm3m 2048^3 381 / 300, 1900x1300x2100 201 / 205.
+Ranges choose_ranges(int eng, int split, int terms, int kblocks, int m, int n, int nprod,
+                     int sms) {
+  const int tblocks = terms * kblocks;
+  auto tiles = [&](const Engine &g) {
+    return ((m + g.tile_p - 1) / g.tile_p) * (long long)((n + g.tile_q - 1) / g.tile_q);
+  };
+  const Engine base = engine(eng, terms, sms), adder = engine(1, terms, sms);
+  int S = split > 0 ? split : choose_ksplit(tiles(base), tblocks, base.slots);
+  if (S > tblocks) S = tblocks > 0 ? tblocks : 1;
+  const int tbs = (tblocks + S - 1) / S;
+  S = (tblocks + tbs - 1) / tbs;
+  Ranges best{};
   double best_us = 1e300;
-  for (int per = S; per >= 1; --per) {
+  for (int per = 1; per <= S; ++per) {
     const int E = (S + per - 1) / per;
     if (per > 1 && (S + per - 2) / (per - 1) == E) continue;  // more even with per - 1
-    const long long waves = (tiles * E + slots - 1) / slots;
+    const bool pairs = E > 1 && per > 1;
+    if (pairs && 2 * E > S) continue;  // no more scratch than one FP32 partial per range
+    const Engine &g = per > 1 ? adder : base;
+    const long long waves = (nprod * tiles(g) * E + g.slots - 1) / g.slots;
     const int tb = per * tbs < tblocks ? per * tbs : tblocks;
-    const double work = tb * t_tb, drains = 1.1 * ((tb + tbs - 1) / tbs);
-    double us = (double)waves * ((work > drains ? work : drains) + 3.0);
-    if (E > 1) us += 2.0 + (double)E * m * n * 8.0 / 6e6;
-    if (us < best_us) best_us = us, best = per;
+    const double work = tb * g.t_tb, drains = 1.0 * ((tb + tbs - 1) / tbs);
+    double us = (double)waves * (work > drains ? work : drains) + 4.0 + 0.7 * (double)(waves - 1);
+    if (E > 1) {
+      const double bytes = (double)E * m * n * nprod * (pairs ? 16.0 : 8.0);
+      us += 2.0 + bytes / (bytes < 64e6 ? 12e6 : 6e6);
+    }
+    if (us < best_us) best_us = us, best = Ranges{per > 1 ? 1 : eng, E, per * tbs, tbs, pairs};
   }
   return best;
 }
 
-// Partials per tile, term blocks per unit and per accumulated range.
-struct Ranges {
-  int E, unit_tb, range_tb;
-};
-
-// The ranges of a product of `tblocks` term blocks: `split` of them (0: chosen for
-// `tiles` tiles on `slots` engines), dealt to units.  nprod: products of that shape
-// in one launch.
-Ranges choose_ranges(int split, int tblocks, long long tiles, int slots, int nprod, double t_tb,
-                     int m, int n) {
-  int S = split > 0 ? split : choose_ksplit(tiles, tblocks, slots);
-  if (S > tblocks) S = tblocks > 0 ? tblocks : 1;
-  const int tbs = (tblocks + S - 1) / S;
-  S = (tblocks + tbs - 1) / tbs;
-  const int per = ranges_per_unit(nprod * tiles, S, tbs, tblocks, slots, t_tb, m, nprod * n);
-  return Ranges{(S + per - 1) / per, per * tbs, tbs};
-}
-
-// One SGEMM product (or nbatch of them) on engine `eng` (see SgCfg).
+// One SGEMM product (or nbatch of them).
 template <class Epi>
-int run_engine(int eng, bool bf16, int terms, const CUtensorMap &tmX, const CUtensorMap &tmY, int m,
+int run_engine(bool bf16, int terms, const CUtensorMap &tmX, const CUtensorMap &tmY, int m,
                int n, int kp, int nbatch, int seg_kb, const Ranges &rg, const Epi &epi, Ctx *cx,
                cudaStream_t s) {
   const char *nm = bf16 ? "sgemm_umma_bf16" : "sgemm_umma_tf32";
@@ -353,8 +399,9 @@ int run_engine(int eng, bool bf16, int terms, const CUtensorMap &tmX, const CUte
   using I3 = std::integral_constant<int, 3>;
   using I128 = std::integral_constant<int, 128>;
   using I256 = std::integral_constant<int, 256>;
-  if (eng == 2) return bf16 ? pair(BF{}, I3{}) : terms == 3 ? pair(TF{}, I3{}) : pair(TF{}, I1{});
-  if (eng == 1)
+  if (rg.eng == 2)
+    return bf16 ? pair(BF{}, I3{}) : terms == 3 ? pair(TF{}, I3{}) : pair(TF{}, I1{});
+  if (rg.eng == 1)
     return bf16         ? single(BF{}, I128{}, I3{})
            : terms == 3 ? single(TF{}, I128{}, I3{})
                         : single(TF{}, I128{}, I1{});
@@ -362,6 +409,9 @@ int run_engine(int eng, bool bf16, int terms, const CUtensorMap &tmX, const CUte
          : terms == 3 ? single(TF{}, I256{}, I3{})
                       : single(TF{}, I256{}, I1{});
 }
+
+// Rows of Y in one TMA box: a CTA's.
+int y_box(int eng) { return eng == 0 ? 256 : 128; }
 
 // Launch as a programmatic dependent of the kernel before it in the stream
 // (the kernel waits for that one's writes with griddepcontrol.wait).
@@ -379,6 +429,18 @@ cudaError_t launch_dependent(void (*kern)(KArgs...), unsigned blocks, int thread
   lc.numAttrs = 1;
   const cudaError_t e = cudaLaunchKernelEx(&lc, kern, args...);
   return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+template <typename T>
+int splitk_reduce(const T *W, long long plane, int ldw, int S, int m, int n, float alpha,
+                  float beta, float *C, int ldc, cudaStream_t s) {
+  const long long blocks = ((long long)((m + 3) / 4) * n + 255) / 256;
+  B2_PROF("sgemm_splitk_reduce", s);
+  // 8 blocks on each of 148 SMs
+  B2_CUDA_TRY(launch_dependent(sgemm_splitk_reduce_kernel<T>,
+                               (unsigned)(blocks < 1184 ? blocks : 1184), 256, s, W, plane, ldw, S,
+                               m, n, alpha, beta, C, ldc));
+  return B2_OK;
 }
 
 SplitOp split_op(const float *X, long long sr, long long sk, int R, void *out) {
@@ -482,8 +544,9 @@ __global__ void __launch_bounds__(256)
 
 // C = alpha (P1 - P2 + i (P3 - P1 - P2)) + beta C from the E partials of each
 // product (plane t*E + e of W), summed in FP64 and rounded once.
+template <typename T>
 __global__ void __launch_bounds__(256)
-    combine3m_tc_kernel(const float *__restrict__ W, long long plane, int ldw, int E, int M, int N,
+    combine3m_tc_kernel(const T *__restrict__ W, long long plane, int ldw, int E, int M, int N,
                         float ar, float ai, float br, float bi, float *__restrict__ C, int ldc) {
   umma::grid_dependency_wait();
   const bool beta_one = br == 1.f && bi == 0.f;
@@ -491,17 +554,17 @@ __global__ void __launch_bounds__(256)
   for (unsigned long long i = blockIdx.x * 256ull + threadIdx.x; i < total;
        i += gridDim.x * 256ull) {
     const int n = (int)(i / (unsigned)M), m = (int)(i - (unsigned long long)n * (unsigned)M);
-    const float *w = W + (long long)n * ldw + m;
+    const T *w = W + (long long)n * ldw + m;
     float *c = C + 2 * ((long long)n * ldc + m);
     float cr = c[0], ci = c[1], p[3];
     if (E == 1) {
 #pragma unroll
-      for (int t = 0; t < 3; ++t) p[t] = w[t * plane];
+      for (int t = 0; t < 3; ++t) p[t] = (float)partial(w[t * plane]);
     } else {
       double acc[3] = {0.0, 0.0, 0.0};
       for (int e = 0; e < E; ++e)
 #pragma unroll
-        for (int t = 0; t < 3; ++t) acc[t] += (double)w[(t * E + e) * plane];
+        for (int t = 0; t < 3; ++t) acc[t] += partial(w[(t * E + e) * plane]);
 #pragma unroll
       for (int t = 0; t < 3; ++t) p[t] = (float)acc[t];
     }
@@ -539,21 +602,19 @@ int cgemm3m_tensor(char ta, char tb, int m, int n, int k, float ar, float ai, fl
   const long long ks = 2LL * kp;
   // engine and K ranges as for one 3xTF32 SGEMM of this shape
   const SgCfg cfg = sgemm_pick_cfg('N', 'N', m, n, k, 1, B2_METHOD_TF32X3);
-  const int eng = (cfg.engine >= 0 && cfg.engine <= 2) ? cfg.engine : 0;
-  const int tile_p = eng == 2 ? 256 : umma::BM, tile_q = eng == 1 ? 128 : 256;
-  const int seg_kb = kp * 4 / umma::KBLOCK_BYTES, kblocks = seg_kb;
-  const long long tiles = ((n + tile_q - 1) / tile_q) * (long long)((m + tile_p - 1) / tile_p);
-  const int slots = eng == 2 ? cx->sm_count / 2 : cx->sm_count;
-  const Ranges rg =
-      choose_ranges(cfg.split, 3 * kblocks, tiles, slots, 3, eng == 1 ? 0.17 : 0.28, m, n);
+  const int seg_kb = kp * 4 / umma::KBLOCK_BYTES;
+  const Ranges rg = choose_ranges((cfg.engine >= 0 && cfg.engine <= 2) ? cfg.engine : 0, cfg.split,
+                                  3, seg_kb, m, n, 3, cx->sm_count);
   const int E = rg.E;
   const int ldw = (int)round_up(m, 32);
   const long long plane = (long long)n * ldw;
   // the split segments of both operands, then the products' sums
   float *Xp = (float *)workspace(
-      cx, WS_3M, (size_t)(3 * (m + (long long)n) * ks + plane * 3 * E) * sizeof(float));
+      cx, WS_3M, (size_t)(3 * (m + (long long)n) * ks) * sizeof(float) +
+                     (size_t)(plane * 3 * E) * rg.bytes());
   if (!Xp) return B2_ERR_NOMEM;
-  float *Yp = Xp + 3 * m * ks, *W = Yp + 3 * n * ks;
+  float *Yp = Xp + 3 * m * ks;
+  void *W = Yp + 3 * n * ks;
   {
     const unsigned kt = (unsigned)kp / 32;
     const unsigned ba = kt * ((unsigned)(m + 63) / 64), bb = kt * ((unsigned)(n + 63) / 64);
@@ -566,15 +627,19 @@ int cgemm3m_tensor(char ta, char tb, int m, int n, int k, float ar, float ai, fl
                                  umma::BM);
   if (rc == B2_OK)
     rc = umma::make_kmajor_map(&tmY, umma::KIND_TF32, Yp, ks, n, 3, ks * 4, (long long)n * ks * 4,
-                               eng == 0 ? 256 : 128);
+                               y_box(rg.eng));
   if (rc != B2_OK) return rc;
-  rc = run_engine(eng, false, 3, tmX, tmY, m, n, kp, 3, seg_kb, rg,
-                  F32PartialEpi{W, plane, ldw, m, n}, cx, s);
+  rc = run_engine(false, 3, tmX, tmY, m, n, kp, 3, seg_kb, rg,
+                  PartialEpi{W, plane, ldw, m, n, rg.pairs}, cx, s);
   if (rc != B2_OK) return rc;
   const long long blocks = ((long long)m * n + 255) / 256;
   B2_PROF("gemm3m_combine", s);
-  B2_CUDA_TRY(launch_dependent(combine3m_tc_kernel, (unsigned)(blocks < 2368 ? blocks : 2368), 256,
-                               s, (const float *)W, plane, ldw, E, m, n, ar, ai, br, bi, C, ldc));
+  const unsigned grid = (unsigned)(blocks < 2368 ? blocks : 2368);
+  B2_CUDA_TRY(rg.pairs ? launch_dependent(combine3m_tc_kernel<float2>, grid, 256, s,
+                                         (const float2 *)W, plane, ldw, E, m, n, ar, ai, br, bi, C,
+                                         ldc)
+                      : launch_dependent(combine3m_tc_kernel<float>, grid, 256, s, (const float *)W,
+                                         plane, ldw, E, m, n, ar, ai, br, bi, C, ldc));
   return B2_OK;
 }
 
@@ -637,45 +702,36 @@ int sgemm_tensor_cfg(char ta, char tb, int m, int n, int k, float alpha, const f
                 : run_split<float>(oa, ob, k, kp, segs, s);
   if (rc != B2_OK) return rc;
   const int kind = bf16 ? umma::KIND_BF16 : umma::KIND_TF32;
-  const int eng = (cfg.engine >= 0 && cfg.engine <= 2) ? cfg.engine : 0;
-  // tile: X rows (m) x Y rows (n) per tile; TMA boxes per CTA
-  const int tile_p = eng == 2 ? 256 : umma::BM, tile_q = eng == 1 ? 128 : 256;
-  const int ybox = eng == 0 ? 256 : 128;
+  const int seg_kb = terms == 3 ? (int)((long long)kp * esz / umma::KBLOCK_BYTES) : 0;
+  const int kblocks = (int)(((long long)kp * esz + umma::KBLOCK_BYTES - 1) / umma::KBLOCK_BYTES);
+  const Ranges rg = choose_ranges((cfg.engine >= 0 && cfg.engine <= 2) ? cfg.engine : 0, cfg.split,
+                                  terms, kblocks, m, n, 1, cx->sm_count);
+  const int E = rg.E;  // partials per tile
   CUtensorMap tmX, tmY;
   rc = umma::make_kmajor_map(&tmX, kind, Xp, ks_, m, 1, ks_ * esz, (long long)m * ks_ * esz,
                              umma::BM);
   if (rc == B2_OK)
-    rc = umma::make_kmajor_map(&tmY, kind, Yp, ks_, n, 1, ks_ * esz, (long long)n * ks_ * esz, ybox);
+    rc = umma::make_kmajor_map(&tmY, kind, Yp, ks_, n, 1, ks_ * esz, (long long)n * ks_ * esz,
+                               y_box(rg.eng));
   if (rc != B2_OK) return rc;
-  const int seg_kb = terms == 3 ? (int)((long long)kp * esz / umma::KBLOCK_BYTES) : 0;
-  const long long tiles = ((n + tile_q - 1) / tile_q) * (long long)((m + tile_p - 1) / tile_p);
-  const int kblocks = (int)(((long long)kp * esz + umma::KBLOCK_BYTES - 1) / umma::KBLOCK_BYTES);
-  const int slots = eng == 2 ? cx->sm_count / 2 : cx->sm_count;
-  const Ranges rg =
-      choose_ranges(cfg.split, terms * kblocks, tiles, slots, 1, eng == 1 ? 0.17 : 0.28, m, n);
-  const int E = rg.E;  // partials per tile
   if (E == 1)
-    return run_engine(eng, bf16, terms, tmX, tmY, m, n, kp, 1, seg_kb, rg,
+    return run_engine(bf16, terms, tmX, tmY, m, n, kp, 1, seg_kb, rg,
                       F32Epi{C, ldc, m, n, alpha, beta}, cx, s);
   // E partial products of K ranges, then one fixed-order reduction.
   const int ldw = (int)round_up(m, 32);
   const long long plane = (long long)n * ldw;
-  float *W = (float *)workspace(cx, WS_MISC, (size_t)plane * E * sizeof(float));
+  void *W = workspace(cx, WS_MISC, (size_t)plane * E * rg.bytes());
   if (!W) return B2_ERR_NOMEM;
-  rc = run_engine(eng, bf16, terms, tmX, tmY, m, n, kp, 1, seg_kb, rg,
-                  F32PartialEpi{W, plane, ldw, m, n}, cx, s);
+  rc = run_engine(bf16, terms, tmX, tmY, m, n, kp, 1, seg_kb, rg,
+                  PartialEpi{W, plane, ldw, m, n, rg.pairs}, cx, s);
   if (rc != B2_OK) return rc;
-  return sgemm_splitk_reduce(W, plane, ldw, E, m, n, alpha, beta, C, ldc, s);
+  return rg.pairs ? splitk_reduce((const float2 *)W, plane, ldw, E, m, n, alpha, beta, C, ldc, s)
+                 : splitk_reduce((const float *)W, plane, ldw, E, m, n, alpha, beta, C, ldc, s);
 }
 
 int sgemm_splitk_reduce(const float *W, long long plane, int ldw, int S, int m, int n,
                         float alpha, float beta, float *C, int ldc, cudaStream_t s) {
-  const long long blocks = ((long long)((m + 3) / 4) * n + 255) / 256;
-  B2_PROF("sgemm_splitk_reduce", s);
-  // 8 blocks on each of 148 SMs
-  B2_CUDA_TRY(launch_dependent(sgemm_splitk_reduce_kernel, (unsigned)(blocks < 1184 ? blocks : 1184),
-                               256, s, W, plane, ldw, S, m, n, alpha, beta, C, ldc));
-  return B2_OK;
+  return splitk_reduce(W, plane, ldw, S, m, n, alpha, beta, C, ldc, s);
 }
 
 }  // namespace b2

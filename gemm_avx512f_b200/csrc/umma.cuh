@@ -10,7 +10,7 @@
 // memory, and the 24x8 FMA register tile of src/kernel/gemm_kernel.S becomes
 // 128 x BN x 32-byte tcgen05.mma instructions accumulating in TMEM.
 //
-// Roles (192 threads, 320 in SUM kernels with BN = 256; one CTA per SM):
+// Roles (192 threads, 320 in SUM kernels; one CTA per SM):
 //   warp 0      TMA producer: fills a STAGES-deep ring of (X, Y) K-blocks.
 //   warp 1      TMEM owner + MMA issuer (one elected lane).
 //   warps 2..   epilogue: tcgen05.ld of their 32-lane quarter of the
@@ -19,10 +19,12 @@
 // overlaps the MMAs of tile i+1.
 // SUM kernels cut a unit's K range into sub-ranges, of term blocks (a K block of a
 // three-term product has three), that go through the two accumulators in turn;
-// the epilogue adds each to FP32 sums in its registers (128 columns a thread: 8
-// epilogue warps for BN = 256) while the next one is multiplied.  The tensor core's accumulation error grows with the length of a
-// chain, so the split forms of SGEMM keep chains short; this keeps them short
-// without writing the partial products to memory.
+// the epilogue adds each to sums in its registers (BN = 128: 64 columns a thread)
+// while the next one is multiplied.  The tensor core's accumulation error grows with
+// the length of a chain, so the split forms of SGEMM keep chains short; this keeps
+// them short without writing the partial products to memory.  The sums carry their
+// rounding errors along and are rounded once, as if they were FP64.  BN = 256 leaves
+// no registers for that: its units are one sub-range.
 //
 // Every mbarrier wait is bounded (Problem::wait_ns of wall time from
 // %globaltimer, 2 s unless a test shortens it); on expiry the waiter stores
@@ -324,45 +326,164 @@ __host__ __device__ constexpr int tmem_cols(int need) {
   return need <= 32 ? 32 : need <= 64 ? 64 : need <= 128 ? 128 : need <= 256 ? 256 : 512;
 }
 
-// Epilogue warps and threads: SUM kernels hold BN / (warps / 4) = 128 sums a thread.
-__host__ __device__ constexpr int epi_warps(int bn, bool sum) { return sum && bn > 128 ? 8 : 4; }
-__host__ __device__ constexpr int threads_for(int bn, bool sum) { return 64 + 32 * epi_warps(bn, sum); }
+// Epilogue warps and threads; a thread of a SUM kernel has BN / 2 columns.
+__host__ __device__ constexpr int epi_warps(bool sum) { return sum ? 8 : 4; }
+__host__ __device__ constexpr int threads_for(bool sum) { return 64 + 32 * epi_warps(sum); }
+// SUM kernels that add several sub-ranges per unit
+__host__ __device__ constexpr bool adds(int bn, bool sum) { return sum && bn <= 128; }
+
+// Two FP32 operations per instruction, each rounded to nearest.
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t a, uint32_t &lo, uint32_t &hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(a));
+}
+
+// A sum of several accumulators is kept at 1/16 (16 ranges cannot pass FLT_MAX on the
+// way to a sum that does not; what that loses below 2^-122 is at most 2^-145): s as
+// FP32 additions give it and e the rounding errors of those additions, bfloat16 pairs
+// (8 bits of something 2^-20 of s at most).
+__device__ __forceinline__ float err_lo(uint32_t e) { return __uint_as_float(e << 16); }
+__device__ __forceinline__ float err_hi(uint32_t e) { return __uint_as_float(e & 0xffff0000u); }
 
 // Epilogue of one work unit of a SUM kernel for one warp: `nsub` accumulators
-// in turn, their columns [c0, c0 + 128) of this lane quarter added up, then
-// handed to the functor 16 columns at a time.  wait(it) waits for accumulator
-// it & 1 (false: abandoned), done(it) frees it.
-template <class Wait, class Done, class Out>
+// in turn (1 where NC is 128), their columns [c0, c0 + NC) of this lane quarter added
+// up, then handed to the functor 16 columns at a time: FP32 values or, where the
+// functor adds several units up later (Epi::PARTIAL and wide), the sums and their
+// errors at 1/16.  wait(it) waits for accumulator it & 1 (false: abandoned), done(it)
+// frees it.
+// An addition's rounding error is exact in FP32 (two-sum, Knuth, TAOCP 4.2.2).
+// 1 us for a sub-range (64 columns a thread).
+template <int NC, class Wait, class Done, class Out>
 __device__ __forceinline__ bool sum_epilogue(uint32_t tmem_quarter, int bn, int c0, int nsub,
-                                             int &it, Wait wait, Done done, Out out) {
-  // 16 columns at a time: 128 sums and one load's registers fit the 168 a
-  // thread that 8 + 2 warps leave
-  float s[8][16];
-  for (int i = 0; i < nsub; ++i, ++it) {
+                                             int &it, bool wide, Wait wait, Done done, Out out) {
+  constexpr int CH = NC / 16;
+  constexpr bool ADDS = NC <= 64;
+  uint64_t s[CH][8];
+  uint32_t e[ADDS ? CH : 1][8];
+  const bool several = ADDS && (nsub > 1 || wide);
+  const uint64_t scale = several ? 0x3d8000003d800000ull : 0x3f8000003f800000ull;  // 1/16 or 1
+  for (int i = 0; i < (ADDS ? nsub : 1); ++i, ++it) {
     if (!__all_sync(0xffffffffu, wait(it))) return false;
     tc_fence_after();
     const uint32_t taddr = tmem_quarter + (uint32_t)((it & 1) * bn + c0);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
+    for (int c = 0; c < CH; ++c) {
       uint32_t v[16];
       tmem_ld16(taddr + (uint32_t)(c * 16), v);
       tmem_ld16_wait(v);
-      if (i == 0) {
+      if constexpr (!ADDS) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) s[c][j] = __uint_as_float(v[j]);
+        for (int j = 0; j < 8; ++j) s[c][j] = pack2(v[2 * j], v[2 * j + 1]);
+      } else if (i == 0) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          s[c][j] = mul2(pack2(v[2 * j], v[2 * j + 1]), scale);
+          e[c][j] = 0;
+        }
       } else {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) s[c][j] += __uint_as_float(v[j]);
+        for (int j = 0; j < 8; ++j) {
+          const uint64_t a = s[c][j], b = pack2(v[2 * j], v[2 * j + 1]);  // b: times scale
+          const uint64_t t = fma2(b, scale, a), nb = sub2(a, t);  // nb: the part of -b in t
+          const uint64_t err = add2(sub2(a, add2(t, nb)), fma2(b, scale, nb));
+          s[c][j] = t;
+          uint32_t lo, hi, r;
+          unpack2(err, lo, hi);
+          asm("cvt.rn.bf16x2.f32 %0, %1, %2;"
+              : "=r"(r)
+              : "f"(__uint_as_float(hi)), "f"(__uint_as_float(lo)));
+          asm("add.rn.bf16x2 %0, %0, %1;" : "+r"(e[c][j]) : "r"(r));
+        }
       }
     }
     tc_fence_before();
     __syncwarp();
     done(it);
   }
+  if constexpr (ADDS && Out::PARTIAL) {
+    if (wide) {
 #pragma unroll
-  for (int c = 0; c < 8; ++c) out(c0 + 16 * c, s[c]);
+      for (int c = 0; c < CH; ++c) {
+        float2 r[16];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          uint32_t lo, hi;
+          unpack2(s[c][j], lo, hi);
+          r[2 * j] = make_float2(__uint_as_float(lo), err_lo(e[c][j]));
+          r[2 * j + 1] = make_float2(__uint_as_float(hi), err_hi(e[c][j]));
+        }
+        out(c0 + 16 * c, r);
+      }
+      return true;
+    }
+  }
+  if constexpr (ADDS) {
+    if (several) {
+      // rounded once; an infinity has a NaN for its error, and is itself
+#pragma unroll
+      for (int c = 0; c < CH; ++c)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const uint64_t r = mul2(add2(s[c][j], pack2(e[c][j] << 16, e[c][j] & 0xffff0000u)),
+                                  0x4180000041800000ull);  // 16
+          uint32_t lo, hi, slo, shi;
+          unpack2(r, lo, hi);
+          unpack2(s[c][j], slo, shi);
+          const float x = __uint_as_float(lo), y = __uint_as_float(hi);
+          s[c][j] = pack2(x == x ? lo : slo, y == y ? hi : shi);
+        }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    float r[16];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      uint32_t lo, hi;
+      unpack2(s[c][j], lo, hi);
+      r[2 * j] = __uint_as_float(lo);
+      r[2 * j + 1] = __uint_as_float(hi);
+    }
+    out(c0 + 16 * c, r);
+  }
   return true;
 }
+
+// A unit's functor call at its tile's place.
+template <class Epi>
+struct SumOut {
+  static constexpr bool PARTIAL = Epi::PARTIAL;
+  const Epi &epi;
+  int ks, p, q;
+  template <typename T>
+  __device__ __forceinline__ void operator()(int c, const T (&v)[16]) const {
+    epi(ks, p, q + c, v);
+  }
+};
 
 // Term blocks [t0, t1) and the K blocks [kb0, kb1) that hold them, of K range ks.
 template <bool SUM, int TERMS>
@@ -385,7 +506,7 @@ __device__ __forceinline__ void unit_range(const Problem &pr, int ks, int &t0, i
 // (epi(p, q0, v0, v1, v2) for NACC = 3: the three real products of the 3M
 // method); no split-K.
 template <int KIND, int BN, int STAGES, class Epi, int NACC = 1, bool SUM = false, int TERMS = 1>
-__global__ void __launch_bounds__(threads_for(BN, SUM), 1)
+__global__ void __launch_bounds__(threads_for(SUM), 1)
     umma_gemm_kernel(const __grid_constant__ CUtensorMap tmX,
                      const __grid_constant__ CUtensorMap tmY, const Problem pr, const Epi epi) {
   using L = SmemLayout<BN, STAGES, TERMS>;
@@ -396,7 +517,7 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
   static_assert(NACC == 1 || NACC == 3, "one accumulator, or three for the 3M products");
   static_assert(NACC == 3 || SETS == 2, "the single-accumulator engine double-buffers");
   constexpr int TCOLS = tmem_cols(SETS * NACC * BN);
-  static_assert(!SUM || (NACC == 1 && BN % 128 == 0), "summed epilogue: 128 columns a thread");
+  static_assert(!SUM || (NACC == 1 && BN % 128 == 0), "64 or 128 columns a thread");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -423,7 +544,7 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);
-      mbar_init(tempty_bar(a), epi_warps(BN, SUM));  // one arrival per epilogue warp
+      mbar_init(tempty_bar(a), epi_warps(SUM));  // one arrival per epilogue warp
     }
     mbar_init(drain_bar, 1);
     *abort_flag = 0;
@@ -604,10 +725,12 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
         int t0, t1, kb0, kb1;
         unit_range<SUM, TERMS>(pr, ks, t0, t1, kb0, kb1);
         const int p = tp * BM + quarter * 32 + lane;
-        epi.prefetch(p - lane, lane, tq * BN + (warp - 2) / 4 * 128);
-        if (!sum_epilogue(
-                tmem_base + ((uint32_t)(quarter * 32) << 16), BN, (warp - 2) / 4 * 128,
-                (t1 - t0 + pr.tb_sub - 1) / pr.tb_sub, it,
+        constexpr int NC = BN / 2;
+        const int c0 = (warp - 2) / 4 * NC;
+        epi.template prefetch<NC>(p - lane, lane, tq * BN + c0);
+        if (!sum_epilogue<NC>(
+                tmem_base + ((uint32_t)(quarter * 32) << 16), BN, c0,
+                (t1 - t0 + pr.tb_sub - 1) / pr.tb_sub, it, epi.wide(),
                 [&](int i) {
                   return mbar_wait(tfull_bar(i & 1), (uint32_t)((i >> 1) & 1), abort_flag, pr.derr,
                                    pr.wait_ns);
@@ -615,7 +738,7 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
                 [&](int i) {
                   if (lane == 0) mbar_arrive(tempty_bar(i & 1));
                 },
-                [&](int c, const float(&v)[16]) { epi(b * pr.ksplit + ks, p, tq * BN + c, v); }))
+                SumOut<Epi>{epi, b * pr.ksplit + ks, p, tq * BN}))
           break;
         continue;
       }
@@ -692,8 +815,8 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
 //   empty[s]  one per CTA; the leader's commit arrives on both (commit
 //             multicast to the pair).
 //   tfull[a]  one per CTA; the leader's commit arrives on both.
-//   tempty[a] only the leader's is used: 8 arrivals, the 4 epilogue warps of
-//             each CTA (remote arrive from the odd CTA).
+//   tempty[a] only the leader's is used: an arrival of each epilogue warp of both
+//             CTAs (remote arrive from the odd CTA).
 // A timeout in either CTA raises the abort flag of both.  The pair meets in a
 // cluster barrier before TMEM is freed, so no MMA of the leader can still be
 // writing the odd CTA's TMEM, and neither CTA leaves while the other's copies
@@ -784,14 +907,14 @@ __device__ __forceinline__ bool mbar_wait_pair(uint32_t bar, uint32_t parity,
 constexpr int PAIR_BM = 2 * BM;  // output rows per pair tile
 
 template <int KIND, int BN, int STAGES, class Epi, bool SUM = false, int TERMS = 1>
-__global__ void __launch_bounds__(threads_for(BN, SUM), 1)
+__global__ void __launch_bounds__(threads_for(SUM), 1)
     umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX,
                           const __grid_constant__ CUtensorMap tmY, const Problem pr,
                           const Epi epi) {
   using L = SmemLayout<BN / 2, STAGES, TERMS>;  // per CTA: 128 X rows + BN/2 Y rows per stage
   static_assert(BN % 32 == 0 && BN >= 64 && BN <= 256, "pair MMA N in [64, 256]");
   static_assert(2 * BN <= 512, "two accumulators must fit in TMEM");
-  static_assert(!SUM || BN % 128 == 0, "summed epilogue: 128 columns a thread");
+  static_assert(!SUM || BN % 128 == 0, "64 or 128 columns a thread");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -825,7 +948,7 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);
-      mbar_init(tempty_bar(a), 2 * epi_warps(BN, SUM));  // the epilogue warps of both CTAs
+      mbar_init(tempty_bar(a), 2 * epi_warps(SUM));  // the epilogue warps of both CTAs
     }
     mbar_init(drain_bar, 1);
     *abort_flag = 0;
@@ -1005,10 +1128,12 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
         int t0, t1, kb0, kb1;
         unit_range<SUM, TERMS>(pr, ks, t0, t1, kb0, kb1);
         const int p = tp * PAIR_BM + (int)rank * BM + quarter * 32 + lane;
-        epi.prefetch(p - lane, lane, tq * BN + (warp - 2) / 4 * 128);
-        if (!sum_epilogue(
-                tmem_base + ((uint32_t)(quarter * 32) << 16), BN, (warp - 2) / 4 * 128,
-                (t1 - t0 + pr.tb_sub - 1) / pr.tb_sub, it,
+        constexpr int NC = BN / 2;
+        const int c0 = (warp - 2) / 4 * NC;
+        epi.template prefetch<NC>(p - lane, lane, tq * BN + c0);
+        if (!sum_epilogue<NC>(
+                tmem_base + ((uint32_t)(quarter * 32) << 16), BN, c0,
+                (t1 - t0 + pr.tb_sub - 1) / pr.tb_sub, it, epi.wide(),
                 [&](int i) {
                   return mbar_wait_pair(tfull_bar(i & 1), (uint32_t)((i >> 1) & 1), abort_flag,
                                         peer_abort, pr.derr, pr.wait_ns);
@@ -1016,7 +1141,7 @@ __global__ void __launch_bounds__(threads_for(BN, SUM), 1)
                 [&](int i) {
                   if (lane == 0) mbar_arrive_remote(map_rank(tempty_bar(i & 1), 0));
                 },
-                [&](int c, const float(&v)[16]) { epi(b * pr.ksplit + ks, p, tq * BN + c, v); }))
+                SumOut<Epi>{epi, b * pr.ksplit + ks, p, tq * BN}))
           break;
         continue;
       }
@@ -1110,7 +1235,8 @@ int launch(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, long lo
            const char *prof_name, int max_ctas = 0, const int *nbatch_dev = nullptr,
            int ksplit = 1, int seg_kb = 0, unsigned seg_x = 0, unsigned seg_y = 0,
            int tb_unit = 0, int tb_sub = 0) {
-  if (SUM && (tb_unit < 1 || tb_sub < 1)) return B2_ERR_ARG;
+  if (SUM && (tb_unit < 1 || tb_sub < 1 || (!adds(BN, SUM) && tb_sub < tb_unit)))
+    return B2_ERR_ARG;
   if (NACC > 1 && (ksplit > 1 || nbatch != NACC || nbatch_dev)) return B2_ERR_ARG;
   using L = SmemLayout<BN, STAGES, TERMS>;
   Problem pr;
@@ -1143,7 +1269,7 @@ int launch(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, long lo
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(threads_for(BN, SUM));
+    cfg.blockDim = dim3(threads_for(SUM));
     cfg.dynamicSmemBytes = L::TOTAL;
     cfg.stream = s;
     cfg.attrs = attr;
@@ -1151,7 +1277,7 @@ int launch(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, long lo
     e = cudaLaunchKernelEx(&cfg, kern, tmX, tmY, pr, epi);
     if (e == cudaSuccess) e = cudaGetLastError();
   } else {
-    kern<<<grid, threads_for(BN, SUM), L::TOTAL, s>>>(tmX, tmY, pr, epi);
+    kern<<<grid, threads_for(SUM), L::TOTAL, s>>>(tmX, tmY, pr, epi);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) return cuda_fail(e, prof_name);
@@ -1166,7 +1292,8 @@ int launch_pair(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, lo
                 int nbatch, const Epi &epi, int device, int *derr, cudaStream_t s,
                 const char *prof_name, const int *nbatch_dev = nullptr, int ksplit = 1,
                 int seg_kb = 0, int tb_unit = 0, int tb_sub = 0) {
-  if (SUM && (tb_unit < 1 || tb_sub < 1)) return B2_ERR_ARG;
+  if (SUM && (tb_unit < 1 || tb_sub < 1 || (!adds(BN, SUM) && tb_sub < tb_unit)))
+    return B2_ERR_ARG;
   using L = SmemLayout<BN / 2, STAGES, TERMS>;
   Problem pr;
   pr.P = P;
@@ -1191,7 +1318,7 @@ int launch_pair(const CUtensorMap &tmX, const CUtensorMap &tmY, int P, int Q, lo
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  cfg.blockDim = dim3(threads_for(BN, SUM));
+  cfg.blockDim = dim3(threads_for(SUM));
   cfg.dynamicSmemBytes = L::TOTAL;
   cfg.stream = s;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;

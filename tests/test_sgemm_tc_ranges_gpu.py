@@ -44,3 +44,41 @@ def test_terms_of_a_k_block_are_chains_of_their_own(cuda, method, engine, m, n):
     a[:, [0, 1, kb, kb + 1]] = [big, 1.0, -big, -1.0]
     b[[0, 1, kb, kb + 1]] = np.array([[s], [s + 1], [s], [s]], np.float32)
     assert (_run(cuda, method, engine, 3, a, b) == 1.0).all()
+
+
+def _in_k_blocks(method, m, n, values):
+    """Operands whose K block i holds the one product values[i][0] * values[i][1]."""
+    kb = KBLOCK[method]
+    a = np.zeros((m, len(values) * kb), np.float32)
+    b = np.zeros((len(values) * kb, n), np.float32)
+    a[:, ::kb] = [x for x, _ in values]
+    b[::kb] = np.array([[y] for _, y in values], np.float32)
+    return a, b
+
+
+@pytest.mark.parametrize("engine", [0, 1, 2])
+@pytest.mark.parametrize("method", sorted(METHOD))
+@pytest.mark.parametrize("log2split", [2, 3])
+@pytest.mark.parametrize("m,n", [(128, 100), (1024, 1024), (2300, 1500)])
+def test_ranges_are_added_as_in_fp64(cuda, method, engine, log2split, m, n):
+    """Eight K blocks in 4 or 8 ranges, one unit per tile (many tiles) or several: the
+    ranges' sums are added with their rounding errors (eight bits of them, where one
+    unit adds several ranges) and rounded once."""
+    zero = (0.0, 0.0)
+
+    def run(first, second, third):
+        # two K blocks apart: different ranges of four as well
+        v = [first, zero, second, zero, third, zero, zero, zero]
+        return _run(cuda, method, engine, log2split, *_in_k_blocks(method, m, n, v))
+
+    # FP32 additions in order would drop the 1
+    assert (run((2.0 ** 14, 2.0 ** 13), (1.0, 1.0), (-2.0 ** 14, 2.0 ** 13)) == 1.0).all()
+    # ... and the last bit here: 2^24 + 1 + 2^-6 lies above the middle of two floats
+    assert (run((2.0 ** 12, 2.0 ** 12), (1.0, 1.0), (2.0 ** -3, 2.0 ** -3)) == 2.0 ** 24 + 2).all()
+    # ... and pass FLT_MAX on the way to a sum that does not
+    x = (2.0 ** 64, 1.5 * 2.0 ** 63)
+    assert (run(x, x, (-x[0], x[1])) == np.float32(1.5 * 2.0 ** 127)).all()
+    assert np.isposinf(run(x, x, zero)).all()
+    if method == "tf32":  # (the split forms make a NaN of an infinite operand's small part)
+        assert np.isposinf(run((np.inf, 1.0), (1.0, 1.0), (-1.0, 2.0))).all()
+        assert np.isnan(run((np.inf, 1.0), (1.0, 1.0), (-np.inf, 1.0))).all()
