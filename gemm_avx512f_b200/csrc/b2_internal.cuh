@@ -109,6 +109,7 @@ struct Fp64Cfg {
   int tile = 0;    // 0: 128x128, 1: 128x64, 2: 64x64, 3: 32x32 (DMMA K 4 only)
   int mmak = 4;    // DMMA K shape: 4, 8 or 16
   int split_k = 1; // >1: K split across CTAs, reduced in FP64 workspace
+  int chain = 0;   // tile 3: K of one chain of additions, a multiple of 16 (0: the slice's)
 };
 int dgemm_fp64(char ta, char tb, int m, int n, int k, double alpha, const double *A, int lda,
                const double *B, int ldb, double beta, double *C, int ldc, cudaStream_t s,

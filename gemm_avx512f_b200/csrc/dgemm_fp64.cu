@@ -23,6 +23,8 @@
 //    slice to arrive adds the partials): the separate reduction is faster on
 //    every shape tried, 14 us against 66 us at 128x128x1024 with 8 slices and
 //    83 us against 118 us at 1024^3 with 4.
+#include <type_traits>
+
 #include "b2_internal.cuh"
 #include "b2_profile.cuh"
 #include "fp64_copy.cuh"
@@ -59,10 +61,18 @@ __device__ __forceinline__ void dmma(double (&c)[4], const double *a, const doub
 // A_KCONT = transA (op(A)(m,k) = A[m*lda+k]); B_KCONT = !transB (op(B)(k,n) = B[n*ldb+k]).
 // Output: when P != nullptr the raw product of this CTA's K range is written to
 // P + z*ldp*N (split-K partial); otherwise C = alpha*acc + beta*C (beta==1: C += alpha*acc).
+// FOLD > 0: the sums of every `fold` blocks of K are chains of their own, added in
+// order.  The chains' sum is held in registers (2, at most four CTAs per SM) or, so that
+// five CTAs of the 32x32 tile fit an SM, in local memory (1: 64 bytes a thread, which
+// stay in L1).  B200: 1024^3 70.4 us in one chain, 72.5 in four with the sum in local
+// memory, 84 with registers bounded to five CTAs; 128x4096x128 in eight chains 9.1 with
+// it in registers, 11 in local memory.
 template <int BM, int BN, int BK, int WM, int WN, int STAGES, int MMAK, bool A_KCONT,
-          bool B_KCONT, bool SH>
-__global__ void __launch_bounds__(WM *WN * 32, BM * BN <= 64 * 64 && MMAK == 4 ? 3 : 1)
-    dgemm_dmma_kernel(int M, int N, int K, int kchunk, double alpha,
+          bool B_KCONT, bool SH, int FOLD>
+__global__ void __launch_bounds__(WM *WN * 32, FOLD == 2                          ? 4
+                                               : BM * BN <= 64 * 64 && MMAK == 4 ? 3
+                                                                                 : 1)
+    dgemm_dmma_kernel(int M, int N, int K, int kchunk, int fold, double alpha,
                       const double *__restrict__ A, int lda, const double *__restrict__ B,
                       int ldb, double beta, double *__restrict__ C, int ldc,
                       double *__restrict__ P, int ldp) {
@@ -212,35 +222,63 @@ __global__ void __launch_bounds__(WM *WN * 32, BM * BN <= 64 * 64 && MMAK == 4 ?
         bf[buf][j][v] = B_KCONT ? Bs[n * (BK + 4) + k] : Bs[k * (BN + 4) + n];
       }
   };
+  using Tot = std::conditional_t<FOLD == 1, volatile double, double>;  // (volatile: local)
+  Tot tot[FOLD ? MT * NTL * 4 : 1];
+  auto end_chain = [&](bool first) {
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+      for (int j = 0; j < NTL; ++j)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          Tot &t = tot[(i * NTL + j) * 4 + v];
+          t = first ? acc[i][j][v] : t + acc[i][j][v];
+          acc[i][j][v] = 0.0;
+        }
+  };
   cp_async_wait<STAGES - 2>();
   __syncthreads();
   if (PIPE) load_frags(0, 0, 0);
   int st = 0, st_fill = STAGES - 1;  // stage being multiplied, stage refilled next
-  for (int kt = 0; kt < KT; ++kt) {
-    const int st_next = st + 1 == STAGES ? 0 : st + 1;
-    // every warp has issued its last reads of stage kt - 1, which is refilled here
-    const bool fill = kt + STAGES - 1 < KT;
+  for (int kt = 0; kt < KT;) {
+    const int chain_end = FOLD ? min(KT, kt + fold) : KT;
+    for (; kt < chain_end; ++kt) {
+      const int st_next = st + 1 == STAGES ? 0 : st + 1;
+      // every warp has issued its last reads of stage kt - 1, which is refilled here
+      const bool fill = kt + STAGES - 1 < KT;
 #pragma unroll
-    for (int ks = 0; ks < KS; ++ks) {
-      const int cur = PIPE ? (ks & 1) : 0;
-      if (!PIPE) load_frags(0, st, ks * MMAK);
-      if (PIPE && ks + 1 < KS) load_frags(cur ^ 1, st, (ks + 1) * MMAK);
-      if (ks == 0 && fill) load_stage(st_fill, kt + STAGES - 1);
-      if (ks + 1 == KS) {
-        cp_async_commit();
-        cp_async_wait<STAGES - 2>();
-        __syncthreads();
-        if (PIPE && kt + 1 < KT) load_frags(cur ^ 1, st_next, 0);
+      for (int ks = 0; ks < KS; ++ks) {
+        const int cur = PIPE ? (ks & 1) : 0;
+        if (!PIPE) load_frags(0, st, ks * MMAK);
+        if (PIPE && ks + 1 < KS) load_frags(cur ^ 1, st, (ks + 1) * MMAK);
+        if (ks == 0 && fill) load_stage(st_fill, kt + STAGES - 1);
+        if (ks + 1 == KS) {
+          cp_async_commit();
+          cp_async_wait<STAGES - 2>();
+          __syncthreads();
+          if (PIPE && kt + 1 < KT) load_frags(cur ^ 1, st_next, 0);
+        }
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+          for (int j = 0; j < NTL; ++j) dmma<MMAK>(acc[i][j], af[cur][i], bf[cur][j]);
       }
+      st = st_next;
+      st_fill = st_fill + 1 == STAGES ? 0 : st_fill + 1;
+    }
+    if (FOLD && kt < KT) end_chain(kt == fold);
+  }
+  cp_async_wait<0>();
+  if constexpr (FOLD) {  // (a slice of one chain has none before it)
+    if (KT > fold) {
 #pragma unroll
       for (int i = 0; i < MT; ++i)
 #pragma unroll
-        for (int j = 0; j < NTL; ++j) dmma<MMAK>(acc[i][j], af[cur][i], bf[cur][j]);
+        for (int j = 0; j < NTL; ++j)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) acc[i][j][v] = tot[(i * NTL + j) * 4 + v] + acc[i][j][v];
     }
-    st = st_next;
-    st_fill = st_fill + 1 == STAGES ? 0 : st_fill + 1;
   }
-  cp_async_wait<0>();
 
   // Epilogue.  Fragment (i, j, v): row g + 8*(v>>1), column 2t + (v&1).
   if (P != nullptr) {
@@ -339,6 +377,8 @@ __global__ void scale_kernel(int M, int N, T beta, T *__restrict__ C, int ldc) {
 
 struct LaunchArgs {
   int M, N, K, kchunk;
+  int fold;  // K blocks of 16 per chain (32x32 tile), 0: one chain
+  bool few;  // at most four CTAs per SM
   double alpha;
   const double *A;
   int lda;
@@ -353,12 +393,12 @@ struct LaunchArgs {
 };
 
 template <int BM, int BN, int BK, int WM, int WN, int STAGES, int MMAK, bool AK, bool BKc,
-          bool SH>
+          bool SH, int FOLD>
 cudaError_t launch_one(const LaunchArgs &a, cudaStream_t s) {
   constexpr int A_ST = AK ? BM * (BK + 4) : BK * (BM + 4);
   constexpr int B_ST = BKc ? BN * (BK + 4) : BK * (BN + 4);
   constexpr size_t SMEM = (size_t)STAGES * (A_ST + B_ST) * sizeof(double);
-  auto kern = dgemm_dmma_kernel<BM, BN, BK, WM, WN, STAGES, MMAK, AK, BKc, SH>;
+  auto kern = dgemm_dmma_kernel<BM, BN, BK, WM, WN, STAGES, MMAK, AK, BKc, SH, FOLD>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)SMEM);
   if (e != cudaSuccess) return e;
@@ -377,20 +417,20 @@ cudaError_t launch_one(const LaunchArgs &a, cudaStream_t s) {
   lc.attrs = attr;
   lc.numAttrs = 1;
   B2_PROF("dgemm_dmma", s);
-  e = cudaLaunchKernelEx(&lc, kern, a.M, a.N, a.K, a.kchunk, a.alpha, a.A, a.lda,
-                                           a.B, a.ldb, a.beta, a.C, a.ldc, a.P, a.ldp);
+  e = cudaLaunchKernelEx(&lc, kern, a.M, a.N, a.K, a.kchunk, a.fold, a.alpha, a.A, a.lda, a.B,
+                         a.ldb, a.beta, a.C, a.ldc, a.P, a.ldp);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-template <int BM, int BN, int WM, int WN, int STAGES, int MMAK, bool SH>
+template <int BM, int BN, int WM, int WN, int STAGES, int MMAK, bool SH, int FOLD = 0>
 cudaError_t launch_layout(bool ak, bool bk, const LaunchArgs &a, cudaStream_t s) {
   // 64x64, both operands K-contiguous: 80 KB in four stages would leave two
   // CTAs per SM; three stages keep three
   constexpr int ST_TN = BM * BN <= 64 * 64 ? 3 : STAGES;
-  if (ak && bk) return launch_one<BM, BN, 16, WM, WN, ST_TN, MMAK, true, true, SH>(a, s);
-  if (ak && !bk) return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, true, false, SH>(a, s);
-  if (!ak && bk) return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, false, true, SH>(a, s);
-  return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, false, false, SH>(a, s);
+  if (ak && bk) return launch_one<BM, BN, 16, WM, WN, ST_TN, MMAK, true, true, SH, FOLD>(a, s);
+  if (ak && !bk) return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, true, false, SH, FOLD>(a, s);
+  if (!ak && bk) return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, false, true, SH, FOLD>(a, s);
+  return launch_one<BM, BN, 16, WM, WN, STAGES, MMAK, false, false, SH, FOLD>(a, s);
 }
 
 template <int MMAK, bool SH>
@@ -399,7 +439,10 @@ cudaError_t launch_tile(int tile, bool ak, bool bk, const LaunchArgs &a, cudaStr
     case 0: return launch_layout<128, 128, 2, 4, 4, MMAK, SH>(ak, bk, a, s);
     case 1: return launch_layout<128, 64, 2, 2, 4, MMAK, SH>(ak, bk, a, s);
     case 3:  // fp64_call_cfg's, DMMA K 4 only
-      if constexpr (MMAK == 4) return launch_layout<32, 32, 2, 2, 4, 4, SH>(ak, bk, a, s);
+      if constexpr (MMAK == 4)
+        return !a.fold  ? launch_layout<32, 32, 2, 2, 4, 4, SH>(ak, bk, a, s)
+               : a.few ? launch_layout<32, 32, 2, 2, 4, 4, SH, 2>(ak, bk, a, s)
+                        : launch_layout<32, 32, 2, 2, 4, 4, SH, 1>(ak, bk, a, s);
       else return cudaErrorInvalidValue;
     default: return launch_layout<64, 64, 2, 2, 4, MMAK, SH>(ak, bk, a, s);
   }
@@ -411,36 +454,48 @@ inline bool is_notrans(char c) { return c == 'N' || c == 'n'; }
 
 namespace {
 
-// Model of the 64x64 tile's time in us over S = 1, 2, 4, 8 slices of K; the best S
-// in *sk.  q = work units (tiles x slices) per SM, each of `kit` K blocks of 16
+// K slices of a product on 64x64 tiles: as many as keep 8 of K each, up to 8, and at
+// most 1024 units (32 MB of partials).  They fill the SMs, and they bound the length
+// of a chain of additions: 512^3 has a relative error of 3.0e-16 in eight chains added
+// up, 7.8e-16 in one.  chain_k is the length that they give, for every form.
+int slices64(int m, int n, int k) {
+  const long long tiles = (long long)((m + 63) / 64) * ((n + 63) / 64);
+  int s = 1;
+  if (tiles < 1024)
+    while (s < 8 && k / (2 * s) >= 8 && tiles * s * 2 <= 1024) s *= 2;
+  return s;
+}
+int slice_k(int k, int slices) { return ((k + slices - 1) / slices + 15) / 16 * 16; }
+int chain_k(int m, int n, int k) {
+  const int s = slices64(m, n, k);
+  return s > 1 ? slice_k(k, s) : k;
+}
+
+// Model of the 64x64 tile's time in us in its K slices.
+// q = work units (tiles x slices) per SM, each of `kit` K blocks of 16
 // that take the FP64 pipe 0.53 us; a lone CTA per SM reaches 74 % of that rate,
 // up to four 91 %, more 95 %; 3 us to fill and drain, 1 us per further wave of
 // three; rows off a 16-byte boundary cost 9 % (shared-memory conflicts).  A
-// split adds a second launch (split_us; 1.5 us on the device and 2 on the host,
-// which bounds a run of small calls: 128x128x128 8.2 us a call in two launches, 6.0
+// split adds a second launch (1.5 us on the device and 2 on the host, which bounds
+// a run of small calls: 128x128x128 8.2 us a call in two launches, 6.0
 // in one) and 64 KB of partials per unit, written and read at about 8 TB/s
 // (they stay in L2).  Measured (B200, us, graph replays):
 //   128x4096x128   S=1 9.2  2 12.4  4 13.0  8 16.2     512^3  26.4 17.1 15.7 17.6
 //   512x1024x512   26.6 26.6 27.3 27.3     2048^3  504 541 551 588
-// (one fixed rule, 8 slices up to 1024 units, took the last column of the
-// first three).
-double model64(int m, int n, int k, int sms, bool shifted, double split_us, int *sk) {
-  const long long tiles = (long long)((m + 63) / 64) * ((n + 63) / 64);
-  double best = 1e300;
-  for (int s = 1; s <= 8; s *= 2) {
-    if (s > 1 && (k < 8 * s || tiles * s > 1024)) break;  // at most 32 MB of partials
-    const long long units = tiles * s, q = (units + sms - 1) / sms;
-    const int kit = ((k + s - 1) / s + 15) / 16;
-    const double rate = q == 1 ? 0.74 : q <= 4 ? 0.91 : 0.95;
-    double us = (double)q * kit * 0.53 / rate * (shifted ? 1.09 : 1.0) + 3.0 +
-                (double)((q + 2) / 3 - 1);
-    if (s > 1) us += split_us + (double)units * 65536.0 / 8e6;
-    if (us < best) best = us, *sk = s;
-  }
-  return best;
+double model64(int m, int n, int k, int sms, bool shifted) {
+  const int s = slices64(m, n, k);
+  const long long units = (long long)((m + 63) / 64) * ((n + 63) / 64) * s;
+  const long long q = (units + sms - 1) / sms;
+  const int kit = ((k + s - 1) / s + 15) / 16;
+  const double rate = q == 1 ? 0.74 : q <= 4 ? 0.91 : 0.95;
+  double us = (double)q * kit * 0.53 / rate * (shifted ? 1.09 : 1.0) + 3.0 +
+              (double)((q + 2) / 3 - 1);
+  if (s > 1) us += 3.5 + (double)units * 65536.0 / 8e6;
+  return us;
 }
 
-// The same for the 32x32 tile: up to five CTAs per SM, 0.24 us per K block for
+// The same for the 32x32 tile, S = 1, 2, 4, 8 and the best S in *sk: up to five CTAs
+// per SM, 0.24 us per K block for
 // one CTA alone on an SM, 0.33 for two, 0.148 each from three on (0.139 a
 // quarter of a 64x64 tile), 0.8 us per further wave of five, 16 KB of partials
 // per unit; 5 % for tiles past an edge, 20 % for shifted rows (40 % for a lone
@@ -449,7 +504,7 @@ double model32(int m, int n, int k, int sms, bool shifted, int *sk) {
   const long long tm = (m + 31) / 32, tn = (n + 31) / 32;
   double best = 1e300;
   for (int s = 1; s <= 8 && tn <= 65535; s *= 2) {
-    if (s > 1 && (k < 8 * s || ((tm + 1) / 2) * ((tn + 1) / 2) * s > 1024)) break;  // as model64
+    if (s > 1 && (k < 8 * s || ((tm + 1) / 2) * ((tn + 1) / 2) * s > 1024)) break;  // as slices64
     const long long units = tm * tn * s, qc = (units + sms - 1) / sms;
     const double q = qc <= 6 ? (double)qc : (double)units / sms;
     const int kit = ((k + s - 1) / s + 15) / 16;
@@ -467,32 +522,33 @@ double model32(int m, int n, int k, int sms, bool shifted, int *sk) {
 
 // The 64x64 tile (three CTAs per SM) is the best of the three tiles of the
 // tuner's list from 1024^3 to 8192^3 and in the exhaustive sweep over M, N, K in
-// [16, 1024]; K in the slices that its model likes best on the device (2 us a
-// second launch: the tuner's configurations are compared by their device time).
+// [16, 1024].
 Fp64Cfg fp64_default_cfg(int m, int n, int k, int sm_count) {
+  (void)sm_count;
   Fp64Cfg c;
   c.tile = 2;
   c.mmak = 4;
-  model64(m, n, k, sm_count > 0 ? sm_count : 148, false, 2.0, &c.split_k);
+  c.split_k = slices64(m, n, k);
   return c;
 }
 
 // A call's own choice (no configuration asked for): the 32x32 tile where the
 // models find it faster.  Four times the tiles fill the SMs where 64x64 ones
-// leave them one chain of K blocks or an uneven last wave; from about 2048^3 on
-// its extra shared reads lose.  B200, us, the better S of each, 64x64 / 32x32:
-//   48x40x64 3.8 / 2.8     256^3 5.9 / 5.1        424x39x1600 16.0 / 10.3
-//   512^3 15.7 / 12.8      900^3 65.3 / 58.3      1024^3 76.3 / 70.8
-//   1536x1024x2048 217 / 211    2048^3 504 / 525  4096^3 3896 / 4083
+// leave them one chain of K blocks or an uneven last wave, in fewer slices, whose
+// chains it adds up itself (64x64 has no registers for that); from about 2048^3 on
+// its extra shared reads lose.  B200, us, 64x64 / 32x32 in the better S of each:
+//   48x40x64 3.7 / 3.0     128x4096x128 15.9 / 9.1    424x39x1600 15.0 / 8.8
+//   512^3 17.1 / 13.3      900^3 65.9 / 59.1          1024^3 75.9 / 72.5
+//   1536x1024x2048 231 / 212    2048^3 504 / 525      4096^3 3896 / 4083
 static Fp64Cfg fp64_call_cfg(int m, int n, int k, int sm_count, bool shifted) {
   const int sms = sm_count > 0 ? sm_count : 148;
   Fp64Cfg c;
   c.mmak = 4;
-  int s64 = 1, s32 = 1;
-  const bool small = model32(m, n, k, sms, shifted, &s32) <
-                     model64(m, n, k, sms, shifted, 3.5, &s64);
+  int s32 = 1;
+  const bool small = model32(m, n, k, sms, shifted, &s32) < model64(m, n, k, sms, shifted);
   c.tile = small ? 3 : 2;
-  c.split_k = small ? s32 : s64;
+  c.split_k = small ? s32 : slices64(m, n, k);
+  c.chain = small ? chain_k(m, n, k) : 0;
   return c;
 }
 
@@ -535,11 +591,10 @@ int dgemm_fp64(char ta, char tb, int m, int n, int k, double alpha, const double
   Fp64Cfg cfg = cfg_in            ? *cfg_in
                 : cx->fp64_override ? fp64_override_cfg()
                                     : fp64_call_cfg(m, n, k, cx->sm_count, !vec2);
-  LaunchArgs a{m, n, k, k, alpha, A, lda, B, ldb, beta, C, ldc, nullptr, 0, 1};
+  LaunchArgs a{m, n, k, k, 0, false, alpha, A, lda, B, ldb, beta, C, ldc, nullptr, 0, 1};
   int splits = cfg.split_k < 1 ? 1 : cfg.split_k;
   if (splits > 1) {
-    int chunk = (k + splits - 1) / splits;
-    chunk = (chunk + 15) / 16 * 16;
+    const int chunk = slice_k(k, splits);
     splits = (k + chunk - 1) / chunk;
     a.kchunk = chunk;
     a.splits = splits;
@@ -553,6 +608,10 @@ int dgemm_fp64(char ta, char tb, int m, int n, int k, double alpha, const double
     } else {
       a.kchunk = k;
     }
+  }
+  if (cfg.chain > 0 && cfg.chain < a.kchunk) {
+    a.fold = cfg.chain / 16;
+    a.few = (long long)((m + 31) / 32) * ((n + 31) / 32) * a.splits <= 4ll * cx->sm_count;
   }
   cudaError_t e;
   const int mk = cfg.mmak;
