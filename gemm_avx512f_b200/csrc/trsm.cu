@@ -35,7 +35,8 @@ constexpr int TI_PLD = TB + 4; // stride of the copied columns (conflict-free DM
 
 // Invert every diagonal block T_b = T[kb:kb+bs, kb:kb+bs] (lower or upper, unit
 // or not); block b goes to Tinv + b*TB*TB (column-major, ld TB, zero outside the
-// triangle and beyond bs).  An upper block is inverted as the lower one it is
+// triangle and beyond bs, and on the diagonal, whose inverse goes to dinv + b*TB).
+// An upper block is inverted as the lower one it is
 // with both indices reversed.  Substitution against the identity in shared
 // memory, in place, 16 columns of T at a time (copied aside as [k][row]): the 16
 // rows of their diagonal block are solved, one thread per column, and taken off
@@ -54,7 +55,7 @@ __device__ __forceinline__ double &tel(double *T, int i, int j) { return T[j * T
 
 __global__ void __launch_bounds__(TI_NT)
     trtri_batched_kernel(const double *__restrict__ A, long long rs, long long cs, int n, int lower,
-                         int unit, double *__restrict__ Tinv) {
+                         int unit, double *__restrict__ Tinv, double *__restrict__ dinv) {
   extern __shared__ __align__(16) double tsm[];
   double *T = tsm;                      // T(i, j) at [j*TB_LD + i], then sums, then the inverse
   double *pan = tsm + TB * TB_LD;       // 16 columns of T, [k][row], this step's and the next's
@@ -181,10 +182,11 @@ __global__ void __launch_bounds__(TI_NT)
     double v = 0.0;
     if (i < bs && j < bs) {
       const int li = lower ? i : bs - 1 - i, lj = lower ? j : bs - 1 - j;
-      if (li >= lj) v = tel(T, li, lj);
+      if (li > lj) v = tel(T, li, lj);
     }
     out[idx] = v;
   }
+  if (tid < TB) dinv[blockIdx.x * TB + tid] = tid < bs ? inv[lower ? tid : bs - 1 - tid] : 0.0;
 }
 
 // ------------------------------------------------------------------ leaf --
@@ -199,10 +201,11 @@ __global__ void __launch_bounds__(TI_NT)
 // -- so that either orientation of T is copied and read 16 bytes at a time, and
 // Z two rows at a time.
 // Bound: L2 -> SM (128 KB of T per step, 64 bytes per clock: 1.07 us) and, wider
-// than 8, the FP64 pipe; reached: 24, 37 and 70 us for 512 rows at 8, 16 and 32
-// (B200).  Each 128-row block as its own memset, GEMM, reduction and copy, with
-// the updates between them as further launches, took 68 us for 512 rows and 1024
-// right-hand sides, 24 now; dtrsm 4096 x 1024 1747 -> 796 us in all.
+// than 8, the FP64 pipe; reached: 25, 41 and 76 us for 512 rows at 8, 16 and 32
+// (B200; 24, 37 and 70 with one chain of additions through a step).  Each 128-row block
+// as its own memset, GEMM, reduction and copy, with the updates between them as further
+// launches, took 68 us for 512 rows and 1024 right-hand sides; dtrsm 4096 x 1024
+// 1374 -> 755 us in all.
 constexpr int LEAF_BLOCKS = 4;  // 512 rows
 constexpr int LEAF_COLS = 32;   // columns of T per ring stage
 template <int W>
@@ -225,8 +228,8 @@ __device__ __forceinline__ int leaf_at(int row, int col) {
 template <int W, bool ROWS>
 __global__ void __launch_bounds__(256, 1)
     trsm_leaf_kernel(const double *__restrict__ A, long long rs, long long cs, int forward, int nr,
-                     const double *__restrict__ Tinv, double *__restrict__ B, long long si,
-                     long long sr, int nrhs) {
+                     const double *__restrict__ Tinv, const double *__restrict__ dinv,
+                     double *__restrict__ B, long long si, long long sr, int nrhs) {
   using L = LeafSmem<W>;
   constexpr int P = L::P, STAGES = L::STAGES, NT = W / 8;
   extern __shared__ __align__(16) double Z[];
@@ -300,21 +303,39 @@ __global__ void __launch_bounds__(256, 1)
     Z[r * P + i] = (i < nr && r0 + r < nrhs) ? B[i * si + (r0 + r) * sr] : 0.0;
   }
   // A DMMA waits for the one before it on the same accumulator: four
-  // independent chains (K steps dealt out in turn), added at a step's end.
+  // independent chains (K steps dealt out in turn).  Every 16 k a chain goes to the
+  // sum: the error of a product of 128 is 3.6 u, not the 8 u of one chain (the slices of
+  // a GEMM of that size are no longer either).
   constexpr int SETS = NT >= 4 ? 1 : 4 / NT;
-  double acc[SETS][NT][4];
+  double acc[SETS][NT][4], sum[NT][4];
+  auto end_chains = [&]() {
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        double x = acc[0][n][v];
+#pragma unroll
+        for (int c = 1; c < SETS; ++c) x += acc[c][n][v];
+        sum[n][v] += x;
+#pragma unroll
+        for (int c = 0; c < SETS; ++c) acc[c][n][v] = 0.0;
+      }
+  };
   // Element (n, v) of a warp's fragment: row wm + 2g + (v >> 1), rhs 8n + 2t + (v & 1)
   __syncthreads();
   int slot = 0;
   for (int kq = 0; kq < nb; ++kq) {
     const int k = forward ? kq : nb - 1 - kq;
 #pragma unroll
-    for (int c = 0; c < SETS; ++c)
+    for (int n = 0; n < NT; ++n)
 #pragma unroll
-      for (int n = 0; n < NT; ++n)
+      for (int v = 0; v < 4; ++v) {
+        sum[n][v] = 0.0;
 #pragma unroll
-        for (int v = 0; v < 4; ++v) acc[c][n][v] = 0.0;
+        for (int c = 0; c < SETS; ++c) acc[c][n][v] = 0.0;
+      }
     double *zk = Z + k * TB + wm + 2 * g;
+    const double d[2] = {dinv[k * TB + wm + 2 * g], dinv[k * TB + wm + 2 * g + 1]};
     for (int jq = 0; jq <= kq; ++jq) {
       const bool diag = jq == kq;
       if (diag && kq > 0) {  // all updates of block k are in: Z_k -= their sum
@@ -322,12 +343,8 @@ __global__ void __launch_bounds__(256, 1)
         for (int n = 0; n < NT; ++n)
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
-            double x = acc[0][n][v];
-#pragma unroll
-            for (int c = 1; c < SETS; ++c) x += acc[c][n][v];
-            zk[(8 * n + 2 * t + (v & 1)) * P + (v >> 1)] -= x;
-#pragma unroll
-            for (int c = 0; c < SETS; ++c) acc[c][n][v] = 0.0;
+            zk[(8 * n + 2 * t + (v & 1)) * P + (v >> 1)] -= sum[n][v];
+            sum[n][v] = 0.0;
           }
         __syncthreads();
       }
@@ -365,24 +382,38 @@ __global__ void __launch_bounds__(256, 1)
                     : "d"(e ? a01 : a00), "d"(e ? a11 : a10), "d"(e ? b.y : b.x));
               }
             }
+            // 8 k a step of s, over SETS chains
+            if (SETS == 1 && (s & 1)) end_chains();
           }
+          if (SETS == 2 || (SETS == 4 && (h & 1))) end_chains();
           if (++slot == STAGES) slot = 0;
         }
       };
       if (ROWS && !diag) mac_block(Yes{});
       else mac_block(No{});
     }
-    // X_k = inv(T_kk) Z_k replaces Z_k once every warp has read it
-    __syncthreads();
+    // X_k = inv(T_kk) Z_k replaces Z_k once every warp has read it.  The diagonal's
+    // term, which may dwarf the others, is added last: one rounding of its size.
 #pragma unroll
     for (int n = 0; n < NT; ++n)
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
-        double x = acc[0][n][v];
-#pragma unroll
-        for (int c = 1; c < SETS; ++c) x += acc[c][n][v];
-        zk[(8 * n + 2 * t + (v & 1)) * P + (v >> 1)] = x;
+        const int r = 8 * n + 2 * t + (v & 1), i = wm + 2 * g + (v >> 1);
+        const double z = zk[r * P + (v >> 1)];
+        double x = fma(d[v >> 1], z, sum[n][v]);
+        if (!isfinite(z)) {  // the zero that stands for the diagonal made a NaN of it
+          const double *ti = Tinv + (long long)k * TB * TB + i, *zr = Z + r * P + k * TB;
+          x = d[v >> 1] * z;
+          for (int j = 0; j < TB; ++j)
+            if (j != i) x = fma(ti[j * TB], zr[j], x);
+        }
+        sum[n][v] = x;
       }
+    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) zk[(8 * n + 2 * t + (v & 1)) * P + (v >> 1)] = sum[n][v];
     __syncthreads();
   }
   asm volatile("cp.async.wait_group 0;\n" ::);
@@ -409,7 +440,8 @@ struct TrsmPlan {
   int method;
   int leaf;
   cudaStream_t s;
-  double *tinv;            // inverted diagonal blocks of T, TB x TB each
+  double *tinv;            // inverted diagonal blocks of T, TB x TB each, zero diagonal
+  double *dinv;            // their diagonals
   bool forward;            // T is lower: blocks are solved in ascending order
   long long rs, cs;        // T(i, j) = A[i*rs + j*cs]
 };
@@ -433,7 +465,7 @@ int launch_leaf(const TrsmPlan &p, int k0, int nr) {
   B2_PROF("trsm_leaf", p.s);
   kern<<<(nrhs + W - 1) / W, 256, smem, p.s>>>(
       p.A + (long long)k0 * (p.rs + p.cs), p.rs, p.cs, p.forward ? 1 : 0, nr,
-      p.tinv + (long long)(k0 / TB) * TB * TB, p.B + (p.left ? k0 : (long long)k0 * p.ldb),
+      p.tinv + (long long)(k0 / TB) * TB * TB, p.dinv + k0, p.B + (p.left ? k0 : (long long)k0 * p.ldb),
       p.left ? 1 : p.ldb, p.left ? p.ldb : 1, nrhs);
   B2_CUDA_TRY(cudaGetLastError());
   return B2_OK;
@@ -538,15 +570,16 @@ int dtrsm_device(char side, char uplo, char transa, char diag, int m, int n, dou
   p.cs = (p.left != p.trans) ? lda : 1;
   const int na = p.left ? m : n;
   const int nblk = (na + TB - 1) / TB;
-  p.tinv = (double *)workspace(cx, WS_TRSM_INV, (size_t)nblk * TB * TB * sizeof(double));
+  p.tinv = (double *)workspace(cx, WS_TRSM_INV, (size_t)nblk * TB * (TB + 1) * sizeof(double));
   if (!p.tinv) return B2_ERR_NOMEM;
+  p.dinv = p.tinv + (size_t)nblk * TB * TB;
   {
     const int smem = (TB * TB_LD + 2 * TI_K * TI_PLD + TB) * (int)sizeof(double);
     B2_CUDA_TRY(cudaFuncSetAttribute(trtri_batched_kernel,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     B2_PROF("trsm_trtri", s);
     trtri_batched_kernel<<<nblk, TI_NT, smem, s>>>(A, p.rs, p.cs, na, p.forward ? 1 : 0,
-                                                   p.unit ? 1 : 0, p.tinv);
+                                                   p.unit ? 1 : 0, p.tinv, p.dinv);
     B2_CUDA_TRY(cudaGetLastError());
   }
   return solve_range(p, 0, na);

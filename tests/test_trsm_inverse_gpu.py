@@ -97,3 +97,33 @@ def test_non_finite_elements_stay_in_their_rows(cuda, side, lower, trans, i, j, 
     assert not np.isfinite(got[hit]).any()
     if bad == np.inf and j == 0:  # one element of that row of the inverse is infinite
         assert np.isinf(got[hit]).all()
+
+
+@pytest.mark.parametrize("row", [0, 40, 127, 200])
+@pytest.mark.parametrize("nrhs", [9, 2500])
+def test_infinite_right_hand_side(cuda, row, nrhs):
+    """An infinity in B stays one in its own row of X, and in its own column."""
+    import torch
+
+    n = 256
+    rng = np.random.default_rng(row)
+    T = np.tril(rng.uniform(0.1, 1, (n, n)))
+    T[np.arange(n), np.arange(n)] += n
+    b = rng.uniform(0.1, 1, (n, nrhs))
+
+    def solve(rhs):
+        a = torch.from_numpy(np.ascontiguousarray(T.T)).to(cuda)
+        x = torch.from_numpy(np.ascontiguousarray(rhs.T)).to(cuda)
+        torch.cuda.synchronize()
+        blas.dtrsm_device("L", "L", "N", "N", n, nrhs, 1.0, a, n, x, n)
+        torch.cuda.synchronize()
+        return x.cpu().numpy().T
+
+    clean = solve(b)
+    for bad in (np.inf, -np.inf, np.nan):
+        rhs = b.copy()
+        rhs[row, 3] = bad
+        got = solve(rhs)
+        assert np.array_equal(got[row, 3], bad, equal_nan=True)
+        others = np.arange(nrhs) != 3
+        assert np.array_equal(got[:, others], clean[:, others])
