@@ -31,7 +31,7 @@ enum WsSlot {
   WS_STAGE_A = 0, WS_STAGE_B, WS_STAGE_C,   // host-pointer staging
   WS_OZ_X, WS_OZ_Y, WS_OZ_R, WS_OZ_SCALE,   // Ozaki slices / residues / exponents
   WS_SPLIT_X, WS_SPLIT_Y,                   // SGEMM split planes
-  WS_TRSM, WS_TRSM_INV, WS_3M, WS_GROUP, WS_ERR, WS_MISC,
+  WS_TRSM, WS_TRSM_INV, WS_TRSM_TMP, WS_3M, WS_GROUP, WS_ERR, WS_MISC,
   WS_KABI_A, WS_KABI_B, WS_KABI_D,         // kernel-ABI unpacked panels / 3M product
   WS_GROUP2,                                // second descriptor slot of one-shot grouped calls
   WS_F32,                                   // FP32 products' K slices, never used by captured calls

@@ -35,7 +35,8 @@ constexpr int TI_PLD = TB + 4; // stride of the copied columns (conflict-free DM
 
 // Invert every diagonal block T_b = T[kb:kb+bs, kb:kb+bs] (lower or upper, unit
 // or not); block b goes to Tinv + b*TB*TB (column-major, ld TB, zero outside the
-// triangle and beyond bs, and on the diagonal, whose inverse goes to dinv + b*TB).
+// triangle and beyond bs, and on the diagonal, whose inverse goes to dinv + b*TB; a
+// block of order up to keep_diag keeps it).
 // An upper block is inverted as the lower one it is
 // with both indices reversed.  Substitution against the identity in shared
 // memory, in place, 16 columns of T at a time (copied aside as [k][row]): the 16
@@ -55,7 +56,8 @@ __device__ __forceinline__ double &tel(double *T, int i, int j) { return T[j * T
 
 __global__ void __launch_bounds__(TI_NT)
     trtri_batched_kernel(const double *__restrict__ A, long long rs, long long cs, int n, int lower,
-                         int unit, double *__restrict__ Tinv, double *__restrict__ dinv) {
+                         int unit, int keep_diag, double *__restrict__ Tinv,
+                         double *__restrict__ dinv) {
   extern __shared__ __align__(16) double tsm[];
   double *T = tsm;                      // T(i, j) at [j*TB_LD + i], then sums, then the inverse
   double *pan = tsm + TB * TB_LD;       // 16 columns of T, [k][row], this step's and the next's
@@ -182,7 +184,7 @@ __global__ void __launch_bounds__(TI_NT)
     double v = 0.0;
     if (i < bs && j < bs) {
       const int li = lower ? i : bs - 1 - i, lj = lower ? j : bs - 1 - j;
-      if (li > lj) v = tel(T, li, lj);
+      if (li > lj || (li == lj && bs <= keep_diag)) v = tel(T, li, lj);
     }
     out[idx] = v;
   }
@@ -442,6 +444,8 @@ struct TrsmPlan {
   cudaStream_t s;
   double *tinv;            // inverted diagonal blocks of T, TB x TB each, zero diagonal
   double *dinv;            // their diagonals
+  double *tmp;             // small_solve's product
+  int sm_count;
   bool forward;            // T is lower: blocks are solved in ascending order
   long long rs, cs;        // T(i, j) = A[i*rs + j*cs]
 };
@@ -471,12 +475,39 @@ int launch_leaf(const TrsmPlan &p, int k0, int nr) {
   return B2_OK;
 }
 
+// A triangle of order up to SMALL against so many right-hand sides that the leaf kernel
+// would take its widest strips: the inverse times all of them as one GEMM, copied back.
+// A leaf takes a step of 128 rows whatever the order, one CTA per SM.  B200, us, whole
+// solves, leaf / GEMM: order 16 by 1000 12.0 / 11.4, by 4096 18.3 / 13.0, by 100000
+// 229 / 39; order 64 by 4096 25.3 / 22.1, by 100000 235 / 86; order 96 by 8192 41.7 /
+// 41.7.
+constexpr int SMALL = 64;
+bool small_many(int nr, int nrhs, int sms) { return nr <= SMALL && nrhs > 16 * sms; }
+
+int small_solve(const TrsmPlan &p, int k0, int nr) {
+  const double *Ti = p.tinv + (long long)(k0 / TB) * TB * TB;
+  const int rows = p.left ? nr : p.m, cols = p.left ? p.n : nr;
+  double *Bk = p.B + (p.left ? k0 : (long long)k0 * p.ldb);
+  // (beta = 0 multiplies what the product's place holds)
+  B2_CUDA_TRY(cudaMemsetAsync(p.tmp, 0, (size_t)rows * cols * sizeof(double), p.s));
+  const int rc = p.left ? dgemm_device('N', 'N', nr, p.n, nr, 1.0, Ti, TB, Bk, p.ldb, 0.0, p.tmp,
+                                       nr, B2_METHOD_FP64, 0, p.s)
+                        : dgemm_device('N', 'T', p.m, nr, nr, 1.0, Bk, p.ldb, Ti,
+                                       TB, 0.0, p.tmp, p.m, B2_METHOD_FP64, 0, p.s);
+  if (rc != B2_OK) return rc;
+  B2_CUDA_TRY(cudaMemcpy2DAsync(Bk, (size_t)p.ldb * sizeof(double), p.tmp,
+                                (size_t)rows * sizeof(double), (size_t)rows * sizeof(double), cols,
+                                cudaMemcpyDeviceToDevice, p.s));
+  return B2_OK;
+}
+
 // Strips of 8, 16 or 32 right-hand sides: the narrowest that one wave of CTAs
 // (one per SM) can take; wider ones lengthen every step (leaf times above).
 int leaf_solve(const TrsmPlan &p, int k0, int nr) {
   const int nrhs = p.left ? p.n : p.m;
-  if (nrhs <= 8 * 148) return launch_leaf<8>(p, k0, nr);
-  if (nrhs <= 16 * 148) return launch_leaf<16>(p, k0, nr);
+  if (nr <= SMALL && p.tmp) return small_solve(p, k0, nr);
+  if (nrhs <= 8 * p.sm_count) return launch_leaf<8>(p, k0, nr);
+  if (nrhs <= 16 * p.sm_count) return launch_leaf<16>(p, k0, nr);
   return launch_leaf<32>(p, k0, nr);
 }
 
@@ -573,13 +604,20 @@ int dtrsm_device(char side, char uplo, char transa, char diag, int m, int n, dou
   p.tinv = (double *)workspace(cx, WS_TRSM_INV, (size_t)nblk * TB * (TB + 1) * sizeof(double));
   if (!p.tinv) return B2_ERR_NOMEM;
   p.dinv = p.tinv + (size_t)nblk * TB * TB;
+  p.sm_count = cx->sm_count;
+  // the last leaf may be a small triangle against many right-hand sides
+  const int last = (na - 1) % p.leaf + 1, nrhs = p.left ? n : m;
+  p.tmp = small_many(last, nrhs, cx->sm_count)
+              ? (double *)workspace(cx, WS_TRSM_TMP, (size_t)last * nrhs * sizeof(double))
+              : nullptr;  // (no scratch: the leaf kernel)
   {
     const int smem = (TB * TB_LD + 2 * TI_K * TI_PLD + TB) * (int)sizeof(double);
     B2_CUDA_TRY(cudaFuncSetAttribute(trtri_batched_kernel,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     B2_PROF("trsm_trtri", s);
     trtri_batched_kernel<<<nblk, TI_NT, smem, s>>>(A, p.rs, p.cs, na, p.forward ? 1 : 0,
-                                                   p.unit ? 1 : 0, p.tinv, p.dinv);
+                                                   p.unit ? 1 : 0, p.tmp ? SMALL : 0, p.tinv,
+                                                   p.dinv);
     B2_CUDA_TRY(cudaGetLastError());
   }
   return solve_range(p, 0, na);
