@@ -374,27 +374,33 @@ void stream_fence() {
 }
 
 // rows x width bytes from src (pitch spitch) to dst (pitch dpitch), split over
-// the pool when large.  to_bounce: dst is a bounce buffer (a DMA reads it next);
-// else src is one, and its lines are evicted once read, so that the DMA that
-// writes it next does not find them in a core's cache.
+// the pool when large, rows too: an operand with long columns has one in a chunk
+// (10^6 x 8 x 8 doubles in whole rows, one thread a chunk: 20.3 ms, 4.9 so).
+// to_bounce: dst is a bounce buffer (a DMA reads it next); else src is one, and its
+// lines are evicted once read, so that the DMA that writes it next does not find them
+// in a core's cache.
 void parallel_copy2d(void *dst, size_t dpitch, const void *src, size_t spitch, size_t width,
                      size_t rows, bool to_bounce) {
   const size_t total = width * rows;
   const bool evict = !to_bounce && host_has_clflushopt();
   size_t tasks = total / (128u << 10);  // a task of 128 KB takes about 10 us
   tasks = tasks < 1 ? 1 : tasks > 16 ? 16 : tasks;
-  if (tasks > rows) tasks = rows ? rows : 1;
   auto body = [&](int t) {
-    const size_t r0 = rows * t / tasks, r1 = rows * (t + 1) / tasks;
-    for (size_t r = r0; r < r1; ++r) {
-      char *d = (char *)dst + r * dpitch;
-      const char *q = (const char *)src + r * spitch;
+    // whole cache lines of the bounce buffer, where the rows follow each other
+    size_t at = total * t / tasks & ~(size_t)63;
+    const size_t end = (size_t)t + 1 == tasks ? total : total * (t + 1) / tasks & ~(size_t)63;
+    while (at < end) {
+      const size_t r = at / width, c = at - r * width;
+      const size_t n = width - c < end - at ? width - c : end - at;
+      char *d = (char *)dst + r * dpitch + c;
+      const char *q = (const char *)src + r * spitch + c;
       if (to_bounce) {
-        stream_copy(d, q, width);
+        stream_copy(d, q, n);
       } else {
-        memcpy(d, q, width);
-        if (evict) host_evict_lines(q, width);
+        memcpy(d, q, n);
+        if (evict) host_evict_lines(q, n);
       }
+      at += n;
     }
     if (to_bounce) stream_fence();
   };
