@@ -477,12 +477,13 @@ struct Split3Op {
 
 // Writes the real part, the imaginary part and their sum of every row of both
 // operands as [big | small] TF32 segments: out[t][r][2*kp], t = 0, 1, 2 (the
-// operands of P1, P2, P3).  One block turns 64 rows x 32 k around.
+// operands of P1, P2, P3), or only part t = `only` (>= 0), to out[0].  One block
+// turns 64 rows x 32 k around.
 // Bound: HBM, 8 bytes read and 24 written per element.  The pre-adds and the
 // splits were passes of their own (20 + 36 bytes per element): 110 -> 31 us at
 // 1900x1300x2100 on B200, the whole product 367 -> 199.
 __global__ void __launch_bounds__(256)
-    split3m_kernel(const Split3Op a, const Split3Op b, unsigned blocks_a, int K, int kp) {
+    split3m_kernel(const Split3Op a, const Split3Op b, unsigned blocks_a, int K, int kp, int only) {
   __shared__ float tr[64][33], ti[64][33];
   umma::grid_dependency_wait();
   const bool second = blockIdx.x >= blocks_a;
@@ -527,6 +528,8 @@ __global__ void __launch_bounds__(256)
     float *dst = out + (long long)r * 2 * kp + k0 + kl;
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
+      if (only >= 0 && t != only) continue;
+      float *to = dst + (only >= 0 ? 0 : t) * plane;
       float big[4], small[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -535,9 +538,8 @@ __global__ void __launch_bounds__(256)
         big[j] = tf32_round(x);
         small[j] = tf32_round(x - big[j]);
       }
-      *reinterpret_cast<float4 *>(dst + t * plane) = make_float4(big[0], big[1], big[2], big[3]);
-      *reinterpret_cast<float4 *>(dst + t * plane + kp) =
-          make_float4(small[0], small[1], small[2], small[3]);
+      *reinterpret_cast<float4 *>(to) = make_float4(big[0], big[1], big[2], big[3]);
+      *reinterpret_cast<float4 *>(to + kp) = make_float4(small[0], small[1], small[2], small[3]);
     }
   }
 }
@@ -603,43 +605,55 @@ int cgemm3m_tensor(char ta, char tb, int m, int n, int k, float ar, float ai, fl
   // engine and K ranges as for one 3xTF32 SGEMM of this shape
   const SgCfg cfg = sgemm_pick_cfg('N', 'N', m, n, k, 1, B2_METHOD_TF32X3);
   const int seg_kb = kp * 4 / umma::KBLOCK_BYTES;
-  const Ranges rg = choose_ranges((cfg.engine >= 0 && cfg.engine <= 2) ? cfg.engine : 0, cfg.split,
-                                  3, seg_kb, m, n, 3, cx->sm_count);
-  const int E = rg.E;
+  Ranges rg = choose_ranges((cfg.engine >= 0 && cfg.engine <= 2) ? cfg.engine : 0, cfg.split, 3,
+                            seg_kb, m, n, 3, cx->sm_count);
   const int ldw = (int)round_up(m, 32);
   const long long plane = (long long)n * ldw;
-  // the split segments of both operands, then the products' sums
-  float *Xp = (float *)workspace(
-      cx, WS_3M, (size_t)(3 * (m + (long long)n) * ks) * sizeof(float) +
-                     (size_t)(plane * 3 * E) * rg.bytes());
+  // The split segments of both operands, then the products' sums.  Where there is no
+  // room for those of all three products, one after another: a set of segments that
+  // they share, and one plane each.
+  auto scratch = [&](int sets) {
+    const size_t seg = (size_t)((m + (long long)n) * ks) * sizeof(float);
+    return (float *)workspace(cx, WS_3M, sets * seg + (size_t)(plane * 3 * rg.E) * rg.bytes());
+  };
+  bool batch = true;
+  float *Xp = scratch(3);
+  if (!Xp) {
+    batch = false;
+    if (rg.E > 1) rg = Ranges{1, 1, 3 * seg_kb, rg.range_tb, false};
+    Xp = scratch(1);
+  }
   if (!Xp) return B2_ERR_NOMEM;
-  float *Yp = Xp + 3 * m * ks;
-  void *W = Yp + 3 * n * ks;
-  {
+  const int sets = batch ? 3 : 1, E = rg.E;
+  float *Yp = Xp + sets * m * ks, *W = Yp + sets * n * ks;
+  CUtensorMap tmX, tmY;
+  int rc = umma::make_kmajor_map(&tmX, umma::KIND_TF32, Xp, ks, m, sets, ks * 4,
+                                 (long long)m * ks * 4, umma::BM);
+  if (rc == B2_OK)
+    rc = umma::make_kmajor_map(&tmY, umma::KIND_TF32, Yp, ks, n, sets, ks * 4,
+                               (long long)n * ks * 4, y_box(rg.eng));
+  for (int t = 0; t < 3 && rc == B2_OK; t += sets) {
     const unsigned kt = (unsigned)kp / 32;
     const unsigned ba = kt * ((unsigned)(m + 63) / 64), bb = kt * ((unsigned)(n + 63) / 64);
-    B2_PROF("gemm3m_prep", s);
-    B2_CUDA_TRY(launch_dependent(split3m_kernel, ba + bb, 256, s, split3_op(A, lda, !tA, cA, m, Xp),
-                                 split3_op(B, ldb, tB, cB, n, Yp), ba, k, kp));
+    {
+      B2_PROF("gemm3m_prep", s);
+      B2_CUDA_TRY(launch_dependent(split3m_kernel, ba + bb, 256, s,
+                                   split3_op(A, lda, !tA, cA, m, Xp),
+                                   split3_op(B, ldb, tB, cB, n, Yp), ba, k, kp, batch ? -1 : t));
+    }
+    rc = run_engine(false, 3, tmX, tmY, m, n, kp, sets, seg_kb, rg,
+                    PartialEpi{W + t * plane, plane, ldw, m, n, rg.pairs}, cx, s);
   }
-  CUtensorMap tmX, tmY;
-  int rc = umma::make_kmajor_map(&tmX, umma::KIND_TF32, Xp, ks, m, 3, ks * 4, (long long)m * ks * 4,
-                                 umma::BM);
-  if (rc == B2_OK)
-    rc = umma::make_kmajor_map(&tmY, umma::KIND_TF32, Yp, ks, n, 3, ks * 4, (long long)n * ks * 4,
-                               y_box(rg.eng));
-  if (rc != B2_OK) return rc;
-  rc = run_engine(false, 3, tmX, tmY, m, n, kp, 3, seg_kb, rg,
-                  PartialEpi{W, plane, ldw, m, n, rg.pairs}, cx, s);
   if (rc != B2_OK) return rc;
   const long long blocks = ((long long)m * n + 255) / 256;
   B2_PROF("gemm3m_combine", s);
   const unsigned grid = (unsigned)(blocks < 2368 ? blocks : 2368);
   B2_CUDA_TRY(rg.pairs ? launch_dependent(combine3m_tc_kernel<float2>, grid, 256, s,
-                                         (const float2 *)W, plane, ldw, E, m, n, ar, ai, br, bi, C,
-                                         ldc)
-                      : launch_dependent(combine3m_tc_kernel<float>, grid, 256, s, (const float *)W,
-                                         plane, ldw, E, m, n, ar, ai, br, bi, C, ldc));
+                                          (const float2 *)W, plane, ldw, E, m, n, ar, ai, br, bi,
+                                          C, ldc)
+                       : launch_dependent(combine3m_tc_kernel<float>, grid, 256, s,
+                                          (const float *)W, plane, ldw, E, m, n, ar, ai, br, bi, C,
+                                          ldc));
   return B2_OK;
 }
 
