@@ -11,13 +11,27 @@ namespace f32copy {
 constexpr int PK = 16;    // k per panel
 constexpr int NT = 256;   // threads that copy it
 
-// `bytes` (0 .. 4 or 16) of one copy, the rest of it zero.
+// `bytes` (0 .. 4 or 16) of one copy, the rest of it zero; the _full ones all of it.
+#ifdef __CUDACC__
 __device__ __forceinline__ void copy16(uint32_t dst, const float *src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
 }
 __device__ __forceinline__ void copy4(uint32_t dst, const float *src, int bytes) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
 }
+__device__ __forceinline__ void copy16_full(uint32_t dst, const float *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
+}
+__device__ __forceinline__ void copy4_full(uint32_t dst, const float *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src));
+}
+#else  // host compilers check the index arithmetic: dst, src, size, bytes
+void host_copy(uint32_t, const void *, int, int);
+inline void copy16(uint32_t dst, const float *src, int bytes) { host_copy(dst, src, 16, bytes); }
+inline void copy4(uint32_t dst, const float *src, int bytes) { host_copy(dst, src, 4, bytes); }
+inline void copy16_full(uint32_t dst, const float *src) { host_copy(dst, src, 16, 16); }
+inline void copy4_full(uint32_t dst, const float *src) { host_copy(dst, src, 4, 4); }
+#endif
 
 // An operand panel of OUTER outer indices x 16 k lies in shared memory as
 // [k][LD].  KCONT: element (o, k) at g[o*ld + k] in memory, else g[k*ld + o].
@@ -97,10 +111,8 @@ __device__ __forceinline__ void run_panel(uint32_t d, const float *p, int ld) {
 #pragma unroll
   for (int e = 0; e < S::COUNT; ++e) {
     const uint32_t de = d + (uint32_t)(S::STEP * e * (KCONT ? 1 : LD)) * 4u;
-    if constexpr (VEC && !KCONT)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(de), "l"(p));
-    else
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(de), "l"(p));
+    if constexpr (VEC && !KCONT) copy16_full(de, p);
+    else copy4_full(de, p);
     p += step;
   }
 }

@@ -7,6 +7,7 @@
 namespace b2 {
 namespace f64copy {
 
+#ifdef __CUDACC__
 template <int BYTES>
 __device__ __forceinline__ void cp_async(uint32_t dst, const void *src, int src_bytes) {
   if constexpr (BYTES == 16) {
@@ -29,6 +30,17 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
+#else  // host compilers check the index arithmetic: dst, src, size, bytes
+void host_copy(uint32_t, const void *, int, int);
+template <int BYTES>
+inline void cp_async(uint32_t dst, const void *src, int src_bytes) {
+  host_copy(dst, src, BYTES, src_bytes);
+}
+template <int BYTES>
+inline void cp_async_full(uint32_t dst, const void *src) {
+  host_copy(dst, src, BYTES, BYTES);
+}
+#endif
 
 // Operand tiles are copied as 16-byte chunks (two elements) of the rows that are
 // contiguous in memory.  SH: the operand's base or leading dimension is odd, so
