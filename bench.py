@@ -237,6 +237,12 @@ def job_tflops(world: int, flops_per_step: float, steps: int, ms: float) -> floa
 def reference_arm(args, rank: int, world: int = 1):
     if rank != 0:
         return None
+    from oracle import oracle as O
+
+    if not (O.ref_available("DGEMM.so") and O.host_has_avx512f()):
+        why = ("this host has no AVX-512F" if O.ref_available("DGEMM.so")
+               else "oracle/_ref/DGEMM.so is not built (make -C oracle ref)")
+        return {"impl": "reference", "unavailable": why, "n_gpus": world}
     os.environ.setdefault("OMP_NUM_THREADS", str(physical_cores()))
     a, b = make_inputs(args.n, args.phi)
     steps = []

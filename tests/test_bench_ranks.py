@@ -83,3 +83,18 @@ def test_gpus_flag_without_a_launcher_starts_that_many_ranks():
     assert len(lines) == 1, res.stdout
     line = json.loads(lines[0])
     assert line["impl"] == "reference" and line["n_gpus"] == 2
+
+
+def test_reference_arm_never_times_the_port(monkeypatch):
+    """Where the reference's own dgemm_ cannot run, the line says so and has no rate."""
+    sys.path.insert(0, ROOT)
+    import bench
+    from oracle import oracle as O
+
+    monkeypatch.setattr(bench, "make_inputs", lambda *a: pytest.fail("inputs made"))
+    for built, avx in ((False, True), (True, False)):
+        monkeypatch.setattr(O, "ref_available", lambda name="DGEMM.so": built)
+        monkeypatch.setattr(O, "host_has_avx512f", lambda: avx)
+        line = bench.reference_arm(None, 0, 2)
+        assert line["impl"] == "reference" and line["n_gpus"] == 2 and line["unavailable"]
+        assert "\n" not in line["unavailable"] and "value" not in line
