@@ -59,8 +59,8 @@ int sgemm_tensor(char ta, char tb, int m, int n, int k, float alpha, const float
                  const float *B, int ldb, float beta, float *C, int ldc, int method,
                  cudaStream_t s);
 // Engine configuration of a tensor-core SGEMM (sgemm_tc.cu): engine 0 =
-// single CTA 128 x 256 / 4 stages, 1 = single CTA 128 x 128 / 6 stages, 2 =
-// CTA pair 256 x 256 / 6 stages; split = K ranges (0 = automatic).
+// single CTA 128 x 256, 1 = single CTA 128 x 128, 2 = CTA pair 256 x 256;
+// split = K ranges (0 = automatic).
 struct SgCfg {
   int engine = 0;
   int split = 0;

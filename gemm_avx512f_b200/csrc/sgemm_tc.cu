@@ -662,20 +662,21 @@ int sgemm_split_tf32x3(const float *X, long long sr, long long sk, int R, int K,
   return run_split<float>(split_op(X, sr, sk, R, out), SplitOp{}, K, kp, 2, s);
 }
 
-// Tensor-core engine of an SGEMM call: 0 = single CTA, 128 x 256 tile, 4
-// stages; 1 = single CTA, 128 x 128 tile, 6 stages; 2 = CTA pair, 256 x 256
-// tile, 6 stages.  split: K ranges (0 = chosen from the tile count).
+// Tensor-core engine of an SGEMM call: 0 = single CTA, 128 x 256 tile; 1 = single
+// CTA, 128 x 128 tile; 2 = CTA pair, 256 x 256 tile; 4, 6 and 6 stages, 2, 3 and 3 of
+// both segments with three terms.  split: K ranges (0 = chosen from the tile count).
 int sgemm_tensor_cfg(char ta, char tb, int m, int n, int k, float alpha, const float *A, int lda,
                      const float *B, int ldb, float beta, float *C, int ldc, int method,
                      const SgCfg &cfg, cudaStream_t s);
 
-// Without selector weights: on the exhaustive sweep of 11000 shapes with M, N,
-// K in [16, 1024] (B200) the 128 x 128 engine with 8 K ranges is the best
-// single configuration of every method (mean regret 2.6 % TF32, 2.0 % TF32x3,
-// 2.3 % BF16x3 against the per-shape best).  Larger products run on the CTA
-// pair with the wave-fitting split: at 4096^3 and 8192^3 it is the fastest
-// engine of every method (8192^3: TF32 688, TF32x3 267, BF16x3 463 TFLOPS,
-// against 622 / 220 / 366 for the single-CTA 128 x 256 engine).
+// Without selector weights: up to 1024 the 128 x 128 engine with 8 K ranges, for
+// its short chains.  On 260 shapes with M, N, K log-uniform in [16, 1024] (B200) its
+// mean regret against the best of the 12 configurations of a shape is 8.0 % (TF32),
+// 10.9 % (TF32x3) and 14.5 % (BF16x3); the fastest single ones have chains two or eight
+// times as long (4 ranges 7.1 and 10.2 %, one 7.0 %).  Larger products run on the CTA
+// pair with the wave-fitting split: at 4096^3 and 8192^3 it is the fastest engine of
+// every method (8192^3: TF32 787, TF32x3 279, BF16x3 485 TFLOPS, against 689 / 230 /
+// 411 for the single-CTA 128 x 256 engine).
 SgCfg sgemm_default_cfg(int m, int n, int k, int method) {
   (void)method;
   if (m <= 1024 && n <= 1024 && k <= 1024) return SgCfg{1, 8};

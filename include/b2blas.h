@@ -217,7 +217,7 @@ B2_API int b2_dgemm_dd(char transa, char transb, int m, int n, int k, double alp
 
 /* Same contract as dtrsm_ on device memory.  update_method selects the GEMM
  * that performs the trailing updates (B2_METHOD_FP64 or B2_METHOD_OZAKI);
- * block = diagonal block order (0 = 128). */
+ * block is accepted and ignored (diagonal blocks have order 128). */
 B2_API int b2_dtrsm(char side, char uplo, char transa, char diag, int m, int n, double alpha,
              const double *A, int lda, double *B, int ldb, int update_method, int block,
              void *stream);
@@ -367,9 +367,9 @@ B2_API int b2_tune_sweep(int nshapes, const int *shapes, int reps, float *out_ms
 
 /* SGEMM configuration space of the tensor-core methods (the selector's dtype
  * 1): config c = method c / 16 (0 = TF32, 1 = TF32X3, 2 = BF16X3) and, for
- * c % 16 < 12, engine (c % 16) / 4 (0 = single CTA 128x256 / 4 stages,
- * 1 = single CTA 128x128 / 6 stages, 2 = CTA pair 256x256 / 6 stages) x
- * split-K 1 << (c % 4); c % 16 >= 12 is unused (B2_ERR_ARG).  Replaces the
+ * c % 16 < 12, engine (c % 16) / 4 (0 = single CTA 128x256, 1 = single CTA
+ * 128x128, 2 = CTA pair 256x256; where adding K ranges within a CTA is the
+ * faster way, 1 does it for 2) x split-K 1 << (c % 4); c % 16 >= 12 is unused (B2_ERR_ARG).  Replaces the
  * compile-time SGEMM block sizes of sgemm_tune.h:6-15. */
 B2_API int b2_sgemm_config(char transa, char transb, int m, int n, int k, float alpha,
                            const float *A, int lda, const float *B, int ldb, float beta,
